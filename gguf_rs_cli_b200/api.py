@@ -45,11 +45,14 @@ class LLM:
 
     def engine(self, n_tokens: int, n_slots: int, max_len: Optional[int] = None) -> Engine:
         """An engine whose cache has at least this room; the one at hand is kept when it
-        is large enough and idle, else a new one replaces it."""
+        is large enough and idle, else a new one replaces it.  A new one would let no sequence grow beyond n_tokens
+        (in whole pages) either, so the one at hand need not: asking it for max_len itself made every call with
+        fewer tokens than the model's longest sequence build cache, workspace and decode graphs anew."""
         key = (n_tokens, n_slots, max_len)
         e = self._engine
         if (e is not None and e.cache.slots.held_count == 0 and e.cache.n_slots >= n_slots
-                and e.cache.n_pages * 64 >= n_tokens and e.cache.max_len >= (max_len or self.spec.max_position)):
+                and e.cache.n_pages * 64 >= n_tokens
+                and e.cache.max_len >= min(max_len or self.spec.max_position, (n_tokens + 63) // 64 * 64)):
             return e
         # too small, or still holding sequences that an interrupted caller left behind: a new one
         self._backend = None
@@ -111,9 +114,12 @@ def generate(llm: LLM, prompt_ids: Sequence[Sequence[int]], max_tokens: int = 51
     params = SamplingParams(temperature, top_k, top_p, rep_penalty, seed)
     backend.profile = bool(profile)
 
+    # an engine that cannot hold `limit` positions of one sequence limits this call as one made for it would
+    context = limit if backend.context_limit >= limit else min(limit, (n_tokens + 63) // 64 * 64)
+
     def clock():
         torch.cuda.synchronize()
         return time.perf_counter()
 
     return generate_ids(backend, prompts, max_tokens, params, stops, max_batch=batch, on_token=on_token, stats=stats,
-                        clock=clock if stats is not None else None, context_limit=limit)
+                        clock=clock if stats is not None else None, context_limit=context)

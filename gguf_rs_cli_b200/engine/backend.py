@@ -3,6 +3,7 @@ from __future__ import annotations
 
 from typing import List, Optional, Sequence
 
+import gc
 import sys
 
 import numpy as np
@@ -69,6 +70,8 @@ def bucket_of(n: int) -> int:
 
 
 class EngineBackend:
+    MAX_GRAPHS = 64          # captured steps that are kept; the one used longest ago goes first
+
     def __init__(self, engine: Engine, use_graphs: bool = True):
         """use_graphs: decode steps run as captured CUDA graphs where every part of the model allows it
         (`graph_class`).  profile: every step runs eagerly with a time stamp after each stage and one line
@@ -77,7 +80,8 @@ class EngineBackend:
         self.use_graphs = use_graphs
         self.profile = False
         self.profile_out = sys.stderr
-        self._graphs = {}
+        self._graphs = {}            # in the order of their last use
+        self._capture_stream = None
         self._batch = None           # (slots of the last decode step, their lengths after it)
         self._last_graph = None
         self.sampler = Sampler(engine.cache, engine.device)
@@ -150,9 +154,13 @@ class EngineBackend:
         if cls is None:
             return None
         key = (bucket_of(n), cls, params.temperature, params.top_k, params.top_p, params.rep_penalty)
-        dg = self._graphs.get(key)
+        dg = self._graphs.pop(key, None)
         if dg is None:
-            dg = self._graphs[key] = DecodeGraph(eng, key[0])
+            if len(self._graphs) >= self.MAX_GRAPHS:
+                torch.cuda.current_stream().synchronize()         # it may still be running
+                self._graphs.pop(next(iter(self._graphs)))
+            dg = DecodeGraph(eng, key[0])
+        self._graphs[key] = dg
         if dg.copied is not None:
             dg.copied.synchronize()
         if (dg.graph is not None and self._last_graph is dg and dg.laid_out_for == slots_t and dg.keys == keys
@@ -183,12 +191,9 @@ class EngineBackend:
                 self.sampler.sample(logits, ctx.slots, dg.keys_dev, params, dg.out_dev)
 
             if dg.graph is None and dg.warm:
-                torch.cuda.current_stream().synchronize()
                 before = native.launch_count()
-                g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g):
-                    body()
-                dg.graph, dg.launches = g, native.launch_count() - before
+                dg.graph = self._capture(body)
+                dg.launches = native.launch_count() - before
             if dg.graph is not None:
                 dg.graph.replay()
                 native.count_launches(dg.launches)
@@ -200,6 +205,28 @@ class EngineBackend:
         self._batch, self._last_graph = (slots_t, lengths + 1), dg
         self.h2d_bytes += h2d
         return self._pending(slots, keys, params, dg.out_dev)
+
+    def _capture(self, body) -> "torch.cuda.CUDAGraph":
+        """`body` captured on a stream of its own.  Not with torch.cuda.graph: that empties the caching allocator first, and
+        giving gigabytes back to the driver in the middle of a request took 0.1 to 1.5 s.  A step allocates nothing here
+        (its buffers were made by the first, eager call); the collector is held so that no graph dies inside the capture."""
+        if self._capture_stream is None:
+            self._capture_stream = torch.cuda.Stream(device=self.engine.device)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        collecting = gc.isenabled()
+        gc.disable()
+        try:
+            with torch.cuda.stream(self._capture_stream):
+                g.capture_begin()
+                try:
+                    body()
+                finally:
+                    g.capture_end()
+        finally:
+            if collecting:
+                gc.enable()
+        return g
 
     def _copied(self, dg: DecodeGraph) -> None:
         if dg.copied is None:

@@ -1,0 +1,66 @@
+"""The host path of a request on the device: the engine that is kept between calls, and the index arrays of a step."""
+import pytest
+import torch
+
+from tests.gpu_util import llm, new_engine, tokens_of
+
+pytestmark = pytest.mark.gpu
+
+
+def _fresh(name, dtype, prompts, **kw):
+    from gguf_rs_cli_b200.api import generate
+    model = llm(name, dtype)
+    model._engine = model._backend = None
+    return generate(model, prompts, stop_token_ids=[], **kw)
+
+
+# 5 + 59 = 64 positions fill a page to its end: an engine made for the call ends such a sequence one token early
+@pytest.mark.parametrize("shape", [((5, 9, 13), 8), ((70, 3), 30), ((5,), 59), ((5, 64), 64)])
+def test_a_kept_engine_answers_as_a_new_one(shape):
+    from gguf_rs_cli_b200.api import generate
+    lens, n = shape
+    prompts = [tokens_of("C", k, 300 + k) for k in lens]
+    want = _fresh("C", "float32", prompts, max_tokens=n)
+    model = llm("C", "float32")
+    made = model._engine
+    assert generate(model, prompts, max_tokens=n, stop_token_ids=[]) == want and model._engine is made
+    # a smaller call is served by the same engine, with the limit that an engine of its own would have had
+    small = [p[:4] for p in prompts]
+    got = generate(model, small, max_tokens=60, stop_token_ids=[])
+    kept = model._engine is made
+    assert got == _fresh("C", "float32", small, max_tokens=60) and (kept or len(lens) == 1 or n < 60)
+
+
+def test_graphs_that_are_kept_are_bounded():
+    from gguf_rs_cli_b200.engine.backend import EngineBackend
+    from gguf_rs_cli_b200.engine.generate import generate_ids
+    from gguf_rs_cli_b200.sampling import SamplingParams
+    backend = EngineBackend(new_engine("A", "float32", n_tokens=256, n_slots=2))
+    backend.MAX_GRAPHS = 2
+    prompt = [tokens_of("A", 6, 1)]
+    want = generate_ids(backend, prompt, 6, SamplingParams(temperature=0.5, seed=1), [])
+    for t in (0.6, 0.7, 0.8):
+        generate_ids(backend, prompt, 6, SamplingParams(temperature=t, seed=1), [])
+        assert len(backend._graphs) <= 2
+    assert generate_ids(backend, prompt, 6, SamplingParams(temperature=0.5, seed=1), []) == want
+
+
+@pytest.mark.parametrize("n", [7, 200])                  # laid out as lists, and as arrays
+@pytest.mark.parametrize("kind", ["list", "numpy", "tensor", "int32", "bool"])
+def test_token_ids_of_every_kind(kind, n):
+    import numpy as np
+    from gguf_rs_cli_b200.engine.step import Entry, StepError
+    ids = tokens_of("C", n, 2)
+    make = {"list": list, "numpy": np.asarray, "tensor": torch.tensor, "int32": lambda x: np.asarray(x, np.int32),
+            "bool": lambda x: [bool(t % 2) for t in x]}[kind]
+    plain = [int(t) for t in make(ids)]
+    eng = new_engine("C", "float32", n_tokens=1024, n_slots=3)
+    s = [eng.open() for _ in range(3)]
+    a = eng.step([Entry(s[0], plain, (n - 1,))]).clone()
+    b = eng.step([Entry(s[1], make(ids), (n - 1,))])
+    assert torch.equal(a, b)
+    if kind != "bool":
+        with pytest.raises(StepError, match="outside the vocabulary"):
+            eng.step([Entry(s[2], make(ids[:-1] + [1000]), ())])
+        with pytest.raises(StepError, match="outside the vocabulary"):
+            eng.step([Entry(s[2], make([-1] + ids), ())])
