@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tc_kernel(con
     // the list holds tiles of 128 queries; this kernel takes them two at a time, from the even ones
     const int b = p.tiles[2 * blockIdx.y], q0 = p.tiles[2 * blockIdx.y + 1];
     if (q0 % AT_PAIR != 0) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int h = blockIdx.x, g = h / (p.nh / p.nkv);
     const int start = p.starts[b], qlen = p.qlens[b], tok0 = p.cu[b] + q0;
     const int last_pos = start + qlen - 1;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tc_kernel(con
     const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 2 * AT_BN;     // + tile * 128 each
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(&q_full, 2 * AT_TILE);
             for (int t = 0; t < 2; ++t)
                 for (int c = 0; c < CHUNKS; ++c)
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tc_kernel(con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_qk = instr_desc_bf16(AT_BM, AT_BN);
             constexpr uint32_t idesc_pv = instr_desc_bf16_b_mn(AT_BM, HD);
             bool ok = mbar_wait(&q_full, 0);

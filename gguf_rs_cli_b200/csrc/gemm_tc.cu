@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
     __shared__ float part_s[128];
     __shared__ float ssq_s[4][BN];          // per epilogue warp and token: sum of squares of the new residual
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     STAMP_IF(threadIdx.x == 0, 0);
     const int kb_total = (p.K + BK - 1) / BK;
     const int token_tiles = (p.T + BN - 1) / BN;
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
     gb_grid_launch_dependents();                    // the next kernel may begin its own prologue
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- producer: TMA loads into the ring, unit after unit without a pause.  The weights do not
             // depend on the kernel before this one, so the first round of weight tiles is requested at
             // once; the activations only after that kernel has finished.
@@ -173,9 +173,10 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMA issue: two accumulators in TMEM, so that unit j+1 is multiplied while unit j is stored
             constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
+            const uint64_t ring_desc = smem_desc_sw128(smem_u32(ring));        // an address further on is added in units of 16 bytes
             int stage = 0, j = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -190,12 +191,10 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
                     if (!mbar_wait(&full_bar[stage], phase)) { atomicExch(p.status, 2); ok = false; break; }
                     STAMP_IF(j == 0 && kb == w.kb_begin, 2);
                     tc_fence_after();
-                    uint32_t a = smem_u32(ring + stage * Cfg::STAGE_BYTES);
-                    uint32_t b = a + A_BYTES;
+                    const uint64_t a = ring_desc + uint64_t(stage) * (Cfg::STAGE_BYTES >> 4), b = a + (A_BYTES >> 4);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        mma_f16(acc, smem_desc_sw128(a + k * UMMA_K * 2), smem_desc_sw128(b + k * UMMA_K * 2), idesc,
-                                (kb > w.kb_begin || k > 0) ? 1u : 0u);
+                        mma_f16(acc, a + k * (UMMA_K * 2 >> 4), b + k * (UMMA_K * 2 >> 4), idesc, (kb > w.kb_begin || k > 0) ? 1u : 0u);
                     mma_commit(&empty_bar[stage]);      // the stage is free once these MMAs have read it
                     if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
                 }

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
     __shared__ float part_s[128];
     __shared__ float ssq_s[4][PBN];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_cta_rank();               // 0: leader
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int kb_total = (p.K + BK - 1) / BK;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
     gb_grid_launch_dependents();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- producer (both CTAs): this CTA's half of W's and of X's rows for every stage
             gb_grid_wait();
             int stage = 0;
@@ -103,9 +103,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             // ---- MMA issue (leader): 256 x 256 x 16 per instruction over the pair
             constexpr uint32_t idesc = instr_desc_bf16(2 * BM, PBN);
+            const uint64_t ring_desc = smem_desc_sw128(smem_u32(ring));        // an address further on is added in units of 16 bytes
             int stage = 0, j = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -117,12 +118,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
                 for (int kb = 0; kb < kb_total; ++kb) {
                     if (!mbar_wait(&full_bar[stage], phase)) { atomicExch(p.status, 2); ok = false; break; }
                     tc_fence_after();
-                    uint32_t a = smem_u32(ring + stage * PSTAGE_BYTES);
-                    uint32_t b = a + A_BYTES;
+                    const uint64_t a = ring_desc + uint64_t(stage) * (PSTAGE_BYTES >> 4), b = a + (A_BYTES >> 4);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        mma_f16_pair(acc, smem_desc_sw128(a + k * UMMA_K * 2), smem_desc_sw128(b + k * UMMA_K * 2), idesc,
-                                     (kb > 0 || k > 0) ? 1u : 0u);
+                        mma_f16_pair(acc, a + k * (UMMA_K * 2 >> 4), b + k * (UMMA_K * 2 >> 4), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     mma_commit_pair(&empty_bar[stage]);
                     if (++stage == PSTAGES) { stage = 0; phase ^= 1; }
                 }

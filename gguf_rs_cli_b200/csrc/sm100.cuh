@@ -8,6 +8,17 @@
 
 namespace sm100 {
 
+// One thread of a converged warp.  Loops that issue TMA loads or MMAs stand behind this and a warp number that is the same in
+// all lanes for the compiler too (warp_index): behind `lane == 0` it cannot know that one thread is left, and whatever the ring's
+// depth and the tile's width, a block of 64 of K then took 0.42 us in every product kernel.  With it 0.28 and less: a 256 x 256
+// tile over K = 4096 27 -> 24 us, 256 x 128 27 -> 15 us; 2048 x 28672 x 4096 350 -> 309 us.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0;
+}
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
