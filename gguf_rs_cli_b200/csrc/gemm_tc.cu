@@ -464,19 +464,29 @@ GB_API int gb_gemm_tc_set_pair(int on) { g_pair = on; return 0; }
 static int g_mode = 0;                // 0: by the rule below, 1: whole tiles only, 2: equal shares of K blocks where tiles are not shared out per tile, 3: equal shares always
 GB_API int gb_gemm_tc_set_mode(int mode) { g_mode = mode; return 0; }
 
-// The same with the number of output features known: a few hundred tokens with few features would
-// give 256-token tiles for less than half of the SMs, so they take 128-token tiles.
-static int tile_for(int T, int N, int sms) {
+// The same with all sizes known.
+static int tile_for(int T, int N, int K, int sms, bool pair) {
     if (g_tile_override > 0) return g_tile_override;
     int bn = gb_gemm_tc_tile(T);
     const long long ft = (N + BM - 1) / BM;
-    if (bn == 256 && 2 * ft * ((T + 255) / 256) <= sms) bn = 128;
     // (A few dozen tokens used to take two half-size token tiles where there are fewer feature tiles than SMs,
     // because the one CTA that finished a shared tile read all its partial tiles.  Since every CTA of a tile of
     // 32 tokens or more finishes a share of it, whole-width tiles are faster: batch 24 to 64 of the 8B shape
     // 3.87 / 3.94 / 4.60 / 4.71 instead of 4.07 / 4.10 / 4.79 / 4.84 ms a step.)
-    // a few hundred tokens: tiles of 64 tokens, two CTAs per SM, as long as all of them fit the device at once
+    if (pair) {
+        // up to 128 tokens: tiles of 64, two CTAs per SM (a CTA with a wide tile streams its operands no faster)
+        if (bn == 128) return 64;
+        // A few hundred tokens go to the kernel that pairs two SMs like thousands (512 x 4096 x 4096 24 instead of 30 us,
+        // 300 x 6144 x 4096 24 instead of 30), but where K is long and the tiles few, CTAs that share tiles of 64 tokens
+        // are faster (200 x 4096 x 14336 51 instead of 57 us, 300 x 2048 x 8192 29 instead of 34; with one CTA a tile 74
+        // instead of 57).
+        if (bn == 256 && K >= 8192 && ft * ((T + 63) / 64) <= sms) return 64;
+        return bn;
+    }
+    // one CTA a tile only: a few hundred tokens with few features would give 256-token tiles for less than half of the SMs, so
+    // they take 128-token tiles; and tiles of 64 tokens, two CTAs per SM, as long as all of them fit the device at once
     // (a CTA with a wide tile streams its operands no faster; measured at 128 to 768 tokens)
+    if (bn == 256 && 2 * ft * ((T + 255) / 256) <= sms) bn = 128;
     if (bn >= 128 && (T <= 128 || ft * ((T + 63) / 64) <= 2LL * sms)) bn = 64;
     return bn;
 }
@@ -490,9 +500,9 @@ struct TcCut {
         p.total_its = int(tiles * kb); p.its_each = p.total_its / n_ctas; p.its_rest = p.total_its % n_ctas;
     }
 };
-static TcCut cut_for(int T, int N, int K, int sms, bool may_share, int n_counters) {
+static TcCut cut_for(int T, int N, int K, int sms, bool may_share, int n_counters, bool may_pair) {
     TcCut c;
-    c.bn = tile_for(T, N, sms);
+    c.bn = tile_for(T, N, K, sms, may_pair && g_pair);
     c.tiles = (long long)((N + BM - 1) / BM) * ((T + c.bn - 1) / c.bn);
     c.kb = (K + BK - 1) / BK;
     const long long slots = (long long)ctas_per_sm(c.bn) * (sms > 0 ? sms : 1);        // CTAs that are resident at once
@@ -534,11 +544,11 @@ static TcCut cut_for(int T, int N, int K, int sms, bool may_share, int n_counter
 }
 
 // CTAs that a product of these sizes runs on, on a device with `sms` SMs, when it may use scratch memory.
-GB_API int gb_gemm_tc_ctas(int T, int N, int K, int sms) { return cut_for(T, N, K, sms, true, 1 << 30).n_ctas; }
+GB_API int gb_gemm_tc_ctas(int T, int N, int K, int sms) { return cut_for(T, N, K, sms, true, 1 << 30, true).n_ctas; }
 
 // Floats of scratch a launch with these sizes needs (0 when no tile is shared between CTAs).
 GB_API long long gb_gemm_tc_scratch_floats(int T, int N, int K, int sms) {
-    return cut_for(T, N, K, sms, true, 1 << 30).scratch_floats;
+    return cut_for(T, N, K, sms, true, 1 << 30, true).scratch_floats;
 }
 
 // Whether the tensor-core kernel takes these operands (bf16, 16-byte aligned, pitches multiples of 8).
@@ -601,7 +611,7 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
                K, ldx, ldw);
     if (T == 0) return 0;
     if (ensure_status()) return 1;
-    const TcCut cut = cut_for(T, N, K, sms, scratch && counters, n_counters);
+    const TcCut cut = cut_for(T, N, K, sms, scratch && counters, n_counters, true);
     GB_REQUIRE(cut.tiles * cut.kb < (1LL << 31) - (1 << 20), "gb_gemm_tc: T=%d N=%d K=%d is more work than the kernel numbers", T, N, K);
     const int bn = cut.bn;
     TcParams p;
@@ -616,7 +626,8 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
     if (bn == 256 && g_pair && cut.cut == CUT_WHOLE) {
         // many tokens: two SMs per 256 x 256 tile, each loading 128 tokens of X per stage; bf16 results leave
         // through shared memory and TMA stores of [16 tokens x 128 features] (64 features after SwiGLU)
-        if (tensor_map_2d(X, T, K, ldx, 128, &mx)) return 1;
+        p.pair_tile = gemm_tc_pair_tile(T, N, sms);
+        if (tensor_map_2d(X, T, K, ldx, p.pair_tile / 2, &mx)) return 1;
         CUtensorMap mo;
         const bool staged = !resid_x && out_dtype == GB_BF16 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
         if (staged && tensor_map_2d(out, T, swiglu_features ? swiglu_features : N, ldo, 16, &mo, swiglu_features ? 64 : 128)) return 1;
@@ -760,7 +771,7 @@ GB_API int gb_gemm_tc_noalloc(const void* X, long long ldx, const void* W, long 
     NoallocDevice* d = nullptr;
     if (noalloc_setup(dev, &d)) return 1;
     // the same cut of the work as gb_gemm_tc makes; tiles that CTAs share need scratch memory and counters
-    const TcCut cut = cut_for(T, N, K, d->sms, true, 1 << 30);
+    const TcCut cut = cut_for(T, N, K, d->sms, true, 1 << 30, false);
     GB_REQUIRE(cut.tiles * cut.kb < (1LL << 31) - (1 << 20), "gb_gemm_tc_noalloc: T=%d N=%d K=%d is more work than the kernel numbers", T, N, K);
     const int bn = cut.bn;
     if (cut.cut != CUT_WHOLE) {

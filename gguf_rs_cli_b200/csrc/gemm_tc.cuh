@@ -59,6 +59,7 @@ struct TcParams {
     // T is the sum of all rows.  The tile whose first token is t multiplies by the features of problem t / group_t.
     // 0: one product.
     int group_t = 0;
+    int pair_tile = 256;  // tokens of a tile of the kernel that pairs two SMs (gemm_tc_pair_tile)
 };
 
 // The work of a product is the sequence of all (tile, K block) pairs, tile after tile: tiles * kb_total
@@ -289,5 +290,7 @@ __device__ __forceinline__ void tc_write_ssq(const TcParams& p, int n0, int t0, 
 // Two CTAs on two SMs per 256 x 256 tile (gemm_tc_pair.cu); taken for steps of many tokens.
 // mo: map of the bf16 output for stores from shared memory (boxes of 16 tokens x 128 features, or x 64 after
 // SwiGLU), or null: results are then stored from registers.
+// pair_tile of the parameters: the x map's boxes have half as many rows.
+int gemm_tc_pair_tile(int T, int N, int sms);
 int gemm_tc_pair_launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap* mo, const void* params,
                         cudaStream_t stream);

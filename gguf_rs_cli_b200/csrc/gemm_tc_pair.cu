@@ -1,6 +1,7 @@
 // The tensor-core product of gemm_tc.cu for steps of many tokens, with two CTAs on two SMs per output tile of
-// 256 features x 256 tokens (tcgen05 cta_group::2).  Each CTA of the pair loads its 128 features of W and its
-// 128 tokens of X for every block of K (32 KB a stage instead of the 48 KB a lone CTA needs for 128 x 256:
+// 256 features x up to 256 tokens (tcgen05 cta_group::2; the width that wastes least of the last round over the device is
+// chosen per product).  Each CTA of the pair loads its 128 features of W and its half of the tile's
+// tokens of X for every block of K (32 KB a stage instead of the 48 KB a lone CTA needs for 128 x 256:
 // a third less traffic from L2 into shared memory, and room for 6 stages), one thread of the even CTA (the
 // leader) issues the MMAs for both, each CTA's TMEM gets its 128 features of the result, and each CTA's four
 // epilogue warps finish those with the code the other kernel uses.
@@ -15,8 +16,8 @@ using namespace sm100;
 
 namespace {
 
-constexpr int PBN = 256;                    // tokens per tile
-constexpr int PHALF = PBN / 2;              // tokens a CTA loads
+constexpr int PBN = 256;                    // most tokens per tile
+constexpr int PHALF = PBN / 2;              // most tokens a CTA loads
 constexpr int PSTAGES = 6;
 constexpr int PSTAGE_BYTES = A_BYTES + PHALF * BK * 2;         // per CTA
 constexpr int POUT_CHUNK = 16 * BM * 2;      // a staged piece of the result: 16 tokens x 128 features of bf16
@@ -25,11 +26,11 @@ constexpr int PSMEM = PSTAGES * PSTAGE_BYTES + POUT_RING * POUT_CHUNK + 1024;
 constexpr int PTMEM_COLS = 2 * PBN;         // two accumulators
 
 struct PairUnit {
-    int n0, t0;                             // first feature and first token of the 256 x 256 tile
+    int n0, t0;                             // first feature and first token of the tile
 };
 // Tiles in the order of gemm_tc.cu's units: token tiles in groups of TILE_GROUP, inside a group feature tile
 // by feature tile with the group's token tiles innermost.
-__device__ __forceinline__ PairUnit pair_unit_of(int u, int feature_tiles, int token_tiles) {
+__device__ __forceinline__ PairUnit pair_unit_of(int u, int feature_tiles, int token_tiles, int bn) {
     const int per_group = TILE_GROUP * feature_tiles;
     const int group = u / per_group, r = u - group * per_group;
     const int group_start = group * TILE_GROUP;
@@ -37,7 +38,7 @@ __device__ __forceinline__ PairUnit pair_unit_of(int u, int feature_tiles, int t
     const int ft = r / group_size;
     PairUnit w;
     w.n0 = ft * (2 * BM);
-    w.t0 = (group_start + (r - ft * group_size)) * PBN;
+    w.t0 = (group_start + (r - ft * group_size)) * bn;
     return w;
 }
 
@@ -59,7 +60,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int kb_total = (p.K + BK - 1) / BK;
     const int feature_tiles = (p.N + 2 * BM - 1) / (2 * BM);
-    const int token_tiles = (p.T + PBN - 1) / PBN;
+    const int bn = p.pair_tile;                             // tokens of a tile, a multiple of 16 up to PBN
+    const int token_tiles = (p.T + bn - 1) / bn;
     const int n_units = feature_tiles * token_tiles;
 
     if (threadIdx.x == 0) {
@@ -87,16 +89,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
             uint32_t phase = 0;
             bool ok = true;
             for (int u = pair; u < n_units && ok; u += n_pairs) {
-                const PairUnit w = pair_unit_of(u, feature_tiles, token_tiles);
+                const PairUnit w = pair_unit_of(u, feature_tiles, token_tiles, bn);
                 // several products in one launch: the tile's tokens belong to one of them, whose features lie
                 // that many times N further down in W
                 const int w_first = p.group_t > 0 ? (w.t0 / p.group_t) * p.N : 0;
                 for (int kb = 0; kb < kb_total; ++kb) {
                     if (!mbar_wait(&empty_bar[stage], phase ^ 1)) { atomicExch(p.status, 1); ok = false; break; }
-                    if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * PSTAGE_BYTES);
+                    if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * A_BYTES + bn * BK * 2);
                     uint8_t* a = ring + stage * PSTAGE_BYTES;
                     tma_load_2d_pair(a, &map_w, kb * BK, w_first + w.n0 + int(rank) * BM, &full_bar[stage]);
-                    tma_load_2d_pair(a + A_BYTES, &map_x, kb * BK, w.t0 + int(rank) * PHALF, &full_bar[stage]);
+                    tma_load_2d_pair(a + A_BYTES, &map_x, kb * BK, w.t0 + int(rank) * (bn >> 1), &full_bar[stage]);
                     if (++stage == PSTAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -104,8 +106,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
         __syncwarp();
     } else if (warp == 1) {
         if (rank == 0 && elect_one()) {
-            // ---- MMA issue (leader): 256 x 256 x 16 per instruction over the pair
-            constexpr uint32_t idesc = instr_desc_bf16(2 * BM, PBN);
+            // ---- MMA issue (leader): 256 x bn x 16 per instruction over the pair
+            const uint32_t idesc = instr_desc_bf16(2 * BM, bn);
             const uint64_t ring_desc = smem_desc_sw128(smem_u32(ring));        // an address further on is added in units of 16 bytes
             int stage = 0, j = 0;
             uint32_t phase = 0;
@@ -136,11 +138,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
         gb_grid_wait();
         int j = 0, piece = 0;
         for (int u = pair; u < n_units; u += n_pairs, ++j) {
-            const PairUnit w = pair_unit_of(u, feature_tiles, token_tiles);
+            const PairUnit w = pair_unit_of(u, feature_tiles, token_tiles, bn);
             const int buf = j & 1;
             const int n0 = w.n0 + int(rank) * BM;
             const int n = n0 + row;
-            const int cols = min(PBN, p.T - w.t0);
+            const int cols = min(bn, p.T - w.t0);
             if (p.row_ssq) tc_token_scales<PBN>(p, w.t0, cols, row, rstd_s, part_s);
             const bool waited = mbar_wait(&acc_full[buf], (j >> 1) & 1);
             if (!waited) {
@@ -207,6 +209,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
 
 }  // namespace
 
+// A tuning aid (process-wide): > 0: tokens of every tile.
+static int g_pair_tile = 0;
+GB_API int gb_gemm_tc_set_pair_tile(int bn) { g_pair_tile = bn; return 0; }
+
 // How many pairs of CTAs of this kernel the device holds at once (0 if it cannot be asked).
 static int pair_slots() {
     static int slots = -1;
@@ -229,6 +235,22 @@ static int pair_slots() {
     return slots;
 }
 
+// Tokens of a tile: the width whose rounds over the device take the least time.  A 256 x bn tile over K takes a time
+// proportional to bn down to about 176 and no less below (4096 deep: 25 us at 256, 18 at 176, 17 at 128: what is left is the
+// loads' pace).  2048 x 6144: 3 rounds of 256 or of 240; 7001 x 4096 x 14336: 7 rounds of 256 (581 us) or of 224 (530 us);
+// 512 x 4096 x 14336: one round of 256 (89 us) or of 160 (65 us).  Of equal costs the widest.
+int gemm_tc_pair_tile(int T, int N, int sms) {
+    if (g_pair_tile > 0) return g_pair_tile;
+    const long long ft = (N + 2 * BM - 1) / (2 * BM), slots = pair_slots() > 0 ? pair_slots() : sms / 2;
+    int best = PBN;
+    long long least = -1;
+    for (int bn = PBN; bn >= 160; bn -= 16) {
+        const long long units = ft * ((T + bn - 1) / bn), cost = (units + slots - 1) / slots * (bn > 176 ? bn : 176);
+        if (least < 0 || cost < least) { least = cost; best = bn; }
+    }
+    return best;
+}
+
 int gemm_tc_pair_launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap* mo, const void* params,
                         cudaStream_t stream) {
     const TcParams& p = *static_cast<const TcParams*>(params);
@@ -240,7 +262,7 @@ int gemm_tc_pair_launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUte
         if (state < 0) cudaGetLastError();
     }
     if (state < 0) return gb_fail("gb_gemm_tc: cannot get %d bytes of shared memory", PSMEM);
-    long long units = (long long)((p.N + 2 * BM - 1) / (2 * BM)) * ((p.T + PBN - 1) / PBN);
+    long long units = (long long)((p.N + 2 * BM - 1) / (2 * BM)) * ((p.T + p.pair_tile - 1) / p.pair_tile);
     long long slots = pair_slots() > 0 ? pair_slots() : p.sms / 2;     // pairs that can be resident at once
     long long rounds = (units + slots - 1) / slots;
     long long pairs = (units + rounds - 1) / rounds;

@@ -222,6 +222,7 @@ _SIGNATURES = {
     "gb_attention_decode_set_pages_kernel": [_I],
     "gb_attention_decode_set_two_warps": [_I],
     "gb_attention_decode_set_stamps": [_P],
+    "gb_gemm_tc_set_pair_tile": [_I],
     "gb_gemm_tc_set_stamps": [_P, _I, _I],
     "gb_attention_decode_scratch_floats": [_I, _I, _I, _I],
     "gb_attention_decode_supported": [_I, _I, _I],

@@ -1,0 +1,70 @@
+"""The products that a size chooses, at the sizes where each can go wrong: the token tiles of the kernel that pairs two SMs."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def K():
+    from gguf_rs_cli_b200 import kernels
+    return kernels
+
+
+def _operands(T, N, Kd, seed, dtype=torch.bfloat16):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    x = torch.randn(T, Kd, generator=g, device=DEV).to(dtype)
+    w = (torch.randn(N, Kd, generator=g, device=DEV) / math.sqrt(Kd)).to(dtype)
+    return x, w, torch.randn(N, generator=g, device=DEV), g
+
+
+def _sum_bound(x, w):
+    """A 32-bit sum of K exact products in any order is off by at most K 2^-24 times the sum of their magnitudes; its bound is
+    never reached, a sixteenth of it still is a hundred times what random signs give."""
+    return x.shape[1] * 2.0 ** -28 * (x.double().abs() @ w.double().abs().T) + 1e-6
+
+
+@pytest.mark.parametrize("tile", [96, 112, 176, 240, 256, 0])
+def test_token_tiles_of_two_sms(tile):
+    """Every width gives the widest tile's results bit for bit (each is one ascending sum), whatever the number of tokens."""
+    from gguf_rs_cli_b200 import native
+    k = K()
+    try:
+        native.call("gb_gemm_tc_set_tile", 256)
+        for T, N, Kd in ((1000, 512, 256), (769, 640, 136), (2049, 300, 64), (300, 30000, 64)):
+            x, w, b, _ = _operands(T, N, Kd, T)
+            w2 = k.interleave_gate_up(w[:N // 2], w[N // 2:N // 2 * 2])
+            got = []
+            for t in (256, tile):
+                native.call("gb_gemm_tc_set_pair_tile", t)
+                outs = [torch.full((T, N), 9.0, device=DEV, dtype=d) for d in (torch.bfloat16, torch.float32)]
+                gated = torch.full((T, N // 2), 9.0, device=DEV, dtype=torch.bfloat16)
+                for o in outs:
+                    k.gemm_tc(x, w, b, o)
+                k.gemm_tc(x, w2, None, gated, swiglu_features=N // 2)
+                got.append(outs + [gated])
+            assert all(torch.equal(a, c) for a, c in zip(*got)), (T, N, Kd)
+            assert ((got[1][1].double() - x.double() @ w.double().T - b.double()).abs() <= _sum_bound(x, w)).all()
+    finally:
+        native.call("gb_gemm_tc_set_pair_tile", 0)
+        native.call("gb_gemm_tc_set_tile", 0)
+    torch.cuda.synchronize()
+    k.check_tc_status()
+
+
+@pytest.mark.parametrize("T", [129, 191, 300, 512, 769])
+def test_a_few_hundred_tokens(T):
+    """Either side of every border of the rule: K at 8,192, more tiles of 64 tokens than SMs."""
+    k = K()
+    for N, Kd in ((256, 8192), (4096, 8192), (640, 8128), (6144, 64), (130, 8200)):
+        x, w, b, _ = _operands(T, N, Kd, T + N)
+        out = torch.empty(T, N, device=DEV)
+        k.gemm_tc(x, w, b, out)
+        assert ((out.double() - x.double() @ w.double().T - b.double()).abs() <= _sum_bound(x, w)).all(), (N, Kd)
+        low = torch.empty(T, N, device=DEV, dtype=torch.bfloat16)
+        k.gemm_tc(x, w, b, low)
+        assert torch.equal(low, out.bfloat16()), (N, Kd)
+    torch.cuda.synchronize()
+    k.check_tc_status()
