@@ -1134,6 +1134,22 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out:
     return out
 
 
+def gemm_f32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    if x.dtype != torch.float32 or w.dtype != torch.float32 or x.stride(1) != 1 or w.stride(1) != 1:
+        return False
+    return bool(native.library().gb_gemm_f32_supported(ptr(x), x.stride(0), ptr(w), w.stride(0), x.shape[1]))
+
+
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
+    """gemm_generic's sums for 32-bit rows that start on 16 bytes."""
+    _cuda(x, w, bias, out)
+    T, K = x.shape
+    assert w.shape[1] == K and x.dtype == w.dtype == torch.float32 and out.shape == (T, w.shape[0]) and out.stride(1) == 1
+    call("gb_gemm_f32", ptr(x), x.stride(0), ptr(w), w.stride(0), ptr(bias), 0 if bias is None else dtype_code(bias), ptr(out),
+         dtype_code(out), out.stride(0), T, w.shape[0], K, stream_ptr())
+    return out
+
+
 GROUPED_TILE = 256               # tokens of a tile of the kernel that pairs two SMs
 
 
@@ -1366,9 +1382,11 @@ def check_tc_status() -> None:
 # ------------------------------------------------------------------ dispatch
 def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
     """The product path of every projection: the tensor-core kernel when dtype and sizes
-    fit it, else the CUDA-core kernel."""
+    fit it, else a CUDA-core kernel (two of them, with the same sums bit for bit)."""
     if gemm_tc_supported(x, w):
         return gemm_tc(x, w, bias, out)
+    if gemm_f32_supported(x, w):
+        return gemm_f32(x, w, bias, out)
     return gemm_generic(x, w, bias, out)
 
 

@@ -222,6 +222,8 @@ _SIGNATURES = {
     "gb_attention_decode_set_pages_kernel": [_I],
     "gb_attention_decode_set_two_warps": [_I],
     "gb_attention_decode_set_stamps": [_P],
+    "gb_gemm_f32": [_P, _L, _P, _L, _P, _I, _P, _I, _L, _I, _I, _I, _P],
+    "gb_gemm_f32_supported": [_P, _L, _P, _L, _I],
     "gb_gemm_tc_set_pair_tile": [_I],
     "gb_gemm_tc_set_stamps": [_P, _I, _I],
     "gb_attention_decode_scratch_floats": [_I, _I, _I, _I],

@@ -1,4 +1,5 @@
-"""The products that a size chooses, at the sizes where each can go wrong: the token tiles of the kernel that pairs two SMs."""
+"""The products that a size chooses, at the sizes where each can go wrong: 32-bit rows that start on 16 bytes (bit for bit the
+general kernel's sums), and the token tiles of the kernel that pairs two SMs."""
 import math
 
 import pytest
@@ -24,6 +25,26 @@ def _sum_bound(x, w):
     """A 32-bit sum of K exact products in any order is off by at most K 2^-24 times the sum of their magnitudes; its bound is
     never reached, a sixteenth of it still is a hundred times what random signs give."""
     return x.shape[1] * 2.0 ** -28 * (x.double().abs() @ w.double().abs().T) + 1e-6
+
+
+@pytest.mark.parametrize("T", [1, 2, 4, 5, 8, 9, 16, 17, 31, 48, 49, 144, 200])
+def test_32_bit_products_are_the_general_kernels_bit_for_bit(T):
+    k = K()
+    for N, Kd in ((64, 64), (130, 176), (1, 4), (257, 132), (3072, 260), (20000, 96)):
+        x, w, b, _ = _operands(T, N, Kd, N + Kd, torch.float32)
+        for bias in (None, b):
+            want, got = torch.empty(T, N, device=DEV), torch.full((T, N + 5), 7.0, device=DEV)[:, :N]
+            k.gemm_generic(x, w, bias, want)
+            assert k.gemm_f32_supported(x, w)
+            k.gemm_f32(x, w, bias, got)
+            assert torch.equal(got, want), (N, Kd)
+    wide = torch.randn(T, 520, device=DEV)
+    w = torch.randn(96, 520, device=DEV)
+    assert not k.gemm_f32_supported(wide[:, 1:513], w[:, :512]) and not k.gemm_f32_supported(wide[:, :510], w[:, :510])
+    want, got = torch.empty(T, 96, device=DEV), torch.empty(T, 96, device=DEV)
+    k.gemm_generic(wide[:, 4:516], w[:, 8:520], None, want)
+    k.gemm_f32(wide[:, 4:516], w[:, 8:520], None, got)
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("tile", [96, 112, 176, 240, 256, 0])
