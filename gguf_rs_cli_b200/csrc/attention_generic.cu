@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
         for (int d = threadIdx.x; d < hdv; d += blockDim.x) gb_store(out, out_dtype, orow + d, 0.f);
         return;
     }
-    __shared__ float qs[MAX_HD];
+    __shared__ __align__(16) float qs[MAX_HD];
     __shared__ float acc_s[AG_WARPS][MAX_HD];
     __shared__ float m_s[AG_WARPS], l_s[AG_WARPS];
     for (int d = threadIdx.x; d < hd; d += blockDim.x) qs[d] = gb_load(q, q_dtype, size_t(t) * ldq + size_t(h) * hd + d);
@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
     // Other rows: each lane walks its own key's row.  Either way the order of the sums is fixed by the sizes alone.
     constexpr int QC = (MAX_HD / 8 + 31) / 32;
     const bool shared_rows = sizeof(TC) == 2 && vec8;
+    const bool quads = sizeof(TC) == 4 && hd % 4 == 0 && (reinterpret_cast<uintptr_t>(kc) & 15) == 0;
     const bool pairs = sizeof(TC) == 2 && hdv % 2 == 0 && v_row % 2 == 0 && (reinterpret_cast<uintptr_t>(vc) & 3) == 0;
     float qr[QC][8];
     if (shared_rows) {
@@ -117,7 +118,22 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
         } else if (valid) {
             const TC* kr = kc + off * hd;
             float dot = 0.f;
-            for (int d = 0; d < hd; ++d) dot = fmaf(qs[d], gb_to_float(kr[d]), dot);
+            if (quads) {
+                // 32-bit rows that start on 16 bytes: the same sum in the same order, four entries a load and eight loads in
+                // flight (entry by entry a row of 64 was sixteen trips to L2 one after the other: 24 us for a few tokens)
+                const float4* k4 = reinterpret_cast<const float4*>(kr);
+                const float4* q4 = reinterpret_cast<const float4*>(qs);
+#pragma unroll 8
+                for (int d = 0; d < hd >> 2; ++d) {
+                    const float4 kk = k4[d], qq = q4[d];
+                    dot = fmaf(qq.x, kk.x, dot);
+                    dot = fmaf(qq.y, kk.y, dot);
+                    dot = fmaf(qq.z, kk.z, dot);
+                    dot = fmaf(qq.w, kk.w, dot);
+                }
+            } else {
+                for (int d = 0; d < hd; ++d) dot = fmaf(qs[d], gb_to_float(kr[d]), dot);
+            }
             s = dot * scale;
         }
         if (softcap > 0.f && valid) s = softcap * tanhf(s / softcap);
@@ -128,6 +144,24 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
         l = l * alpha + gb_warp_sum(pj);
 #pragma unroll
         for (int c = 0; c < C; ++c) acc[c] *= alpha;
+        if (sizeof(TC) == 4 && MAX_HD <= 256) {
+            // the same sums with eight keys' values asked for at a time; a key without weight is not read (its row may
+            // never have been written) and adds nothing
+            for (int j0 = 0; j0 < 32; j0 += 8) {
+                float pv[8], vv[8][C];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    pv[e] = __shfl_sync(0xffffffffu, pj, j0 + e);
+                    const TC* vr = vc + __shfl_sync(0xffffffffu, off, j0 + e) * v_row;
+#pragma unroll
+                    for (int c = 0; c < C; ++c) vv[e][c] = pv[e] != 0.f && lane + 32 * c < hdv ? gb_to_float(vr[lane + 32 * c]) : 0.f;
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) acc[c] = fmaf(pv[e], vv[e][c], acc[c]);
+            }
+        } else
         for (int jj = 0; jj < 32; ++jj) {
             float pv = __shfl_sync(0xffffffffu, pj, jj);
             long long o = __shfl_sync(0xffffffffu, off, jj);
@@ -217,7 +251,9 @@ GB_API int gb_attention_generic(const void* q, int q_dtype, long long ldq, void*
         (const TC*)kcache, (const TC*)vcache, window, scale, head_pages, window > 0 ? keep_first : 0, gate, gate_dtype, ldg, gate_per_head, sink, sink_values, chunk, slopes, softcap, out_scale)
     const bool small = hd <= 256 && hdv <= 256, mid = hd <= AG_MID_HD && hdv <= AG_MID_HD;
     if (cache_dtype == GB_F32) {
-        if (small) AG_LAUNCH(float, 256);
+        if (hd <= 64 && hdv <= 64) AG_LAUNCH(float, 64);
+        else if (hd <= 128 && hdv <= 128) AG_LAUNCH(float, 128);
+        else if (small) AG_LAUNCH(float, 256);
         else if (mid) AG_LAUNCH(float, AG_MID_HD);
         else AG_LAUNCH(float, AG_MAX_HD);
     } else {
