@@ -132,6 +132,23 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
         const int kk = warp * AD_KEYS_PER_WARP + key_in_warp;
         const int j = pg * GB_PAGE + kk;
         const bool valid = j <= pos && (j >= lo || j < keep);
+        // This warp's 16 rows of values are asked for before its keys are used (heads of up to 128, up to four of them: 32 registers): with a
+        // page or two per CTA the time is the trips to memory one after the other, and this takes four of six off.
+        const __nv_bfloat16* vp = p.vc + page_off + size_t(warp * AD_KEYS_PER_WARP) * hd;
+        const int first_key = pg * GB_PAGE + warp * AD_KEYS_PER_WARP;
+        auto seen = [&](int k) {                       // uniform over the warp; unwritten rows are never read
+            const int jk = first_key + k;
+            return jk <= pos && (jk >= lo || jk < keep);
+        };
+        constexpr bool EARLY = HC <= 2 && GT <= 4;
+        unsigned vr[EARLY ? AD_KEYS_PER_WARP : 1][HC];
+        if constexpr (EARLY) {
+#pragma unroll
+            for (int k = 0; k < AD_KEYS_PER_WARP; ++k)
+#pragma unroll
+                for (int c = 0; c < HC; ++c)
+                    vr[k][c] = seen(k) && 2 * lane + 64 * c < hd ? __ldg(reinterpret_cast<const unsigned*>(vp + size_t(k) * hd + 2 * lane + 64 * c)) : 0u;
+        }
         // ---- scores of this warp's 16 keys; two lanes share a key and take its 16-byte chunks in turn
         float s[GT];
 #pragma unroll
@@ -175,23 +192,11 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
         }
         __syncwarp();
         // ---- weighted values: lane owns dimensions 2*lane + 64*c, +1
-        const __nv_bfloat16* vp = p.vc + page_off + size_t(warp * AD_KEYS_PER_WARP) * hd;
 #pragma unroll
         for (int gi = 0; gi < GT; ++gi)
 #pragma unroll
             for (int c = 0; c < HC; ++c) { acc[gi][c][0] *= alpha[gi]; acc[gi][c][1] *= alpha[gi]; }
-        const int first_key = pg * GB_PAGE + warp * AD_KEYS_PER_WARP;
-#pragma unroll 4
-        for (int k = 0; k < AD_KEYS_PER_WARP; ++k) {
-            const int jk = first_key + k;
-            if (jk > pos || (jk < lo && jk >= keep)) continue;          // uniform over the warp; unwritten rows are never read
-            float2 vf[HC];
-#pragma unroll
-            for (int c = 0; c < HC; ++c) {
-                int d = 2 * lane + 64 * c;
-                vf[c] = make_float2(0.f, 0.f);
-                if (d < hd) vf[c] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(vp + size_t(k) * hd + d));
-            }
+        auto mix = [&](int k, const float2 (&vf)[HC]) {
 #pragma unroll
             for (int gi = 0; gi < GT; ++gi) {
                 float pv = ps[warp][gi][k];
@@ -200,6 +205,29 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
                     acc[gi][c][0] = fmaf(pv, vf[c].x, acc[gi][c][0]);
                     acc[gi][c][1] = fmaf(pv, vf[c].y, acc[gi][c][1]);
                 }
+            }
+        };
+        if constexpr (EARLY) {
+#pragma unroll
+            for (int k = 0; k < AD_KEYS_PER_WARP; ++k) {
+                if (!seen(k)) continue;
+                float2 vf[HC];
+#pragma unroll
+                for (int c = 0; c < HC; ++c) vf[c] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&vr[k][c]));
+                mix(k, vf);
+            }
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < AD_KEYS_PER_WARP; ++k) {
+                if (!seen(k)) continue;
+                float2 vf[HC];
+#pragma unroll
+                for (int c = 0; c < HC; ++c) {
+                    int d = 2 * lane + 64 * c;
+                    vf[c] = make_float2(0.f, 0.f);
+                    if (d < hd) vf[c] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(vp + size_t(k) * hd + d));
+                }
+                mix(k, vf);
             }
         }
         __syncwarp();
@@ -249,8 +277,10 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
         int gi = i / hd, d = i - gi * hd;
         const float* rec = p.scratch + (size_t(t) * p.nh + h0 + gi) * p.splits * (hd + 2);
         float M = -INFINITY;
+#pragma unroll 8
         for (int s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd));
         float L = 0.f, o = 0.f;
+#pragma unroll 8
         for (int s = 0; s < p.splits; ++s) {
             float ms = __ldcg(rec + s * (hd + 2) + hd);
             float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);

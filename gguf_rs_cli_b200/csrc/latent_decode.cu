@@ -22,6 +22,7 @@ constexpr int LD_THREADS = LD_WARPS * 32;
 constexpr int LD_MAX_HEADS = 16;                    // heads per token: at most 2 per warp (with 32 heads the general
                                                     // kernel's block per head was measured faster: 0.774 against 0.799 ms a step)
 constexpr int LD_HW = LD_MAX_HEADS / LD_WARPS;
+constexpr int LD_MAX_SPLITS = 64;
 constexpr int LD_MAX_C = 512;                       // entries of the value: at most 8 pairs per lane
 constexpr int LD_PAIRS = LD_MAX_C / 64;
 
@@ -175,6 +176,8 @@ __device__ __forceinline__ void lm_split3(float p, float& hi, float& mid, float&
 
 __global__ void __launch_bounds__(LM_THREADS) latent_decode_mma_kernel(const LdParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    gb_grid_launch_dependents();
+    gb_grid_wait();
     const int t = blockIdx.x, split = blockIdx.y;
     const int b = p.seq_of[t];
     if (b < 0) return;
@@ -189,12 +192,15 @@ __global__ void __launch_bounds__(LM_THREADS) latent_decode_mma_kernel(const LdP
     const int kb0 = kbf + split * per, kb1 = min(kbf + nkb, kb0 + per);
     const int* trow = p.table + size_t(b) * p.table_width;
     const int pieces = HDK / 8;
-    for (int i = threadIdx.x; i < 16 * pieces; i += LM_THREADS) {
-        const int r = i / pieces, c8 = i - r * pieces;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (r < H) v = *reinterpret_cast<const uint4*>(p.q + size_t(t) * p.ldq + size_t(r) * HDK + 8 * c8);
-        *reinterpret_cast<uint4*>(qt + r * KS + 8 * c8) = v;
-    }
+    // A warp copies a row: the queries with the first tile of keys, all in flight at once (16 bytes a copy; piece by piece
+    // through registers, 18 copies a thread in turn, a tile took longer to come than to use).
+    auto copy = [&](__nv_bfloat16* dst, const __nv_bfloat16* src, bool valid) {
+        for (int c8 = lane; c8 < pieces; c8 += 32) {
+            const unsigned d = unsigned(__cvta_generic_to_shared(dst + 8 * c8));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (valid ? 8 * c8 : 0)), "r"(valid ? 16 : 0) : "memory");
+        }
+    };
+    for (int r = warp; r < 16; r += LM_THREADS / 32) copy(qt + r * KS, p.q + size_t(t) * p.ldq + size_t(r < H ? r : 0) * HDK, r < H);
     const int CW = C / 4, ot = CW / 8;                 // this warp's value columns [warp * CW, +CW): ot tiles of 8
     const float sl2 = p.scale * 1.4426950408889634f;
     float o[LM_MAX_OT][4];
@@ -204,12 +210,13 @@ __global__ void __launch_bounds__(LM_THREADS) latent_decode_mma_kernel(const LdP
 
     for (int kb = kb0; kb < kb1; ++kb) {
         __syncthreads();
-        for (int i = threadIdx.x; i < 32 * pieces; i += LM_THREADS) {
-            const int r = i / pieces, c8 = i - r * pieces, j = kb * 32 + r;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (j <= pos && j >= lo) v = *reinterpret_cast<const uint4*>(p.cache + gb_kv_offset(trow, p.ring_pages, j, 0, 1, HDK) + 8 * c8);
-            *reinterpret_cast<uint4*>(kt + r * KS + 8 * c8) = v;
+        for (int r = warp; r < 32; r += LM_THREADS / 32) {
+            const int j = kb * 32 + r;
+            const bool valid = j <= pos && j >= lo;
+            copy(kt + r * KS, p.cache + (valid ? gb_kv_offset(trow, p.ring_pages, j, 0, 1, HDK) : 0), valid);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         // ---- S = Q K^T: 16 heads x 32 keys, as four tiles of 8 keys
         float s[4][4];
@@ -314,35 +321,53 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ scratch, co
                                            __nv_bfloat16* __restrict__ out, long long ldo, int H, int C, int splits,
                                            const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, long long ldg) {
     const int t = blockIdx.x, h = blockIdx.y;
+    gb_grid_launch_dependents();
+    gb_grid_wait();
     __nv_bfloat16* o = out + size_t(t) * ldo + size_t(h) * C;
     if (seq_of[t] < 0) {
         for (int c = threadIdx.x; c < C; c += blockDim.x) o[c] = __float2bfloat16_rn(0.f);
         return;
     }
+    // every split's factor once: e^(m_s - M), at most LD_MAX_SPLITS of them
+    __shared__ float w[LD_MAX_SPLITS], sums[LD_MAX_SPLITS], total[2];
     const float* base = scratch + (size_t(t) * H + h) * splits * (C + 2);
+    for (int s = threadIdx.x; s < splits; s += blockDim.x) {
+        w[s] = base[size_t(s) * (C + 2) + C];
+        sums[s] = base[size_t(s) * (C + 2) + C + 1];
+    }
+    __syncthreads();
     float M = -INFINITY;
-    for (int s = 0; s < splits; ++s) M = fmaxf(M, base[size_t(s) * (C + 2) + C]);
-    float L = 0.f;
-    for (int s = 0; s < splits; ++s) {
-        const float ms = base[size_t(s) * (C + 2) + C];
-        if (ms != -INFINITY) L += base[size_t(s) * (C + 2) + C + 1] * expf(ms - M);
-    }
-    float f = 1.f;                       // what the sums are multiplied by: a sink above every score brings them down to its level
-    if (sink && M != -INFINITY) {
-        const float sv = sink[h];
-        if (sv > M) {
-            f = expf(M - sv);
-            L = L * f + 1.f;
-        } else {
-            L += expf(sv - M);
+    for (int s = 0; s < splits; ++s) M = fmaxf(M, w[s]);
+    __syncthreads();
+    for (int s = threadIdx.x; s < splits; s += blockDim.x) w[s] = w[s] == -INFINITY ? 0.f : expf(w[s] - M);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float L = 0.f;
+        for (int s = 0; s < splits; ++s)
+            if (w[s] != 0.f) L += sums[s] * w[s];
+        float f = 1.f;                   // what the sums are multiplied by: a sink above every score brings them down to its level
+        if (sink && M != -INFINITY) {
+            const float sv = sink[h];
+            if (sv > M) {
+                f = expf(M - sv);
+                L = L * f + 1.f;
+            } else {
+                L += expf(sv - M);
+            }
         }
+        if (gate) f *= 1.f / (1.f + expf(-__bfloat162float(gate[size_t(t) * ldg + h])));
+        total[0] = f;
+        total[1] = L;
     }
-    if (gate) f *= 1.f / (1.f + expf(-__bfloat162float(gate[size_t(t) * ldg + h])));
+    __syncthreads();
+    const float f = total[0], L = total[1];
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
         float v = 0.f;
+        // a split without keys has left nothing (its record may hold anything)
+#pragma unroll 16
         for (int s = 0; s < splits; ++s) {
-            const float ms = base[size_t(s) * (C + 2) + C];
-            if (ms != -INFINITY) v += base[size_t(s) * (C + 2) + c] * expf(ms - M);
+            const float x = base[size_t(s) * (C + 2) + c];        // loaded whatever the factor, so that sixteen are on their way
+            v += w[s] != 0.f ? x * w[s] : 0.f;
         }
         o[c] = __float2bfloat16_rn(v * f / L);
     }
@@ -380,10 +405,11 @@ GB_API int gb_latent_decode(const void* q, long long ldq, void* out, long long l
                             const void* gate, long long ldg, cudaStream_t stream) {
     GB_REQUIRE(window >= 0, "gb_latent_decode: a negative window");
     GB_REQUIRE(gb_latent_decode_supported(H, C, R, GB_BF16, GB_BF16), "gb_latent_decode: sizes heads=%d kv_rank=%d rot_dim=%d are not supported", H, C, R);
-    GB_REQUIRE(splits >= 1 && splits <= 65535 && scratch && table_width > 0 && ring_pages > 0, "gb_latent_decode: bad arguments");
+    GB_REQUIRE(splits >= 1 && splits <= LD_MAX_SPLITS && scratch && table_width > 0 && ring_pages > 0, "gb_latent_decode: bad arguments");
     GB_REQUIRE((ldq % 2) == 0 && (reinterpret_cast<uintptr_t>(cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(scratch) & 7) == 0,
                "gb_latent_decode: misaligned operands");
     if (T == 0) return 0;
+    const int merge_threads = C >= 512 ? 512 : (C + 31) / 32 * 32;          // an entry a thread, all splits' numbers on their way
     LdParams p;
     p.q = (const __nv_bfloat16*)q; p.cache = (const __nv_bfloat16*)cache; p.seq_of = seq_of; p.pos = pos; p.table = table;
     p.scratch = scratch; p.ldq = ldq; p.H = H; p.C = C; p.R = R; p.splits = splits; p.table_width = table_width;
@@ -396,9 +422,9 @@ GB_API int gb_latent_decode(const void* q, long long ldq, void* out, long long l
                 return gb_fail("gb_latent_decode: cannot get %zu bytes of shared memory", smem_mma);
             configured_mma = true;
         }
-        latent_decode_mma_kernel<<<dim3(T, splits), LM_THREADS, smem_mma, stream>>>(p);
+        gb_launch(latent_decode_mma_kernel, dim3(T, splits), dim3(LM_THREADS), smem_mma, stream, p);
         GB_LAUNCH_OK("gb_latent_decode (tensor cores)");
-        latent_decode_merge_kernel<<<dim3(T, H), 128, 0, stream>>>(scratch, seq_of, (__nv_bfloat16*)out, ldo, H, C, splits, sink, (const __nv_bfloat16*)gate, ldg);
+        gb_launch(latent_decode_merge_kernel, dim3(T, H), dim3(merge_threads), 0, stream, (const float*)scratch, seq_of, (__nv_bfloat16*)out, ldo, H, C, splits, sink, (const __nv_bfloat16*)gate, ldg);
         GB_LAUNCH_OK("gb_latent_decode (merge)");
         return 0;
     }
@@ -411,7 +437,7 @@ GB_API int gb_latent_decode(const void* q, long long ldq, void* out, long long l
     }
     latent_decode_kernel<<<dim3(T, splits), LD_THREADS, smem, stream>>>(p);
     GB_LAUNCH_OK("gb_latent_decode");
-    latent_decode_merge_kernel<<<dim3(T, H), 128, 0, stream>>>(scratch, seq_of, (__nv_bfloat16*)out, ldo, H, C, splits, sink, (const __nv_bfloat16*)gate, ldg);
+    latent_decode_merge_kernel<<<dim3(T, H), merge_threads, 0, stream>>>(scratch, seq_of, (__nv_bfloat16*)out, ldo, H, C, splits, sink, (const __nv_bfloat16*)gate, ldg);
     GB_LAUNCH_OK("gb_latent_decode (merge)");
     return 0;
 }

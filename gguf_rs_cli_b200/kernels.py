@@ -676,9 +676,9 @@ def latent_decode_supported(n_heads: int, kv_rank: int, rot_dim: int, dtype: tor
 
 
 def latent_decode_class(max_kv: int) -> int:
-    """Class of a decode step for the latent decode kernel: half of the longest sequence's blocks of 32 keys, rounded
+    """Class of a decode step for the latent decode kernel: the longest sequence's blocks of 32 keys, rounded
     down to one of a few values; steps of one class split their keys alike."""
-    return _split_class(((max_kv + 31) // 32) // 2)
+    return _split_class((max_kv + 31) // 32)
 
 
 def latent_decode(qa: torch.Tensor, out: torch.Tensor, n_heads: int, kv_rank: int, rot_dim: int, ctx, table: torch.Tensor,
@@ -686,7 +686,7 @@ def latent_decode(qa: torch.Tensor, out: torch.Tensor, n_heads: int, kv_rank: in
                   gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Latent attention of single tokens: qa [T, heads*(kv_rank + rot_dim)] (queries in the latent's space, then the
     rotated part), cache rows [kv_rank + rot_dim]; out [T, heads*kv_rank] is the mix of the rows' first kv_rank
-    entries.  One pass over each token's rows serves all heads; the rows are split over CTAs (two blocks of 32 keys or
+    entries.  One pass over each token's rows serves all heads; the rows are split over CTAs (a block of 32 keys or
     more per split, while two CTAs per SM hold the step) and merged in order.  window: the last `window` positions only;
     sink_values float32 [heads]: one more key without a value of that score in the denominator; gate bfloat16 [T, heads]:
     a head's result times its sigmoid."""
@@ -1191,12 +1191,12 @@ def decode_split_class_cuda(max_kv: int) -> int:
 
 
 def decode_split_class_exact(max_kv: int) -> int:
-    """Class of a decode step of the normalised attention on the CUDA-core decode kernel: half of the pages."""
-    return _split_class(((max_kv + 63) // 64) // 2)
+    """Class of a decode step of the normalised attention on the CUDA-core decode kernel: its pages."""
+    return _split_class((max_kv + 63) // 64)
 
 
 def decode_splits_exact(T: int, n_heads: int, n_kv_heads: int, max_kv: int, sms: int) -> int:
-    """Splits of each sequence's pages for that kernel: two pages or more per split while all CTAs fit the device at
+    """Splits of each sequence's pages for that kernel: a page or more per split while all CTAs fit the device at
     once with two per SM (the rule of decode_splits leaves a step of 8 sequences of 512 positions at 32 CTAs)."""
     group = n_heads // n_kv_heads
     tile = 8 if group >= 8 else 4 if group > 2 else group
