@@ -3,15 +3,15 @@
 // bit for bit, whatever the sizes, so a row's result does not depend on the rows beside it; only the loads differ.
 //
 // Few tokens (gemm_f32_few_kernel): the time is the weights' way from memory, and one output's chain of K additions, each
-// waiting for the one before and for its operands (5.5 ns a step of K as measured).  Every CTA has the same few rows of W
-// with all of K, copied asynchronously as far ahead as shared memory allows; a thread has one row and one to four tokens.  On
-// 2,048 x 8,192 at 2 tokens gemm_generic's 64-row tiles kept 32 SMs busy, each with one load in flight per thread: 645 us,
-// here 52 (16,384 x 2,048: 223 and 31; a head of 128,256 x 2,048: 1,188 and 186, where its bytes take 160).  Requests by TMA
-// with the adding warps by themselves were no faster (54, 28 and 161 us) and slower at 8 tokens (96 instead of 57 us).
+// waiting for the one before.  Every CTA has the same few rows of W with all of K, copied asynchronously as far ahead as
+// shared memory allows; a thread has one row and one to four tokens.  On 2,048 x 8,192 at 2 tokens gemm_generic's 64-row
+// tiles kept 32 SMs busy, each with one load in flight per thread: 645 us, here 38 (16,384 x 2,048: 223 and 29; a head of
+// 128,256 x 2,048: 1,188 and 180, where its bytes take 160).
 // More tokens (gemm_f32_tile_kernel): bound by the FMA pipes; tiles of 64 features by 16 to 64 tokens, chosen so that the
 // tiles fill the device, 4 x 2 to 4 x 8 outputs a thread, operands copied asynchronously three blocks of K ahead (a block
 // is multiplied in a fifth of the time that memory takes to answer).  At 144 tokens 16,384 x 2,048 takes 265 us (gemm_generic
-// 602), 2,048 x 8,192 225 (613).
+// 602), 2,048 x 8,192 225 (613).  Eight blocks ahead, twice the threads with half the outputs each, and operands loaded a
+// step ahead were no faster: 63 to 69 us instead of 65 at 3,072 x 2,048 and 144 tokens.
 #include "common.cuh"
 
 namespace {
@@ -26,6 +26,13 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 // ------------------------------------------------------------------------------------------------------ few tokens
 constexpr int FF_THREADS = 256, FF_KC = 128, FF_LD = FF_KC + 4, FF_MAX_T = 16, FF_MAX_ROWS = 64;
 constexpr int FF_RING = 3 * (FF_MAX_ROWS + FF_MAX_T) * FF_LD * 4;      // the most shared memory of a CTA
+
+// 16 bytes of shared memory, loaded where it stands in the program.
+__device__ __forceinline__ float4 ff_lds(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
 
 // TT: tokens of a thread.  STAGES: chunks of K in the ring.  rows: features of a tile; CTA c takes tiles c, c + CTAs, ...
 template <int TT, int STAGES>
@@ -42,11 +49,14 @@ __global__ void __launch_bounds__(FF_THREADS, 2) gemm_f32_few_kernel(const float
     gb_grid_launch_dependents();
     gb_grid_wait();
     int c_item = 0, c_chunk = 0, c_stage = 0, c_n0 = int(blockIdx.x) * rows;      // the next item to be copied
+    // The warps that add have their hands full; where they are few, the others copy (2,048 x 8,192 48 -> 37 us).
+    const int adders = (rows * ((T + TT - 1) / TT) + 31) >> 5;
+    const int first = adders <= FF_THREADS / 128 ? adders : 0, copiers = FF_THREADS / 32 - first, warp = tid >> 5;
     auto copy = [&] {
-        if (c_item < n_items) {
+        if (warp >= first && c_item < n_items) {
             const int n0 = c_n0, k = c_chunk * FF_KC + piece;
             float* s = smem + c_stage * stage_floats;
-            for (int r = tid >> 5; r < rows + T; r += FF_THREADS / 32) {
+            for (int r = warp - first; r < rows + T; r += copiers) {
                 const bool is_w = r < rows;
                 const bool valid = k < K && (!is_w || n0 + r < N);
                 const float* src = is_w ? W + size_t(valid ? n0 + r : 0) * ldw : X + size_t(r - rows) * ldx;
@@ -74,21 +84,40 @@ __global__ void __launch_bounds__(FF_THREADS, 2) gemm_f32_few_kernel(const float
 #pragma unroll
                 for (int j = 0; j < TT; ++j) acc[j] = 0.f;
             }
-            const float4* w4 = reinterpret_cast<const float4*>(s + r * FF_LD);
-            const float4* x4[TT];
+            const unsigned wa = unsigned(__cvta_generic_to_shared(s + r * FF_LD));
+            unsigned xa[TT];
 #pragma unroll
-            for (int j = 0; j < TT; ++j) x4[j] = reinterpret_cast<const float4*>(s + (rows + min(t0 + j, T - 1)) * FF_LD);
-#pragma unroll 8
-            for (int k = 0; k < FF_KC / 4; ++k) {
-                const float4 w = w4[k];
+            for (int j = 0; j < TT; ++j) xa[j] = unsigned(__cvta_generic_to_shared(s + (rows + min(t0 + j, T - 1)) * FF_LD));
+            // Sixteen steps of K at a time, the next sixteen's operands in registers while these are added: a step is one addition
+            // behind another (4.2 cycles), and with the loads left to the compiler, next to their uses, it took 8.3.
+            float4 wv[2][4], xv[2][TT][4];
+            auto fetch = [&](int g, int buf) {
 #pragma unroll
-                for (int j = 0; j < TT; ++j) {
-                    const float4 x = x4[j][k];
-                    acc[j] = fmaf(x.x, w.x, acc[j]);
-                    acc[j] = fmaf(x.y, w.y, acc[j]);
-                    acc[j] = fmaf(x.z, w.z, acc[j]);
-                    acc[j] = fmaf(x.w, w.w, acc[j]);
+                for (int c = 0; c < 4; ++c) {
+                    wv[buf][c] = ff_lds(wa + g * 64 + c * 16);
+#pragma unroll
+                    for (int j = 0; j < TT; ++j) xv[buf][j][c] = ff_lds(xa[j] + g * 64 + c * 16);
                 }
+            };
+            auto add = [&](int buf) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int j = 0; j < TT; ++j) {
+                        const float4 w = wv[buf][c], x = xv[buf][j][c];
+                        acc[j] = fmaf(x.x, w.x, acc[j]);
+                        acc[j] = fmaf(x.y, w.y, acc[j]);
+                        acc[j] = fmaf(x.z, w.z, acc[j]);
+                        acc[j] = fmaf(x.w, w.w, acc[j]);
+                    }
+            };
+            fetch(0, 0);
+#pragma unroll
+            for (int g = 0; g < FF_KC / 16; g += 2) {
+                fetch(g + 1, 1);
+                add(0);
+                if (g + 2 < FF_KC / 16) fetch(g + 2, 0);
+                add(1);
             }
         }
         if (++chunk == chunks) {
@@ -247,14 +276,16 @@ GB_API int gb_gemm_f32(const float* X, long long ldx, const float* W, long long 
     if (T == 0) return 0;
     const int sms = sm_count();
     if (T <= FF_MAX_T) {
-        const int tt = T <= 4 ? 1 : T <= 8 ? 2 : 4, groups = (T + tt - 1) / tt;
-        const int most = FF_THREADS / groups < FF_MAX_ROWS ? FF_THREADS / groups : FF_MAX_ROWS;
         // two CTAs an SM, or one where that leaves each fewer rows than there are tokens to copy beside them
         int ctas = 2 * sms;
         if ((N + ctas - 1) / ctas < T) ctas = sms;
         int rounds = 1;
-        while ((N + (long long)rounds * ctas - 1) / ((long long)rounds * ctas) > most) ++rounds;
+        while ((N + (long long)rounds * ctas - 1) / ((long long)rounds * ctas) > FF_MAX_ROWS) ++rounds;
         const int rows = int((N + (long long)rounds * ctas - 1) / ((long long)rounds * ctas)), tiles = (N + rows - 1) / rows;
+        // A token a thread where two warps hold them all (2,048 x 8,192 at 4 tokens 41 us, 60 with four a thread), else up to
+        // four: the row's operands are then read once for all (a head of 128,256 x 2,048 at 4 tokens 219 us, 265 with one).
+        int tt = 1;
+        while (tt < 4 && rows * ((T + tt - 1) / tt) > 64) tt *= 2;
         const int grid = tiles < ctas ? tiles : ctas;
         // as deep a ring as lets two CTAs share an SM: what is on its way has to cover memory's latency
         const size_t stage = size_t(rows + T) * FF_LD * sizeof(float);
