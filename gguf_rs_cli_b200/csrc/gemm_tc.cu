@@ -476,11 +476,13 @@ static int tile_for(int T, int N, int K, int sms, bool pair) {
     if (pair) {
         // up to 128 tokens: tiles of 64, two CTAs per SM (a CTA with a wide tile streams its operands no faster)
         if (bn == 128) return 64;
-        // A few hundred tokens go to the kernel that pairs two SMs like thousands (512 x 4096 x 4096 24 instead of 30 us,
-        // 300 x 6144 x 4096 24 instead of 30), but where K is long and the tiles few, CTAs that share tiles of 64 tokens
-        // are faster (200 x 4096 x 14336 51 instead of 57 us, 300 x 2048 x 8192 29 instead of 34; with one CTA a tile 74
-        // instead of 57).
-        if (bn == 256 && K >= 8192 && ft * ((T + 63) / 64) <= sms) return 64;
+        // A few hundred tokens go to the kernel that pairs two SMs like thousands (512 x 4096 x 4096 21 us, 26 with tiles of 64
+        // tokens; 300 x 6144 x 4096 22 and 27), but a tile of that kernel takes what its K takes, however few there are: where
+        // K is long enough for several CTAs to share every tile of 64 tokens, those are faster (300 x 256 x 2048 9.4 against
+        // 11.1 us, 130 x 2048 x 4096 14.1 against 18.4, 200 x 4096 x 14336 47 against 55).  The two meet at 40 tiles for
+        // K = 2048 (11.4 and 11.8 us), 96 for 4096 (18.9 and 19.5), 148 for 8192 (35.1 and 35.6); at K = 1024 never.
+        const long long tiles = ft * ((T + 63) / 64);
+        if (bn == 256 && K >= 2048 && tiles <= sms && tiles <= K / 48) return 64;
         return bn;
     }
     // one CTA a tile only: a few hundred tokens with few features would give 256-token tiles for less than half of the SMs, so

@@ -77,9 +77,9 @@ def test_token_tiles_of_two_sms(tile):
 
 @pytest.mark.parametrize("T", [129, 191, 300, 512, 769])
 def test_a_few_hundred_tokens(T):
-    """Either side of every border of the rule: K at 8,192, more tiles of 64 tokens than SMs."""
+    """Either side of every border of the rule: K at 2,048, tiles of 64 tokens per K, more of them than SMs."""
     k = K()
-    for N, Kd in ((256, 8192), (4096, 8192), (640, 8128), (6144, 64), (130, 8200)):
+    for N, Kd in ((256, 8192), (4096, 8192), (640, 2040), (640, 2048), (1300, 2048), (6144, 64), (130, 8200)):
         x, w, b, _ = _operands(T, N, Kd, T + N)
         out = torch.empty(T, N, device=DEV)
         k.gemm_tc(x, w, b, out)
