@@ -108,18 +108,17 @@ def generate(llm: LLM, prompt_ids: Sequence[Sequence[int]], max_tokens: int = 51
     limit = min(ctx_len or llm.spec.max_position, llm.spec.max_position)
     batch = min(max_batch, len(prompts))
     longest = sorted((min(len(p) + max_tokens, limit) for p in prompts), reverse=True)[:batch]
-    n_tokens = sum(((n + 63) // 64) * 64 for n in longest)
+    # a sequence ends at its engine's last position but one, so a request of one sequence whose tokens fill a page to its end
+    # gets a page more: what ends it is max_tokens or the model's limit, never the engine that happens to be at hand
+    n_tokens = max(sum(((n + 63) // 64) * 64 for n in longest), (min(longest[0] + 1, limit) + 63) // 64 * 64)
     backend = llm.backend(n_tokens=n_tokens, n_slots=batch, max_len=limit)
     stops = llm.spec.stop_token_ids if stop_token_ids is None else stop_token_ids
     params = SamplingParams(temperature, top_k, top_p, rep_penalty, seed)
     backend.profile = bool(profile)
-
-    # an engine that cannot hold `limit` positions of one sequence limits this call as one made for it would
-    context = limit if backend.context_limit >= limit else min(limit, (n_tokens + 63) // 64 * 64)
 
     def clock():
         torch.cuda.synchronize()
         return time.perf_counter()
 
     return generate_ids(backend, prompts, max_tokens, params, stops, max_batch=batch, on_token=on_token, stats=stats,
-                        clock=clock if stats is not None else None, context_limit=context)
+                        clock=clock if stats is not None else None, context_limit=limit)

@@ -255,3 +255,31 @@ def test_decode_split_rule_is_fixed_within_a_graph_class():
     # eight sequences split in two from about 1,500 positions on, sixteen never: one CTA per SM is kept
     assert [kernels.decode_splits(8, 32, 8, n, sms, True) for n in (1024, 1600, 2048, 8000)] == [1, 2, 2, 2]
     assert kernels.decode_splits(16, 32, 8, 4096, sms, True) == 1 and kernels.decode_splits(4, 32, 8, 4096, sms, True) == 4
+
+
+class _HostEngine:
+    """What `LLM.engine` and `generate` look at of an engine, without a device."""
+
+    def __init__(self, model, n_tokens, n_slots, max_len=None):
+        from types import SimpleNamespace
+        pages = (n_tokens + 63) // 64
+        self.cache = SimpleNamespace(n_slots=n_slots, n_pages=pages, max_len=min(max_len or model.spec.max_position, 64 * pages),
+                                     slots=SimpleNamespace(held_count=0))
+
+
+# (prompts' lengths, max_tokens, ctx_len, ids): 5 + 59 fills a page to its end; 200 is the model's limit and 64 and 65 a caller's, where
+# the reference's rule (position >= context - 1) ends a sequence
+@pytest.mark.parametrize("lens, n, ctx, want", [([5], 59, None, 59), ([5], 58, None, 58), ([5], 60, None, 60), ([64], 64, None, 64),
+                                                ([5, 7], 59, None, 59), ([5], 59, 64, 58), ([5], 200, None, 194), ([1], 63, 65, 63)])
+@pytest.mark.parametrize("before", [None, (3, 40), (70, 20), (5, 59), (30, 500)])
+def test_ids_do_not_depend_on_the_engine_at_hand(lens, n, ctx, want, before, monkeypatch):
+    from types import SimpleNamespace
+    from gguf_rs_cli_b200 import api
+    monkeypatch.setattr(api, "Engine", _HostEngine)
+    monkeypatch.setattr(api, "EngineBackend", lambda e: Scripted(n_slots=e.cache.n_slots, context_limit=e.cache.max_len))
+    model = SimpleNamespace(spec=SimpleNamespace(max_position=200, stop_token_ids=[]))
+    llm = api.LLM(model, {})
+    if before:
+        api.generate(llm, [[1] * before[0]] * 2, max_tokens=before[1])
+    out = api.generate(llm, [[1] * k for k in lens], max_tokens=n, ctx_len=ctx)
+    assert [len(o) for o in out] == [want] * len(lens)
