@@ -315,5 +315,11 @@ class EngineBackend:
         self.engine.check()
         return pending.out_host[:pending.n].tolist()
 
+    def settle(self) -> None:
+        """Waits for every step that was launched, read or not: its buffers are then anybody's, on any stream."""
+        for event in self._events:
+            event.synchronize()
+        torch.cuda.current_stream(self.engine.device).synchronize()       # a step that failed before its event was recorded
+
     def run(self, slots: List[int], feeds: List[List[int]], keys: List[int], params: SamplingParams) -> List[int]:
         return self.finish(self.begin(slots, feeds, keys, params))

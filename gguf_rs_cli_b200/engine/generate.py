@@ -76,6 +76,7 @@ def generate_ids(backend, prompts: Sequence[Sequence[int]], max_tokens: int, par
                                when each may grow by n tokens; at least 1 or an error
     backend.open() -> slot     backend.close(slot)
     backend.run(slots, feeds, keys, params) -> one sampled token per sequence
+    backend.settle()           where it has one: waits for the steps in flight (a call that is interrupted leaves none behind)
     """
     params.validate()
     stops = set(int(s) for s in stop_token_ids)
@@ -150,6 +151,12 @@ def generate_ids(backend, prompts: Sequence[Sequence[int]], max_tokens: int, par
                 elif live:
                     rows, counts = live, [1] * len(live)
                     pending = steps.begin([s.slot for s in rows], [s.feed for s in rows], [keys[s.request] for s in rows], params)
+        except BaseException:
+            # the engine outlives this call, and the next one may run on another stream: nothing orders it behind a step
+            # that is still in flight
+            if hasattr(backend, "settle"):
+                backend.settle()
+            raise
         finally:
             # a step, a callback or the cache may raise: whatever the batch still holds is given back
             for s in live:

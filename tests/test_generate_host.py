@@ -235,6 +235,27 @@ def test_a_failure_with_a_step_in_flight_gives_every_slot_back():
     assert not b.state and sorted(b.free) == [0, 1, 2]
 
 
+def test_an_interrupted_call_leaves_no_step_in_flight():
+    """The next call has the same buffers, perhaps on another stream: the step that ran ahead is waited for before slots are
+    given back, whatever interrupts the call."""
+    class Settling(ScriptedAhead):
+        def settle(self):
+            self.in_flight.clear()
+            self.log.append(("settle", -1))
+
+    def boom(i, tok):
+        if tok == 12:
+            raise KeyboardInterrupt
+    b = Settling(n_slots=3)
+    with pytest.raises(KeyboardInterrupt):
+        generate_ids(b, [[10], [20], [30]], max_tokens=5, on_token=boom)
+    assert not b.in_flight and not b.state
+    assert [e[0] for e in b.log[-5:]] == ["ahead", "settle", "close", "close", "close"]
+    b = Settling(n_slots=3)
+    generate_ids(b, [[10], [20], [30]], max_tokens=5)
+    assert not b.in_flight and ("settle", -1) not in b.log          # a call that ends has read every step
+
+
 def test_decode_split_rule_is_fixed_within_a_graph_class():
     """A captured decode graph is keyed by the class of the longest sequence: within a class the number of page
     splits must not change, for any batch size, and it never asks for more CTAs than the rule allows."""
