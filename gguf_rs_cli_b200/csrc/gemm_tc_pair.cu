@@ -24,6 +24,7 @@ constexpr int POUT_CHUNK = 16 * BM * 2;      // a staged piece of the result: 16
 constexpr int POUT_RING = 4;                // pieces in flight to global memory
 constexpr int PSMEM = PSTAGES * PSTAGE_BYTES + POUT_RING * POUT_CHUNK + 1024;
 constexpr int PTMEM_COLS = 2 * PBN;         // two accumulators
+constexpr int PMAX_DEVICES = 64;
 
 struct PairUnit {
     int n0, t0;                             // first feature and first token of the tile
@@ -213,10 +214,28 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
 static int g_pair_tile = 0;
 GB_API int gb_gemm_tc_set_pair_tile(int bn) { g_pair_tile = bn; return 0; }
 
-// How many pairs of CTAs of this kernel the device holds at once (0 if it cannot be asked).
-static int pair_slots() {
-    static int slots = -1;
-    if (slots < 0) {
+// Raises the kernel's shared-memory limit on the current device, on its first call there; 0: done.
+static int pair_ready(int* dev) {
+    static bool configured[PMAX_DEVICES] = {};
+    if (cudaGetDevice(dev) != cudaSuccess || *dev < 0 || *dev >= PMAX_DEVICES) return gb_fail("gb_gemm_tc: no usable current device");
+    if (!configured[*dev]) {
+        if (cudaFuncSetAttribute(gemm_tc_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(gemm_tc_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM) != cudaSuccess) {
+            cudaGetLastError();
+            return gb_fail("gb_gemm_tc: cannot get %d bytes of shared memory", PSMEM);
+        }
+        configured[*dev] = true;
+    }
+    return 0;
+}
+
+// How many pairs of CTAs of this kernel the current device holds at once (0 if it cannot be asked; then it is asked again).  The
+// question is refused for more shared memory than the kernel's limit, so that comes first.
+GB_API int gb_gemm_tc_pair_slots() {
+    static int slots[PMAX_DEVICES] = {};
+    int dev = 0;
+    if (pair_ready(&dev)) return 0;
+    if (slots[dev] == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2);
         cfg.blockDim = dim3(TC_THREADS);
@@ -230,9 +249,14 @@ static int pair_slots() {
         cfg.numAttrs = 1;
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_kernel<true>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-        slots = n;
+        slots[dev] = n;
     }
-    return slots;
+    return slots[dev];
+}
+
+static long long pair_slots(int sms) {
+    const int n = gb_gemm_tc_pair_slots();
+    return n > 0 ? n : sms / 2;
 }
 
 // Tokens of a tile: the width whose rounds over the device take the least time.  A 256 x bn tile over K takes a time
@@ -241,7 +265,7 @@ static int pair_slots() {
 // 512 x 4096 x 14336: one round of 256 (89 us) or of 160 (65 us).  Of equal costs the widest.
 int gemm_tc_pair_tile(int T, int N, int sms) {
     if (g_pair_tile > 0) return g_pair_tile;
-    const long long ft = (N + 2 * BM - 1) / (2 * BM), slots = pair_slots() > 0 ? pair_slots() : sms / 2;
+    const long long ft = (N + 2 * BM - 1) / (2 * BM), slots = pair_slots(sms);
     int best = PBN;
     long long least = -1;
     for (int bn = PBN; bn >= 160; bn -= 16) {
@@ -254,16 +278,10 @@ int gemm_tc_pair_tile(int T, int N, int sms) {
 int gemm_tc_pair_launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap* mo, const void* params,
                         cudaStream_t stream) {
     const TcParams& p = *static_cast<const TcParams*>(params);
-    static int state = 0;                          // 1: ready, -1: refused
-    if (state == 0) {
-        state = cudaFuncSetAttribute(gemm_tc_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM) == cudaSuccess &&
-                        cudaFuncSetAttribute(gemm_tc_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM) == cudaSuccess
-                    ? 1 : -1;
-        if (state < 0) cudaGetLastError();
-    }
-    if (state < 0) return gb_fail("gb_gemm_tc: cannot get %d bytes of shared memory", PSMEM);
+    int dev = 0;
+    if (pair_ready(&dev)) return 1;
     long long units = (long long)((p.N + 2 * BM - 1) / (2 * BM)) * ((p.T + p.pair_tile - 1) / p.pair_tile);
-    long long slots = pair_slots() > 0 ? pair_slots() : p.sms / 2;     // pairs that can be resident at once
+    long long slots = pair_slots(p.sms);                                // pairs that can be resident at once
     long long rounds = (units + slots - 1) / slots;
     long long pairs = (units + rounds - 1) / rounds;
     cudaLaunchConfig_t cfg = {};

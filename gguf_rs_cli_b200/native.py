@@ -225,6 +225,7 @@ _SIGNATURES = {
     "gb_gemm_f32": [_P, _L, _P, _L, _P, _I, _P, _I, _L, _I, _I, _I, _P],
     "gb_gemm_f32_supported": [_P, _L, _P, _L, _I],
     "gb_gemm_tc_set_pair_tile": [_I],
+    "gb_gemm_tc_pair_slots": [],
     "gb_gemm_tc_set_stamps": [_P, _I, _I],
     "gb_attention_decode_scratch_floats": [_I, _I, _I, _I],
     "gb_attention_decode_supported": [_I, _I, _I],

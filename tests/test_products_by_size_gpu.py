@@ -75,6 +75,23 @@ def test_token_tiles_of_two_sms(tile):
     k.check_tc_status()
 
 
+def test_pairs_of_sms_are_counted_before_the_first_product():
+    """The width of a tile goes by how many pairs the device holds, asked before the kernel's first launch in a process."""
+    import subprocess
+    import sys
+    code = """if True:
+        import torch
+        from gguf_rs_cli_b200 import kernels, native
+        x = torch.zeros(1024, 256, device="cuda", dtype=torch.bfloat16)
+        first = native.library().gb_gemm_tc_pair_slots()
+        kernels.gemm_tc(x, x, None, torch.empty(1024, 1024, device="cuda"))
+        torch.cuda.synchronize()
+        assert 0 < first == native.library().gb_gemm_tc_pair_slots() <= torch.cuda.get_device_properties(0).multi_processor_count // 2
+    """
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+
 @pytest.mark.parametrize("T", [129, 191, 300, 512, 769])
 def test_a_few_hundred_tokens(T):
     """Either side of every border of the rule: K at 2,048, tiles of 64 tokens per K, more of them than SMs."""
