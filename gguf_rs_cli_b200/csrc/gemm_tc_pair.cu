@@ -210,9 +210,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
 
 }  // namespace
 
-// A tuning aid (process-wide): > 0: tokens of every tile.
+// A tuning aid (process-wide): > 0: tokens of every tile, in the steps that the MMA and the output's pieces of 16 tokens allow.
 static int g_pair_tile = 0;
-GB_API int gb_gemm_tc_set_pair_tile(int bn) { g_pair_tile = bn; return 0; }
+GB_API int gb_gemm_tc_set_pair_tile(int bn) {
+    GB_REQUIRE(bn == 0 || (bn >= 32 && bn <= PBN && bn % 16 == 0), "gb_gemm_tc_set_pair_tile: %d is no multiple of 16 from 32 to %d", bn, PBN);
+    g_pair_tile = bn;
+    return 0;
+}
 
 // Raises the kernel's shared-memory limit on the current device, on its first call there; 0: done.
 static int pair_ready(int* dev) {

@@ -25,3 +25,15 @@ def test_the_ordinary_library_has_no_time_stamps():
     for entry, args in (("gb_gemm_tc_set_stamps", (0, 0, 0)), ("gb_attention_decode_set_stamps", (0,))):
         with pytest.raises(native.NativeError, match="without -DGB_STAMPS"):
             native.call(entry, *args)
+
+
+def test_a_tile_width_that_the_kernel_cannot_run_is_refused():
+    import pytest
+    try:
+        for bn in (32, 176, 256, 0):
+            native.call("gb_gemm_tc_set_pair_tile", bn)
+        for bn in (-16, 1, 16, 100, 168, 264, 272, 512):
+            with pytest.raises(native.NativeError, match="multiple of 16"):
+                native.call("gb_gemm_tc_set_pair_tile", bn)
+    finally:
+        native.call("gb_gemm_tc_set_pair_tile", 0)
