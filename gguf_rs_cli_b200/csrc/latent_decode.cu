@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(LM_THREADS) latent_decode_mma_kernel(const LdP
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (valid ? 8 * c8 : 0)), "r"(valid ? 16 : 0) : "memory");
         }
     };
-    for (int r = warp; r < 16; r += LM_THREADS / 32) copy(qt + r * KS, p.q + size_t(t) * p.ldq + size_t(r < H ? r : 0) * HDK, r < H);
+    if (kb0 < kb1)                                     // a split without blocks asks for nothing: only the loop below waits
+        for (int r = warp; r < 16; r += LM_THREADS / 32) copy(qt + r * KS, p.q + size_t(t) * p.ldq + size_t(r < H ? r : 0) * HDK, r < H);
     const int CW = C / 4, ot = CW / 8;                 // this warp's value columns [warp * CW, +CW): ot tiles of 8
     const float sl2 = p.scale * 1.4426950408889634f;
     float o[LM_MAX_OT][4];

@@ -1,0 +1,51 @@
+"""Latent attention of single tokens, the two kernels and their merge, against 64-bit sums."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+SIZES = [(16, 512, 64), (5, 64, 16), (3, 40, 24)]            # heads, kv_rank, rot_dim: tensor cores twice, CUDA cores
+
+
+def _step(lens, H, C, R, seed=0):
+    """A step of one token per sequence: queries, cache pages in any order, and what the kernels read of a context."""
+    from gguf_rs_cli_b200.parts.base import Workspace
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    T, width = len(lens), (max(lens) + 63) // 64
+    q = torch.randn(T, H * (C + R), generator=g, device=DEV).bfloat16()
+    cache = torch.randn(T * width, 1, 64, C + R, generator=g, device=DEV).bfloat16()
+    table = torch.randperm(T * width, generator=g, device=DEV).int().view(T, width)
+    ctx = SimpleNamespace(max_kv=max(lens), ws=Workspace(DEV), seq_of=torch.arange(T, device=DEV, dtype=torch.int32),
+                          pos=torch.tensor([n - 1 for n in lens], device=DEV, dtype=torch.int32))
+    return q, cache, table, ctx
+
+
+def _plain(q, cache, table, lens, H, C, R, scale, window=0):
+    out = []
+    for t, n in enumerate(lens):
+        rows = cache[table[t].long()].reshape(-1, C + R)[:n].double()
+        s = q[t].double().view(H, C + R) @ rows.T * scale
+        if window:
+            s[:, :max(0, n - window)] = -torch.inf
+        out.append((torch.softmax(s, -1) @ rows[:, :C]).flatten())
+    return torch.stack(out)
+
+
+def _check(got, want):
+    """Half a unit in the last place of bfloat16 is 2^-9 of a value; sums of a few thousand 32-bit terms are far below the other half."""
+    assert ((got.double() - want).abs() <= 2 ** -8 * want.abs().amax(1, keepdim=True)).all()
+
+
+@pytest.mark.parametrize("H, C, R", SIZES)
+@pytest.mark.parametrize("lens", [[1], [1, 1000, 33, 64, 740], [32, 65, 2], [736] * 4, [300] * 40])
+def test_unequal_lengths_in_one_step(H, C, R, lens):
+    """Splits follow the longest sequence: a short one leaves most of its splits without keys."""
+    from gguf_rs_cli_b200 import kernels
+    q, cache, table, ctx = _step(lens, H, C, R)
+    scale = (C + R) ** -0.5
+    for window in (0, 45):
+        out = torch.full((len(lens), H * C), 7.0, device=DEV, dtype=torch.bfloat16)
+        kernels.latent_decode(q, out, H, C, R, ctx, table, table.shape[1], cache, scale, window=window)
+        _check(out, _plain(q, cache, table, lens, H, C, R, scale, window))
