@@ -22,7 +22,7 @@ constexpr int LD_THREADS = LD_WARPS * 32;
 constexpr int LD_MAX_HEADS = 16;                    // heads per token: at most 2 per warp (with 32 heads the general
                                                     // kernel's block per head was measured faster: 0.774 against 0.799 ms a step)
 constexpr int LD_HW = LD_MAX_HEADS / LD_WARPS;
-constexpr int LD_MAX_SPLITS = 64;
+constexpr int LD_MERGED = 64;                       // splits whose factors a CTA of the merge holds at a time
 constexpr int LD_MAX_C = 512;                       // entries of the value: at most 8 pairs per lane
 constexpr int LD_PAIRS = LD_MAX_C / 64;
 
@@ -329,24 +329,46 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ scratch, co
         for (int c = threadIdx.x; c < C; c += blockDim.x) o[c] = __float2bfloat16_rn(0.f);
         return;
     }
-    // every split's factor once: e^(m_s - M), at most LD_MAX_SPLITS of them
-    __shared__ float w[LD_MAX_SPLITS], sums[LD_MAX_SPLITS], total[2];
+    // every split's factor once, e^(m_s - M), LD_MERGED splits at a time (no wrapper asks for more than one such group)
+    __shared__ float w[LD_MERGED], sums[LD_MERGED], total[2];
     const float* base = scratch + (size_t(t) * H + h) * splits * (C + 2);
-    for (int s = threadIdx.x; s < splits; s += blockDim.x) {
-        w[s] = base[size_t(s) * (C + 2) + C];
-        sums[s] = base[size_t(s) * (C + 2) + C + 1];
-    }
-    __syncthreads();
+    auto load = [&](int s0) {                // a group's maxima and sums; how many they are
+        const int n = min(LD_MERGED, splits - s0);
+        for (int s = threadIdx.x; s < n; s += blockDim.x) {
+            w[s] = base[size_t(s0 + s) * (C + 2) + C];
+            sums[s] = base[size_t(s0 + s) * (C + 2) + C + 1];
+        }
+        __syncthreads();
+        return n;
+    };
     float M = -INFINITY;
-    for (int s = 0; s < splits; ++s) M = fmaxf(M, w[s]);
-    __syncthreads();
-    for (int s = threadIdx.x; s < splits; s += blockDim.x) w[s] = w[s] == -INFINITY ? 0.f : expf(w[s] - M);
-    __syncthreads();
+    for (int s0 = 0; s0 < splits; s0 += LD_MERGED) {
+        const int n = load(s0);
+        for (int s = 0; s < n; ++s) M = fmaxf(M, w[s]);
+        __syncthreads();
+    }
+    const int c = threadIdx.x;               // an entry a thread
+    float v = 0.f, L = 0.f;                  // L: the first thread's
+    for (int s0 = 0; s0 < splits; s0 += LD_MERGED) {
+        const int n = splits > LD_MERGED ? load(s0) : splits;             // a single group is still there
+        for (int s = threadIdx.x; s < n; s += blockDim.x) w[s] = w[s] == -INFINITY ? 0.f : expf(w[s] - M);
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int s = 0; s < n; ++s)
+                if (w[s] != 0.f) L += sums[s] * w[s];
+        if (c < C) {
+            // a split without keys has left nothing (its record may hold anything)
+            const float* x0 = base + size_t(s0) * (C + 2) + c;
+#pragma unroll 16
+            for (int s = 0; s < n; ++s) {
+                const float x = x0[size_t(s) * (C + 2)];      // loaded whatever the factor, so that sixteen are on their way
+                v += w[s] != 0.f ? x * w[s] : 0.f;
+            }
+        }
+        __syncthreads();
+    }
     if (threadIdx.x == 0) {
-        float L = 0.f;
-        for (int s = 0; s < splits; ++s)
-            if (w[s] != 0.f) L += sums[s] * w[s];
-        float f = 1.f;                   // what the sums are multiplied by: a sink above every score brings them down to its level
+        float f = 1.f;                       // what the sums are multiplied by: a sink above every score brings them down to its level
         if (sink && M != -INFINITY) {
             const float sv = sink[h];
             if (sv > M) {
@@ -361,17 +383,7 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ scratch, co
         total[1] = L;
     }
     __syncthreads();
-    const float f = total[0], L = total[1];
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        float v = 0.f;
-        // a split without keys has left nothing (its record may hold anything)
-#pragma unroll 16
-        for (int s = 0; s < splits; ++s) {
-            const float x = base[size_t(s) * (C + 2) + c];        // loaded whatever the factor, so that sixteen are on their way
-            v += w[s] != 0.f ? x * w[s] : 0.f;
-        }
-        o[c] = __float2bfloat16_rn(v * f / L);
-    }
+    if (c < C) o[c] = __float2bfloat16_rn(v * total[0] / total[1]);
 }
 
 }  // namespace
@@ -406,11 +418,11 @@ GB_API int gb_latent_decode(const void* q, long long ldq, void* out, long long l
                             const void* gate, long long ldg, cudaStream_t stream) {
     GB_REQUIRE(window >= 0, "gb_latent_decode: a negative window");
     GB_REQUIRE(gb_latent_decode_supported(H, C, R, GB_BF16, GB_BF16), "gb_latent_decode: sizes heads=%d kv_rank=%d rot_dim=%d are not supported", H, C, R);
-    GB_REQUIRE(splits >= 1 && splits <= LD_MAX_SPLITS && scratch && table_width > 0 && ring_pages > 0, "gb_latent_decode: bad arguments");
+    GB_REQUIRE(splits >= 1 && splits <= 65535 && scratch && table_width > 0 && ring_pages > 0, "gb_latent_decode: bad arguments");
     GB_REQUIRE((ldq % 2) == 0 && (reinterpret_cast<uintptr_t>(cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(scratch) & 7) == 0,
                "gb_latent_decode: misaligned operands");
     if (T == 0) return 0;
-    const int merge_threads = C >= 512 ? 512 : (C + 31) / 32 * 32;          // an entry a thread, all splits' numbers on their way
+    const int merge_threads = (C + 31) / 32 * 32;          // an entry a thread, the splits' numbers on their way together
     LdParams p;
     p.q = (const __nv_bfloat16*)q; p.cache = (const __nv_bfloat16*)cache; p.seq_of = seq_of; p.pos = pos; p.table = table;
     p.scratch = scratch; p.ldq = ldq; p.H = H; p.C = C; p.R = R; p.splits = splits; p.table_width = table_width;

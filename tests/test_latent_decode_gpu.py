@@ -49,3 +49,26 @@ def test_unequal_lengths_in_one_step(H, C, R, lens):
         out = torch.full((len(lens), H * C), 7.0, device=DEV, dtype=torch.bfloat16)
         kernels.latent_decode(q, out, H, C, R, ctx, table, table.shape[1], cache, scale, window=window)
         _check(out, _plain(q, cache, table, lens, H, C, R, scale, window))
+
+
+@pytest.mark.parametrize("H, C, R", SIZES)
+@pytest.mark.parametrize("splits", [1, 2, 63, 64, 65, 128, 129, 300])
+def test_any_number_of_splits(H, C, R, splits):
+    """The merge holds 64 splits' factors at a time; the entry takes as many as a grid has rows."""
+    from gguf_rs_cli_b200 import native
+    from gguf_rs_cli_b200.native import call, ptr, stream_ptr
+    lens = [4500, 70, 1]
+    q, cache, table, ctx = _step(lens, H, C, R, seed=splits)
+    g = torch.Generator(device=DEV).manual_seed(splits)
+    sink, gate = torch.randn(H, generator=g, device=DEV), torch.randn(3, H, generator=g, device=DEV).bfloat16()
+    scale = (C + R) ** -0.5
+    scratch = torch.full((native.library().gb_latent_decode_scratch_floats(3, H, C, splits),), torch.nan, device=DEV)
+    out = torch.full((3, H * C), 7.0, device=DEV, dtype=torch.bfloat16)
+    call("gb_latent_decode", ptr(q), q.stride(0), ptr(out), out.stride(0), 3, H, C, R, ptr(ctx.seq_of), ptr(ctx.pos), ptr(table),
+         table.shape[1], table.shape[1], ptr(cache), float(scale), splits, ptr(scratch), 0, ptr(sink), ptr(gate), gate.stride(0), stream_ptr())
+    want = []
+    for t, n in enumerate(lens):
+        rows = cache[table[t].long()].reshape(-1, C + R)[:n].double()
+        s = torch.cat([q[t].double().view(H, C + R) @ rows.T * scale, sink.double()[:, None]], 1)
+        want.append(((torch.softmax(s, -1)[:, :-1] @ rows[:, :C]) * torch.sigmoid(gate[t].double())[:, None]).flatten())
+    _check(out, torch.stack(want))
