@@ -351,18 +351,19 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ scratch, co
     float v = 0.f, L = 0.f;                  // L: the first thread's
     for (int s0 = 0; s0 < splits; s0 += LD_MERGED) {
         const int n = splits > LD_MERGED ? load(s0) : splits;             // a single group is still there
-        for (int s = threadIdx.x; s < n; s += blockDim.x) w[s] = w[s] == -INFINITY ? 0.f : expf(w[s] - M);
+        // -1: a split without keys, which has left nothing (its record may hold anything).  A factor that is too small for 32 bits
+        // is 0 and is used all the same, so that a split's infinities and NaN are not lost behind one with larger scores.
+        for (int s = threadIdx.x; s < n; s += blockDim.x) w[s] = w[s] == -INFINITY ? -1.f : expf(w[s] - M);
         __syncthreads();
         if (threadIdx.x == 0)
             for (int s = 0; s < n; ++s)
-                if (w[s] != 0.f) L += sums[s] * w[s];
+                if (!(w[s] < 0.f)) L = fmaf(sums[s], w[s], L);
         if (c < C) {
-            // a split without keys has left nothing (its record may hold anything)
             const float* x0 = base + size_t(s0) * (C + 2) + c;
 #pragma unroll 16
             for (int s = 0; s < n; ++s) {
                 const float x = x0[size_t(s) * (C + 2)];      // loaded whatever the factor, so that sixteen are on their way
-                v += w[s] != 0.f ? x * w[s] : 0.f;
+                v = w[s] < 0.f ? v : fmaf(x, w[s], v);
             }
         }
         __syncthreads();

@@ -72,3 +72,19 @@ def test_any_number_of_splits(H, C, R, splits):
         s = torch.cat([q[t].double().view(H, C + R) @ rows.T * scale, sink.double()[:, None]], 1)
         want.append(((torch.softmax(s, -1)[:, :-1] @ rows[:, :C]) * torch.sigmoid(gate[t].double())[:, None]).flatten())
     _check(out, torch.stack(want))
+
+
+@pytest.mark.parametrize("H, C, R", SIZES)
+def test_a_nan_is_not_lost_behind_larger_scores(H, C, R):
+    """The first 32 keys' scores are 200 below the others', so that their split's factor e^-200 is 0 in 32 bits; a NaN in one of
+    those rows has to reach the result as it does in one pass over all keys."""
+    from gguf_rs_cli_b200 import kernels
+    lens = [256, 256]                                 # eight blocks of keys, eight splits
+    q, cache, table, ctx = _step(lens, H, C, R)
+    q[:], cache[:] = 1.0, 0.0
+    for t in range(2):
+        cache[table[t, 0].long(), 0, :32, 0] = -200.0
+    cache[table[1, 0].long(), 0, 7, 1] = torch.nan
+    out = torch.full((2, H * C), 7.0, device=DEV, dtype=torch.bfloat16)
+    kernels.latent_decode(q, out, H, C, R, ctx, table, table.shape[1], cache, 1.0)
+    assert (out[0] == 0).all() and out[1].isnan().all()
