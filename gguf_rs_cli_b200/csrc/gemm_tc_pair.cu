@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_pair_kernel(const __gri
                     tmem_ld16(taddr + c0, v);
                     tc_finish_chunk<PBN>(p, n0, w.t0, n, row, lane, quarter, bias, waited, c0, cols, v, rstd_s, ssq_s);
                 }
-                if (p.resid_x) tc_write_ssq<PBN>(p, n0, w.t0, row, 0, cols, ssq_s);
+                // where the last tile's features end in its first half, the other CTA has none: no sums to write, and no room for them
+                if (p.resid_x && n0 < p.N) tc_write_ssq<PBN>(p, n0, w.t0, row, 0, cols, ssq_s);
             }
             tc_fence_before();
             __syncwarp();

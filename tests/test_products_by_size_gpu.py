@@ -75,6 +75,22 @@ def test_token_tiles_of_two_sms(tile):
     k.check_tc_status()
 
 
+@pytest.mark.parametrize("T", [129, 300, 769, 2049])
+@pytest.mark.parametrize("N", [64, 128, 200, 300, 640])
+def test_residual_sums_stay_inside_their_rows(T, N):
+    """A pair's second CTA has no features where the last tile's end in its first half: it writes no sums of squares, which would
+    lie behind the ceil(N/128) rows that the caller gave."""
+    k = K()
+    x, w, b, _ = _operands(T, N, 64, T + N)
+    tiles = (N + 127) // 128
+    resid, copy = torch.ones(T, N, device=DEV), torch.empty(T, N, device=DEV, dtype=torch.bfloat16)
+    ssq = torch.full((tiles + 2, T), 7.0, device=DEV)
+    k.gemm_tc(x, w, b, None, resid_x=resid, resid_xb=copy, ssq_out=ssq)
+    assert (ssq[tiles:] == 7.0).all() and torch.equal(copy, resid.bfloat16())
+    sums = torch.nn.functional.pad(resid.double().pow(2), (0, -N % 128)).view(T, -1, 128).sum(2).t()
+    assert ((ssq[:tiles].double() - sums).abs() <= 2.0 ** -17 * sums).all()      # 128 squares, an addition off by 2^-24 of the sum at most
+
+
 def test_pairs_of_sms_are_counted_before_the_first_product():
     """The width of a tile goes by how many pairs the device holds, asked before the kernel's first launch in a process."""
     import subprocess
