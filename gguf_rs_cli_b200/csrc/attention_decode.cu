@@ -15,6 +15,8 @@
 
 #include "common.cuh"
 
+GB_API int gb_sm_count();
+
 namespace {
 
 constexpr int AD_THREADS = 128;
@@ -63,8 +65,10 @@ __device__ __forceinline__ void unpack8(uint4 v, float* f) {
     }
 }
 
-template <int GT, int HC>
-__global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p) {
+// PER_SM: CTAs that an SM has to hold (0: as many as the registers leave).
+template <int GT, int HC, int PER_SM = 0>
+__global__ void __launch_bounds__(AD_THREADS, PER_SM) attention_decode_kernel(AdParams p) {
+    constexpr bool EARLY = HC <= 2 && GT <= 4;
     gb_grid_launch_dependents();
     gb_grid_wait();
     const int t = blockIdx.x;
@@ -132,17 +136,18 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
         const int kk = warp * AD_KEYS_PER_WARP + key_in_warp;
         const int j = pg * GB_PAGE + kk;
         const bool valid = j <= pos && (j >= lo || j < keep);
-        // This warp's 16 rows of values are asked for before its keys are used (heads of up to 128, up to four of them: 32 registers): with a
-        // page or two per CTA the time is the trips to memory one after the other, and this takes four of six off.
-        const __nv_bfloat16* vp = p.vc + page_off + size_t(warp * AD_KEYS_PER_WARP) * hd;
-        const int first_key = pg * GB_PAGE + warp * AD_KEYS_PER_WARP;
+        // EARLY: this warp's 16 rows of values are asked for before its keys are used: with a page or two per CTA the time is the trips to
+        // memory one after the other, and this takes four of six off (4 sequences of 739 positions, 4 KV heads of 128, one split, us:
+        // groups of 1 58 -> 26, of 4 71 -> 41).  It is for heads of up to 128, up to four of them: it takes 16 or 32 registers, and
+        // what they displace costs the larger instances more CTAs than the trips are worth (groups of 8 with heads of 128, 64
+        // sequences of 1,000: 244, and 412 with their loop compiled the other way at 144 registers instead of 114).
         auto seen = [&](int k) {                       // uniform over the warp; unwritten rows are never read
-            const int jk = first_key + k;
+            const int jk = pg * GB_PAGE + warp * AD_KEYS_PER_WARP + k;
             return jk <= pos && (jk >= lo || jk < keep);
         };
-        constexpr bool EARLY = HC <= 2 && GT <= 4;
         unsigned vr[EARLY ? AD_KEYS_PER_WARP : 1][HC];
         if constexpr (EARLY) {
+            const __nv_bfloat16* vp = p.vc + page_off + size_t(warp * AD_KEYS_PER_WARP) * hd;
 #pragma unroll
             for (int k = 0; k < AD_KEYS_PER_WARP; ++k)
 #pragma unroll
@@ -196,6 +201,7 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
         for (int gi = 0; gi < GT; ++gi)
 #pragma unroll
             for (int c = 0; c < HC; ++c) { acc[gi][c][0] *= alpha[gi]; acc[gi][c][1] *= alpha[gi]; }
+        const int first_key = pg * GB_PAGE + warp * AD_KEYS_PER_WARP;
         auto mix = [&](int k, const float2 (&vf)[HC]) {
 #pragma unroll
             for (int gi = 0; gi < GT; ++gi) {
@@ -217,9 +223,11 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
                 mix(k, vf);
             }
         } else {
+            const __nv_bfloat16* vp = p.vc + page_off + size_t(warp * AD_KEYS_PER_WARP) * hd;
 #pragma unroll 4
             for (int k = 0; k < AD_KEYS_PER_WARP; ++k) {
-                if (!seen(k)) continue;
+                const int jk = first_key + k;
+                if (jk > pos || (jk < lo && jk >= keep)) continue;
                 float2 vf[HC];
 #pragma unroll
                 for (int c = 0; c < HC; ++c) {
@@ -227,7 +235,15 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
                     vf[c] = make_float2(0.f, 0.f);
                     if (d < hd) vf[c] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(vp + size_t(k) * hd + d));
                 }
-                mix(k, vf);
+#pragma unroll
+                for (int gi = 0; gi < GT; ++gi) {
+                    float pv = ps[warp][gi][k];
+#pragma unroll
+                    for (int c = 0; c < HC; ++c) {
+                        acc[gi][c][0] = fmaf(pv, vf[c].x, acc[gi][c][0]);
+                        acc[gi][c][1] = fmaf(pv, vf[c].y, acc[gi][c][1]);
+                    }
+                }
             }
         }
         __syncwarp();
@@ -276,16 +292,49 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
     for (int i = threadIdx.x; i < heads * hd; i += AD_THREADS) {
         int gi = i / hd, d = i - gi * hd;
         const float* rec = p.scratch + (size_t(t) * p.nh + h0 + gi) * p.splits * (hd + 2);
-        float M = -INFINITY;
+        // The splits' numbers are added in order; how many are on their way together is chosen per instance, by what it costs the
+        // loop over the pages in registers (us, 1 x 4,000 positions in 32 splits and 8 x 500 in 4): groups of 8 with heads of
+        // 128 83 and 38 with the compiler's own unrolling, 60 and 47 by eights and the rest one by one, 58 and 38 as here.
+        float M = -INFINITY, L = 0.f, o = 0.f;
+        if constexpr (EARLY) {
 #pragma unroll 8
-        for (int s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd));
-        float L = 0.f, o = 0.f;
+            for (int s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd));
 #pragma unroll 8
-        for (int s = 0; s < p.splits; ++s) {
-            float ms = __ldcg(rec + s * (hd + 2) + hd);
-            float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);
-            L += __ldcg(rec + s * (hd + 2) + hd + 1) * wgt;
-            o += __ldcg(rec + s * (hd + 2) + d) * wgt;
+            for (int s = 0; s < p.splits; ++s) {
+                float ms = __ldcg(rec + s * (hd + 2) + hd);
+                float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);
+                L += __ldcg(rec + s * (hd + 2) + hd + 1) * wgt;
+                o += __ldcg(rec + s * (hd + 2) + d) * wgt;
+            }
+        } else if constexpr (GT == 8 && HC >= 2) {
+            auto largest = [&](int s) { M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd)); };
+            auto add = [&](int s) {
+                float ms = __ldcg(rec + s * (hd + 2) + hd);
+                float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);
+                L += __ldcg(rec + s * (hd + 2) + hd + 1) * wgt;
+                o += __ldcg(rec + s * (hd + 2) + d) * wgt;
+            };
+            auto in_order = [&](auto& each) {
+                int s = 0;
+                for (; s + 8 <= p.splits; s += 8)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) each(s + e);
+                for (; s + 4 <= p.splits; s += 4)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) each(s + e);
+                if (s + 2 <= p.splits) { each(s); each(s + 1); s += 2; }
+                if (s < p.splits) each(s);
+            };
+            in_order(largest);
+            in_order(add);
+        } else {
+            for (int s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd));
+            for (int s = 0; s < p.splits; ++s) {
+                float ms = __ldcg(rec + s * (hd + 2) + hd);
+                float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);
+                L += __ldcg(rec + s * (hd + 2) + hd + 1) * wgt;
+                o += __ldcg(rec + s * (hd + 2) + d) * wgt;
+            }
         }
         if (p.sink && M != -INFINITY) L += exp2f((p.sink_values ? p.sink_values[h0 + gi] * 1.4426950408889634f : 0.f) - M);
         p.out[size_t(t) * p.ldo + size_t(h0 + gi) * hd + d] = __float2bfloat16_rn(ad_gated(p, t, h0 + gi, d, o / L));
@@ -294,7 +343,14 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(AdParams p
 }
 
 template <int GT, int HC> int launch_ad(const AdParams& p, dim3 grid, cudaStream_t stream) {
-    gb_launch(attention_decode_kernel<GT, HC>, grid, dim3(AD_THREADS), 0, stream, p);
+    // Groups of up to 4 with heads of up to 64 need 140 registers, three CTAs an SM; more CTAs than that run in 96, five an SM
+    // (64 x 200 positions, 8 KV heads 28 -> 21 us, 256 x 60 28 -> 22, 64 x 1,000 113 -> 81), fewer are faster with them all
+    // (8 x 500 24 us, 28 in 96).
+    constexpr int FIVE = GT == 4 && HC == 1 ? 5 : 0;
+    if (FIVE && (long long)grid.x * grid.y * grid.z > 3LL * gb_sm_count())
+        gb_launch(attention_decode_kernel<GT, HC, FIVE>, grid, dim3(AD_THREADS), 0, stream, p);
+    else
+        gb_launch(attention_decode_kernel<GT, HC>, grid, dim3(AD_THREADS), 0, stream, p);
     GB_LAUNCH_OK("gb_attention_decode");
     return 0;
 }
