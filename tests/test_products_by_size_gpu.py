@@ -30,7 +30,8 @@ def _sum_bound(x, w):
 @pytest.mark.parametrize("T", [1, 2, 4, 5, 8, 9, 16, 17, 31, 48, 49, 144, 200])
 def test_32_bit_products_are_the_general_kernels_bit_for_bit(T):
     k = K()
-    for N, Kd in ((64, 64), (130, 176), (1, 4), (257, 132), (3072, 260), (20000, 96)):
+    # the last two: few tokens take several tiles a CTA with several pieces of K each
+    for N, Kd in ((64, 64), (130, 176), (1, 4), (257, 132), (3072, 260), (20000, 96), (20000, 260), (40000, 516)):
         x, w, b, _ = _operands(T, N, Kd, N + Kd, torch.float32)
         for bias in (None, b):
             want, got = torch.empty(T, N, device=DEV), torch.full((T, N + 5), 7.0, device=DEV)[:, :N]
@@ -47,7 +48,7 @@ def test_32_bit_products_are_the_general_kernels_bit_for_bit(T):
     assert torch.equal(got, want)
 
 
-@pytest.mark.parametrize("tile", [96, 112, 176, 240, 256, 0])
+@pytest.mark.parametrize("tile", [96, 112, 176, 192, 208, 224, 240, 256, 0])
 def test_token_tiles_of_two_sms(tile):
     """Every width gives the widest tile's results bit for bit (each is one ascending sum), whatever the number of tokens."""
     from gguf_rs_cli_b200 import native
@@ -65,9 +66,24 @@ def test_token_tiles_of_two_sms(tile):
                 for o in outs:
                     k.gemm_tc(x, w, b, o)
                 k.gemm_tc(x, w2, None, gated, swiglu_features=N // 2)
-                got.append(outs + [gated])
+                # a norm's factor per token, and a sum into the residual stream with its copy and the new sums of squares
+                scaled, resid = torch.full((T, N), 9.0, device=DEV), torch.ones(T, N, device=DEV)
+                copy, ssq = torch.empty(T, N, device=DEV, dtype=torch.bfloat16), torch.empty((N + 127) // 128, T, device=DEV)
+                parts = x.float().pow(2).view(T, 2, Kd // 2).sum(2).t().contiguous()
+                k.gemm_tc(x, w, None, scaled, row_ssq=parts, ssq_parts=2, norm_size=Kd, eps=1e-5)
+                k.gemm_tc(x, w, b, None, resid_x=resid, resid_xb=copy, ssq_out=ssq)
+                got.append(outs + [gated, scaled, resid, copy, ssq])
             assert all(torch.equal(a, c) for a, c in zip(*got)), (T, N, Kd)
-            assert ((got[1][1].double() - x.double() @ w.double().T - b.double()).abs() <= _sum_bound(x, w)).all()
+            plain = x.double() @ w.double().T
+            outs, scaled, resid, copy, ssq = got[1][:2], *got[1][3:]
+            assert ((outs[1].double() - plain - b.double()).abs() <= _sum_bound(x, w)).all()
+            rstd = (x.double().pow(2).mean(1, keepdim=True) + 1e-5).rsqrt()
+            # the factor itself is a 32-bit reciprocal root of a 32-bit mean: 2^-20 of the result covers both
+            assert ((scaled.double() - plain * rstd).abs() <= _sum_bound(x, w) * rstd + 2.0 ** -20 * (plain * rstd).abs()).all()
+            assert ((resid.double() - 1 - plain - b.double()).abs() <= _sum_bound(x, w) + 2.0 ** -22 * resid.double().abs()).all()
+            assert torch.equal(copy, resid.bfloat16())
+            sums = torch.nn.functional.pad(resid.double().pow(2), (0, -N % 128)).view(T, -1, 128).sum(2).t()
+            assert ((ssq.double() - sums).abs() <= 2.0 ** -17 * sums).all()      # 128 squares, each addition off by at most 2^-24 of the sum
     finally:
         native.call("gb_gemm_tc_set_pair_tile", 0)
         native.call("gb_gemm_tc_set_tile", 0)

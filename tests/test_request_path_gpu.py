@@ -14,21 +14,28 @@ def _fresh(name, dtype, prompts, **kw):
     return generate(model, prompts, stop_token_ids=[], **kw)
 
 
-# 5 + 59 = 64 positions fill a page to its end: an engine made for the call ends such a sequence one token early
+# 5 + 59 = 64 positions fill a page to its end: no engine may end such a sequence early
 @pytest.mark.parametrize("shape", [((5, 9, 13), 8), ((70, 3), 30), ((5,), 59), ((5, 64), 64)])
 def test_a_kept_engine_answers_as_a_new_one(shape):
     from gguf_rs_cli_b200.api import generate
     lens, n = shape
     prompts = [tokens_of("C", k, 300 + k) for k in lens]
     want = _fresh("C", "float32", prompts, max_tokens=n)
+    assert [len(w) for w in want] == [n] * len(lens)
     model = llm("C", "float32")
     made = model._engine
     assert generate(model, prompts, max_tokens=n, stop_token_ids=[]) == want and model._engine is made
-    # a smaller call is served by the same engine, with the limit that an engine of its own would have had
+    # a smaller call is served by the same engine
     small = [p[:4] for p in prompts]
-    got = generate(model, small, max_tokens=60, stop_token_ids=[])
-    kept = model._engine is made
-    assert got == _fresh("C", "float32", small, max_tokens=60) and (kept or len(lens) == 1 or n < 60)
+    got = generate(model, small, max_tokens=n, stop_token_ids=[])
+    assert model._engine is made and [len(g) for g in got] == [n] * len(lens)
+    assert got == _fresh("C", "float32", small, max_tokens=n)
+    # and both by one that holds the model's longest sequence
+    generate(model, [tokens_of("C", 900, 9)] * 3, max_tokens=124, stop_token_ids=[])
+    made = model._engine
+    assert made.cache.max_len == model.spec.max_position
+    assert generate(model, prompts, max_tokens=n, stop_token_ids=[]) == want
+    assert generate(model, small, max_tokens=n, stop_token_ids=[]) == got and model._engine is made
 
 
 def test_graphs_that_are_kept_are_bounded():
@@ -64,3 +71,25 @@ def test_token_ids_of_every_kind(kind, n):
             eng.step([Entry(s[2], make(ids[:-1] + [1000]), ())])
         with pytest.raises(StepError, match="outside the vocabulary"):
             eng.step([Entry(s[2], make([-1] + ids), ())])
+
+
+def test_an_interrupted_request_leaves_nothing_in_flight():
+    """... and the next one, on another stream, has its buffers to itself."""
+    from gguf_rs_cli_b200.api import generate
+    prompts = [tokens_of("C", k, 400 + k) for k in (90, 40)]
+    want = _fresh("C", "bfloat16", prompts, max_tokens=20)
+    model = llm("C", "bfloat16")
+    made = model._engine
+
+    def boom(request, token):
+        if len(seen) == 9:
+            raise RuntimeError("callback")
+        seen.append(token)
+    for _ in range(3):
+        seen = []
+        with pytest.raises(RuntimeError, match="callback"):
+            generate(model, prompts, max_tokens=20, stop_token_ids=[], on_token=boom)
+        assert torch.cuda.current_stream().query()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            assert generate(model, prompts, max_tokens=20, stop_token_ids=[]) == want and model._engine is made
+            torch.cuda.synchronize()
