@@ -626,7 +626,7 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
     CUtensorMap mw, mx;
     if (tensor_map_2d(W, N, K, ldw, BM, &mw)) return 1;
     if (bn == 256 && g_pair && cut.cut == CUT_WHOLE) {
-        // many tokens: two SMs per 256 x 256 tile, each loading 128 tokens of X per stage; bf16 results leave
+        // more than 128 tokens: two SMs per tile of 256 features, each loading half of the tile's tokens of X per stage; bf16 results leave
         // through shared memory and TMA stores of [16 tokens x 128 features] (64 features after SwiGLU)
         p.pair_tile = gemm_tc_pair_tile(T, N, sms);
         if (tensor_map_2d(X, T, K, ldx, p.pair_tile / 2, &mx)) return 1;
@@ -772,7 +772,8 @@ GB_API int gb_gemm_tc_noalloc(const void* X, long long ldx, const void* W, long 
     if (cudaGetDevice(&dev) != cudaSuccess) return gb_fail("gb_gemm_tc_noalloc: no current device");
     NoallocDevice* d = nullptr;
     if (noalloc_setup(dev, &d)) return 1;
-    // the same cut of the work as gb_gemm_tc makes; tiles that CTAs share need scratch memory and counters
+    // one CTA a tile: up to 128 tokens the cut that gb_gemm_tc makes, from 129 on (where that one pairs SMs) its own tiles and shares
+    // of K; tiles that CTAs share need scratch memory and counters
     const TcCut cut = cut_for(T, N, K, d->sms, true, 1 << 30, false);
     GB_REQUIRE(cut.tiles * cut.kb < (1LL << 31) - (1 << 20), "gb_gemm_tc_noalloc: T=%d N=%d K=%d is more work than the kernel numbers", T, N, K);
     const int bn = cut.bn;

@@ -287,7 +287,7 @@ __device__ __forceinline__ void tc_write_ssq(const TcParams& p, int n0, int t0, 
 
 }  // namespace
 
-// Two CTAs on two SMs per 256 x 256 tile (gemm_tc_pair.cu); taken for steps of many tokens.
+// Two CTAs on two SMs per tile of 256 features (gemm_tc_pair.cu); taken for steps of more than 128 tokens.
 // mo: map of the bf16 output for stores from shared memory (boxes of 16 tokens x 128 features, or x 64 after
 // SwiGLU), or null: results are then stored from registers.
 // pair_tile of the parameters: the x map's boxes have half as many rows.

@@ -265,16 +265,17 @@ static long long pair_slots(int sms) {
 }
 
 // Tokens of a tile: the width whose rounds over the device take the least time.  A 256 x bn tile over K takes a time
-// proportional to bn down to about 176 and no less below (4096 deep: 25 us at 256, 18 at 176, 17 at 128: what is left is the
-// loads' pace).  2048 x 6144: 3 rounds of 256 or of 240; 7001 x 4096 x 14336: 7 rounds of 256 (581 us) or of 224 (530 us);
-// 512 x 4096 x 14336: one round of 256 (89 us) or of 160 (65 us).  Of equal costs the widest.
+// proportional to bn down to about 176 and hardly less below (512 x 4096 x 4096, one round: 29.5 us at 256, 23.6 at 176, 22.2 at 160,
+// 21.4 at 128: what is left is the loads' pace), and a narrower one reads W more often, so 176 is the narrowest.  2048 x 6144 x 4096:
+// four rounds of 176 74 us, three of 240 80, three of 256 84; 7001 x 4096 x 14336: seven rounds of 224 639, seven of 256 726;
+// 512 x 4096 x 14336: one round of 176 58, of 256 84.  Of equal costs the widest.
 int gemm_tc_pair_tile(int T, int N, int sms) {
     if (g_pair_tile > 0) return g_pair_tile;
     const long long ft = (N + 2 * BM - 1) / (2 * BM), slots = pair_slots(sms);
     int best = PBN;
     long long least = -1;
-    for (int bn = PBN; bn >= 160; bn -= 16) {
-        const long long units = ft * ((T + bn - 1) / bn), cost = (units + slots - 1) / slots * (bn > 176 ? bn : 176);
+    for (int bn = PBN; bn >= 176; bn -= 16) {
+        const long long units = ft * ((T + bn - 1) / bn), cost = (units + slots - 1) / slots * bn;
         if (least < 0 || cost < least) { least = cost; best = bn; }
     }
     return best;

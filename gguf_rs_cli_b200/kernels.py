@@ -677,7 +677,8 @@ def latent_decode_supported(n_heads: int, kv_rank: int, rot_dim: int, dtype: tor
 
 def latent_decode_class(max_kv: int) -> int:
     """Class of a decode step for the latent decode kernel: the longest sequence's blocks of 32 keys, rounded
-    down to one of a few values; steps of one class split their keys alike."""
+    down to one of a few values; steps of one class split their keys alike.  Where the number of blocks is no class itself, some
+    CTAs take two blocks and the last ones none: 23 blocks on 16 splits are eleven CTAs of two, one of one and four without."""
     return _split_class((max_kv + 31) // 32)
 
 
@@ -1191,7 +1192,8 @@ def decode_split_class_cuda(max_kv: int) -> int:
 
 
 def decode_split_class_exact(max_kv: int) -> int:
-    """Class of a decode step of the normalised attention on the CUDA-core decode kernel: its pages."""
+    """Class of a decode step of the normalised attention on the CUDA-core decode kernel: its pages, rounded down to one of a
+    few values (where that is no class itself, some CTAs take two pages)."""
     return _split_class((max_kv + 63) // 64)
 
 
