@@ -293,18 +293,48 @@ __global__ void __launch_bounds__(AD_THREADS, PER_SM) attention_decode_kernel(Ad
         int gi = i / hd, d = i - gi * hd;
         const float* rec = p.scratch + (size_t(t) * p.nh + h0 + gi) * p.splits * (hd + 2);
         // The splits' numbers are added in order; how many are on their way together is chosen per instance, by what it costs the
-        // loop over the pages in registers (us, 1 x 4,000 positions in 32 splits and 8 x 500 in 4): groups of 8 with heads of
-        // 128 83 and 38 with the compiler's own unrolling, 60 and 47 by eights and the rest one by one, 58 and 38 as here.
+        // loop over the pages in registers.  A loop unrolled by eight takes what is left of 4, 6 or 12 splits one by one.  Groups of 4
+        // ask for eight, there or not, where the splits are no multiple of eight (heads of 128, 4 KV heads, 4 sequences of 420 and 715
+        // positions in 6 and 12 splits: 25.5 -> 17.4 and 24.6 -> 20.5 us); groups of 8 take eight, four, two (heads of 128, 8 KV heads,
+        // 8 x 500 positions in 4 splits and 1 x 4,000 in 32: 38 and 83 us with the compiler's own unrolling, 47 and 60 by eights, 38
+        // and 58 so); the others lose more in the loop over the pages.
         float M = -INFINITY, L = 0.f, o = 0.f;
         if constexpr (EARLY) {
+            if (GT == 4 && (p.splits & 7)) {
+                for (int s0 = 0; s0 < p.splits; s0 += 8) {
+                    float ms[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) ms[e] = s0 + e < p.splits ? __ldcg(rec + (s0 + e) * (hd + 2) + hd) : -INFINITY;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) M = fmaxf(M, ms[e]);
+                }
+                for (int s0 = 0; s0 < p.splits; s0 += 8) {
+                    float ms[8], ls[8], os[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float* r = rec + (s0 + e) * (hd + 2);
+                        const bool there = s0 + e < p.splits;
+                        ms[e] = there ? __ldcg(r + hd) : -INFINITY;
+                        ls[e] = there ? __ldcg(r + hd + 1) : 0.f;
+                        os[e] = there ? __ldcg(r + d) : 0.f;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float wgt = ms[e] == -INFINITY ? 0.f : exp2f(ms[e] - M);
+                        L += ls[e] * wgt;
+                        o += os[e] * wgt;
+                    }
+                }
+            } else {
 #pragma unroll 8
-            for (int s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd));
+                for (int s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd));
 #pragma unroll 8
-            for (int s = 0; s < p.splits; ++s) {
-                float ms = __ldcg(rec + s * (hd + 2) + hd);
-                float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);
-                L += __ldcg(rec + s * (hd + 2) + hd + 1) * wgt;
-                o += __ldcg(rec + s * (hd + 2) + d) * wgt;
+                for (int s = 0; s < p.splits; ++s) {
+                    float ms = __ldcg(rec + s * (hd + 2) + hd);
+                    float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);
+                    L += __ldcg(rec + s * (hd + 2) + hd + 1) * wgt;
+                    o += __ldcg(rec + s * (hd + 2) + d) * wgt;
+                }
             }
         } else if constexpr (GT == 8 && HC >= 2) {
             auto largest = [&](int s) { M = fmaxf(M, __ldcg(rec + s * (hd + 2) + hd)); };
