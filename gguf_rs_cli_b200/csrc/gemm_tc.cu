@@ -464,8 +464,8 @@ GB_API int gb_gemm_tc_set_pair(int on) { g_pair = on; return 0; }
 static int g_mode = 0;                // 0: by the rule below, 1: whole tiles only, 2: equal shares of K blocks where tiles are not shared out per tile, 3: equal shares always
 GB_API int gb_gemm_tc_set_mode(int mode) { g_mode = mode; return 0; }
 
-// The same with all sizes known.
-static int tile_for(int T, int N, int K, int sms, bool pair) {
+// The same with all sizes known.  gated: gate and up features in pairs (W of N rows gives N / 2 results).
+static int tile_for(int T, int N, int K, int sms, bool pair, bool gated) {
     if (g_tile_override > 0) return g_tile_override;
     int bn = gb_gemm_tc_tile(T);
     const long long ft = (N + BM - 1) / BM;
@@ -477,12 +477,18 @@ static int tile_for(int T, int N, int K, int sms, bool pair) {
         // up to 128 tokens: tiles of 64, two CTAs per SM (a CTA with a wide tile streams its operands no faster)
         if (bn == 128) return 64;
         // A few hundred tokens go to the kernel that pairs two SMs like thousands (512 x 4096 x 4096 21 us, 26 with tiles of 64
-        // tokens; 300 x 6144 x 4096 22 and 27), but a tile of that kernel takes what its K takes, however few there are: where
-        // K is long enough for several CTAs to share every tile of 64 tokens, those are faster (300 x 256 x 2048 9.4 against
-        // 11.1 us, 130 x 2048 x 4096 14.1 against 18.4, 200 x 4096 x 14336 47 against 55).  The two meet at 40 tiles for
-        // K = 2048 (11.4 and 11.8 us), 96 for 4096 (18.9 and 19.5), 148 for 8192 (35.1 and 35.6); at K = 1024 never.
+        // tokens; 300 x 6144 x 4096 22 and 27), but a tile of that kernel takes what its K and its epilogue take, however few tiles
+        // there are.  Where several CTAs can share every tile of 64 tokens, those are faster, the more so for 32-bit results, whose
+        // epilogue is longer; the line is one for both types, so that a bfloat16 result is the 32-bit one, rounded.  Tiles of 64 tokens
+        // over the kernel for pairs, bfloat16 and 32-bit results: K = 512 1.05 and 1.0 up to 72 tiles; 1024 1.03 and 0.87; 1536 1.05 and
+        // 0.82; 2048 0.94 and 0.74, and 1.2 and 0.95 from 80 to 96; 3072 0.82 and 0.67, and 1.05 and 0.87 from 80 to 96; 4096 0.93 and 0.8
+        // from 80 to 96, 1.06 and 0.93 from 112 on; 8192 0.9 and 0.8 from 112 to 148.  More tiles are not shared: 1.2 and 0.95 to 1.1.
         const long long tiles = ft * ((T + 63) / 64);
-        if (bn == 256 && K >= 2048 && tiles <= sms && tiles <= K / 48) return 64;
+        const int few = K / 36 + 11 > sms / 2 ? K / 36 + 11 : sms / 2;       // 96 for 3072, 124 for 4096, all from 4900 on
+        if (bn == 256 && K >= 1024 && tiles <= sms && tiles <= few) return 64;
+        // The gate's epilogue is longer still and stands alone behind a single round: 0.35 to 0.95 as long wherever two CTAs an SM hold
+        // all tiles of 64 tokens (200 x 2048 x 2048 13 instead of 28 us, 300 x 2048 x 3072 20 instead of 35), 1.2 to 1.9 beyond.
+        if (bn == 256 && gated && tiles <= 2LL * sms) return 64;
         return bn;
     }
     // one CTA a tile only: a few hundred tokens with few features would give 256-token tiles for less than half of the SMs, so
@@ -502,9 +508,9 @@ struct TcCut {
         p.total_its = int(tiles * kb); p.its_each = p.total_its / n_ctas; p.its_rest = p.total_its % n_ctas;
     }
 };
-static TcCut cut_for(int T, int N, int K, int sms, bool may_share, int n_counters, bool may_pair) {
+static TcCut cut_for(int T, int N, int K, int sms, bool may_share, int n_counters, bool may_pair, bool gated) {
     TcCut c;
-    c.bn = tile_for(T, N, K, sms, may_pair && g_pair);
+    c.bn = tile_for(T, N, K, sms, may_pair && g_pair, gated);
     c.tiles = (long long)((N + BM - 1) / BM) * ((T + c.bn - 1) / c.bn);
     c.kb = (K + BK - 1) / BK;
     const long long slots = (long long)ctas_per_sm(c.bn) * (sms > 0 ? sms : 1);        // CTAs that are resident at once
@@ -545,12 +551,14 @@ static TcCut cut_for(int T, int N, int K, int sms, bool may_share, int n_counter
     return c;
 }
 
-// CTAs that a product of these sizes runs on, on a device with `sms` SMs, when it may use scratch memory.
-GB_API int gb_gemm_tc_ctas(int T, int N, int K, int sms) { return cut_for(T, N, K, sms, true, 1 << 30, true).n_ctas; }
+// CTAs that a product of these sizes (without gates) runs on, on a device with `sms` SMs, when it may use scratch memory.
+GB_API int gb_gemm_tc_ctas(int T, int N, int K, int sms) { return cut_for(T, N, K, sms, true, 1 << 30, true, false).n_ctas; }
 
-// Floats of scratch a launch with these sizes needs (0 when no tile is shared between CTAs).
+// Floats of scratch a launch with these sizes needs, gated or not (0 when no tile is shared between CTAs).
 GB_API long long gb_gemm_tc_scratch_floats(int T, int N, int K, int sms) {
-    return cut_for(T, N, K, sms, true, 1 << 30, true).scratch_floats;
+    const long long plain = cut_for(T, N, K, sms, true, 1 << 30, true, false).scratch_floats;
+    const long long gated = cut_for(T, N, K, sms, true, 1 << 30, true, true).scratch_floats;
+    return plain > gated ? plain : gated;
 }
 
 // Whether the tensor-core kernel takes these operands (bf16, 16-byte aligned, pitches multiples of 8).
@@ -613,7 +621,7 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
                K, ldx, ldw);
     if (T == 0) return 0;
     if (ensure_status()) return 1;
-    const TcCut cut = cut_for(T, N, K, sms, scratch && counters, n_counters, true);
+    const TcCut cut = cut_for(T, N, K, sms, scratch && counters, n_counters, true, swiglu_features > 0);
     GB_REQUIRE(cut.tiles * cut.kb < (1LL << 31) - (1 << 20), "gb_gemm_tc: T=%d N=%d K=%d is more work than the kernel numbers", T, N, K);
     const int bn = cut.bn;
     TcParams p;
@@ -774,7 +782,7 @@ GB_API int gb_gemm_tc_noalloc(const void* X, long long ldx, const void* W, long 
     if (noalloc_setup(dev, &d)) return 1;
     // one CTA a tile: up to 128 tokens the cut that gb_gemm_tc makes, from 129 on (where that one pairs SMs) its own tiles and shares
     // of K; tiles that CTAs share need scratch memory and counters
-    const TcCut cut = cut_for(T, N, K, d->sms, true, 1 << 30, false);
+    const TcCut cut = cut_for(T, N, K, d->sms, true, 1 << 30, false, false);
     GB_REQUIRE(cut.tiles * cut.kb < (1LL << 31) - (1 << 20), "gb_gemm_tc_noalloc: T=%d N=%d K=%d is more work than the kernel numbers", T, N, K);
     const int bn = cut.bn;
     if (cut.cut != CUT_WHOLE) {

@@ -126,9 +126,11 @@ def test_pairs_of_sms_are_counted_before_the_first_product():
 
 @pytest.mark.parametrize("T", [129, 191, 300, 512, 769])
 def test_a_few_hundred_tokens(T):
-    """Either side of every border of the rule: K at 2,048, tiles of 64 tokens per K, more of them than SMs."""
+    """Either side of every border of the rule: K at 1,024, tiles of 64 tokens per K, more of them than SMs, and for gated products
+    than twice as many.  A bfloat16 result is the 32-bit one, rounded, whichever kernel a size takes."""
     k = K()
-    for N, Kd in ((256, 8192), (4096, 8192), (640, 2040), (640, 2048), (1300, 2048), (6144, 64), (130, 8200)):
+    for N, Kd in ((256, 8192), (4096, 8192), (640, 2040), (640, 2048), (1300, 2048), (6144, 64), (130, 8200), (256, 1016), (256, 1024),
+                  (1500, 1024), (3000, 3072), (4096, 4096)):
         x, w, b, _ = _operands(T, N, Kd, T + N)
         out = torch.empty(T, N, device=DEV)
         k.gemm_tc(x, w, b, out)
@@ -136,5 +138,15 @@ def test_a_few_hundred_tokens(T):
         low = torch.empty(T, N, device=DEV, dtype=torch.bfloat16)
         k.gemm_tc(x, w, b, low)
         assert torch.equal(low, out.bfloat16()), (N, Kd)
+    for F, Kd in ((100, 1024), (520, 1024), (1024, 512), (3000, 256), (4736, 136)):
+        x, w, _, _ = _operands(T, 2 * F, Kd, T + F)
+        gate, up = (x.double() @ w[i * F:(i + 1) * F].double().T for i in (0, 1))
+        want = torch.nn.functional.silu(gate) * up
+        got = torch.empty(T, F, device=DEV)
+        k.gemm_tc(x, k.interleave_gate_up(w[:F], w[F:]), None, got, swiglu_features=F)
+        assert (got.double() - want).norm() <= 1e-5 * want.norm(), (F, Kd)           # 32-bit sums of up to 1,024 terms
+        low = torch.empty(T, F, device=DEV, dtype=torch.bfloat16)
+        k.gemm_tc(x, k.interleave_gate_up(w[:F], w[F:]), None, low, swiglu_features=F)
+        assert torch.equal(low, got.bfloat16()), (F, Kd)
     torch.cuda.synchronize()
     k.check_tc_status()
