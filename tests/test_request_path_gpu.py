@@ -93,3 +93,19 @@ def test_an_interrupted_request_leaves_nothing_in_flight():
         with torch.cuda.stream(torch.cuda.Stream()):
             assert generate(model, prompts, max_tokens=20, stop_token_ids=[]) == want and model._engine is made
             torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("lens", [[1] * 130, [1, 200, 1, 33, 5, 129, 32], [40, 3], [2] * 70 + [129] + [1] * 3, [33] * 5])
+def test_index_arrays_of_long_and_short_sequences_side_by_side(lens):
+    """Laid out as arrays, as lists and as both in turn: in 32-bit mode every sequence's logits are those of a step of its own."""
+    from gguf_rs_cli_b200.engine.step import Entry
+    eng = new_engine("C", "float32", n_tokens=sum((n + 63) // 64 * 64 for n in lens), n_slots=len(lens))
+    prompts = [tokens_of("C", n, 500 + k) for k, n in enumerate(lens)]
+    slots = [eng.open() for _ in lens]
+    together = eng.step([Entry(s, p, (len(p) - 1,)) for s, p in zip(slots, prompts)]).clone()
+    for s in slots:
+        eng.close(s)
+    for row, p in list(zip(together, prompts))[::7] + [(together[-1], prompts[-1])]:
+        s = eng.open()
+        assert torch.equal(row, eng.step([Entry(s, p, (len(p) - 1,))])[0])
+        eng.close(s)
