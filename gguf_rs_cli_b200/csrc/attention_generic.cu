@@ -24,8 +24,11 @@ constexpr int AG_WARPS = 8;
 
 // hd: entries of a query and of a key; hdv: entries of a value (and of a head's result); a value row starts
 // every v_row entries of the value storage, which lets the values be the first hdv entries of the key rows
-// themselves (attention over one shared latent row per position).  MAX_HD bounds both sizes.
-template <typename TC, int MAX_HD>
+// themselves (attention over one shared latent row per position).  MAX_HD bounds both sizes.  EARLY: the instance for 32-bit key rows
+// that start on 16 bytes, with many loads in flight in few warps.  It takes other rows too, and is the better one for them while its
+// two CTAs an SM hold the step (2 tokens of 700 positions, 16 heads of 130: 48 us against 58); entry by entry keys want more warps
+// than that (64 of 1,000: 443 against 336, 10 heads of 250 542 against 449; 64 of 1,000, 8 heads of 66: 165 against 126).
+template <typename TC, int MAX_HD, bool EARLY>
 __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
     const void* __restrict__ q, int q_dtype, long long ldq, void* __restrict__ out, int out_dtype, long long ldo,
     int nh, int nkv, int hd, int hdv, int v_row, const int* __restrict__ seq_of, const int* __restrict__ pos,
@@ -40,7 +43,7 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
         for (int d = threadIdx.x; d < hdv; d += blockDim.x) gb_store(out, out_dtype, orow + d, 0.f);
         return;
     }
-    __shared__ __align__(16) float qs[MAX_HD];
+    __shared__ alignas(EARLY ? 16 : 4) float qs[MAX_HD];     // whole loads of it only beside those of a key: 1.05 to 1.25 times as long otherwise
     __shared__ float acc_s[AG_WARPS][MAX_HD];
     __shared__ float m_s[AG_WARPS], l_s[AG_WARPS];
     for (int d = threadIdx.x; d < hd; d += blockDim.x) qs[d] = gb_load(q, q_dtype, size_t(t) * ldq + size_t(h) * hd + d);
@@ -54,6 +57,7 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
     const int* trow = table + size_t(b) * table_width;
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int C = MAX_HD / 32;
+    constexpr bool BATCHED = sizeof(TC) == 4 && (EARLY ? MAX_HD <= 256 : MAX_HD <= 64);
     float acc[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) acc[c] = 0.f;
@@ -64,7 +68,7 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
     // Other rows: each lane walks its own key's row.  Either way the order of the sums is fixed by the sizes alone.
     constexpr int QC = (MAX_HD / 8 + 31) / 32;
     const bool shared_rows = sizeof(TC) == 2 && vec8;
-    const bool quads = sizeof(TC) == 4 && hd % 4 == 0 && (reinterpret_cast<uintptr_t>(kc) & 15) == 0;
+    const bool quads = EARLY && hd % 4 == 0 && (reinterpret_cast<uintptr_t>(kc) & 15) == 0;
     const bool pairs = sizeof(TC) == 2 && hdv % 2 == 0 && v_row % 2 == 0 && (reinterpret_cast<uintptr_t>(vc) & 3) == 0;
     float qr[QC][8];
     if (shared_rows) {
@@ -119,8 +123,8 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
             const TC* kr = kc + off * hd;
             float dot = 0.f;
             if (quads) {
-                // 32-bit rows that start on 16 bytes: the same sum in the same order, four entries a load and eight loads in
-                // flight (entry by entry a row of 64 was sixteen trips to L2 one after the other: 24 us for a few tokens)
+                // the same sum in the same order, four entries a load and eight loads in flight
+                // (entry by entry a row of 64 was sixteen trips to L2 one after the other: 24 us for a few tokens)
                 const float4* k4 = reinterpret_cast<const float4*>(kr);
                 const float4* q4 = reinterpret_cast<const float4*>(qs);
 #pragma unroll 8
@@ -144,7 +148,7 @@ __global__ void __launch_bounds__(AG_WARPS * 32) attention_generic_kernel(
         l = l * alpha + gb_warp_sum(pj);
 #pragma unroll
         for (int c = 0; c < C; ++c) acc[c] *= alpha;
-        if (sizeof(TC) == 4 && MAX_HD <= 256) {
+        if (BATCHED) {
             // the same sums with eight keys' values asked for at a time; a key without weight is not read (its row may
             // never have been written) and adds nothing
             for (int j0 = 0; j0 < 32; j0 += 8) {
@@ -245,21 +249,33 @@ GB_API int gb_attention_generic(const void* q, int q_dtype, long long ldq, void*
     GB_REQUIRE(!gate || gb_is_dtype(gate_dtype), "gb_attention_generic: bad gate dtype");
     if (T == 0) return 0;
     dim3 grid(T, nh);
-#define AG_LAUNCH(TC, MAX_HD)                                                                                     \
-    attention_generic_kernel<TC, MAX_HD><<<grid, AG_WARPS * 32, 0, stream>>>(                                     \
+#define AG_LAUNCH(TC, MAX_HD, EARLY)                                                                              \
+    attention_generic_kernel<TC, MAX_HD, EARLY><<<grid, AG_WARPS * 32, 0, stream>>>(                              \
         q, q_dtype, ldq, out, out_dtype, ldo, nh, nkv, hd, hdv, v_row, seq_of, pos, table, table_width, ring_pages, \
         (const TC*)kcache, (const TC*)vcache, window, scale, head_pages, window > 0 ? keep_first : 0, gate, gate_dtype, ldg, gate_per_head, sink, sink_values, chunk, slopes, softcap, out_scale)
     const bool small = hd <= 256 && hdv <= 256, mid = hd <= AG_MID_HD && hdv <= AG_MID_HD;
-    if (cache_dtype == GB_F32) {
-        if (hd <= 64 && hdv <= 64) AG_LAUNCH(float, 64);
-        else if (hd <= 128 && hdv <= 128) AG_LAUNCH(float, 128);
-        else if (small) AG_LAUNCH(float, 256);
-        else if (mid) AG_LAUNCH(float, AG_MID_HD);
-        else AG_LAUNCH(float, AG_MAX_HD);
+    bool early = cache_dtype == GB_F32 && hd % 4 == 0 && (reinterpret_cast<uintptr_t>(kcache) & 15) == 0;
+    if (cache_dtype == GB_F32 && !early && mid) {
+        int dev = 0, sms = 0;
+        early = cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+                (long long)T * nh <= 2LL * sms;
+    }
+    if (early) {
+        if (hd <= 64 && hdv <= 64) AG_LAUNCH(float, 64, true);
+        else if (hd <= 128 && hdv <= 128) AG_LAUNCH(float, 128, true);
+        else if (small) AG_LAUNCH(float, 256, true);
+        else if (mid) AG_LAUNCH(float, AG_MID_HD, true);
+        else AG_LAUNCH(float, AG_MAX_HD, true);
+    } else if (cache_dtype == GB_F32) {
+        if (hd <= 64 && hdv <= 64) AG_LAUNCH(float, 64, false);
+        else if (hd <= 128 && hdv <= 128) AG_LAUNCH(float, 128, false);
+        else if (small) AG_LAUNCH(float, 256, false);
+        else if (mid) AG_LAUNCH(float, AG_MID_HD, false);
+        else AG_LAUNCH(float, AG_MAX_HD, false);
     } else {
-        if (small) AG_LAUNCH(__nv_bfloat16, 256);
-        else if (mid) AG_LAUNCH(__nv_bfloat16, AG_MID_HD);
-        else AG_LAUNCH(__nv_bfloat16, AG_MAX_HD);
+        if (small) AG_LAUNCH(__nv_bfloat16, 256, false);
+        else if (mid) AG_LAUNCH(__nv_bfloat16, AG_MID_HD, false);
+        else AG_LAUNCH(__nv_bfloat16, AG_MAX_HD, false);
     }
 #undef AG_LAUNCH
     GB_LAUNCH_OK("gb_attention_generic");
