@@ -22,6 +22,7 @@ constexpr int LD_THREADS = LD_WARPS * 32;
 constexpr int LD_MAX_HEADS = 16;                    // heads per token: at most 2 per warp (with 32 heads the general
                                                     // kernel's block per head was measured faster: 0.774 against 0.799 ms a step)
 constexpr int LD_HW = LD_MAX_HEADS / LD_WARPS;
+constexpr int LD_FEW = 8;                           // splits that every thread of the merge weighs for itself
 constexpr int LD_MERGED = 64;                       // splits whose factors a CTA of the merge holds at a time
 constexpr int LD_MAX_C = 512;                       // entries of the value: at most 8 pairs per lane
 constexpr int LD_PAIRS = LD_MAX_C / 64;
@@ -192,16 +193,19 @@ __global__ void __launch_bounds__(LM_THREADS) latent_decode_mma_kernel(const LdP
     const int kb0 = kbf + split * per, kb1 = min(kbf + nkb, kb0 + per);
     const int* trow = p.table + size_t(b) * p.table_width;
     const int pieces = HDK / 8;
-    // A warp copies a row: the queries with the first tile of keys, all in flight at once (16 bytes a copy; piece by piece
-    // through registers, 18 copies a thread in turn, a tile took longer to come than to use).
+    // The queries with the first tile of keys, all in flight at once (16 bytes a copy; piece by piece through registers, 18 copies a
+    // thread in turn, a tile took longer to come than to use).  As many lanes a row as it has pieces: with a warp for each
+    // row, ten pieces (64 + 16 entries) left two thirds of it idle.
+    const int row_lanes = pieces > 16 ? 32 : pieces > 8 ? 16 : 8, piece = threadIdx.x & (row_lanes - 1);
+    const int row0 = threadIdx.x / row_lanes, rows = LM_THREADS / row_lanes;
     auto copy = [&](__nv_bfloat16* dst, const __nv_bfloat16* src, bool valid) {
-        for (int c8 = lane; c8 < pieces; c8 += 32) {
+        for (int c8 = piece; c8 < pieces; c8 += row_lanes) {
             const unsigned d = unsigned(__cvta_generic_to_shared(dst + 8 * c8));
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (valid ? 8 * c8 : 0)), "r"(valid ? 16 : 0) : "memory");
         }
     };
     if (kb0 < kb1)                                     // a split without blocks asks for nothing: only the loop below waits
-        for (int r = warp; r < 16; r += LM_THREADS / 32) copy(qt + r * KS, p.q + size_t(t) * p.ldq + size_t(r < H ? r : 0) * HDK, r < H);
+        for (int r = row0; r < 16; r += rows) copy(qt + r * KS, p.q + size_t(t) * p.ldq + size_t(r < H ? r : 0) * HDK, r < H);
     const int CW = C / 4, ot = CW / 8;                 // this warp's value columns [warp * CW, +CW): ot tiles of 8
     const float sl2 = p.scale * 1.4426950408889634f;
     float o[LM_MAX_OT][4];
@@ -211,10 +215,12 @@ __global__ void __launch_bounds__(LM_THREADS) latent_decode_mma_kernel(const LdP
 
     for (int kb = kb0; kb < kb1; ++kb) {
         __syncthreads();
-        for (int r = warp; r < 32; r += LM_THREADS / 32) {
+        // half a page, one after the other (asked row by row, the table and the ring's remainder stood in front of every copy)
+        const __nv_bfloat16* rows0 = p.cache + gb_kv_offset(trow, p.ring_pages, kb * 32, 0, 1, HDK);
+        for (int r = row0; r < 32; r += rows) {
             const int j = kb * 32 + r;
             const bool valid = j <= pos && j >= lo;
-            copy(kt + r * KS, p.cache + (valid ? gb_kv_offset(trow, p.ring_pages, j, 0, 1, HDK) : 0), valid);
+            copy(kt + r * KS, rows0 + (valid ? r * HDK : 0), valid);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -329,9 +335,50 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ scratch, co
         for (int c = threadIdx.x; c < C; c += blockDim.x) o[c] = __float2bfloat16_rn(0.f);
         return;
     }
+    const float* base = scratch + (size_t(t) * H + h) * splits * (C + 2);
+    const int c = threadIdx.x;               // an entry a thread
+    // what the sums are multiplied by, and their denominator with a sink: one above every score brings them down to its level
+    auto finish = [&](float M, float& L) {
+        float f = 1.f;
+        if (sink && M != -INFINITY) {
+            const float sv = sink[h];
+            if (sv > M) {
+                f = expf(M - sv);
+                L = L * f + 1.f;
+            } else {
+                L += expf(sv - M);
+            }
+        }
+        if (gate) f *= 1.f / (1.f + expf(-__bfloat162float(gate[size_t(t) * ldg + h])));
+        return f;
+    };
+    float M = -INFINITY, v = 0.f, L = 0.f;
+    if (splits <= LD_FEW) {
+        // every thread for itself, all of its numbers asked for at once: with so few splits the barriers below cost more than the
+        // factors that they share (64 tokens, 3 heads, 4 splits: 2 us)
+        float ms[LD_FEW], ls[LD_FEW], x[LD_FEW];
+#pragma unroll
+        for (int s = 0; s < LD_FEW; ++s) {
+            const float* r = base + size_t(s) * (C + 2);
+            ms[s] = s < splits ? r[C] : -INFINITY;
+            ls[s] = s < splits ? r[C + 1] : 0.f;
+            x[s] = s < splits && c < C ? r[c] : 0.f;
+        }
+#pragma unroll
+        for (int s = 0; s < LD_FEW; ++s) M = fmaxf(M, ms[s]);
+#pragma unroll
+        for (int s = 0; s < LD_FEW; ++s) {
+            if (ms[s] == -INFINITY) continue;                // no keys: its record may hold anything
+            const float w = expf(ms[s] - M);
+            L = fmaf(ls[s], w, L);
+            v = fmaf(x[s], w, v);
+        }
+        const float f = finish(M, L);
+        if (c < C) o[c] = __float2bfloat16_rn(v * f / L);
+        return;
+    }
     // every split's factor once, e^(m_s - M), LD_MERGED splits at a time (no wrapper asks for more than one such group)
     __shared__ float w[LD_MERGED], sums[LD_MERGED], total[2];
-    const float* base = scratch + (size_t(t) * H + h) * splits * (C + 2);
     auto load = [&](int s0) {                // a group's maxima and sums; how many they are
         const int n = min(LD_MERGED, splits - s0);
         for (int s = threadIdx.x; s < n; s += blockDim.x) {
@@ -341,14 +388,11 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ scratch, co
         __syncthreads();
         return n;
     };
-    float M = -INFINITY;
     for (int s0 = 0; s0 < splits; s0 += LD_MERGED) {
         const int n = load(s0);
         for (int s = 0; s < n; ++s) M = fmaxf(M, w[s]);
         __syncthreads();
     }
-    const int c = threadIdx.x;               // an entry a thread
-    float v = 0.f, L = 0.f;                  // L: the first thread's
     for (int s0 = 0; s0 < splits; s0 += LD_MERGED) {
         const int n = splits > LD_MERGED ? load(s0) : splits;             // a single group is still there
         // -1: a split without keys, which has left nothing (its record may hold anything).  A factor that is too small for 32 bits
@@ -368,19 +412,8 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ scratch, co
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        float f = 1.f;                       // what the sums are multiplied by: a sink above every score brings them down to its level
-        if (sink && M != -INFINITY) {
-            const float sv = sink[h];
-            if (sv > M) {
-                f = expf(M - sv);
-                L = L * f + 1.f;
-            } else {
-                L += expf(sv - M);
-            }
-        }
-        if (gate) f *= 1.f / (1.f + expf(-__bfloat162float(gate[size_t(t) * ldg + h])));
-        total[0] = f;
+    if (threadIdx.x == 0) {                  // L: the first thread's
+        total[0] = finish(M, L);
         total[1] = L;
     }
     __syncthreads();

@@ -6,7 +6,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
-SIZES = [(16, 512, 64), (5, 64, 16), (3, 40, 24)]            # heads, kv_rank, rot_dim: tensor cores twice, CUDA cores
+# heads, kv_rank, rot_dim: tensor cores (32, 16, 8 and 32 lanes a row), then CUDA cores
+SIZES = [(16, 512, 64), (5, 64, 16), (2, 64, 0), (8, 128, 32), (3, 40, 24)]
 
 
 def _step(lens, H, C, R, seed=0):
@@ -52,9 +53,9 @@ def test_unequal_lengths_in_one_step(H, C, R, lens):
 
 
 @pytest.mark.parametrize("H, C, R", SIZES)
-@pytest.mark.parametrize("splits", [1, 2, 63, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("splits", [1, 2, 7, 8, 9, 63, 64, 65, 128, 129, 300])
 def test_any_number_of_splits(H, C, R, splits):
-    """The merge holds 64 splits' factors at a time; the entry takes as many as a grid has rows."""
+    """The merge holds 64 splits' factors at a time, up to 8 in registers; the entry takes as many as a grid has rows."""
     from gguf_rs_cli_b200 import native
     from gguf_rs_cli_b200.native import call, ptr, stream_ptr
     lens = [4500, 70, 1]
