@@ -150,3 +150,13 @@ def test_a_few_hundred_tokens(T):
         assert torch.equal(low, got.bfloat16()), (F, Kd)
     torch.cuda.synchronize()
     k.check_tc_status()
+
+
+@pytest.mark.parametrize("N, K", [(1000, 16), (1001, 16), (1001, 20), (4096, 4)])
+@pytest.mark.parametrize("T", [1, 17])
+def test_products_of_one_block_of_k_are_the_same_bits_on_either_kernel(T, N, K):
+    from gguf_rs_cli_b200 import kernels as k
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x, w = torch.randn(T, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    outs = [f(x, w, None, torch.empty(T, N, device="cuda")) for f in (k.gemm, k.gemm_f32, k.gemm_generic)]
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
