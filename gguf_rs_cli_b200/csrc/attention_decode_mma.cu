@@ -3,9 +3,8 @@
 // one 16-row MMA tile (groups larger than 16 take several tiles), so one pass over the
 // keys and values serves the whole group with a handful of instructions per page:
 // S = Q K^T and O += P V through mma.sync m16n8k16 (bf16 in, f32 accumulate), softmax
-// in 32-bit registers.  A CTA is (token, KV head tile, split of the token's pages); its
-// 4 warps each take 16 of a page's 64 keys (or its 2 warps 16 of half a page's 32, four
-// such CTAs on an SM); pages stream through a 3-stage cp.async ring.  The warps' results
+// in 32-bit registers.  A CTA is (token, KV head tile, split of the token's pages); its warps take 16 keys
+// at a time, copied to shared memory by cp.async while the ones before them are worked on.  The warps' results
 // are merged in warp order, the splits' results by the CTA that arrives last, in split
 // order (scratch memory + a counter; nobody waits).
 // Same arithmetic as src/model/llama.rs:374-394.  Other head sizes take the CUDA-core
@@ -43,7 +42,10 @@ struct DmParams {
     float* scratch;              // [T, nh, splits, hd + 2]
     int* counters;
     long long ldq, ldo;
-    int nh, nkv, table_width, ring_pages, window, splits;
+    int nh, nkv, table_width, ring_pages, window;
+    int T;                       // tokens of the step
+    int splits, split_pages;     // the grid's splits of a sequence, and how many pages a split has at least
+    int slots;                   // CTAs that the device holds at once, for the rule of dm_splits (0: split_pages alone)
     float scale_log2;
     // rotation and cache write in the same kernel (rotate != 0): q, k_new and v_new are the products as they
     // come from the projection; the kernel rotates q on its way into shared memory, and the CTA that reads a
@@ -86,34 +88,62 @@ template <int HD> __device__ __forceinline__ int dm_swz(int row, int chunk) {
     return row * HD + (((chunk & ~7) | ((chunk ^ row) & 7)) << 3);
 }
 
+// The first page and the number of pages that a token at `pos` sees.
+__device__ __forceinline__ void dm_pages(int pos, int window, int& first, int& n) {
+    first = (window > 0 ? max(0, pos - window + 1) : 0) >> GB_PAGE_SHIFT;
+    n = (pos >> GB_PAGE_SHIFT) - first + 1;
+}
+
+// How a sequence of n_pages pages is split: into equal splits of at least split_pages pages, and of no fewer than a CTA would have
+// if all pages of the step were dealt out equally over the device, no more splits than the grid has.  So the lengths of the
+// step's sequences decide, not the longest one's: equal sequences that fill the device are left whole, a long one beside short
+// ones is shared by many CTAs, and CTAs without pages leave at once.  (Every warp reads the step's positions for itself, while
+// the kernel in front still runs.)
+__device__ __forceinline__ void dm_splits(const DmParams& p, int n_pages, int& live, int& pg_each) {
+    int least = p.split_pages;
+    if (p.splits > 1 && p.slots > 0) {
+        long long total = 0;
+        for (int i = threadIdx.x & 31; i < p.T; i += 32) {
+            int first, n;
+            dm_pages(p.pos[i], p.window, first, n);
+            if (p.seq_of[i] >= 0) total += n;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        least = max(least, int((total * gridDim.y + p.slots - 1) / p.slots));
+    }
+    live = max(1, min(p.splits, n_pages / least));
+    pg_each = (n_pages + live - 1) / live;
+    live = (n_pages + pg_each - 1) / pg_each;
+}
+
 // The partial results of a (token, head tile)'s splits, merged in split order into the output: every split
-// left, per head, its unnormalised sum of values, its maximum (in units of log2) and its sum of weights.
+// left, per head, its unnormalised sum of values, its maximum (in units of log2) and its sum of weights.  Eight splits'
+// records are asked for together, and all three numbers of a record: a round of eight costs one trip to L2.
 template <int HD>
-__device__ __forceinline__ void dm_merge_splits(const DmParams& p, int t, int h0, int heads, int tid, int threads) {
+__device__ __forceinline__ void dm_merge_splits(const DmParams& p, int live, int t, int h0, int heads, int tid, int threads) {
     for (int i = tid; i < heads * HD; i += threads) {
         const int r = i / HD, d = i - r * HD;
         const float* rec = p.scratch + (size_t(t) * p.nh + h0 + r) * p.splits * (HD + 2);
-        float M = -INFINITY;
-        for (int s0 = 0; s0 < p.splits; s0 += 8) {
-            float mv[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) mv[j] = s0 + j < p.splits ? __ldcg(rec + (s0 + j) * (HD + 2) + HD) : -INFINITY;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) M = fmaxf(M, mv[j]);
-        }
-        float L = 0.f, acc = 0.f;
-        for (int s0 = 0; s0 < p.splits; s0 += 8) {
-            float mv[8], lv[8], ov[8];
+        float M = -INFINITY, L = 0.f, acc = 0.f;
+        for (int s0 = 0; s0 < live; s0 += 8) {
+            float mv[8], lv[8], ov[8], top = M;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                bool ok = s0 + j < p.splits;
+                const bool ok = s0 + j < live;
                 mv[j] = ok ? __ldcg(rec + (s0 + j) * (HD + 2) + HD) : -INFINITY;
                 lv[j] = ok ? __ldcg(rec + (s0 + j) * (HD + 2) + HD + 1) : 0.f;
                 ov[j] = ok ? __ldcg(rec + (s0 + j) * (HD + 2) + d) : 0.f;
             }
 #pragma unroll
+            for (int j = 0; j < 8; ++j) top = fmaxf(top, mv[j]);
+            const float old = M == -INFINITY ? 0.f : exp2f(M - top);
+            L *= old;
+            acc *= old;
+            M = top;
+#pragma unroll
             for (int j = 0; j < 8; ++j) {
-                float wgt = mv[j] == -INFINITY ? 0.f : exp2f(mv[j] - M);
+                const float wgt = mv[j] == -INFINITY ? 0.f : exp2f(mv[j] - M);
                 L += lv[j] * wgt;
                 acc += ov[j] * wgt;
             }
@@ -122,9 +152,9 @@ __device__ __forceinline__ void dm_merge_splits(const DmParams& p, int t, int h0
     }
 }
 
-// WARPS warps take 16 keys each of a unit of WARPS * 16 keys: a whole page with four warps, half a page with two.
-// The CTA of two warps needs half the shared memory, so four of them fit an SM where two of the other do: steps
-// with more CTAs than fit the device at once in the one shape and no more than fit in the other run in one round.
+// Four warps take 16 keys each of a page at a time, with a block-wide barrier per page: for heads of 64 with more than two CTAs
+// for each SM (64 sequences of 500 positions, 8 KV heads: 14.4 us where the kernel below takes 18.6) and for
+// heads of 128 with more than four.
 template <int HD, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) attention_decode_mma_kernel(DmParams p) {
     constexpr int CH = HD / 8, KS = HD / 16, OT = HD / 8, HALF = HD / 2;
@@ -167,9 +197,11 @@ __global__ void __launch_bounds__(WARPS * 32) attention_decode_mma_kernel(DmPara
     }
     const int pos = p.pos[t];
     const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
-    const int first_page = lo >> GB_PAGE_SHIFT, n_pages = (pos >> GB_PAGE_SHIFT) - first_page + 1;
-    const int pg_begin = first_page + int((long long)split * n_pages / p.splits);
-    const int pg_end = first_page + int((long long)(split + 1) * n_pages / p.splits);
+    int first_page, n_pages, live, pg_each;
+    dm_pages(pos, p.window, first_page, n_pages);
+    dm_splits(p, n_pages, live, pg_each);
+    if (split >= live) return;                             // this sequence is not as long as others: nothing to do
+    const int pg_begin = first_page + split * pg_each, pg_end = min(pg_begin + pg_each, first_page + n_pages);
     // the split's units; those of its pages that lie wholly before the window or behind the token are left out
     const int u_begin = max(pg_begin * UPP, lo / UK), u_end = min(pg_end * UPP, pos / UK + 1);
     const int* trow = p.table + size_t(b) * p.table_width;
@@ -400,7 +432,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_decode_mma_kernel(DmPara
             L += l_s[w][r] * wgt;
             acc += merge_o[(size_t(w) * DM_ROWS + r) * MS + d] * wgt;
         }
-        if (p.splits == 1) {
+        if (live == 1) {
             p.out[size_t(t) * p.ldo + size_t(h0 + r) * HD + d] = __float2bfloat16_rn(acc / L);
         } else {
             float* rec = p.scratch + ((size_t(t) * p.nh + h0 + r) * p.splits + split) * (HD + 2);
@@ -409,33 +441,35 @@ __global__ void __launch_bounds__(WARPS * 32) attention_decode_mma_kernel(DmPara
         }
     }
     STAMP_IF(threadIdx.x == 0, 6);
-    if (p.splits == 1) return;
+    if (live == 1) return;
     __threadfence();
     __syncthreads();
     if (tid == 0) {
         int old = atomicAdd(&p.counters[t * gridDim.y + blockIdx.y], 1);
-        last_flag = (old == p.splits - 1);
+        last_flag = (old == live - 1);
     }
     __syncthreads();
     if (!last_flag) return;                               // the others' records are read from L2 (__ldcg): no fence here
-    dm_merge_splits<HD>(p, t, h0, heads, tid, THREADS);
+    dm_merge_splits<HD>(p, live, t, h0, heads, tid, THREADS);
     if (tid == 0) p.counters[t * gridDim.y + blockIdx.y] = 0;
 }
 
-// The same attention for steps with so few (token, KV head) pairs that the device is mostly idle and a CTA's
-// time is the latency of its pages one after the other: twelve warps, each taking quarter pages of 16 keys (warp
-// w: quarters w, w + 12, ...) into two slots of shared memory of its own in turn, so that six pages are on their
-// way at once, a warp's next quarter arrives while it works on this one, and nobody waits for a block-wide
-// barrier per page.  One CTA per SM (24 slots of 16 keys and values); a sequence's pages may be split over
-// several CTAs as in the other kernel.
-constexpr int PW_WARPS = 12;
-constexpr int PW_THREADS = PW_WARPS * 32;
+// The same attention with warps that wait for nobody: warp w takes quarter pages of 16 keys (quarters w, w + warps, ...) into
+// slots of shared memory of its own in turn, so that its next quarters arrive while it works on this one, and there is no
+// block-wide barrier per page: a CTA's time is what bounds a step whose CTAs are few or unequal, and most of that time
+// was barriers and table look-ups (320 CTAs over six sequences of 355 to 2,000 positions 72 -> 34 us a layer with four warps of three
+// slots against the kernel above with two warps, 31 with the splits of dm_splits; six of 700 28.6 -> 17).  Shapes, for heads of 128:
+//   12 warps x 2 slots, one CTA an SM: no more CTAs than SMs (six pages on their way at once);
+//   4 x 3, two an SM: up to two CTAs for each SM;     4 x 2, three an SM: up to three (eight sequences of 1,000, 40 KV heads 40 -> 28.6 us);
+//   2 x 3, four an SM: up to four (64 sequences of 33 to 112 positions, 8 KV heads 10.2 -> 9.3 us, of 520 28.1 -> 27.3).
+// Heads of 64: 12 x 2 in the first case; up to two CTAs for each SM 6 x 2 (32 sequences of 700 positions, 8 KV heads 16.0 -> 11.0 us),
+// where no sequence has more than 7 pages 4 x 3 (100 positions 4.4 us, 5.0 with 6 x 2).
 constexpr int PW_KEYS = 16;                 // keys per slot
-constexpr int PW_SLOTS = 2;                 // slots per warp
 constexpr int PW_UPP = GB_PAGE / PW_KEYS;   // slots' worth of keys per page
 
-template <int HD>
-__global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmParams p) {
+template <int HD, int PW_WARPS, int PW_SLOTS>
+__global__ void __launch_bounds__(PW_WARPS * 32, PW_WARPS == 4 && PW_SLOTS == 2 ? 3 : 1) attention_decode_pages_kernel(DmParams p) {
+    constexpr int PW_THREADS = PW_WARPS * 32;
     constexpr int CH = HD / 8, KS = HD / 16, OT = HD / 8, HALF = HD / 2;
     constexpr int PAGE_ELEMS = GB_PAGE * HD, SLOT_ELEMS = PW_KEYS * HD;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -471,18 +505,20 @@ __global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmPa
     }
     const int pos = p.pos[t];
     const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
-    const int first_page = lo >> GB_PAGE_SHIFT, n_pages = (pos >> GB_PAGE_SHIFT) - first_page + 1;
-    const int pg_begin = first_page + int((long long)split * n_pages / p.splits);
-    const int pg_end = first_page + int((long long)(split + 1) * n_pages / p.splits);
+    int first_page, n_pages, live, pg_each;
+    dm_pages(pos, p.window, first_page, n_pages);
+    dm_splits(p, n_pages, live, pg_each);
+    if (split >= live) return;                             // this sequence is not as long as others: nothing to do
+    const int pg_begin = first_page + split * pg_each, pg_end = min(pg_begin + pg_each, first_page + n_pages);
     const int* trow = p.table + size_t(b) * p.table_width;
     const bool own_kv = p.rotate && p.k_new != nullptr;
     // quarter pages u of the sequence (16 keys each), those of this split's pages that hold a key the token sees
     const int u_first = max(pg_begin * PW_UPP, lo / PW_KEYS), u_end = min(pg_end * PW_UPP, pos / PW_KEYS + 1);
 
-    auto load_quarter = [&](int u, int slot) {
+    auto page_of = [&](int u) { return u < u_end ? trow[(u / PW_UPP) % p.ring_pages] : 0; };
+    auto load_quarter = [&](int u, int slot, int phys) {
         if (u < u_end) {
-            const int pg = u / PW_UPP, row0 = (u % PW_UPP) * PW_KEYS;
-            const int phys = trow[pg % p.ring_pages];
+            const int row0 = (u % PW_UPP) * PW_KEYS;
             const size_t off = (size_t(phys) * p.nkv + g) * size_t(PAGE_ELEMS) + size_t(row0) * HD;
             __nv_bfloat16* kt = ks + (warp * PW_SLOTS + slot) * SLOT_ELEMS;
             __nv_bfloat16* vt = vs + (warp * PW_SLOTS + slot) * SLOT_ELEMS;
@@ -496,41 +532,84 @@ __global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmPa
         }
         dm_commit();                                       // one group per call, also an empty one: the waits count groups
     };
-    // every warp's first two quarters are asked for at once
+    // every warp's first quarters are asked for at once; the page of the one after them is looked up ahead of its turn (the
+    // table's entry is a trip to L2 that the copies would wait for)
     int u = u_first + warp;
-    load_quarter(u, 0);
-    load_quarter(u + PW_WARPS, 1);
-    // the rotation's cosines and sines, one pair index per thread (the position is known before the kernel in
-    // front has finished)
-    if (p.rotate && tid < HALF) {
-        const int half = p.inv_freq ? p.rotary_dim / 2 : 0;
-        float sn = 0.f, cs = 1.f;
-        if (tid < half) sincosf(float(pos) * p.inv_freq[tid], &sn, &cs);
-        cs_s[tid] = cs;
-        sn_s[tid] = sn;
+#pragma unroll
+    for (int k = 0; k < PW_SLOTS; ++k) load_quarter(u + k * PW_WARPS, k, page_of(u + k * PW_WARPS));
+    int next_page = page_of(u + PW_SLOTS * PW_WARPS);
+    // What else does not need the kernel in front: the rotation's cosines and sines, one pair index per thread (the
+    // position is known), the rows of the tile beyond the group, and where the token's own row lies.
+    const int half = p.rotate && p.inv_freq ? p.rotary_dim / 2 : 0;
+    auto pair_of = [&](int pi, int& d0, int& d1) {           // pair pi of a row: inside the rotation, unchanged beyond it
+        d0 = pi < half ? (p.pairing ? 2 * pi : pi) : 2 * pi;
+        d1 = pi < half ? (p.pairing ? 2 * pi + 1 : pi + half) : 2 * pi + 1;
+    };
+    constexpr int OWN = HALF / 32;                           // pairs of the own row per lane
+    const int own_u = pos / PW_KEYS;
+    const bool own_warp = own_kv && own_u >= u_first && own_u < u_end && (own_u - u_first) % PW_WARPS == warp;
+    size_t own_dst = 0;
+    if (own_warp)
+        own_dst = (size_t(trow[(pos >> GB_PAGE_SHIFT) % p.ring_pages]) * p.nkv + g) * size_t(PAGE_ELEMS) + size_t(pos & (GB_PAGE - 1)) * HD;
+    if (p.rotate) {
+        if (tid < HALF) {
+            float sn = 0.f, cs = 1.f;
+            if (tid < half) sincosf(float(pos) * p.inv_freq[tid], &sn, &cs);
+            cs_s[tid] = cs;
+            sn_s[tid] = sn;
+        }
+        for (int i = heads * CH + tid; i < DM_ROWS * CH; i += PW_THREADS) *reinterpret_cast<uint4*>(qs + i * 8) = make_uint4(0, 0, 0, 0);
+        __syncthreads();
     }
     STAMP_IF(threadIdx.x == 0, 1);
     if (early) gb_grid_wait();
     STAMP_IF(threadIdx.x == 0, 2);
 
+    // the token's own key and value, asked for by the warp that will put them into their quarter page
+    __nv_bfloat16 own_k[OWN][2];
+    __nv_bfloat162 own_v[OWN];
+    if (own_warp) {
+        const size_t src = size_t(t) * p.ldq + size_t(g) * HD;
+#pragma unroll
+        for (int e = 0; e < OWN; ++e) {
+            const int pi = lane + 32 * e;
+            int d0, d1;
+            pair_of(pi, d0, d1);
+            own_k[e][0] = p.k_new[src + d0];
+            own_k[e][1] = p.k_new[src + d1];
+            own_v[e] = *reinterpret_cast<const __nv_bfloat162*>(p.v_new + src + 2 * pi);
+        }
+    }
     // the queries
     if (p.rotate) {
-        const int half = p.inv_freq ? p.rotary_dim / 2 : 0;
-        __syncthreads();
-        for (int idx = tid; idx < DM_ROWS * HALF; idx += PW_THREADS) {
-            const int r = idx / HALF, pi = idx - r * HALF;
-            const int d0 = pi < half ? (p.pairing ? 2 * pi : pi) : 2 * pi;
-            const int d1 = pi < half ? (p.pairing ? 2 * pi + 1 : pi + half) : 2 * pi + 1;
-            float x0 = 0.f, x1 = 0.f;
-            if (r < heads) {
-                const __nv_bfloat16* src = p.q + size_t(t) * p.ldq + size_t(h0 + r) * HD;
-                x0 = __bfloat162float(src[d0]);
-                x1 = __bfloat162float(src[d1]);
+        // four pairs of a thread are asked for together (a trip to L2 each, and nothing else to do meanwhile)
+        for (int i0 = tid; i0 < heads * HALF; i0 += 4 * PW_THREADS) {
+            float x0[4], x1[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int idx = i0 + j * PW_THREADS;
+                x0[j] = x1[j] = 0.f;
+                if (idx < heads * HALF) {
+                    int d0, d1;
+                    pair_of(idx % HALF, d0, d1);
+                    const __nv_bfloat16* src = p.q + size_t(t) * p.ldq + size_t(h0 + idx / HALF) * HD;
+                    x0[j] = __bfloat162float(src[d0]);
+                    x1[j] = __bfloat162float(src[d1]);
+                }
             }
-            float y0, y1;
-            gb_rotate(x0, x1, cs_s[pi], sn_s[pi], y0, y1);
-            qs[dm_swz<HD>(r, d0 >> 3) + (d0 & 7)] = __float2bfloat16_rn(y0);
-            qs[dm_swz<HD>(r, d1 >> 3) + (d1 & 7)] = __float2bfloat16_rn(y1);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int idx = i0 + j * PW_THREADS;
+                if (idx < heads * HALF) {
+                    const int r = idx / HALF, pi = idx % HALF;
+                    int d0, d1;
+                    pair_of(pi, d0, d1);
+                    float y0, y1;
+                    gb_rotate(x0[j], x1[j], cs_s[pi], sn_s[pi], y0, y1);
+                    qs[dm_swz<HD>(r, d0 >> 3) + (d0 & 7)] = __float2bfloat16_rn(y0);
+                    qs[dm_swz<HD>(r, d1 >> 3) + (d1 & 7)] = __float2bfloat16_rn(y1);
+                }
+            }
         }
     } else {
         for (int i = tid; i < DM_ROWS * CH; i += PW_THREADS) {
@@ -552,36 +631,31 @@ __global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmPa
     for (int k = 0; k < KS; ++k)
         dm_ldmatrix_x4(qf[k][0], qf[k][1], qf[k][2], qf[k][3], qs + dm_swz<HD>(lane & 15, 2 * k + (lane >> 4)));
 
-    for (int it = 0; u < u_end; u += PW_WARPS, ++it) {
-        const int slot = it & 1;
+    for (int slot = 0; u < u_end; u += PW_WARPS) {
         __nv_bfloat16* kt = ks + (warp * PW_SLOTS + slot) * SLOT_ELEMS;
         __nv_bfloat16* vt = vs + (warp * PW_SLOTS + slot) * SLOT_ELEMS;
         dm_wait<PW_SLOTS - 1>();                            // all groups but the newest: this quarter is there
         __syncwarp();
-        if (own_kv && u == pos / PW_KEYS) {
+        if (own_warp && u == own_u) {
             // the token's own key (rotated) and value: into the quarter page in shared memory, and by the first
             // head tile of the KV head into the cache
             const int r = pos & (PW_KEYS - 1);
-            const int half = p.inv_freq ? p.rotary_dim / 2 : 0;
             const bool writes = (blockIdx.y % gtiles) == 0;
-            const size_t src = size_t(t) * p.ldq + size_t(g) * HD;
-            const size_t dst = (size_t(trow[(pos >> GB_PAGE_SHIFT) % p.ring_pages]) * p.nkv + g) * size_t(PAGE_ELEMS) +
-                               size_t(pos & (GB_PAGE - 1)) * HD;
-            for (int pi = lane; pi < HALF; pi += 32) {
-                const int d0 = pi < half ? (p.pairing ? 2 * pi : pi) : 2 * pi;
-                const int d1 = pi < half ? (p.pairing ? 2 * pi + 1 : pi + half) : 2 * pi + 1;
+#pragma unroll
+            for (int e = 0; e < OWN; ++e) {
+                const int pi = lane + 32 * e, ev = 2 * pi;
+                int d0, d1;
+                pair_of(pi, d0, d1);
                 float r0, r1;
-                gb_rotate(__bfloat162float(p.k_new[src + d0]), __bfloat162float(p.k_new[src + d1]), cs_s[pi], sn_s[pi], r0, r1);
+                gb_rotate(__bfloat162float(own_k[e][0]), __bfloat162float(own_k[e][1]), cs_s[pi], sn_s[pi], r0, r1);
                 const __nv_bfloat16 y0 = __float2bfloat16_rn(r0), y1 = __float2bfloat16_rn(r1);
                 kt[dm_swz<HD>(r, d0 >> 3) + (d0 & 7)] = y0;
                 kt[dm_swz<HD>(r, d1 >> 3) + (d1 & 7)] = y1;
-                const int e = 2 * pi;
-                const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(p.v_new + src + e);
-                *reinterpret_cast<__nv_bfloat162*>(vt + dm_swz<HD>(r, e >> 3) + (e & 7)) = x;
+                *reinterpret_cast<__nv_bfloat162*>(vt + dm_swz<HD>(r, ev >> 3) + (ev & 7)) = own_v[e];
                 if (writes) {
-                    p.kc_w[dst + d0] = y0;
-                    p.kc_w[dst + d1] = y1;
-                    *reinterpret_cast<__nv_bfloat162*>(p.vc_w + dst + e) = x;
+                    p.kc_w[own_dst + d0] = y0;
+                    p.kc_w[own_dst + d1] = y1;
+                    *reinterpret_cast<__nv_bfloat162*>(p.vc_w + own_dst + ev) = own_v[e];
                 }
             }
             __syncwarp();
@@ -589,16 +663,20 @@ __global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmPa
         // the slot's 16 keys, as the other kernel treats a warp's 16 keys of a page
         {
             constexpr int key_base = 0;
-            float s[2][4];
+            float s[2][4], s2[2][4];                         // even and odd steps of the head: half as long a chain of products
 #pragma unroll
-            for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+            for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = s2[j][0] = s2[j][1] = s2[j][2] = s2[j][3] = 0.f;
 #pragma unroll
             for (int k = 0; k < KS; ++k) {
                 unsigned b0, b1, b2, b3;
                 dm_ldmatrix_x4(b0, b1, b2, b3, kt + dm_swz<HD>(key_base + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1)));
-                dm_mma(s[0], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b0, b1);
-                dm_mma(s[1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b2, b3);
+                dm_mma(k & 1 ? s2[0] : s[0], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b0, b1);
+                dm_mma(k & 1 ? s2[1] : s[1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b2, b3);
             }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[j][e] += s2[j][e];
             const int key0 = u * PW_KEYS + key_base + 2 * (lane & 3);
             float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
@@ -626,18 +704,22 @@ __global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmPa
             m0 = mn0;
             m1 = mn1;
             const unsigned pa0 = dm_pack(p00, p01), pa1 = dm_pack(p02, p03), pa2 = dm_pack(p10, p11), pa3 = dm_pack(p12, p13);
+            if (__any_sync(0xffffffffu, a0 != 1.f || a1 != 1.f)) {        // some row's maximum has grown
+#pragma unroll
+                for (int i = 0; i < OT; ++i) { o[i][0] *= a0; o[i][1] *= a0; o[i][2] *= a1; o[i][3] *= a1; }
+            }
 #pragma unroll
             for (int i2 = 0; i2 < OT / 2; ++i2) {
                 unsigned b0, b1, b2, b3;
                 dm_ldmatrix_x4_trans(b0, b1, b2, b3, vt + dm_swz<HD>(key_base + (lane & 15), 2 * i2 + (lane >> 4)));
-                o[2 * i2][0] *= a0; o[2 * i2][1] *= a0; o[2 * i2][2] *= a1; o[2 * i2][3] *= a1;
-                o[2 * i2 + 1][0] *= a0; o[2 * i2 + 1][1] *= a0; o[2 * i2 + 1][2] *= a1; o[2 * i2 + 1][3] *= a1;
                 dm_mma(o[2 * i2], pa0, pa1, pa2, pa3, b0, b1);
                 dm_mma(o[2 * i2 + 1], pa0, pa1, pa2, pa3, b2, b3);
             }
         }
         __syncwarp();                                        // the slot may be loaded again
-        load_quarter(u + PW_SLOTS * PW_WARPS, slot);
+        load_quarter(u + PW_SLOTS * PW_WARPS, slot, next_page);
+        next_page = page_of(u + (PW_SLOTS + 1) * PW_WARPS);
+        if (++slot == PW_SLOTS) slot = 0;
     }
     STAMP_AFTER_IF(threadIdx.x == 0, 4, o[0][0]);
     dm_wait<0>();
@@ -675,7 +757,7 @@ __global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmPa
             L += l_s[w][r] * wgt;
             acc += merge_o[(size_t(w) * DM_ROWS + r) * MS + d] * wgt;
         }
-        if (p.splits == 1) {
+        if (live == 1) {
             p.out[size_t(t) * p.ldo + size_t(h0 + r) * HD + d] = __float2bfloat16_rn(acc / L);
         } else {
             float* rec = p.scratch + ((size_t(t) * p.nh + h0 + r) * p.splits + split) * (HD + 2);
@@ -684,29 +766,29 @@ __global__ void __launch_bounds__(PW_THREADS) attention_decode_pages_kernel(DmPa
         }
     }
     STAMP_IF(threadIdx.x == 0, 6);
-    if (p.splits == 1) return;
+    if (live == 1) return;
     // ---- the splits of a (token, head tile) are merged by the CTA that finishes last, in split order
     __threadfence();
     __syncthreads();
     if (tid == 0) {
         int old = atomicAdd(&p.counters[t * gridDim.y + blockIdx.y], 1);
-        last_flag = (old == p.splits - 1);
+        last_flag = (old == live - 1);
     }
     __syncthreads();
     if (!last_flag) return;                               // the others' records are read from L2 (__ldcg): no fence here
-    dm_merge_splits<HD>(p, t, h0, heads, tid, PW_THREADS);
+    dm_merge_splits<HD>(p, live, t, h0, heads, tid, PW_THREADS);
     if (tid == 0) p.counters[t * gridDim.y + blockIdx.y] = 0;
 }
 
-template <int HD> int launch_pw(const DmParams& p, dim3 grid, cudaStream_t stream) {
-    constexpr int SMEM = (DM_ROWS + 2 * PW_WARPS * PW_SLOTS * PW_KEYS) * HD * 2;
+template <int HD, int WARPS, int SLOTS> int launch_pw(const DmParams& p, dim3 grid, cudaStream_t stream) {
+    constexpr int SMEM = (DM_ROWS + 2 * WARPS * SLOTS * PW_KEYS) * HD * 2;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(attention_decode_pages_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+        if (cudaFuncSetAttribute(attention_decode_pages_kernel<HD, WARPS, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
             return gb_fail("gb_attention_decode_mma: cannot get %d bytes of shared memory", SMEM);
         configured = true;
     }
-    gb_launch(attention_decode_pages_kernel<HD>, grid, dim3(PW_THREADS), SMEM, stream, p);
+    gb_launch(attention_decode_pages_kernel<HD, WARPS, SLOTS>, grid, dim3(WARPS * 32), SMEM, stream, p);
     GB_LAUNCH_OK("gb_attention_decode_mma");
     return 0;
 }
@@ -748,18 +830,19 @@ GB_API int gb_attention_decode_mma_supported(int hd, int cache_dtype, int q_dtyp
 }
 
 // Same contract as gb_attention_decode; counters: T * nkv * ceil(G/16) zeroed ints when splits > 1;
-// scratch: T * nh * splits * (hd + 2) floats.  With rotate != 0 the kernel also does what gb_rope_kv_write does
+// scratch: T * nh * splits * (hd + 2) floats; split_pages: a split has no fewer pages; short_seqs: no sequence has more than
+// 7 pages (it chooses among CTA shapes only).  With rotate != 0 the kernel also does what gb_rope_kv_write does
 // for these tokens: q, k_new, v_new (rows ldq apart, as the projection left them; k_new and v_new null for a
 // mixer that reads another run's cache) are rotated by pos * inv_freq (inv_freq null: no rotation) and the
 // token's key and value are written at its position of the cache.  q itself stays as it was.
 static int decode_mma(const void* q, long long ldq, void* out, long long ldo, int T, int nh, int nkv, int hd,
                       const int* seq_of, const int* pos, const int* table, int table_width, int ring_pages,
-                      void* kcache, void* vcache, int window, float scale, int splits, float* scratch,
+                      void* kcache, void* vcache, int window, float scale, int splits, int split_pages, int short_seqs, float* scratch,
                       int* counters, int n_counters, int rotate, const void* k_new, const void* v_new,
                       const float* inv_freq, int rotary_dim, int pairing, cudaStream_t stream) {
     GB_REQUIRE(gb_attention_decode_mma_supported(hd, GB_BF16, GB_BF16), "gb_attention_decode_mma: head_dim %d is not 64 or 128", hd);
     GB_REQUIRE(nh > 0 && nkv > 0 && nh % nkv == 0, "gb_attention_decode_mma: %d heads are not a multiple of %d KV heads", nh, nkv);
-    GB_REQUIRE(window >= 0 && ring_pages > 0 && table_width > 0 && splits >= 1, "gb_attention_decode_mma: bad cache geometry");
+    GB_REQUIRE(window >= 0 && ring_pages > 0 && table_width > 0 && splits >= 1 && split_pages >= 1, "gb_attention_decode_mma: bad cache geometry");
     GB_REQUIRE((ldq % 8) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 && (reinterpret_cast<uintptr_t>(kcache) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(vcache) & 15) == 0, "gb_attention_decode_mma: misaligned operands");
     if (T == 0) return 0;
@@ -771,7 +854,7 @@ static int decode_mma(const void* q, long long ldq, void* out, long long ldo, in
     p.q = (const __nv_bfloat16*)q; p.out = (__nv_bfloat16*)out; p.kc = (const __nv_bfloat16*)kcache;
     p.vc = (const __nv_bfloat16*)vcache; p.seq_of = seq_of; p.pos = pos; p.table = table; p.scratch = scratch;
     p.counters = counters; p.ldq = ldq; p.ldo = ldo; p.nh = nh; p.nkv = nkv; p.table_width = table_width;
-    p.ring_pages = ring_pages; p.window = window; p.splits = splits; p.scale_log2 = scale * 1.4426950408889634f;
+    p.ring_pages = ring_pages; p.window = window; p.T = T; p.splits = splits; p.split_pages = split_pages; p.scale_log2 = scale * 1.4426950408889634f;
     p.rotate = rotate; p.k_new = (const __nv_bfloat16*)k_new; p.v_new = (const __nv_bfloat16*)v_new;
     p.kc_w = (__nv_bfloat16*)kcache; p.vc_w = (__nv_bfloat16*)vcache; p.inv_freq = inv_freq;
     p.rotary_dim = rotary_dim; p.pairing = pairing;
@@ -779,22 +862,34 @@ static int decode_mma(const void* q, long long ldq, void* out, long long ldo, in
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_pages_kernel && (long long)T * nkv * gtiles * splits <= sms)       // few CTAs: a CTA's latency is the step's
-        return hd == 64 ? launch_pw<64>(p, grid, stream) : launch_pw<128>(p, grid, stream);
-    // Heads of 128: two CTAs of four warps fit an SM, or four CTAs of two warps.  A step with more CTAs than fit
-    // in the first shape, and no more than fit in the second, runs in one round with the second.
-    const long long ctas = (long long)T * nkv * gtiles * splits;
-    if (hd == 128 && g_two_warps && (g_two_warps == 2 || (ctas > 2LL * sms && ctas <= 4LL * sms)))
-        return launch_dm<128, 2>(p, grid, stream);
+    // shapes of a CTA: see attention_decode_pages_kernel.  p.slots: CTAs of the shape that the device holds
+    const long long columns = (long long)T * nkv * gtiles;
+    const bool two = hd == 128 && g_two_warps == 2;
+    p.slots = 0;
+    if (g_pages_kernel && columns * splits <= sms)
+        return hd == 64 ? launch_pw<64, 12, 2>(p, grid, stream) : launch_pw<128, 12, 2>(p, grid, stream);
+    if (g_pages_kernel && columns <= 2LL * sms && !two) {
+        p.slots = 2 * sms;
+        if (hd == 64) return short_seqs ? launch_pw<64, 4, 3>(p, grid, stream) : launch_pw<64, 6, 2>(p, grid, stream);
+        return launch_pw<128, 4, 3>(p, grid, stream);
+    }
+    if (g_pages_kernel && hd == 128 && columns <= 3LL * sms && !two) {
+        p.slots = 3 * sms;
+        return launch_pw<128, 4, 2>(p, grid, stream);
+    }
+    if (two || (hd == 128 && g_pages_kernel && g_two_warps && columns <= 4LL * sms)) {
+        p.slots = 4 * sms;
+        return launch_pw<128, 2, 3>(p, grid, stream);
+    }
     return hd == 64 ? launch_dm<64, 4>(p, grid, stream) : launch_dm<128, 4>(p, grid, stream);
 }
 
 GB_API int gb_attention_decode_mma(const void* q, long long ldq, void* out, long long ldo, int T, int nh, int nkv, int hd,
                                    const int* seq_of, const int* pos, const int* table, int table_width,
                                    int ring_pages, const void* kcache, const void* vcache, int window, float scale,
-                                   int splits, float* scratch, int* counters, int n_counters, cudaStream_t stream) {
+                                   int splits, int split_pages, int short_seqs, float* scratch, int* counters, int n_counters, cudaStream_t stream) {
     return decode_mma(q, ldq, out, ldo, T, nh, nkv, hd, seq_of, pos, table, table_width, ring_pages, (void*)kcache,
-                      (void*)vcache, window, scale, splits, scratch, counters, n_counters, 0, nullptr, nullptr, nullptr,
+                      (void*)vcache, window, scale, splits, split_pages, short_seqs, scratch, counters, n_counters, 0, nullptr, nullptr, nullptr,
                       0, 0, stream);
 }
 
@@ -802,13 +897,13 @@ GB_API int gb_attention_decode_mma_rope(const void* q, const void* k_new, const 
                                         long long ldo, int T, int nh, int nkv, int hd, int rotary_dim, int pairing,
                                         const float* inv_freq, const int* seq_of, const int* pos, const int* table,
                                         int table_width, int ring_pages, void* kcache, void* vcache, int window,
-                                        float scale, int splits, float* scratch, int* counters, int n_counters,
+                                        float scale, int splits, int split_pages, int short_seqs, float* scratch, int* counters, int n_counters,
                                         cudaStream_t stream) {
     GB_REQUIRE(rotary_dim >= 0 && rotary_dim <= hd && rotary_dim % 2 == 0,
                "gb_attention_decode_mma_rope: rotary_dim %d must be even and at most head_dim %d", rotary_dim, hd);
     GB_REQUIRE((k_new == nullptr) == (v_new == nullptr), "gb_attention_decode_mma_rope: k and v must both be given or both be null");
     GB_REQUIRE(!v_new || (reinterpret_cast<uintptr_t>(v_new) & 3) == 0, "gb_attention_decode_mma_rope: misaligned v");
     return decode_mma(q, ldq, out, ldo, T, nh, nkv, hd, seq_of, pos, table, table_width, ring_pages, kcache, vcache,
-                      window, scale, splits, scratch, counters, n_counters, 1, k_new, v_new, inv_freq, rotary_dim,
+                      window, scale, splits, split_pages, short_seqs, scratch, counters, n_counters, 1, k_new, v_new, inv_freq, rotary_dim,
                       pairing, stream);
 }

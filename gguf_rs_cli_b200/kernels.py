@@ -3,7 +3,7 @@ stream.  Nothing here computes; a missing or failing library raises NativeError.
 """
 from __future__ import annotations
 
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 
@@ -1232,6 +1232,29 @@ def decode_splits(T: int, n_heads: int, n_kv_heads: int, max_kv: int, sms: int, 
     return _split_class(min(room, cls // 3))
 
 
+MANY_SPLITS, SPLIT_PAGES = 4, 4
+
+
+def decode_sharing(T: int, n_heads: int, n_kv_heads: int, head_dim: int, max_kv: int, sms: int) -> Tuple[int, int]:
+    """(splits of the grid, pages that a split has at least) for a step of the tensor-core kernels; like decode_splits a
+    function of the step's class and its CTAs.
+
+    More CTAs than SMs: the grid has room for four splits of each sequence, and the kernel decides from the lengths which
+    sequences use them (a split has no fewer pages than a CTA has when all pages are dealt out equally, and at least four).  Six
+    sequences of 355 to 2,000 positions with 40 KV heads: 34 us a layer whole, 31 with up to four splits; twenty of up to
+    3,000 with 8: 46 and 31; equal ones stay whole (45.1 us against 44.2 at 32 of 2,000).  Below 16 pages the CTAs that
+    leave at once cost more than the splits give (64 sequences of up to 112 positions: 9.3 us, 13.6 with room for four splits), for
+    heads of 64 they always do (32 of 20 to 1,500 positions 16.7 and 21.5 us), and with more than four CTAs for each SM the rounds
+    even the lengths out by themselves."""
+    group = n_heads // n_kv_heads
+    ctas = T * n_kv_heads * ((group + 15) // 16)
+    if ctas <= sms:
+        return decode_splits(T, n_heads, n_kv_heads, max_kv, sms, True), 1
+    if head_dim == 64 or ctas > 4 * sms or decode_split_class(max_kv) < 4:
+        return 1, 1
+    return MANY_SPLITS, SPLIT_PAGES
+
+
 def attention_decode_mma_supported(q: torch.Tensor, kcache: torch.Tensor, head_dim: int) -> bool:
     return bool(native.library().gb_attention_decode_mma_supported(head_dim, dtype_code(kcache), dtype_code(q)))
 
@@ -1243,7 +1266,7 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv_head
                      rope: Optional[tuple] = None, keep_first: int = 0, head_pages: int = 0,
                      gate: Optional[torch.Tensor] = None, sink: bool = False, sink_values: Optional[torch.Tensor] = None,
                      chunk: int = 0, slopes: Optional[torch.Tensor] = None, softcap: float = 0.0,
-                     out_scale: float = 1.0) -> torch.Tensor:
+                     out_scale: float = 1.0, split_pages: int = 1) -> torch.Tensor:
     """One token per sequence over the bf16 cache; all heads of a group share one pass over
     the keys and values.  mma: the tensor-core kernel (head sizes 64 and 128; the default
     where it fits) or the CUDA-core one (any head size that is a multiple of 16).
@@ -1268,8 +1291,13 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv_head
     if mma is None:
         mma = attention_decode_mma_supported(q, kcache, head_dim)
     entry = "gb_attention_decode_mma" if mma else "gb_attention_decode"
+    longest = max_kv if max_kv else table.shape[1] * 64
+    short = int(decode_split_class(longest) < 2)
     if splits is None:
-        splits = decode_splits(T, n_heads, n_kv_heads, max_kv if max_kv else table.shape[1] * 64, sc.sms, mma)
+        if mma:
+            splits, split_pages = decode_sharing(T, n_heads, n_kv_heads, head_dim, longest, sc.sms)
+        else:
+            splits = decode_splits(T, n_heads, n_kv_heads, longest, sc.sms, False)
     need = lib.gb_attention_decode_scratch_floats(T, n_heads, head_dim, splits)
     scratch = counters = None
     if need:
@@ -1282,7 +1310,7 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv_head
         assert mma and (k is None or (k.stride(0) == q.stride(0) and v.stride(0) == q.stride(0) and k.dtype == q.dtype))
         call("gb_attention_decode_mma_rope", ptr(q), ptr(k), ptr(v), q.stride(0), ptr(out), out.stride(0), T, n_heads,
              n_kv_heads, head_dim, rotary_dim, pairing, ptr(inv_freq), ptr(seq_of), ptr(pos), ptr(table), table.shape[1],
-             ring_pages, ptr(kcache), ptr(vcache), int(window or 0), float(scale), splits, ptr(scratch), ptr(counters),
+             ring_pages, ptr(kcache), ptr(vcache), int(window or 0), float(scale), splits, split_pages, short, ptr(scratch), ptr(counters),
              0 if counters is None else counters.numel(), stream_ptr())
         return out
     if kept:
@@ -1294,7 +1322,8 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv_head
         return out
     call(entry, ptr(q), q.stride(0), ptr(out), out.stride(0), T, n_heads, n_kv_heads, head_dim,
          ptr(seq_of), ptr(pos), ptr(table), table.shape[1], ring_pages, ptr(kcache), ptr(vcache), int(window or 0),
-         float(scale), splits, ptr(scratch), ptr(counters), 0 if counters is None else counters.numel(), stream_ptr())
+         float(scale), splits, *((split_pages, short) if mma else ()), ptr(scratch), ptr(counters),
+         0 if counters is None else counters.numel(), stream_ptr())
     return out
 
 
