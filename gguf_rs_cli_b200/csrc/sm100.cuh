@@ -326,5 +326,7 @@ __host__ __device__ constexpr uint32_t instr_desc_bf16(int M, int N) {
 // Tensor map of a row-major bf16 matrix [rows, cols] with pitch ld (elements): boxes of box_rows x 64
 // columns, 128-byte swizzle, zero fill outside.  Host side; returns 0 or sets the error text.
 int tensor_map_bf16_2d(const void* ptr, long long rows, long long cols, long long ld, int box_rows, CUtensorMap* out);
+// The same of 32-bit floats: boxes of box_rows x 32 columns.
+int tensor_map_f32_2d(const void* ptr, long long rows, long long cols, long long ld, int box_rows, CUtensorMap* out);
 
 }  // namespace sm100

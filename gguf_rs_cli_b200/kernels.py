@@ -3,6 +3,7 @@ stream.  Nothing here computes; a missing or failing library raises NativeError.
 """
 from __future__ import annotations
 
+import threading
 from typing import Optional, Tuple
 
 import torch
@@ -1151,6 +1152,47 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     return out
 
 
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
+    """32-bit operands on the tensor cores, three bfloat16 terms each; the same operands as gemm_f32."""
+    _cuda(x, w, bias, out)
+    T, K = x.shape
+    N = w.shape[0]
+    assert w.shape[1] == K and x.dtype == w.dtype == torch.float32 and out.shape == (T, N) and out.stride(1) == 1
+    sms = tc_scratch(x.device).sms
+    counters, scratch = _f32_counters(x.device), None
+    need = native.library().gb_gemm_f32_tc_scratch_floats(T, N, K, sms, 0 if counters is None else counters.numel())
+    if need:
+        scratch = torch.empty(need, dtype=torch.float32, device=x.device)
+    call("gb_gemm_f32_tc", ptr(x), x.stride(0), ptr(w), w.stride(0), ptr(bias), 0 if bias is None else dtype_code(bias), ptr(out),
+         dtype_code(out), out.stride(0), T, N, K, ptr(scratch), ptr(counters), 0 if counters is None else counters.numel(), sms, stream_ptr())
+    return out
+
+
+_f32_counter_buffers, _f32_counter_rows, _f32_counter_lock = {}, {}, threading.Lock()
+F32_COUNTER_STREAMS = 64         # 16 KB each; launches on further streams share no tiles
+
+
+def _f32_counters(device) -> Optional[torch.Tensor]:
+    """Arrival counters of the 32-bit tensor-core products on the current stream, zero between launches.  Products on different
+    streams may run at the same time, so each stream has its own; all are allocated at a device's first product, so that a
+    stream's first may be one that is being captured."""
+    index = torch.device(device).index or 0
+    key = (index, stream_ptr())
+    got = _f32_counter_rows.get(key)
+    if got is not None:
+        return got
+    with _f32_counter_lock:
+        if index not in _f32_counter_buffers:
+            if torch.cuda.is_current_stream_capturing():
+                return None
+            _f32_counter_buffers[index] = torch.zeros(F32_COUNTER_STREAMS, _TcScratch.COUNTERS, dtype=torch.int32, device=device)
+            torch.cuda.synchronize(index)                             # zero for every stream
+        taken = sum(k[0] == index for k in _f32_counter_rows)
+        if key not in _f32_counter_rows and taken < F32_COUNTER_STREAMS:
+            _f32_counter_rows[key] = _f32_counter_buffers[index][taken]
+        return _f32_counter_rows.get(key)
+
+
 GROUPED_TILE = 256               # tokens of a tile of the kernel that pairs two SMs
 
 
@@ -1404,6 +1446,12 @@ def check_tc_status() -> None:
         raise native.NativeError(f"a tensor-core product gave up waiting (code {code}: 1 a stage never came free, "
                                  f"2 a load never arrived, 3/4 an accumulator never completed, 5 a CTA that shares a tile never arrived); "
                                  f"its output is invalid")
+    code = lib.gb_gemm_f32_tc_status()
+    if code:
+        lib.gb_gemm_f32_tc_status_clear()
+        for counters in _f32_counter_buffers.values():
+            counters.zero_()
+        raise native.NativeError(f"a 32-bit tensor-core product gave up waiting (code {code}); its output is invalid")
     code = lib.gb_attention_tc_status()
     if code:
         lib.gb_attention_tc_status_clear()
@@ -1411,11 +1459,23 @@ def check_tc_status() -> None:
 
 
 # ------------------------------------------------------------------ dispatch
+def _f32_on_tensor_cores(w: torch.Tensor) -> bool:
+    """Whether 32-bit products with this matrix run on the tensor cores: for every number of tokens or for none, so that a row's
+    result does not depend on the rows beside it.  Tensor cores over CUDA cores at 1, 2, 4, 16 and 187 tokens, us: 3072 x 2048 12.4 / 13.4,
+    12.6 / 12.3, 12.7 / 16.9, 13 / 36, 23 / 123; 2048 x 8192 22 / 36, 22 / 42, 22 / 41, 22 / 80, 45 / 414; 16384 x 2048 35 / 24, 35 / 27,
+    35 / 33, 36 / 63, 80 / 390; 2048 x 2048 11 / 12.5 ... 20 / 114; 1024 x 1024 7.8 / 7.4 ... 16 tokens 7.7 / 8.6, 17 7.8 / 19.6.  Smaller matrices are
+    faster on CUDA cores (512 x 512 7.0 / 4.2), and so is a head, which sees few tokens (128256 x 2048 203 / 180)."""
+    N, K = w.shape
+    return K >= 1024 and N * K >= 1 << 20 and N <= 1 << 16
+
+
 def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
-    """The product path of every projection: the tensor-core kernel when dtype and sizes
+    """The product path of every projection: a tensor-core kernel when dtype and sizes
     fit it, else a CUDA-core kernel (two of them, with the same sums bit for bit)."""
     if gemm_tc_supported(x, w):
         return gemm_tc(x, w, bias, out)
+    if gemm_f32_supported(x, w) and _f32_on_tensor_cores(w):
+        return gemm_f32_tc(x, w, bias, out)
     # one block of 16 of K and thousands of features: gemm_generic has nothing to wait for (16 x 16384 x 16 3.2 us, 6.8 in gemm_f32;
     # 1000 x 4096 x 16 9.4 and 12.5), and from K = 20 on gemm_f32 takes 0.7 to 0.8 as long in the mean
     if gemm_f32_supported(x, w) and not (x.shape[1] <= 16 and w.shape[0] > 1000):

@@ -1,0 +1,111 @@
+"""32-bit products on the tensor cores: every tile width, its edges, shared tiles, operands that are not finite, and the
+distance from 64 bits beside the one-thread sums of the CUDA-core kernel."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _operands(T, N, K, seed, positive=False):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    x, w = torch.randn(T, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV) / math.sqrt(K)
+    return (x.abs(), w.abs()) if positive else (x, w)
+
+
+# widths of 32, 64, 96, 128, 160 and 192 tokens, several of them, K that ends inside a block, one block, shared tiles and whole ones
+@pytest.mark.parametrize("T", [1, 16, 17, 32, 33, 64, 96, 97, 128, 160, 187, 192, 193, 400])
+@pytest.mark.parametrize("N, K", [(128, 512), (130, 2048), (3000, 516), (257, 4), (20000, 548), (2048, 4096)])
+@pytest.mark.parametrize("positive", [False, True])
+def test_closer_to_64_bits_than_one_thread(T, N, K, positive):
+    from gguf_rs_cli_b200 import kernels as k
+    x, w = _operands(T, N, K, T + N + K, positive)
+    bias = torch.randn(N, device=DEV) if K == 516 else None
+    want = x.double() @ w.double().T
+    if bias is not None:
+        want += bias.double()
+    got, plain = torch.full((T, N + 4), 7.0, device=DEV)[:, :N], torch.empty(T, N, device=DEV)
+    k.gemm_f32_tc(x, w, bias, got)
+    k.gemm_f32(x, w, bias, plain)
+    torch.cuda.synchronize()
+    k.check_tc_status()
+    e, e_plain = [float((a.double() - want).norm() / want.norm()) for a in (got, plain)]
+    # a result is rounded once (2^-25 in the mean of a binade's ends) and the sums of 32 that it adds are; the terms left out are 2^-23
+    assert e <= max(1.1 * e_plain, 1.5e-7) and e < 4e-7, (e, e_plain)
+    assert (got._base[:, N:] == 7.0).all()
+    again, low = torch.empty_like(plain), torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
+    k.gemm_f32_tc(x, w, bias, again)
+    k.gemm_f32_tc(x, w, bias, low)
+    assert torch.equal(again, got) and torch.equal(low, got.bfloat16())          # the order of the sums is fixed; counters are back at zero
+
+
+def test_rows_of_larger_matrices_and_the_dispatch():
+    from gguf_rs_cli_b200 import kernels as k
+    x, w = _operands(40, 1030, 1032, 3)
+    for K, tc in ((1024, True), (1020, False)):
+        xs, ws = x[:, 4:4 + K], w[:, 8:8 + K]
+        got, direct = torch.empty(40, 1030, device=DEV), torch.empty(40, 1030, device=DEV)
+        k.gemm(xs, ws, None, got)
+        (k.gemm_f32_tc if tc else k.gemm_generic)(xs, ws, None, direct)
+        want = xs.double() @ ws.double().T
+        assert torch.equal(direct, got) and float((got.double() - want).norm() / want.norm()) < (4e-7 if tc else 2e-6)
+
+
+@pytest.mark.parametrize("N, K", [(1024, 1024), (2048, 8192), (3072, 2048), (20000, 2048), (40000, 1024), (1030, 1100)])
+def test_a_rows_result_does_not_depend_on_the_rows_beside_it(N, K):
+    """One, two, four CTAs' share of K, or sixteen, tiles of every width: the same bits for a token, alone or among others."""
+    from gguf_rs_cli_b200 import kernels as k
+    x, w = _operands(450, N, K, N + K)
+    want = torch.empty(450, N, device=DEV)
+    k.gemm(x, w, None, want)
+    for lo, hi in ((0, 1), (3, 5), (0, 16), (1, 18), (0, 33), (7, 80), (0, 100), (10, 140), (0, 192), (50, 243), (100, 450)):
+        got = torch.empty(hi - lo, N, device=DEV)
+        k.gemm(x[lo:hi], w, None, got)
+        assert torch.equal(got, want[lo:hi]), (lo, hi)
+    torch.cuda.synchronize()
+    k.check_tc_status()
+
+
+def test_operands_that_are_not_finite_and_large_ones():
+    """Infinities, NaN (with a payload in its last bits only), numbers next to the largest, and subnormal ones: what one thread's sum gives."""
+    from gguf_rs_cli_b200 import kernels as k
+    x, w = _operands(50, 200, 640, 5)
+    x[3, 100], x[7, 5], x[9, 639] = math.inf, -math.inf, math.nan
+    x[11, 50] = torch.tensor(0x7F800001, dtype=torch.int32).view(torch.float32)
+    x[20, :] = 0.0
+    x[20, 3], w[17, 3] = 3.4e38, 1.0
+    x[21, 4], w[18, 4] = 3.4e38, 4.0
+    x[22] *= 1e-39
+    w[30, 9] = math.inf
+    x[23, 9] = 0.0
+    got, want = torch.empty(50, 200, device=DEV), torch.empty(50, 200, device=DEV)
+    k.gemm_f32_tc(x, w, None, got)
+    k.gemm_generic(x, w, None, want)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    inf = want.isinf()
+    assert torch.equal(got[inf], want[inf]) and inf.any() and want.isnan().any()
+    # a row's error is measured against its own size; row 22 holds sums of subnormal numbers, taken one product behind another like
+    # gemm_generic's unless nothing is left of them at all (below 2^-126)
+    fin = want.isfinite()
+    a, b = torch.where(fin, got, 0.0).double(), torch.where(fin, want, 0.0).double()
+    assert ((a - b).norm(dim=1) <= 2e-6 * b.norm(dim=1) + 2.0 ** -126).all()
+    assert torch.equal(got[22][got[22] != 0], want[22][got[22] != 0]) and (got[22] != 0).sum() > 100
+
+
+def test_streams_have_counters_of_their_own():
+    from gguf_rs_cli_b200 import kernels as k
+    x, w = _operands(100, 2048, 2048, 9)
+    want = torch.empty(100, 2048, device=DEV)
+    k.gemm_f32_tc(x, w, None, want)
+    torch.cuda.synchronize()
+    streams, outs = [torch.cuda.Stream() for _ in range(2)], []
+    for _ in range(20):
+        for s in streams:
+            with torch.cuda.stream(s):
+                outs.append(torch.empty(100, 2048, device=DEV))
+                k.gemm_f32_tc(x, w, None, outs[-1])
+    torch.cuda.synchronize()
+    k.check_tc_status()
+    assert all(torch.equal(o, want) for o in outs)
