@@ -51,31 +51,115 @@ __device__ __forceinline__ bool epilogue_any(bool flag) {
 }
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-// v[jj] = the sum over a shared tile's CTAs, in ascending order, of token c0 + jj of this thread's feature: S partial
-// tiles x C tokens of loads in flight at a time (every round of loads costs a trip to L2, and the kernel after
-// this one waits for it: few CTAs on a tile take more tokens per round).  base: the first CTA's first slot, at
-// this thread's feature.
-template <int BN, int S, int C>
-__device__ __forceinline__ void sum_partials(const float* base, int first_which, int n_ctas, int c0, int cols, float (&v)[16]) {
+// What only some products need, kept out of the way of the others (every SM runs the code below from a cold instruction cache).
+// Arguments by value: a reference to the kernel's parameters would copy them to local memory, 10 us a layer.
+__device__ __noinline__ float4 shared_bias(const void* bias, int dtype, int n) {
+    return make_float4(gb_load(bias, dtype, n), gb_load(bias, dtype, n + 1), gb_load(bias, dtype, n + 2), gb_load(bias, dtype, n + 3));
+}
+// Even features are gates, odd ones the matching up features; at: the place of the first pair's result, left: results from there on in the row.
+__device__ __noinline__ void shared_gated(void* out, int dtype, size_t at, int left, int act, float g0, float u0, float g1, float u1) {
+    if (left > 0) gb_store(out, dtype, at, gb_gate_act(g0, act) * u0);
+    if (left > 1) gb_store(out, dtype, at + 1, gb_gate_act(g1, act) * u1);
+}
+// The sum of one feature of one token, for rows that take no accesses of four values and for features next to the matrix's end.
+__device__ __noinline__ float shared_sum(const float* part, size_t stride, const float* first, int n_ctas) {
+    float v = __ldcg(first);
+    for (int s = 1; s < n_ctas; ++s) v += __ldcg(part + s * stride);
+    return v;
+}
+
+// The tokens c_lo .. c_hi - 1 of a shared tile, finished by one of its CTAs: the sums of all its CTAs, in ascending order, and the
+// last steps (as tc_finish_chunk).  A warp has a token and a lane four neighbouring features of it, so that a token's row of a
+// partial tile, of the residual stream and of the result is one access of a warp, TOK tokens with SUMS CTAs' sums each are
+// asked for at once, and the sum of squares needs no other warp.  (A feature a thread, 16 tokens each, took a trip to L2 for every
+// 8 tokens: 5 us behind the last CTA's arrival at 64 tokens.)
+// base: the first CTA's first slot.
+template <int BN, int TOK, int SUMS>
+__device__ __forceinline__ void finish_shared(const TcParams& p, const float* base, int first_which, int n_ctas, int n0, int t0, int c_lo, int c_hi,
+                                              int warp4, int lane, const float* rstd_s) {
+    constexpr size_t STRIDE = 2 * BN * BM;                   // between two CTAs' first slots
+    const int n = n0 + 4 * lane;
+    const float* part = base + 4 * lane;
+    const float* first = part + first_which * (BN * BM);
+    if (!p.vec || n0 + BM > p.N) {                           // uniform over the CTA
+        for (int c = c_lo + warp4; c < c_hi; c += 4) {
+            const float scale = p.row_ssq ? rstd_s[c] : 1.f;
+            float sq = 0.f, gate = 0.f;
+#pragma unroll 1
+            for (int e = 0; e < 4; ++e) {
+                if (n + e >= p.N) break;
+                float v = shared_sum(part + c * BM + e, STRIDE, first + c * BM + e, n_ctas) * scale;
+                if (p.bias) v += gb_load(p.bias, p.bias_dtype, n + e);
+                if (p.swiglu) {                              // N is a multiple of 128
+                    if (e & 1) shared_gated(p.out, p.out_dtype, size_t(t0 + c) * p.ldo + ((n + e) >> 1), min(1, p.N_out - ((n + e) >> 1)), p.swiglu, gate, v, 0.f, 0.f);
+                    gate = v;
+                } else if (p.resid_x) {
+                    const size_t at = size_t(t0 + c) * p.ld_x + n + e;
+                    v = fmaf(p.resid_scale, v, __ldcg(p.resid_x + at));
+                    p.resid_x[at] = v;
+                    p.resid_xb[at] = __float2bfloat16_rn(v);
+                    sq = fmaf(v, v, sq);
+                } else {
+                    gb_store(p.out, p.out_dtype, size_t(t0 + c) * p.ldo + n + e, v);
+                }
+            }
+            if (p.resid_x) {
+                sq = gb_warp_sum(sq);
+                if (lane == 0) p.ssq_out[size_t(n0 / BM) * p.T + t0 + c] = sq;
+            }
+        }
+        return;
+    }
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.bias) bias = shared_bias(p.bias, p.bias_dtype, n);
+    for (int c0 = c_lo + warp4; c0 < c_hi; c0 += 4 * TOK) {
+        float4 v[TOK], x[TOK];
 #pragma unroll
-    for (int jj = 0; jj < 16; ++jj) v[jj] = 0.f;
+        for (int i = 0; i < TOK; ++i) {
+            const int c = c0 + 4 * i;
+            v[i] = x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (p.resid_x && c < c_hi) x[i] = __ldcg(reinterpret_cast<const float4*>(p.resid_x + size_t(t0 + c) * p.ld_x + n));
+        }
+        for (int s0 = 0; s0 < n_ctas; s0 += SUMS) {
+            float4 ld[TOK][SUMS];
 #pragma unroll
-    for (int j0 = 0; j0 < 16; j0 += C) {
-        if (c0 + j0 >= cols) break;
-        for (int s0 = 0; s0 < n_ctas; s0 += S) {
-            float ld[S][C];
+            for (int i = 0; i < TOK; ++i) {
+                const float* at = part + size_t(s0) * STRIDE + (c0 + 4 * i) * BM;
 #pragma unroll
-            for (int si = 0; si < S; ++si) {
-                const int s = s0 + si;
-                const float* part = base + (size_t(s) * 2 + (s == 0 ? first_which : 0)) * (BN * BM);
-#pragma unroll
-                for (int jj = 0; jj < C; ++jj)
-                    ld[si][jj] = (s < n_ctas && c0 + j0 + jj < cols) ? __ldcg(part + (c0 + j0 + jj) * BM) : 0.f;
+                for (int e = 0; e < SUMS; ++e) {
+                    const float* a = e == 0 && s0 == 0 ? first + (c0 + 4 * i) * BM : at + e * STRIDE;
+                    ld[i][e] = s0 + e < n_ctas && c0 + 4 * i < c_hi ? __ldcg(reinterpret_cast<const float4*>(a)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
             }
 #pragma unroll
-            for (int si = 0; si < S; ++si)
+            for (int i = 0; i < TOK; ++i)
 #pragma unroll
-                for (int jj = 0; jj < C; ++jj) v[j0 + jj] += ld[si][jj];
+                for (int e = 0; e < SUMS; ++e) { v[i].x += ld[i][e].x; v[i].y += ld[i][e].y; v[i].z += ld[i][e].z; v[i].w += ld[i][e].w; }
+        }
+#pragma unroll
+        for (int i = 0; i < TOK; ++i) {
+            const int c = c0 + 4 * i;
+            if (c >= c_hi) break;                            // uniform over the warp
+            const float scale = p.row_ssq ? rstd_s[c] : 1.f;
+            float4 r = make_float4(v[i].x * scale, v[i].y * scale, v[i].z * scale, v[i].w * scale);
+            if (p.swiglu) {
+                shared_gated(p.out, p.out_dtype, size_t(t0 + c) * p.ldo + (n >> 1), p.N_out - (n >> 1), p.swiglu, r.x, r.y, r.z, r.w);
+                continue;
+            }
+            r.x += bias.x; r.y += bias.y; r.z += bias.z; r.w += bias.w;
+            if (p.resid_x) {
+                const size_t at = size_t(t0 + c) * p.ld_x + n;
+                r = make_float4(fmaf(p.resid_scale, r.x, x[i].x), fmaf(p.resid_scale, r.y, x[i].y), fmaf(p.resid_scale, r.z, x[i].z),
+                                fmaf(p.resid_scale, r.w, x[i].w));
+                *reinterpret_cast<float4*>(p.resid_x + at) = r;
+                *reinterpret_cast<uint2*>(p.resid_xb + at) = gb_pack4(r);
+                const float sq = gb_warp_sum(r.x * r.x + r.y * r.y + (r.z * r.z + r.w * r.w));
+                if (lane == 0) p.ssq_out[size_t(n0 / BM) * p.T + t0 + c] = sq;
+            } else {
+                const size_t at = size_t(t0 + c) * p.ldo + n;
+                if (p.out_dtype == GB_F32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at) = r;
+                else *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + at) = gb_pack4(r);
+            }
         }
     }
 }
@@ -83,7 +167,7 @@ __device__ __forceinline__ void sum_partials(const float* base, int first_which,
 // Time stamps (builds with -DGB_STAMPS): slots of a CTA of the one product whose N and K were asked for.
 // 0 entry, 1 the wait for the kernel in front is over, 2 the first operands are there, 3 the last MMA is committed,
 // 4 the accumulator is seen complete, 5 partial sums stored and fenced, 6 counted (and the tile's other CTAs seen),
-// 7 the sharers' sums of the first 16 tokens are there, 8 the tile (or this CTA's share) is finished, 9 exit.
+// 8 the tile (or this CTA's share) is finished, 9 exit.
 #ifdef GB_STAMPS
 __device__ long long* g_stamps = nullptr;
 __device__ int g_stamps_n = 0, g_stamps_k = 0;
@@ -219,13 +303,13 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
             const int cols = min(BN, p.T - w.t0);       // valid tokens of this tile
             const bool whole = w.kb_begin == 0 && w.kb_end == kb_total;
             // What the kernel before left for this tile is fetched while the products still run: the sums of
-            // squares behind the tokens' scales and, in the 16-token kernel, this thread's row of the residual
+            // squares behind the tokens' scales and, for a tile of its own of 16 tokens, this thread's row of the residual
             // stream (each a trip to L2 that the kernel after this one would otherwise wait for).
             float bias = 0.f;
             if (p.bias && n < p.N) bias = gb_load(p.bias, p.bias_dtype, n);
             if (p.row_ssq) tc_token_scales<BN>(p, w.t0, cols, row, rstd_s, part_s);
             float x_early[16];
-            if (BN == 16 && p.resid_x) {
+            if (BN == 16 && p.resid_x && whole) {
 #pragma unroll
                 for (int c = 0; c < 16; ++c)
                     x_early[c] = (n < p.N && c < cols) ? __ldcg(p.resid_x + size_t(w.t0 + c) * p.ld_x + n) : 0.f;
@@ -308,39 +392,20 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
                     finish = last_flag != 0;
                 }
             }
-            if (finish) {
-                for (int c0 = c_lo & ~15; c0 < c_hi; c0 += 16) {
-                    float v[16], xv[16];
-                    bool have_x = false;
-                    if (whole) {
-                        tmem_ld16(taddr + c0, v);
-                    } else {
-                        // the last CTA of a shared tile: its rows of the residual stream are asked for with the
-                        // partial sums, not after them (one trip to L2 instead of two for every 16 tokens; tiles of 16
-                        // tokens have them already, and with tiles of 32 it measured slower: 5.17 against 5.07 ms
-                        // a step at 64 tokens, where tiles of 64 gain 0.05 of 5.9 ms at 128 tokens)
-                        if (BN >= 64 && p.resid_x) {
-#pragma unroll
-                            for (int jj = 0; jj < 16; ++jj)
-                                xv[jj] = (n < p.N && c0 + jj >= c_lo && c0 + jj < c_hi)
-                                             ? __ldcg(p.resid_x + size_t(w.t0 + c0 + jj) * p.ld_x + n) : 0.f;
-                            have_x = true;
-                        }
-                        const float* base = p.scratch + size_t(first_cta) * 2 * (BN * BM) + row;
-                        if (n_ctas <= 4) sum_partials<BN, 4, 16>(base, first_which, n_ctas, c0, c_hi, v);
-                        else sum_partials<BN, 8, 8>(base, first_which, n_ctas, c0, c_hi, v);
-                        STAMP_AFTER_IF(threadIdx.x == 64 && c0 == (c_lo & ~15), 7, v[0] + v[7]);
-                    }
-                    if constexpr (BN == 16)
-                        tc_finish_chunk<BN>(p, w.n0, w.t0, n, row, lane, quarter, bias, true, c0, c_hi, v, rstd_s, ssq_s,
-                                            p.resid_x ? x_early : nullptr, c_lo);
-                    else
-                        tc_finish_chunk<BN>(p, w.n0, w.t0, n, row, lane, quarter, bias, true, c0, c_hi, v, rstd_s, ssq_s,
-                                            have_x ? xv : nullptr, c_lo);
+            if (finish && whole) {
+                for (int c0 = 0; c0 < cols; c0 += 16) {
+                    float v[16];
+                    tmem_ld16(taddr + c0, v);
+                    tc_finish_chunk<BN>(p, w.n0, w.t0, n, row, lane, quarter, bias, true, c0, cols, v, rstd_s, ssq_s,
+                                        BN == 16 && p.resid_x ? x_early : nullptr);
                 }
-                if (p.resid_x) tc_write_ssq<BN>(p, w.n0, w.t0, row, c_lo, c_hi, ssq_s);
+                if (p.resid_x) tc_write_ssq<BN>(p, w.n0, w.t0, row, 0, cols, ssq_s);
                 STAMP_IF(threadIdx.x == 64, 8);
-                if (!whole && !sliced && threadIdx.x == 64) p.counters[w.tile] = 0;       // ready for the next launch
+            } else if (finish) {
+                finish_shared<BN, 2, 8>(p, p.scratch + size_t(first_cta) * 2 * (BN * BM), first_which, n_ctas, w.n0, w.t0, c_lo, c_hi,
+                                                    warp - 2, lane, rstd_s);
+                STAMP_IF(threadIdx.x == 64, 8);
+                if (!sliced && threadIdx.x == 64) p.counters[w.tile] = 0;       // ready for the next launch
             }
             if (sliced) {
                 // the last of the tile's CTAs to have read the others' sums puts the counter back for the next launch
@@ -629,6 +694,8 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
     p.ldo = ldo; p.out_dtype = out_dtype; p.bias_dtype = bias_dtype; p.T = T; p.N = N; p.K = K;
     p.swiglu = swiglu_features > 0 ? gate_act : 0; p.N_out = swiglu_features; p.sms = sms;
     cut.fill(p);
+    p.vec = resid_x ? gb_aligned(resid_x, 16) && gb_aligned(resid_xb, 8) && ld_x % 4 == 0 : gb_aligned(out, 16) && ldo % 4 == 0;
+    p.vec = p.vec && gb_aligned(scratch, 16);
     p.row_ssq = row_ssq; p.ssq_parts = ssq_parts; p.norm_size = norm_size; p.eps = eps;
     p.resid_x = resid_x; p.resid_xb = (__nv_bfloat16*)resid_xb; p.ssq_out = ssq_out; p.ld_x = ld_x; p.resid_scale = resid_scale;
     CUtensorMap mw, mx;
@@ -799,6 +866,7 @@ GB_API int gb_gemm_tc_noalloc(const void* X, long long ldx, const void* W, long 
     p.ldo = ldo; p.out_dtype = out_dtype; p.bias_dtype = bias_dtype; p.T = T; p.N = N; p.K = K;
     p.swiglu = 0; p.N_out = 0; p.sms = d->sms;
     cut.fill(p);
+    p.vec = gb_aligned(out, 16) && ldo % 4 == 0;
     p.row_ssq = nullptr; p.ssq_parts = 0; p.norm_size = 0; p.eps = 0.f;
     p.resid_x = nullptr; p.resid_xb = nullptr; p.ssq_out = nullptr; p.ld_x = 0; p.resid_scale = 1.f;
     CUtensorMap mw, mx;

@@ -59,6 +59,7 @@ struct TcParams {
     // T is the sum of all rows.  The tile whose first token is t multiplies by the features of problem t / group_t.
     // 0: one product.
     int group_t = 0;
+    bool vec = false;     // scratch memory and the rows that the epilogue of a shared tile reads and writes take accesses of four values
     int pair_tile = 256;  // tokens of a tile of the kernel that pairs two SMs (gemm_tc_pair_tile)
 };
 
