@@ -137,6 +137,9 @@ __device__ __forceinline__ float gb_gate_act(float z, int act) {
     return z / (1.f + expf(-z));
 }
 
+// Dynamic tanh of one value: tanh(alpha v) * w + b, the last two in one rounding, so that every kernel gives the same bits.
+__device__ __forceinline__ float gb_dyt(float v, float alpha, float w, float b) { return fmaf(tanhf(alpha * v), w, b); }
+
 // An expert's gated unit.  limit > 0: with clamped inputs, g <- min(g, limit), u <- clamp(u, -limit, limit),
 // g sigmoid(1.702 g) (u + 1).  limit 0: the plain unit g sigmoid(g) u.
 __device__ __forceinline__ float gb_act_glu(float g, float u, float limit) {

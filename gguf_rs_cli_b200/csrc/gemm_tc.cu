@@ -74,7 +74,7 @@ __device__ __noinline__ float shared_sum(const float* part, size_t stride, const
 // asked for at once, and the sum of squares needs no other warp.  (A feature a thread, 16 tokens each, took a trip to L2 for every
 // 8 tokens: 5 us behind the last CTA's arrival at 64 tokens.)
 // base: the first CTA's first slot.
-template <int BN, int TOK, int SUMS>
+template <int BN, int TOK, int SUMS, bool DYT>
 __device__ __forceinline__ void finish_shared(const TcParams& p, const float* base, int first_which, int n_ctas, int n0, int t0, int c_lo, int c_hi,
                                               int warp4, int lane, const float* rstd_s) {
     constexpr size_t STRIDE = 2 * BN * BM;                   // between two CTAs' first slots
@@ -97,13 +97,13 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
                     const size_t at = size_t(t0 + c) * p.ld_x + n + e;
                     v = fmaf(p.resid_scale, v, __ldcg(p.resid_x + at));
                     p.resid_x[at] = v;
-                    p.resid_xb[at] = __float2bfloat16_rn(v);
+                    p.resid_xb[at] = __float2bfloat16_rn(DYT ? gb_dyt(v, p.dyt_alpha, gb_load(p.dyt_w, p.dyt_dtype, n + e), gb_load(p.dyt_b, p.dyt_dtype, n + e)) : v);
                     sq = fmaf(v, v, sq);
                 } else {
                     gb_store(p.out, p.out_dtype, size_t(t0 + c) * p.ldo + n + e, v);
                 }
             }
-            if (p.resid_x) {
+            if (p.resid_x && !DYT) {
                 sq = gb_warp_sum(sq);
                 if (lane == 0) p.ssq_out[size_t(n0 / BM) * p.T + t0 + c] = sq;
             }
@@ -112,6 +112,11 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
     }
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.bias) bias = shared_bias(p.bias, p.bias_dtype, n);
+    float4 dyt_w = bias, dyt_b = bias;
+    if (DYT) {
+        dyt_w = shared_bias(p.dyt_w, p.dyt_dtype, n);
+        dyt_b = shared_bias(p.dyt_b, p.dyt_dtype, n);
+    }
     for (int c0 = c_lo + warp4; c0 < c_hi; c0 += 4 * TOK) {
         float4 v[TOK], x[TOK];
 #pragma unroll
@@ -152,6 +157,12 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
                 r = make_float4(fmaf(p.resid_scale, r.x, x[i].x), fmaf(p.resid_scale, r.y, x[i].y), fmaf(p.resid_scale, r.z, x[i].z),
                                 fmaf(p.resid_scale, r.w, x[i].w));
                 *reinterpret_cast<float4*>(p.resid_x + at) = r;
+                if (DYT) {
+                    *reinterpret_cast<uint2*>(p.resid_xb + at) =
+                        gb_pack4(make_float4(gb_dyt(r.x, p.dyt_alpha, dyt_w.x, dyt_b.x), gb_dyt(r.y, p.dyt_alpha, dyt_w.y, dyt_b.y),
+                                             gb_dyt(r.z, p.dyt_alpha, dyt_w.z, dyt_b.z), gb_dyt(r.w, p.dyt_alpha, dyt_w.w, dyt_b.w)));
+                    continue;
+                }
                 *reinterpret_cast<uint2*>(p.resid_xb + at) = gb_pack4(r);
                 const float sq = gb_warp_sum(r.x * r.x + r.y * r.y + (r.z * r.z + r.w * r.w));
                 if (lane == 0) p.ssq_out[size_t(n0 / BM) * p.T + t0 + c] = sq;
@@ -184,7 +195,8 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     return v;
 }
 
-template <int BN>
+// DYT: the residual epilogue is followed by a dynamic tanh (a kernel of its own: the branch and its code would cost the others).
+template <int BN, bool DYT>
 __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                 const __grid_constant__ CUtensorMap map_x, TcParams p) {
     using Cfg = TileCfg<BN>;
@@ -396,13 +408,13 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
                 for (int c0 = 0; c0 < cols; c0 += 16) {
                     float v[16];
                     tmem_ld16(taddr + c0, v);
-                    tc_finish_chunk<BN>(p, w.n0, w.t0, n, row, lane, quarter, bias, true, c0, cols, v, rstd_s, ssq_s,
+                    tc_finish_chunk<BN, DYT>(p, w.n0, w.t0, n, row, lane, quarter, bias, true, c0, cols, v, rstd_s, ssq_s,
                                         BN == 16 && p.resid_x ? x_early : nullptr);
                 }
-                if (p.resid_x) tc_write_ssq<BN>(p, w.n0, w.t0, row, 0, cols, ssq_s);
+                if (p.resid_x && !DYT) tc_write_ssq<BN>(p, w.n0, w.t0, row, 0, cols, ssq_s);
                 STAMP_IF(threadIdx.x == 64, 8);
             } else if (finish) {
-                finish_shared<BN, 2, 8>(p, p.scratch + size_t(first_cta) * 2 * (BN * BM), first_which, n_ctas, w.n0, w.t0, c_lo, c_hi,
+                finish_shared<BN, 2, 8, DYT>(p, p.scratch + size_t(first_cta) * 2 * (BN * BM), first_which, n_ctas, w.n0, w.t0, c_lo, c_hi,
                                                     warp - 2, lane, rstd_s);
                 STAMP_IF(threadIdx.x == 64, 8);
                 if (!sliced && threadIdx.x == 64) p.counters[w.tile] = 0;       // ready for the next launch
@@ -498,7 +510,7 @@ int ensure_status() {
 
 constexpr int MAX_DEVICES = 64;
 
-template <int BN>
+template <int BN, bool DYT = false>
 int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, cudaStream_t stream, bool pdl = true) {
     using Cfg = TileCfg<BN>;
     // the shared-memory limit is an attribute of the function on each device; the first launch of a tile width
@@ -507,11 +519,11 @@ int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, c
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return gb_fail("gb_gemm_tc: no usable current device");
     if (!configured[dev]) {
-        if (cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemm_tc_kernel<BN, DYT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
             return gb_fail("gb_gemm_tc: cannot get %d bytes of shared memory", Cfg::SMEM);
         configured[dev] = true;
     }
-    gb_launch_opt(gemm_tc_kernel<BN>, dim3(p.n_ctas), dim3(TC_THREADS), Cfg::SMEM, stream, pdl, mw, mx, p);
+    gb_launch_opt(gemm_tc_kernel<BN, DYT>, dim3(p.n_ctas), dim3(TC_THREADS), Cfg::SMEM, stream, pdl, mw, mx, p);
     GB_LAUNCH_OK("gb_gemm_tc");
     return 0;
 }
@@ -641,16 +653,18 @@ GB_API int gb_gemm_tc_supported(const void* X, long long ldx, const void* W, lon
 // rows pad the last tile), F = swiglu_features, and
 // out[t,f] = act(gate_f) * up_f has F columns (src/model/llama.rs:399-401 in the product's epilogue); act is
 // SiLU, or what gate_act names (GbGateAct) in gb_gemm_tc_fused.
+struct TcDyt { const void* w; const void* b; int dtype; float alpha; };
 static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long ldw, const void* bias, int bias_dtype,
                         void* out, int out_dtype, long long ldo, int T, int N, int K, float* scratch, int* counters,
                         int n_counters, int sms, int swiglu_features, int gate_act, const float* row_ssq, int ssq_parts, int norm_size,
-                        float eps, float* resid_x, void* resid_xb, float* ssq_out, long long ld_x, float resid_scale, cudaStream_t stream);
+                        float eps, float* resid_x, void* resid_xb, float* ssq_out, long long ld_x, float resid_scale, const TcDyt* dyt,
+                        cudaStream_t stream);
 
 GB_API int gb_gemm_tc(const void* X, long long ldx, const void* W, long long ldw, const void* bias, int bias_dtype,
                       void* out, int out_dtype, long long ldo, int T, int N, int K, float* scratch, int* counters,
                       int n_counters, int sms, int swiglu_features, cudaStream_t stream) {
     return gemm_tc_impl(X, ldx, W, ldw, bias, bias_dtype, out, out_dtype, ldo, T, N, K, scratch, counters, n_counters, sms,
-                        swiglu_features, GB_ACT_SILU, nullptr, 0, 0, 0.f, nullptr, nullptr, nullptr, 0, 1.f, stream);
+                        swiglu_features, GB_ACT_SILU, nullptr, 0, 0, 0.f, nullptr, nullptr, nullptr, 0, 1.f, nullptr, stream);
 }
 
 // The same product with a deferred RMS norm on its input and/or a residual epilogue:
@@ -668,13 +682,26 @@ GB_API int gb_gemm_tc_fused(const void* X, long long ldx, const void* W, long lo
     GB_REQUIRE(!resid_x || (resid_xb && ssq_out && ld_x >= N && !swiglu_features), "gb_gemm_tc_fused: bad residual parameters");
     GB_REQUIRE(!swiglu_features || gate_act == GB_ACT_SILU || gate_act == GB_ACT_GELU_TANH, "gb_gemm_tc_fused: unknown gate activation %d", gate_act);
     return gemm_tc_impl(X, ldx, W, ldw, bias, bias_dtype, out, out_dtype, ldo, T, N, K, scratch, counters, n_counters, sms,
-                        swiglu_features, gate_act, row_ssq, ssq_parts, norm_size, eps, resid_x, resid_xb, ssq_out, ld_x, resid_scale, stream);
+                        swiglu_features, gate_act, row_ssq, ssq_parts, norm_size, eps, resid_x, resid_xb, ssq_out, ld_x, resid_scale, nullptr, stream);
+}
+
+// The residual epilogue in front of a dynamic tanh: x += resid_scale * (result + bias) in place, and `rows` (bf16, the pitch of x) gets
+// tanh(alpha x) * w + b, what the sublayer behind it reads.  For steps that one CTA a tile takes (up to 128 tokens).
+GB_API int gb_gemm_tc_dyt(const void* X, long long ldx, const void* W, long long ldw, const void* bias, int bias_dtype, int T, int N, int K,
+                          float* scratch, int* counters, int n_counters, int sms, float* resid_x, void* rows, long long ld_x, float resid_scale,
+                          const void* dyt_w, const void* dyt_b, int dyt_dtype, float alpha, cudaStream_t stream) {
+    GB_REQUIRE(resid_x && rows && ld_x >= N && dyt_w && dyt_b && gb_is_dtype(dyt_dtype), "gb_gemm_tc_dyt: bad residual or tanh parameters");
+    GB_REQUIRE(T <= 128, "gb_gemm_tc_dyt: T=%d is more than 128", T);
+    const TcDyt dyt{dyt_w, dyt_b, dyt_dtype, alpha};
+    return gemm_tc_impl(X, ldx, W, ldw, bias, bias_dtype, nullptr, GB_BF16, 0, T, N, K, scratch, counters, n_counters, sms, 0, GB_ACT_SILU, nullptr,
+                        0, 0, 0.f, resid_x, rows, nullptr, ld_x, resid_scale, &dyt, stream);
 }
 
 static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long ldw, const void* bias, int bias_dtype,
                         void* out, int out_dtype, long long ldo, int T, int N, int K, float* scratch, int* counters,
                         int n_counters, int sms, int swiglu_features, int gate_act, const float* row_ssq, int ssq_parts, int norm_size,
-                        float eps, float* resid_x, void* resid_xb, float* ssq_out, long long ld_x, float resid_scale, cudaStream_t stream) {
+                        float eps, float* resid_x, void* resid_xb, float* ssq_out, long long ld_x, float resid_scale, const TcDyt* dyt,
+                        cudaStream_t stream) {
     GB_REQUIRE(gb_is_dtype(out_dtype) && (!bias || gb_is_dtype(bias_dtype)), "gb_gemm_tc: bad dtype");
     GB_REQUIRE(T >= 0 && N > 0 && K > 0, "gb_gemm_tc: bad sizes T=%d N=%d K=%d", T, N, K);
     GB_REQUIRE(swiglu_features >= 0 && (resid_x || ldo >= (swiglu_features ? swiglu_features : N)), "gb_gemm_tc: output pitch %lld too small", ldo);
@@ -700,6 +727,17 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
     p.resid_x = resid_x; p.resid_xb = (__nv_bfloat16*)resid_xb; p.ssq_out = ssq_out; p.ld_x = ld_x; p.resid_scale = resid_scale;
     CUtensorMap mw, mx;
     if (tensor_map_2d(W, N, K, ldw, BM, &mw)) return 1;
+    if (dyt) {
+        p.dyt_w = dyt->w; p.dyt_b = dyt->b; p.dyt_dtype = dyt->dtype; p.dyt_alpha = dyt->alpha;
+        if (tensor_map_2d(X, T, K, ldx, bn, &mx)) return 1;
+        switch (bn) {
+            case 16: return launch_tc<16, true>(mw, mx, p, stream);
+            case 32: return launch_tc<32, true>(mw, mx, p, stream);
+            case 64: return launch_tc<64, true>(mw, mx, p, stream);
+            case 128: return launch_tc<128, true>(mw, mx, p, stream);
+            default: return launch_tc<256, true>(mw, mx, p, stream);
+        }
+    }
     if (bn == 256 && g_pair && cut.cut == CUT_WHOLE) {
         // more than 128 tokens: two SMs per tile of 256 features, each loading half of the tile's tokens of X per stage; bf16 results leave
         // through shared memory and TMA stores of [16 tokens x 128 features] (64 features after SwiGLU)

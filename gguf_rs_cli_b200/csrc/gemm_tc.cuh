@@ -59,6 +59,11 @@ struct TcParams {
     // T is the sum of all rows.  The tile whose first token is t multiplies by the features of problem t / group_t.
     // 0: one product.
     int group_t = 0;
+    // dynamic tanh behind the residual update: resid_xb gets tanh(dyt_alpha x) * dyt_w + dyt_b, no sums of squares (kernels of their own)
+    const void* dyt_w = nullptr;
+    const void* dyt_b = nullptr;
+    int dyt_dtype = 0;
+    float dyt_alpha = 0.f;
     bool vec = false;     // scratch memory and the rows that the epilogue of a shared tile reads and writes take accesses of four values
     int pair_tile = 256;  // tokens of a tile of the kernel that pairs two SMs (gemm_tc_pair_tile)
 };
@@ -214,7 +219,7 @@ __device__ __forceinline__ float tc_warp_sum16(const float (&v)[16], int lane) {
 // The last steps for 16 columns (tokens c0 .. c0+15 of the tile, those from c_lo on and below c_end being the
 // caller's to finish) of this thread's feature row n = n0 + row: v[jj] holds the finished sum of column c0 + jj.
 // x_early: the 16 values of the residual stream at these places if the caller has read them already, else null.
-template <int BN>
+template <int BN, bool DYT = false>
 __device__ __forceinline__ void tc_finish_chunk(const TcParams& p, int n0, int t0, int n, int row, int lane, int quarter,
                                                 float bias, bool waited, int c0, int c_end, float (&v)[16],
                                                 const float* rstd_s, float (*ssq_s)[BN], const float* x_early = nullptr,
@@ -232,6 +237,8 @@ __device__ __forceinline__ void tc_finish_chunk(const TcParams& p, int n0, int t
         for (int jj = 0; jj < 16; ++jj)
             xv[jj] = x_early ? x_early[jj]
                              : (n < p.N && mine(c0 + jj)) ? __ldcg(p.resid_x + size_t(t0 + c0 + jj) * p.ld_x + n) : 0.f;
+        float dyt_w = 0.f, dyt_b = 0.f;
+        if (DYT && n < p.N) { dyt_w = gb_load(p.dyt_w, p.dyt_dtype, n); dyt_b = gb_load(p.dyt_b, p.dyt_dtype, n); }
 #pragma unroll
         for (int jj = 0; jj < 16; ++jj) {
             float sq = 0.f;
@@ -239,11 +246,12 @@ __device__ __forceinline__ void tc_finish_chunk(const TcParams& p, int n0, int t
                 const size_t at = size_t(t0 + c0 + jj) * p.ld_x + n;
                 const float xn = fmaf(p.resid_scale, v[jj] + bias, xv[jj]);
                 p.resid_x[at] = xn;
-                p.resid_xb[at] = __float2bfloat16_rn(xn);
+                p.resid_xb[at] = __float2bfloat16_rn(DYT ? gb_dyt(xn, p.dyt_alpha, dyt_w, dyt_b) : xn);
                 sq = xn * xn;
             }
             v[jj] = sq;
         }
+        if (DYT) return;
         const float sq = tc_warp_sum16(v, lane);
         const int jj = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
         if ((lane & 1) == 0 && mine(c0 + jj)) ssq_s[quarter][c0 + jj] = sq;

@@ -19,7 +19,7 @@ __global__ void add_dyt_kernel(float* __restrict__ x, const void* __restrict__ d
         float v = xr[i];
         for (int d = 0; d < n_delta; ++d) v += gb_load(delta, delta_dtype, d * delta_stride + size_t(s) * E + i);
         if (write_x && n_delta) xr[i] = v;
-        gb_store(out, out_dtype, size_t(r) * E + i, tanhf(alpha * v) * gb_load(w, w_dtype, i) + gb_load(b, w_dtype, i));
+        gb_store(out, out_dtype, size_t(r) * E + i, gb_dyt(v, alpha, gb_load(w, w_dtype, i), gb_load(b, w_dtype, i)));
     }
 }
 

@@ -1136,6 +1136,25 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out:
     return out
 
 
+def gemm_tc_dyt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], resid_x: torch.Tensor, rows: torch.Tensor, weight: torch.Tensor,
+                dyt_bias: torch.Tensor, alpha: float, resid_scale: float = 1.0) -> torch.Tensor:
+    """resid_x += resid_scale * (x w^T + bias) in place (f32 [T, N]) and rows [T, N] (bfloat16) = tanh(alpha resid_x) * weight + dyt_bias: a
+    residual product and the dynamic tanh behind it, for up to 128 tokens."""
+    _cuda(x, w, bias, resid_x, rows, weight, dyt_bias)
+    T, K = x.shape
+    N = w.shape[0]
+    assert w.shape[1] == K and x.dtype == w.dtype == rows.dtype == torch.bfloat16 and resid_x.dtype == torch.float32
+    assert resid_x.shape == rows.shape == (T, N) and resid_x.stride(1) == rows.stride(1) == 1 and resid_x.stride(0) == rows.stride(0)
+    assert weight.numel() == dyt_bias.numel() == N and weight.dtype == dyt_bias.dtype and weight.is_contiguous() and dyt_bias.is_contiguous()
+    sc = tc_scratch(x.device)
+    need = native.library().gb_gemm_tc_scratch_floats(T, N, K, sc.sms)
+    share = need and sc.fits(need)
+    call("gb_gemm_tc_dyt", ptr(x), x.stride(0), ptr(w), w.stride(0), ptr(bias), 0 if bias is None else dtype_code(bias), T, N, K,
+         ptr(sc.floats) if share else None, ptr(sc.counters) if share else None, sc.counters.numel() if share else 0, sc.sms, ptr(resid_x),
+         ptr(rows), resid_x.stride(0), float(resid_scale), ptr(weight), ptr(dyt_bias), dtype_code(weight), float(alpha), stream_ptr())
+    return rows
+
+
 def gemm_f32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
     if x.dtype != torch.float32 or w.dtype != torch.float32 or x.stride(1) != 1 or w.stride(1) != 1:
         return False

@@ -188,6 +188,9 @@ class Stream:
         # The norm that the next run's block applies first (set by the decoder before every run; None behind the last),
         # and, when a block's last kernel has already applied it, (that norm, its rows): valid while x is unchanged.
         self.next_norm = None
+        # The norm that reads x after the sublayer that runs now, if its block tells: a product that adds the sublayer's term to x
+        # may apply it in the same pass (`normed`).
+        self.after = None
         self.normed: Optional[Tuple[object, torch.Tensor]] = None
 
     def drop_shadow(self) -> None:

@@ -52,11 +52,12 @@ class PreNormBlock:
         try:
             self._forward(stream, ctx, run)
         finally:
-            stream.term_scale = 1.0
+            stream.term_scale, stream.after = 1.0, None
 
     def _forward(self, stream: Stream, ctx: StepContext, run: RunView) -> None:
         h = self._norm("mixer", stream, ctx)
         ctx.mark("norm")
+        stream.after = stream.next_norm if self.feed_forward is None else self.norms["feed_forward"]
         if getattr(self.mixer, "accepts_residual", False):
             term = self.mixer.forward(h, ctx, run, residual=stream)
         else:
@@ -66,6 +67,7 @@ class PreNormBlock:
             return
         h = self._norm("feed_forward", stream, ctx)
         ctx.mark("ff_norm")
+        stream.after = stream.next_norm
         if getattr(self.feed_forward, "accepts_residual", False):
             term = self.feed_forward.forward(h, ctx, residual=stream)
         elif self.unsummed:
@@ -75,13 +77,14 @@ class PreNormBlock:
         self._add(stream, term)
 
     def _norm(self, name: str, stream: Stream, ctx: StepContext):
-        if self.absorbed[name]:
-            return self.norms[name].apply(stream, ctx, absorbed=True)
-        return self.norms[name].apply(stream, ctx)
+        h = self.norms[name].apply(stream, ctx, absorbed=True) if self.absorbed[name] else self.norms[name].apply(stream, ctx)
+        stream.normed = None
+        return h
 
     def _add(self, stream: Stream, term) -> None:
         """A part that has added its term to the stream itself returns None."""
         if term is not None:
+            stream.normed = None
             stream.pending, stream.pending_scale = term, self.scale
             stream.drop_shadow()
 

@@ -33,7 +33,8 @@ class Linear:
                  residual: Optional[Stream] = None, activation: Optional[str] = None) -> Optional[torch.Tensor]:
         """x: rows [T, in], or a DeferredNorm (then the product applies the norm's scale).  With
         `residual`, and where the tensor-core product can do it, the result is added to the stream in
-        the product's epilogue (x += the stream's term_scale times the result, shadow left for the next norm) and None is returned.  activation
+        the product's epilogue (x += the stream's term_scale times the result, shadow left for the next norm, or that norm's rows
+        where it is a dynamic tanh) and None is returned.  activation
         (kernels.UNARY_ACTS): applied to every result by a kernel behind the product (in the tensor-core product's
         epilogue the branch cost every model's decode step 4.5%: 3.28 against 3.13 ms on the Llama-3.1-8B shape)."""
         T = x.shape[0]
@@ -42,6 +43,14 @@ class Linear:
         if residual is not None and T <= FUSE_MAX_TOKENS and self.tensor_core() \
                 and kernels.gemm_tc_supported(rows, self.weight) and residual.x.shape == (T, self.out_features):
             xb = ctx.ws.get("stream.xb", residual.x.shape, torch.bfloat16)
+            epilogue = getattr(residual.after, "product_epilogue", None)
+            if epilogue is not None and not norm:
+                # the norm behind this term needs nothing but x: its rows instead of the bfloat16 copy of x
+                kernels.gemm_tc_dyt(rows, self.weight, self.bias, residual.x, xb, *epilogue(), resid_scale=residual.term_scale)
+                residual.pending, residual.normed = None, (residual.after, xb)
+                residual.drop_shadow()
+                return None
+            residual.normed = None
             parts = (self.out_features + 127) // 128
             ssq = ctx.ws.get("stream.ssq", (parts, T), torch.float32)
             kernels.gemm_tc(rows, self.weight, self.bias, None, resid_x=residual.x, resid_xb=xb, ssq_out=ssq,

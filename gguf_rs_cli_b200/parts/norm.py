@@ -151,10 +151,19 @@ class DynamicTanh(Part):
 
     graph_class = ()
 
+    def product_epilogue(self) -> tuple:
+        """(weight, bias, alpha): what a residual product needs to apply this norm to the x that it writes."""
+        return self.weight, self.bias, self.alpha
+
     def apply(self, stream: Stream, ctx: StepContext, rows: Optional[torch.Tensor] = None, buffer: str = "normed",
               absorbed: bool = False):
         """Adds the stream's pending term into x (32-bit) and returns tanh(alpha x) * weight + bias of all rows,
-        or of `rows` only (x is then left as it is)."""
+        or of `rows` only (x is then left as it is).  Where the product in front has applied this norm already (`Stream.normed`), its rows."""
+        if rows is None and stream.normed is not None and stream.normed[0] is self and stream.pending is None and not stream.more:
+            h, stream.normed = stream.normed[1], None
+            return h
+        if rows is None:
+            stream.normed = None
         if stream.more or stream.pending_scale != 1.0 or isinstance(stream.pending, RoutedRows):
             raise RuntimeError("dyt: this norm adds one pending term only, as it is")
         n = stream.x.shape[0] if rows is None else rows.numel()
