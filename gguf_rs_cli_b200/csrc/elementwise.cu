@@ -382,6 +382,39 @@ GB_API int gb_swiglu(const void* gu, long long ld, void* out, int T, int F, int 
     return 0;
 }
 
+// ------------------------------------------------------- from one step to the next
+// Behind the sampling of a captured step of single tokens: every sequence's token, position and length become the next step's,
+// and the sampled tokens go to the one of two host buffers (mapped, pinned) whose turn it is.  One launch at the end of the graph in the
+// place of three copies between two graphs (tokens to the host, index arrays to the device, tokens into them), each of which kept the
+// device idle for 8 to 10 us.
+__global__ void __launch_bounds__(256) step_tail_kernel(const int* __restrict__ out, const int* __restrict__ seq_of, int* __restrict__ tokens,
+                                                        int* __restrict__ pos, int* __restrict__ starts, int n, int* __restrict__ turn,
+                                                        int* host0, int* host1) {
+    gb_grid_launch_dependents();
+    gb_grid_wait();
+    const int now = *turn;
+    int* host = now ? host1 : host0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int t = out[i];
+        host[i] = t;
+        if (seq_of[i] >= 0) {                          // padding stays as it is
+            tokens[i] = t;
+            ++pos[i];
+            ++starts[i];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *turn = now ^ 1;
+}
+
+GB_API int gb_step_tail(const int* out, const int* seq_of, int* tokens, int* pos, int* starts, int n, int* turn, int* host0, int* host1,
+                        cudaStream_t stream) {
+    GB_REQUIRE(n > 0 && out && seq_of && tokens && pos && starts && turn && host0 && host1, "gb_step_tail: bad arguments");
+    gb_launch(step_tail_kernel, dim3(1), dim3(256), 0, stream, out, seq_of, tokens, pos, starts, n, turn, host0, host1);
+    GB_LAUNCH_OK("gb_step_tail");
+    return 0;
+}
+
 // ------------------------------------------------------------- per-slot state
 // Zeroes one slot's row in every region of a byte arena: region r starts at table[2r] and holds rows of
 // table[2r+1] bytes (a multiple of 4), one per slot.  blockIdx.x is the region; its row is shared out over gridDim.y blocks.

@@ -9,6 +9,7 @@ import sys
 import numpy as np
 import torch
 
+from .. import kernels
 from ..cache.pool import PAGE, CacheFull, pages_for
 from ..parts.base import HostBatch
 from ..sampling.params import SamplingParams
@@ -19,7 +20,8 @@ from .step import Engine, Entry, StepError
 class DecodeGraph:
     """One captured decode step (model + sampling) for a padded batch size and one set of
     sampling options.  Its index arrays live in buffers of its own, so replaying it needs
-    one host-to-device copy and one graph launch."""
+    one host-to-device copy and one graph launch.  The step's last kernel moves the index arrays on by one token, feeds the
+    sampled tokens back and writes them to the host: while the same sequences go on, one step is one graph launch."""
 
     def __init__(self, engine: Engine, bucket: int):
         self.bucket = bucket
@@ -28,6 +30,10 @@ class DecodeGraph:
         self.keys_host = torch.zeros(bucket, dtype=torch.int64).pin_memory()
         self.keys_dev = torch.zeros(bucket, dtype=torch.int64, device=engine.device)
         self.out_dev = torch.zeros(bucket, dtype=torch.int32, device=engine.device)
+        # where a step's tokens go on the host: two steps may be in flight
+        self.out_hosts = [torch.zeros(bucket, dtype=torch.int32).pin_memory() for _ in range(2)]
+        self.turn_dev = torch.zeros(1, dtype=torch.int32, device=engine.device)
+        self.turn = 0
         self.graph = None
         self.warm = False
         self.launches = 0
@@ -122,15 +128,20 @@ class EngineBackend:
         self._batch = self._last_graph = None
         self.engine.close(slot)
 
-    def _pending(self, slots, keys, params, out_dev) -> Pending:
-        """Asks for the step's tokens on the host and marks the place in the stream where they are there."""
+    def _pending(self, slots, keys, params, out_dev, dg: Optional[DecodeGraph] = None) -> Pending:
+        """Marks the place in the stream where the step's tokens are on the host: the last kernel of a DecodeGraph's step writes
+        them there, others are copied."""
         i = self._turn
         self._turn = 1 - i
         n = len(slots)
-        self._out_hosts[i][:n].copy_(out_dev[:n], non_blocking=True)
+        if dg is not None:
+            host, dg.turn = dg.out_hosts[dg.turn], 1 - dg.turn
+        else:
+            host = self._out_hosts[i]
+            host[:n].copy_(out_dev[:n], non_blocking=True)
         self._events[i].record()
         self.d2h_bytes += 4 * n
-        return Pending(slots, keys, params, out_dev, self._out_hosts[i], self._events[i])
+        return Pending(slots, keys, params, out_dev, host, self._events[i])
 
     def _launch_decode_graph(self, slots, tokens, keys, params, after: Optional[Pending] = None) -> Optional[Pending]:
         """A step of single tokens through a captured graph: the first call of a batch size
@@ -161,10 +172,19 @@ class EngineBackend:
                 self._graphs.pop(next(iter(self._graphs)))
             dg = DecodeGraph(eng, key[0])
         self._graphs[key] = dg
+        same = (dg.graph is not None and self._last_graph is dg and dg.laid_out_for == slots_t and dg.keys == keys and dg.plan_words == 0)
+        if same and after is not None and after.out_dev is dg.out_dev and bool((lengths % PAGE).all()):
+            # the step in front has left everything in place for this one
+            self._check_room(longest)
+            dg.graph.replay()
+            native.count_launches(dg.launches)
+            for s in slots:
+                cache.lengths[s] += 1
+            self._batch = (slots_t, lengths + 1)
+            return self._pending(slots, keys, params, dg.out_dev, dg)
         if dg.copied is not None:
             dg.copied.synchronize()
-        if (dg.graph is not None and self._last_graph is dg and dg.laid_out_for == slots_t and dg.keys == keys
-                and dg.plan_words == 0):
+        if same:
             self._advance_in_place(dg, slots, tokens, lengths)
             self._feed_from(dg, after, n)
             dg.graph.replay()
@@ -189,6 +209,7 @@ class EngineBackend:
             def body():
                 logits = eng.model.forward(ctx, eng.runs, want_rows)
                 self.sampler.sample(logits, ctx.slots, dg.keys_dev, params, dg.out_dev)
+                kernels.step_tail(dg.out_dev, ctx.seq_of, ctx.tokens, ctx.pos, ctx.starts, dg.turn_dev, dg.out_hosts)
 
             if dg.graph is None and dg.warm:
                 before = native.launch_count()
@@ -204,7 +225,11 @@ class EngineBackend:
             h2d = ctx.host["h2d_bytes"] + 8 * dg.bucket
         self._batch, self._last_graph = (slots_t, lengths + 1), dg
         self.h2d_bytes += h2d
-        return self._pending(slots, keys, params, dg.out_dev)
+        return self._pending(slots, keys, params, dg.out_dev, dg)
+
+    def _check_room(self, longest: int) -> None:
+        if longest + 1 > self.engine.cache.max_len:
+            raise CacheFull(f"a sequence would exceed the longest sequence allowed ({self.engine.cache.max_len})")
 
     def _capture(self, body) -> "torch.cuda.CUDAGraph":
         """`body` captured on a stream of its own.  Not with torch.cuda.graph: that empties the caching allocator first, and
@@ -245,8 +270,7 @@ class EngineBackend:
         eng, cache, n = self.engine, self.engine.cache, len(slots)
         if tokens is not None and (tokens.min() < 0 or tokens.max() >= eng.vocab_size):
             raise StepError(f"a token id of {tokens.tolist()} is outside the vocabulary (0..{eng.vocab_size - 1})")
-        if int(lengths.max()) + 1 > cache.max_len:
-            raise CacheFull(f"a sequence would exceed the longest sequence allowed ({cache.max_len})")
+        self._check_room(int(lengths.max()))
         fresh = np.nonzero(lengths % PAGE == 0)[0]               # these enter a new page (where their group still grows)
         if fresh.size:
             cache.reserve([slots[b] for b in fresh], [1] * fresh.size)

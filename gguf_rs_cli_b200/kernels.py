@@ -1019,6 +1019,18 @@ def zero_rows(arena: torch.Tensor, table: torch.Tensor, slot: int) -> None:
     call("gb_zero_rows", ptr(arena), ptr(table), table.shape[0], int(slot), stream_ptr())
 
 
+def step_tail(out: torch.Tensor, seq_of: torch.Tensor, tokens: torch.Tensor, pos: torch.Tensor, starts: torch.Tensor, turn: torch.Tensor,
+              hosts) -> None:
+    """What follows the sampling of a step of single tokens: out[i] becomes tokens[i], pos[i] and starts[i] go up by one (where seq_of[i] is
+    not negative), and out goes to hosts[turn] (two pinned host buffers); turn changes.  All int32."""
+    n = seq_of.numel()
+    _cuda(out, seq_of, tokens, pos, starts, turn)
+    for t in (out, seq_of, tokens, pos, starts, turn, *hosts):
+        assert t.dtype == torch.int32 and t.is_contiguous()
+    assert all(h.is_pinned() and h.numel() >= n for h in hosts) and min(out.numel(), tokens.numel(), pos.numel(), starts.numel()) >= n
+    call("gb_step_tail", ptr(out), ptr(seq_of), ptr(tokens), ptr(pos), ptr(starts), n, ptr(turn), ptr(hosts[0]), ptr(hosts[1]), stream_ptr())
+
+
 def gemm_generic(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
     """out[t,n] = sum_k x[t,k] w[n,k] + bias[n], 32-bit FMAs on the CUDA cores."""
     _cuda(x, w, bias, out)
