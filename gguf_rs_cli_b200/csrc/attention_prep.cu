@@ -18,11 +18,14 @@ __global__ void qk_norm_kv_write_kernel(void* __restrict__ q, const void* __rest
                                         const int* __restrict__ pos, const int* __restrict__ table, int table_width,
                                         int ring_pages, void* __restrict__ kcache, void* __restrict__ vcache,
                                         int cache_dtype) {
+    gb_grid_launch_dependents();
+    gb_grid_wait();
     const int t = blockIdx.x;
     const int b = seq_of[t];
     if (b < 0) return;
     const int p = pos[t];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    // few tokens: a warp a head, the heads over several blocks (one block a token took 7.5 us for 4 tokens of 24 heads)
+    const int warp = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, warps = gridDim.y * (blockDim.x >> 5);
     const size_t row = size_t(t) * size_t(ld);
     const int* trow = table + size_t(b) * table_width;
     const float temp = coef != 0.f ? 1.f + coef * logf(float((p + 1) / every) + 1.f) : 1.f;
@@ -69,8 +72,11 @@ GB_API int gb_qk_norm_kv_write(void* q, const void* k, const void* v, int dtype,
     GB_REQUIRE((k == nullptr) == (v == nullptr), "gb_qk_norm_kv_write: k and v must both be given or both be null");
     GB_REQUIRE(!k || (table && kcache && vcache && ring_pages > 0 && table_width >= 1), "gb_qk_norm_kv_write: cache missing");
     if (T == 0) return 0;
-    qk_norm_kv_write_kernel<<<T, 128, 0, stream>>>(q, k, v, dtype, ld, H, G, D, Dv, normalise, eps, coef, every > 0 ? every : 1,
-                                                   seq_of, pos, table, table_width, ring_pages, kcache, vcache, cache_dtype);
+    const bool few = T <= GB_FEW_TOKENS;
+    const int slices = few ? ((k ? H + 2 * G : H) + 3) / 4 : 1;
+    GB_REQUIRE(slices <= 65535, "gb_qk_norm_kv_write: too many heads (%d)", H);
+    gb_launch_opt(qk_norm_kv_write_kernel, dim3(T, slices), dim3(128), 0, stream, few, q, k, v, dtype, ld, H, G, D, Dv, normalise, eps, coef,
+                  every > 0 ? every : 1, seq_of, pos, table, table_width, ring_pages, kcache, vcache, cache_dtype);
     GB_LAUNCH_OK("gb_qk_norm_kv_write");
     return 0;
 }
@@ -272,6 +278,9 @@ __global__ void __launch_bounds__(WARPS * 32) head_matmul_kernel(const TX* __res
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int o = blockIdx.z * 32 + lane;
     const int nt = min(HM_TOKENS, T - t0);
+    // The product behind the values' matrices (many inputs) asks for its weights meanwhile; the latent attention behind the keys' must not
+    // start among this kernel's CTAs: two of its own then share SMs while others are empty (15 -> 24 us).
+    if (WARPS == 16) gb_grid_launch_dependents();
     for (int idx = threadIdx.x; idx < HM_TOKENS * I; idx += WARPS * 32) {
         const int tt = idx / I, i = idx - tt * I;
         xt[idx] = tt < nt ? gb_to_float(x[size_t(t0 + tt) * ldx + size_t(h) * xs + i]) : 0.f;

@@ -60,6 +60,11 @@ static inline cudaError_t gb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 bl
     return gb_launch_opt(kernel, grid, block, smem, stream, true, static_cast<Args&&>(args)...);
 }
 
+// Steps of up to this many tokens launch their small kernels programmatically too (gb_launch_opt): there a kernel's start and end are
+// most of its time, and the product behind it asks for its weights meanwhile (the hybrid 1B design's recurrent layer at
+// four sequences, from its rows prepared to its o product done: 27 -> 23 us); with thousands of blocks each block pays for the wait.
+constexpr int GB_FEW_TOKENS = 64;
+
 static inline bool gb_is_dtype(int d) { return d == GB_F32 || d == GB_BF16; }
 static inline size_t gb_dtype_size(int d) { return d == GB_F32 ? 4 : 2; }
 

@@ -241,6 +241,8 @@ struct DeltaPrepParams {
 
 // One warp per item: items 0..H-1 are the heads (decays, beta, values), items H..H+G-1 the q/k heads.
 __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaPrepParams p) {
+    gb_grid_launch_dependents();
+    gb_grid_wait();
     const int t = blockIdx.x, item = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= p.H + p.G) return;
     const int D = p.D, DA = p.DA;
@@ -295,6 +297,7 @@ __device__ __forceinline__ void dr_cp16(float* dst, const float* src) {
 template <int NR>
 __global__ void __launch_bounds__(128) delta_rule_kernel(const DeltaRuleParams p) {
     extern __shared__ __align__(16) float sm[];
+    gb_grid_launch_dependents();                        // the wait comes behind the state's loads: an earlier step left it
     const int b = blockIdx.x, h = blockIdx.y;
     const int slot = p.slots[b], n = p.qlens[b];
     if (slot < 0 || n <= 0) return;
@@ -314,6 +317,7 @@ __global__ void __launch_bounds__(128) delta_rule_kernel(const DeltaRuleParams p
         const int i = r * NR + m;
         S[m] = (i < D && col_ok) ? sp[size_t(i) * Dv + j] : 0.f;
     }
+    gb_grid_wait();
     for (int i = threadIdx.x; i < 2 * TC * TOK; i += 128) sm[i] = 0.f;      // what no copy reaches stays zero
     __syncthreads();
     const int t0 = p.cu[b];
@@ -428,7 +432,8 @@ GB_API int gb_delta_rule(const void* q, const void* k, const void* v, int dtype,
     pp.vf = pp.gb + size_t(T) * H * (DA + 4);
     pp.ld = ld; pp.ld_beta = ld_beta; pp.ld_a = ld_a; pp.dtype = dtype; pp.w_dtype = w_dtype;
     pp.H = H; pp.G = G; pp.D = D; pp.Dv = Dv; pp.DA = DA; pp.VA = VA; pp.q_scale = q_scale;
-    delta_prep_kernel<<<dim3(T, (H + G + 3) / 4), 128, 0, stream>>>(pp);
+    const bool pdl = T <= GB_FEW_TOKENS;
+    gb_launch_opt(delta_prep_kernel, dim3(T, (H + G + 3) / 4), dim3(128), 0, stream, pdl, pp);
     GB_LAUNCH_OK("gb_delta_rule (prepare)");
     DeltaRuleParams p;
     p.qk = pp.qk; p.gb = pp.gb; p.vf = pp.vf; p.state = state; p.out = out; p.cu = cu; p.slots = slots; p.qlens = qlens;
@@ -452,10 +457,10 @@ GB_API int gb_delta_rule(const void* q, const void* k, const void* v, int dtype,
     }
     dim3 grid(B, H, (Dv + CB - 1) / CB);
     GB_REQUIRE(grid.z <= 65535 && H <= 65535, "gb_delta_rule: too many heads or value columns");
-    if (NR == 8) delta_rule_kernel<8><<<grid, 128, smem, stream>>>(p);
-    else if (NR == 16) delta_rule_kernel<16><<<grid, 128, smem, stream>>>(p);
-    else if (NR == 32) delta_rule_kernel<32><<<grid, 128, smem, stream>>>(p);
-    else delta_rule_kernel<64><<<grid, 128, smem, stream>>>(p);
+    if (NR == 8) gb_launch_opt(delta_rule_kernel<8>, grid, dim3(128), smem, stream, pdl, p);
+    else if (NR == 16) gb_launch_opt(delta_rule_kernel<16>, grid, dim3(128), smem, stream, pdl, p);
+    else if (NR == 32) gb_launch_opt(delta_rule_kernel<32>, grid, dim3(128), smem, stream, pdl, p);
+    else gb_launch_opt(delta_rule_kernel<64>, grid, dim3(128), smem, stream, pdl, p);
     GB_LAUNCH_OK("gb_delta_rule");
     return 0;
 }
@@ -469,6 +474,8 @@ __global__ void gated_head_norm_kernel(const float* __restrict__ o, long long ld
                                        int gate_dtype, long long ldg, const void* __restrict__ w, int w_dtype, float eps,
                                        void* __restrict__ out, int out_dtype, long long ld_out, long long items, int H, int Dv,
                                        int gate_act, int w_per_head, int gate_first) {
+    gb_grid_launch_dependents();
+    gb_grid_wait();
     const long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= items) return;
     const int lane = threadIdx.x & 31;
@@ -547,8 +554,8 @@ GB_API int gb_gated_head_norm(const float* o, long long ldo, const void* gate, i
         GB_LAUNCH_OK("gb_gated_head_norm");
         return 0;
     }
-    gated_head_norm_kernel<<<unsigned((items + 3) / 4), 128, 0, stream>>>(o, ldo, gate, gate_dtype, ldg, w, w_dtype, eps, out,
-                                                                          out_dtype, ld_out, items, H, Dv, gate_act, w_per_head, gate_first);
+    gb_launch_opt(gated_head_norm_kernel, dim3(unsigned((items + 3) / 4)), dim3(128), 0, stream, T <= GB_FEW_TOKENS, o, ldo, gate, gate_dtype, ldg, w, w_dtype, eps,
+                  out, out_dtype, ld_out, items, H, Dv, gate_act, w_per_head, gate_first);
     GB_LAUNCH_OK("gb_gated_head_norm");
     return 0;
 }

@@ -35,7 +35,7 @@ GB_API int gb_embed(const void* table, int table_dtype, const int* tokens, int T
 // The same, and for the deferred norm of the first layer: xb[t,:] = bf16(x[t,:]) and ssq[t] = sum(x[t,:]^2).
 __global__ void embed_shadow_kernel(const void* __restrict__ table, int table_dtype, const int* __restrict__ tokens,
                                     int E, int V, float scale, float* __restrict__ out, __nv_bfloat16* __restrict__ xb,
-                                    float* __restrict__ ssq) {
+                                    float* __restrict__ ssq, bool vec) {
     __shared__ float red[32];
     gb_grid_launch_dependents();
     gb_grid_wait();
@@ -44,11 +44,32 @@ __global__ void embed_shadow_kernel(const void* __restrict__ table, int table_dt
     bool ok = tok >= 0 && tok < V;
     size_t base = size_t(ok ? tok : 0) * E;
     float ss = 0.f;
-    for (int i = threadIdx.x; i < E; i += blockDim.x) {
-        float v = ok ? gb_load(table, table_dtype, base + i) * scale : 0.f;
-        out[size_t(t) * E + i] = v;
-        xb[size_t(t) * E + i] = __float2bfloat16_rn(v);
-        ss += v * v;
+    if (vec) {                                   // four entries a thread, all of them asked for before the first is stored (4096: 12 us entry by entry)
+        for (int i0 = 4 * threadIdx.x; i0 < E; i0 += 16 * blockDim.x) {
+            float4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + 4 * j * blockDim.x;
+                v[j] = ok && i < E ? gb_load4(table, table_dtype, base + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + 4 * j * blockDim.x;
+                v[j] = make_float4(v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale);
+                if (i < E) {
+                    *reinterpret_cast<float4*>(out + size_t(t) * E + i) = v[j];
+                    *reinterpret_cast<uint2*>(xb + size_t(t) * E + i) = gb_pack4(v[j]);
+                }
+                ss += (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
+            }
+        }
+    } else {
+        for (int i = threadIdx.x; i < E; i += blockDim.x) {
+            float v = ok ? gb_load(table, table_dtype, base + i) * scale : 0.f;
+            out[size_t(t) * E + i] = v;
+            xb[size_t(t) * E + i] = __float2bfloat16_rn(v);
+            ss += v * v;
+        }
     }
     ss = gb_warp_sum(ss);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
@@ -65,7 +86,8 @@ GB_API int gb_embed_shadow(const void* table, int table_dtype, const int* tokens
     GB_REQUIRE(gb_is_dtype(table_dtype), "gb_embed_shadow: bad table dtype %d", table_dtype);
     GB_REQUIRE(T >= 0 && E > 0 && V > 0 && xb && ssq, "gb_embed_shadow: bad arguments");
     if (T == 0) return 0;
-    gb_launch(embed_shadow_kernel, dim3(T), dim3(256), 0, stream, table, table_dtype, tokens, E, V, scale, out, (__nv_bfloat16*)xb, ssq);
+    const bool vec = E % 4 == 0 && gb_aligned(table, 4 * gb_dtype_size(table_dtype)) && gb_aligned(out, 16) && gb_aligned(xb, 8);
+    gb_launch(embed_shadow_kernel, dim3(T), dim3(256), 0, stream, table, table_dtype, tokens, E, V, scale, out, (__nv_bfloat16*)xb, ssq, vec);
     GB_LAUNCH_OK("gb_embed_shadow");
     return 0;
 }

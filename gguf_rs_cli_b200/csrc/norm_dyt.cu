@@ -12,6 +12,8 @@ __global__ void add_dyt_kernel(float* __restrict__ x, const void* __restrict__ d
                                size_t delta_stride, const int* __restrict__ rows, int E, const void* __restrict__ w,
                                const void* __restrict__ b, int w_dtype, float alpha, void* __restrict__ out,
                                int out_dtype, int write_x) {
+    gb_grid_launch_dependents();
+    gb_grid_wait();
     const int r = blockIdx.x;
     const int s = rows ? rows[r] : r;
     float* xr = x + size_t(s) * E;
@@ -33,8 +35,8 @@ GB_API int gb_add_dyt(float* x, const void* delta, int delta_dtype, int n_delta,
     const int threads = 128;
     int slices = (E + threads - 1) / threads;
     slices = slices > 16 ? 16 : slices;
-    add_dyt_kernel<<<dim3(n_rows, slices), threads, 0, stream>>>(x, delta, delta_dtype, n_delta, size_t(delta_stride), rows, E, w, b,
-                                                   w_dtype, alpha, out, out_dtype, write_x);
+    gb_launch_opt(add_dyt_kernel, dim3(n_rows, slices), dim3(threads), 0, stream, n_rows <= GB_FEW_TOKENS, x, delta, delta_dtype, n_delta, size_t(delta_stride), rows, E, w,
+                  b, w_dtype, alpha, out, out_dtype, write_x);
     GB_LAUNCH_OK("gb_add_dyt");
     return 0;
 }
