@@ -297,7 +297,8 @@ __device__ __forceinline__ void dr_cp16(float* dst, const float* src) {
 template <int NR>
 __global__ void __launch_bounds__(128) delta_rule_kernel(const DeltaRuleParams p) {
     extern __shared__ __align__(16) float sm[];
-    gb_grid_launch_dependents();                        // the wait comes behind the state's loads: an earlier step left it
+    gb_grid_launch_dependents();                        // the state too is read behind the wait: of two calls one behind the other the second may start
+    gb_grid_wait();                                     // while the first still runs (the kernel between them waits, but says at its start that it has begun)
     const int b = blockIdx.x, h = blockIdx.y;
     const int slot = p.slots[b], n = p.qlens[b];
     if (slot < 0 || n <= 0) return;
@@ -317,7 +318,6 @@ __global__ void __launch_bounds__(128) delta_rule_kernel(const DeltaRuleParams p
         const int i = r * NR + m;
         S[m] = (i < D && col_ok) ? sp[size_t(i) * Dv + j] : 0.f;
     }
-    gb_grid_wait();
     for (int i = threadIdx.x; i < 2 * TC * TOK; i += 128) sm[i] = 0.f;      // what no copy reaches stays zero
     __syncthreads();
     const int t0 = p.cu[b];
