@@ -51,6 +51,20 @@ __device__ __forceinline__ bool epilogue_any(bool flag) {
 }
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
+// Time stamps (builds with -DGB_STAMPS): slots of a CTA of the one product whose N and K were asked for.
+// 0 entry, 1 the wait for the kernel in front is over, 2 the first operands are there, 3 the last MMA is committed,
+// 4 the accumulator is seen complete, 5 partial sums stored and fenced, 6 counted (and the tile's other CTAs seen),
+// 7 the sharers' sums of its first tokens are there, 8 the tile (or this CTA's share) is finished, 9 exit.
+#ifdef GB_STAMPS
+__device__ long long* g_stamps = nullptr;
+__device__ int g_stamps_n = 0, g_stamps_k = 0;
+#define STAMP_IF(cond, k) if (cond) GB_STAMP_WRITE((p.N == g_stamps_n && p.K == g_stamps_k) ? g_stamps : nullptr, blockIdx.x, k)
+#define STAMP_AFTER_IF(cond, k, val) if (cond) GB_STAMP_WRITE_AFTER((p.N == g_stamps_n && p.K == g_stamps_k) ? g_stamps : nullptr, blockIdx.x, k, val)
+#else
+#define STAMP_IF(cond, k)
+#define STAMP_AFTER_IF(cond, k, val)
+#endif
+
 // What only some products need, kept out of the way of the others (every SM runs the code below from a cold instruction cache).
 // Arguments by value: a reference to the kernel's parameters would copy them to local memory, 10 us a layer.
 __device__ __noinline__ float4 shared_bias(const void* bias, int dtype, int n) {
@@ -141,6 +155,7 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
 #pragma unroll
                 for (int e = 0; e < SUMS; ++e) { v[i].x += ld[i][e].x; v[i].y += ld[i][e].y; v[i].z += ld[i][e].z; v[i].w += ld[i][e].w; }
         }
+        STAMP_AFTER_IF(threadIdx.x == 64 && c0 == c_lo + warp4, 7, v[0].x);
 #pragma unroll
         for (int i = 0; i < TOK; ++i) {
             const int c = c0 + 4 * i;
@@ -174,20 +189,6 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
         }
     }
 }
-
-// Time stamps (builds with -DGB_STAMPS): slots of a CTA of the one product whose N and K were asked for.
-// 0 entry, 1 the wait for the kernel in front is over, 2 the first operands are there, 3 the last MMA is committed,
-// 4 the accumulator is seen complete, 5 partial sums stored and fenced, 6 counted (and the tile's other CTAs seen),
-// 8 the tile (or this CTA's share) is finished, 9 exit.
-#ifdef GB_STAMPS
-__device__ long long* g_stamps = nullptr;
-__device__ int g_stamps_n = 0, g_stamps_k = 0;
-#define STAMP_IF(cond, k) if (cond) GB_STAMP_WRITE((p.N == g_stamps_n && p.K == g_stamps_k) ? g_stamps : nullptr, blockIdx.x, k)
-#define STAMP_AFTER_IF(cond, k, val) if (cond) GB_STAMP_WRITE_AFTER((p.N == g_stamps_n && p.K == g_stamps_k) ? g_stamps : nullptr, blockIdx.x, k, val)
-#else
-#define STAMP_IF(cond, k)
-#define STAMP_AFTER_IF(cond, k, val)
-#endif
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     int v;
