@@ -1,4 +1,5 @@
-// The matrix product of the 32-bit mode for rows that start on 16 bytes: out[t,n] = sum_k X[t,k] W[n,k] (+ bias[n]),
+// The matrix product of the 32-bit mode for rows that start on 16 bytes and matrices that are too small for the tensor cores
+// (gemm_f32_tc.cu) or a head: out[t,n] = sum_k X[t,k] W[n,k] (+ bias[n]),
 // every product and sum a 32-bit FMA, every output summed by one thread in ascending k.  That is gemm_generic.cu's sum,
 // bit for bit, whatever the sizes, so a row's result does not depend on the rows beside it; only the loads differ.
 //

@@ -1,8 +1,8 @@
 """A dense projection y = x W^T (+ b) with W stored [out, in] as in the model folder
 (src/tensor/dequant.rs:258-259).  The reference does these products with its own
 kernels, not a library (src/gpu/f32_gemv.glsl, src/tensor/dequant.rs:315-317); so does
-this: the tensor-core kernel where its sizes fit, the CUDA-core kernel otherwise and
-everywhere in 32-bit mode.
+this: the tensor-core kernel where its sizes fit, the CUDA-core kernel otherwise; in 32-bit mode
+the larger matrices run on the tensor cores too, with all 24 bits of both operands.
 """
 from __future__ import annotations
 
