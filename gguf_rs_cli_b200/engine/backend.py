@@ -27,12 +27,16 @@ class DecodeGraph:
         self.bucket = bucket
         n = engine.meta_size(bucket)
         self.meta = (torch.empty(n, dtype=torch.int32).pin_memory(), torch.empty(n, dtype=torch.int32, device=engine.device))
-        self.keys_host = torch.zeros(bucket, dtype=torch.int64).pin_memory()
-        self.keys_dev = torch.zeros(bucket, dtype=torch.int64, device=engine.device)
+        # the sequences' keys and, behind them, the turn of the host buffers below
+        self.keys_host = torch.zeros(bucket + 1, dtype=torch.int64).pin_memory()
+        self.keys_and_turn = torch.zeros(bucket + 1, dtype=torch.int64, device=engine.device)
+        self.keys_dev = self.keys_and_turn[:bucket]
         self.out_dev = torch.zeros(bucket, dtype=torch.int32, device=engine.device)
-        # where a step's tokens go on the host: two steps may be in flight
+        # Where a step's tokens go on the host: two steps may be in flight.  Whose turn it is, is the host's to say (`turn`): every
+        # step that is laid out anew takes it to the device with its keys, and the device's own count (the step's last kernel
+        # moves it on) holds only from there to the next one, over launches that the host has counted too.
         self.out_hosts = [torch.zeros(bucket, dtype=torch.int32).pin_memory() for _ in range(2)]
-        self.turn_dev = torch.zeros(1, dtype=torch.int32, device=engine.device)
+        self.turn_dev = self.keys_and_turn[bucket:].view(torch.int32)[:1]
         self.turn = 0
         self.graph = None
         self.warm = False
@@ -154,8 +158,12 @@ class EngineBackend:
         eng, n = self.engine, len(slots)
         cache = eng.cache
         slots_t = tuple(slots)
-        if self._batch is not None and self._batch[0] == slots_t:
-            lengths = self._batch[1]
+        # Known again once this step is launched and counted: after an interruption anywhere in between the next step is laid out
+        # anew, from the cache's lengths and the host's turn.
+        batch, last = self._batch, self._last_graph
+        self._batch = self._last_graph = None
+        if batch is not None and batch[0] == slots_t:
+            lengths = batch[1]
         else:
             lengths = np.array([cache.length(s) for s in slots], dtype=np.int64)
         # what a captured graph fixes (grids that depend on the lengths, a part's host-side choices) is the
@@ -172,7 +180,7 @@ class EngineBackend:
                 self._graphs.pop(next(iter(self._graphs)))
             dg = DecodeGraph(eng, key[0])
         self._graphs[key] = dg
-        same = (dg.graph is not None and self._last_graph is dg and dg.laid_out_for == slots_t and dg.keys == keys and dg.plan_words == 0)
+        same = (dg.graph is not None and last is dg and dg.laid_out_for == slots_t and dg.keys == keys and dg.plan_words == 0)
         if same and after is not None and after.out_dev is dg.out_dev and bool((lengths % PAGE).all()):
             # the step in front has left everything in place for this one
             self._check_room(longest)
@@ -180,8 +188,7 @@ class EngineBackend:
             native.count_launches(dg.launches)
             for s in slots:
                 cache.lengths[s] += 1
-            self._batch = (slots_t, lengths + 1)
-            return self._pending(slots, keys, params, dg.out_dev, dg)
+            return self._counted(slots_t, lengths, keys, params, dg)
         if dg.copied is not None:
             dg.copied.synchronize()
         if same:
@@ -202,7 +209,8 @@ class EngineBackend:
             dg.plan_words = ctx.host["plan_words"]
             dg.keys = list(keys)
             dg.keys_host[:n] = torch.tensor(keys, dtype=torch.int64)
-            dg.keys_dev.copy_(dg.keys_host, non_blocking=True)
+            dg.keys_host[dg.bucket] = dg.turn
+            dg.keys_and_turn.copy_(dg.keys_host, non_blocking=True)
             self._copied(dg)
             self._feed_from(dg, after, n)
 
@@ -222,10 +230,15 @@ class EngineBackend:
                 body()
                 dg.warm = True
             cache.advance(slots, [1] * n)
-            h2d = ctx.host["h2d_bytes"] + 8 * dg.bucket
-        self._batch, self._last_graph = (slots_t, lengths + 1), dg
+            h2d = ctx.host["h2d_bytes"] + 8 * (dg.bucket + 1)
         self.h2d_bytes += h2d
-        return self._pending(slots, keys, params, dg.out_dev, dg)
+        return self._counted(slots_t, lengths, keys, params, dg)
+
+    def _counted(self, slots_t, lengths, keys, params, dg: DecodeGraph) -> Pending:
+        """A captured step that has been launched: only from here on may the next one go on from it."""
+        pending = self._pending(slots_t, keys, params, dg.out_dev, dg)
+        self._batch, self._last_graph = (slots_t, lengths + 1), dg
+        return pending
 
     def _check_room(self, longest: int) -> None:
         if longest + 1 > self.engine.cache.max_len:

@@ -95,6 +95,33 @@ def test_an_interrupted_request_leaves_nothing_in_flight():
             torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("at", [1, 2, 3, 4, 5, 6, 9, 26, 27])
+def test_a_request_interrupted_behind_a_launch_leaves_the_next_ones_ids(at):
+    """The interruption comes when the device has the step and the host has not counted it: behind the prompts' step, the eager step,
+    the captured one, those that follow on the device and those of a page border (lengths 90 and 40: the step behind 64 and 128 tokens)."""
+    from gguf_rs_cli_b200.api import generate
+    from gguf_rs_cli_b200.engine.backend import EngineBackend
+    prompts = [tokens_of("C", k, 400 + k) for k in (90, 40)]
+    want = _fresh("C", "bfloat16", prompts, max_tokens=40)
+    model = llm("C", "bfloat16")
+    for warm in (False, True):
+        if not warm:                               # nothing is captured; then everything is
+            model._engine = model._backend = None
+        calls, real = [], EngineBackend._pending
+
+        def boom(self, *args, **kw):
+            calls.append(1)
+            if len(calls) == at:
+                raise KeyboardInterrupt
+            return real(self, *args, **kw)
+        with pytest.MonkeyPatch.context() as m:
+            m.setattr(EngineBackend, "_pending", boom)
+            with pytest.raises(KeyboardInterrupt):
+                generate(model, prompts, max_tokens=40, stop_token_ids=[])
+        for _ in range(2):
+            assert generate(model, prompts, max_tokens=40, stop_token_ids=[]) == want
+
+
 @pytest.mark.parametrize("lens", [[1] * 130, [1, 200, 1, 33, 5, 129, 32], [40, 3], [2] * 70 + [129] + [1] * 3, [33] * 5])
 def test_index_arrays_of_long_and_short_sequences_side_by_side(lens):
     """Laid out as arrays, as lists and as both in turn: in 32-bit mode every sequence's logits are those of a step of its own."""
