@@ -75,12 +75,6 @@ __device__ __noinline__ void shared_gated(void* out, int dtype, size_t at, int l
     if (left > 0) gb_store(out, dtype, at, gb_gate_act(g0, act) * u0);
     if (left > 1) gb_store(out, dtype, at + 1, gb_gate_act(g1, act) * u1);
 }
-// The sum of one feature of one token, for rows that take no accesses of four values and for features next to the matrix's end.
-__device__ __noinline__ float shared_sum(const float* part, size_t stride, const float* first, int n_ctas) {
-    float v = __ldcg(first);
-    for (int s = 1; s < n_ctas; ++s) v += __ldcg(part + s * stride);
-    return v;
-}
 
 // The tokens c_lo .. c_hi - 1 of a shared tile, finished by one of its CTAs: the sums of all its CTAs, in ascending order, and the
 // last steps (as tc_finish_chunk).  A warp has a token and a lane four neighbouring features of it, so that a token's row of a
@@ -92,29 +86,46 @@ template <int BN, int TOK, int SUMS, bool DYT>
 __device__ __forceinline__ void finish_shared(const TcParams& p, const float* base, int first_which, int n_ctas, int n0, int t0, int c_lo, int c_hi,
                                               int warp4, int lane, const float* rstd_s) {
     constexpr size_t STRIDE = 2 * BN * BM;                   // between two CTAs' first slots
-    const int n = n0 + 4 * lane;
-    const float* part = base + 4 * lane;
-    const float* first = part + first_which * (BN * BM);
-    if (!p.vec || n0 + BM > p.N) {                           // uniform over the CTA
+    if (!p.vec) {
+        // Rows that take no accesses of four values: a lane's four features lie 32 apart (a gated product is not among these).
         for (int c = c_lo + warp4; c < c_hi; c += 4) {
-            const float scale = p.row_ssq ? rstd_s[c] : 1.f;
-            float sq = 0.f, gate = 0.f;
-#pragma unroll 1
+            const float* at = base + c * BM + lane;
+            const size_t row = size_t(t0 + c);
+            float v[4], x[4];
+#pragma unroll
             for (int e = 0; e < 4; ++e) {
-                if (n + e >= p.N) break;
-                float v = shared_sum(part + c * BM + e, STRIDE, first + c * BM + e, n_ctas) * scale;
-                if (p.bias) v += gb_load(p.bias, p.bias_dtype, n + e);
-                if (p.swiglu) {                              // N is a multiple of 128
-                    if (e & 1) shared_gated(p.out, p.out_dtype, size_t(t0 + c) * p.ldo + ((n + e) >> 1), min(1, p.N_out - ((n + e) >> 1)), p.swiglu, gate, v, 0.f, 0.f);
-                    gate = v;
-                } else if (p.resid_x) {
-                    const size_t at = size_t(t0 + c) * p.ld_x + n + e;
-                    v = fmaf(p.resid_scale, v, __ldcg(p.resid_x + at));
-                    p.resid_x[at] = v;
-                    p.resid_xb[at] = __float2bfloat16_rn(DYT ? gb_dyt(v, p.dyt_alpha, gb_load(p.dyt_w, p.dyt_dtype, n + e), gb_load(p.dyt_b, p.dyt_dtype, n + e)) : v);
-                    sq = fmaf(v, v, sq);
+                const int n = n0 + lane + 32 * e;
+                v[e] = 0.f;
+                x[e] = p.resid_x && n < p.N ? __ldcg(p.resid_x + row * p.ld_x + n) : 0.f;
+            }
+            for (int s0 = 0; s0 < n_ctas; s0 += 4) {
+                float ld[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float* a = at + (s0 + i == 0 ? first_which * (BN * BM) : (s0 + i) * STRIDE);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) ld[i][e] = s0 + i < n_ctas ? __ldcg(a + 32 * e) : 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) v[e] += ld[i][e];
+            }
+            const float scale = p.row_ssq ? rstd_s[c] : 1.f;
+            float sq = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int n = n0 + lane + 32 * e;
+                if (n >= p.N) break;
+                float r = v[e] * scale;
+                if (p.bias) r += gb_load(p.bias, p.bias_dtype, n);
+                if (p.resid_x) {
+                    r = fmaf(p.resid_scale, r, x[e]);
+                    p.resid_x[row * p.ld_x + n] = r;
+                    p.resid_xb[row * p.ld_x + n] = __float2bfloat16_rn(DYT ? gb_dyt(r, p.dyt_alpha, gb_load(p.dyt_w, p.dyt_dtype, n), gb_load(p.dyt_b, p.dyt_dtype, n)) : r);
+                    sq = fmaf(r, r, sq);
                 } else {
-                    gb_store(p.out, p.out_dtype, size_t(t0 + c) * p.ldo + n + e, v);
+                    gb_store(p.out, p.out_dtype, row * p.ldo + n, r);
                 }
             }
             if (p.resid_x && !DYT) {
@@ -124,10 +135,14 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
         }
         return;
     }
+    const int n = n0 + 4 * lane;
+    const bool in = n < p.N;                                 // N is a multiple of four here: all of a lane's features are, or none
+    const float* part = base + 4 * lane;
+    const float* first = part + first_which * (BN * BM);
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.bias) bias = shared_bias(p.bias, p.bias_dtype, n);
+    if (p.bias && in) bias = shared_bias(p.bias, p.bias_dtype, n);
     float4 dyt_w = bias, dyt_b = bias;
-    if (DYT) {
+    if (DYT && in) {
         dyt_w = shared_bias(p.dyt_w, p.dyt_dtype, n);
         dyt_b = shared_bias(p.dyt_b, p.dyt_dtype, n);
     }
@@ -137,7 +152,7 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
         for (int i = 0; i < TOK; ++i) {
             const int c = c0 + 4 * i;
             v[i] = x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p.resid_x && c < c_hi) x[i] = __ldcg(reinterpret_cast<const float4*>(p.resid_x + size_t(t0 + c) * p.ld_x + n));
+            if (p.resid_x && in && c < c_hi) x[i] = __ldcg(reinterpret_cast<const float4*>(p.resid_x + size_t(t0 + c) * p.ld_x + n));
         }
         for (int s0 = 0; s0 < n_ctas; s0 += SUMS) {
             float4 ld[TOK][SUMS];
@@ -171,17 +186,17 @@ __device__ __forceinline__ void finish_shared(const TcParams& p, const float* ba
                 const size_t at = size_t(t0 + c) * p.ld_x + n;
                 r = make_float4(fmaf(p.resid_scale, r.x, x[i].x), fmaf(p.resid_scale, r.y, x[i].y), fmaf(p.resid_scale, r.z, x[i].z),
                                 fmaf(p.resid_scale, r.w, x[i].w));
-                *reinterpret_cast<float4*>(p.resid_x + at) = r;
+                if (in) *reinterpret_cast<float4*>(p.resid_x + at) = r;
                 if (DYT) {
-                    *reinterpret_cast<uint2*>(p.resid_xb + at) =
+                    if (in) *reinterpret_cast<uint2*>(p.resid_xb + at) =
                         gb_pack4(make_float4(gb_dyt(r.x, p.dyt_alpha, dyt_w.x, dyt_b.x), gb_dyt(r.y, p.dyt_alpha, dyt_w.y, dyt_b.y),
                                              gb_dyt(r.z, p.dyt_alpha, dyt_w.z, dyt_b.z), gb_dyt(r.w, p.dyt_alpha, dyt_w.w, dyt_b.w)));
                     continue;
                 }
-                *reinterpret_cast<uint2*>(p.resid_xb + at) = gb_pack4(r);
-                const float sq = gb_warp_sum(r.x * r.x + r.y * r.y + (r.z * r.z + r.w * r.w));
+                if (in) *reinterpret_cast<uint2*>(p.resid_xb + at) = gb_pack4(r);
+                const float sq = gb_warp_sum(in ? r.x * r.x + r.y * r.y + (r.z * r.z + r.w * r.w) : 0.f);
                 if (lane == 0) p.ssq_out[size_t(n0 / BM) * p.T + t0 + c] = sq;
-            } else {
+            } else if (in) {
                 const size_t at = size_t(t0 + c) * p.ldo + n;
                 if (p.out_dtype == GB_F32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at) = r;
                 else *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + at) = gb_pack4(r);
@@ -714,7 +729,7 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
                K, ldx, ldw);
     if (T == 0) return 0;
     if (ensure_status()) return 1;
-    const TcCut cut = cut_for(T, N, K, sms, scratch && counters, n_counters, true, swiglu_features > 0);
+    const TcCut cut = cut_for(T, N, K, sms, scratch && gb_aligned(scratch, 16) && counters, n_counters, true, swiglu_features > 0);
     GB_REQUIRE(cut.tiles * cut.kb < (1LL << 31) - (1 << 20), "gb_gemm_tc: T=%d N=%d K=%d is more work than the kernel numbers", T, N, K);
     const int bn = cut.bn;
     TcParams p;
@@ -722,8 +737,9 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
     p.ldo = ldo; p.out_dtype = out_dtype; p.bias_dtype = bias_dtype; p.T = T; p.N = N; p.K = K;
     p.swiglu = swiglu_features > 0 ? gate_act : 0; p.N_out = swiglu_features; p.sms = sms;
     cut.fill(p);
-    p.vec = resid_x ? gb_aligned(resid_x, 16) && gb_aligned(resid_xb, 8) && ld_x % 4 == 0 : gb_aligned(out, 16) && ldo % 4 == 0;
-    p.vec = p.vec && gb_aligned(scratch, 16);
+    // (a gated product's results are stored one by one)
+    p.vec = swiglu_features || (N % 4 == 0 && (resid_x ? gb_aligned(resid_x, 16) && gb_aligned(resid_xb, 8) && ld_x % 4 == 0
+                                                       : gb_aligned(out, 16) && ldo % 4 == 0));
     p.row_ssq = row_ssq; p.ssq_parts = ssq_parts; p.norm_size = norm_size; p.eps = eps;
     p.resid_x = resid_x; p.resid_xb = (__nv_bfloat16*)resid_xb; p.ssq_out = ssq_out; p.ld_x = ld_x; p.resid_scale = resid_scale;
     CUtensorMap mw, mx;
@@ -905,7 +921,7 @@ GB_API int gb_gemm_tc_noalloc(const void* X, long long ldx, const void* W, long 
     p.ldo = ldo; p.out_dtype = out_dtype; p.bias_dtype = bias_dtype; p.T = T; p.N = N; p.K = K;
     p.swiglu = 0; p.N_out = 0; p.sms = d->sms;
     cut.fill(p);
-    p.vec = gb_aligned(out, 16) && ldo % 4 == 0;
+    p.vec = N % 4 == 0 && gb_aligned(out, 16) && ldo % 4 == 0;
     p.row_ssq = nullptr; p.ssq_parts = 0; p.norm_size = 0; p.eps = 0.f;
     p.resid_x = nullptr; p.resid_xb = nullptr; p.ssq_out = nullptr; p.ld_x = 0; p.resid_scale = 1.f;
     CUtensorMap mw, mx;

@@ -160,3 +160,32 @@ def test_products_of_one_block_of_k_are_the_same_bits_on_either_kernel(T, N, K):
     x, w = torch.randn(T, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
     outs = [f(x, w, None, torch.empty(T, N, device="cuda")) for f in (k.gemm, k.gemm_f32, k.gemm_generic)]
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("T", [1, 4, 16, 17, 64, 127])
+@pytest.mark.parametrize("N", [6672, 2624, 132, 1030, 2047])
+def test_shared_tiles_at_a_matrixs_edge(N, T):
+    """The last tile's features, where several CTAs share a tile: the bits of the same matrix with rows of zeros up to a whole tile, for
+    rows that take accesses of four values and rows that do not; nothing is written beside them."""
+    k = K()
+    x, w, b, g = _operands(T, N, 2048, N + T)
+    P = (N + 127) // 128 * 128
+    wp, bp = torch.zeros(P, 2048, device=DEV, dtype=w.dtype), torch.zeros(P, device=DEV)
+    wp[:N], bp[:N] = w, b
+    for pitch in (N, (N + 7) // 4 * 4, N + 3):
+        for dtype in (torch.float32, torch.bfloat16):
+            want, got = torch.empty(T, P, device=DEV, dtype=dtype), torch.full((T, pitch), 9.0, device=DEV, dtype=dtype)
+            k.gemm_tc(x, wp, bp, want)
+            k.gemm_tc(x, w, b, got[:, :N])
+            assert torch.equal(got[:, :N], want[:, :N]) and (got[:, N:] == 9.0).all(), (pitch, dtype)
+        start, parts = torch.randn(T, P, generator=g, device=DEV), P // 128
+        full, fullb, ssq_full = start.clone(), torch.empty(T, P, device=DEV, dtype=torch.bfloat16), torch.empty(parts, T, device=DEV)
+        k.gemm_tc(x, wp, bp, None, resid_x=full, resid_xb=fullb, ssq_out=ssq_full, resid_scale=0.5)
+        res, resb = torch.full((T, pitch), 9.0, device=DEV), torch.full((T, pitch), 9.0, device=DEV, dtype=torch.bfloat16)
+        res[:, :N], ssq = start[:, :N], torch.full((parts, T), 9.0, device=DEV)
+        k.gemm_tc(x, w, b, None, resid_x=res[:, :N], resid_xb=resb[:, :N], ssq_out=ssq, resid_scale=0.5)
+        assert torch.equal(res[:, :N], full[:, :N]) and torch.equal(resb[:, :N], fullb[:, :N])
+        assert (res[:, N:] == 9.0).all() and (resb[:, N:] == 9.0).all()
+        want = torch.nn.functional.pad(full[:, :N].double() ** 2, (0, P - N)).view(T, parts, 128).sum(2).T
+        # 128 squares, each rounded once, and their sum in any order: 128 roundings at most
+        assert ((ssq.double() - want).abs() <= 129 * 2.0 ** -24 * want).all()
