@@ -1,28 +1,30 @@
-// The matrix product of the 32-bit mode on the tensor cores, for more tokens than gemm_f32's few:
+// The matrix product of the 32-bit mode on the tensor cores, for the larger matrices and every number of tokens:
 //   out[t,n] = sum_k X[t,k] W[n,k] (+ bias[n]), operands and results in 32 bits.
 //
-// Every operand is cut into three bfloat16 terms of eight bits each (x = h + m + l, exactly: 24 bits by truncation), and
-// six of the nine products of terms are taken: hh, hm, mh, hl, lh, mm.  What is left out is 2^-23 of a product and less.
-// The tensor core's own 32-bit additions are not relied on for long sums: a block of 32 of K is summed there (its ten small
-// products first, so that only two additions meet a sum of full size), and the blocks' sums are added one behind another
-// in registers, rounded to nearest.  Against 64 bits the result is 2 to 10 times closer than one thread's ascending sum (K = 256 1.2e-7
-// of the result's norm against 2.8e-7, 2048 1.4e-7 and 8.1e-7, 8192 1.6e-7 and 1.6e-6).  Results that are not finite (an infinite
-// operand times a term that is zero) and results below 2^-96 (the terms of operands of that size reach the end of the exponents' range: operands
-// of 1e-34 would give 6e-7, of 1e-36 5e-5) are summed again one product behind another, as gemm_generic does; an exact zero stays.
+// Every operand is cut into three bfloat16 terms, each the rest rounded to nearest, so that nothing is left behind the third (x = h + m + l: the
+// scheme of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", 2019), and eight
+// of the nine products of terms are taken; l l, 2^-36 of a product, is left out.  The tensor core cuts its 32-bit sums instead of rounding them, so it
+// is given little to cut: a block of 32 of K has a sum of its own for h h, whose products have 16 bits, and the blocks' sums are added in
+// registers, rounded to nearest; the seven small products are summed in a second accumulator over a piece of K, where a lost bit is 2^-8 of
+// that, and added behind its last block.  Against 64 bits (2,048 of K, 32-bit FMAs one behind another in brackets, of the result's norm): one term in a row
+// 2.5e-8 (2.5e-8), 4 side by side 2.7e-8 (4.2e-8), 4 far apart 4.5e-8 (4.1e-8), 16 3.7e-8 and 6.9e-8 (7.5e-8), all 9.8e-8 (8.1e-7).
+// (One accumulator for all products: one term 4.9e-8, and 2 to 15 % less time.)
+// Results that are not finite (an infinite operand times a term that is zero) and results below 2^-96 (the terms of operands of that size
+// reach the end of the exponents' range: operands of 1e-34 would give 6e-7, of 1e-36 5e-5) are summed again one product behind another, as gemm_generic
+// does; an exact zero stays.
 //
 // A row's result does not depend on the rows beside it: a block's sum is the same whatever the tile's width, and K is cut into pieces
 // by the matrix's sizes alone (fx_pieces), whose sums are added in order.
 //
-// What bounds it: a block of 128 features x 192 tokens x 32 of K takes 1,150 cycles of tensor core (six products for each 32-bit
-// one) and 2,300 in all: the warps' chain from a block's copy through its conversion (W's terms into tensor memory, X's into
-// shared memory) and the sums of an earlier block.  Without the sums it takes 15 % less, without X's conversion 15 %, with one product
-// instead of six 1 %.  W is the A operand from tensor memory because shared memory would be busy for 1,700 cycles with its reads beside X's.
-// Microseconds, gemm_f32 in brackets: 187 tokens 16,384 x 2,048 84 (390), 2,048 x 8,192 45 (414), 3,072 x 2,048 26 (123), 2,048 x 2,048 22
-// (114 at 100 tokens); 2 tokens 35 (27), 22 (42), 12.6 (12.3), 10.8 (14.5), where two CTAs an SM each stream their share of W; 1 to 16 tokens are the same.
+// What bounds it: a block of 128 features x 192 tokens x 32 of K takes 1,540 cycles of tensor core (eight products for each 32-bit one), 1,670 of
+// shared memory (the loads, X's conversion, the products' reads of X) and 2,500 in all.  Few tokens: the loads; without conversion and sums 39 us of 41 at 16,384 x 2,048.
+// W is the A operand from tensor memory because shared memory would be busy for 1,700 cycles more with its reads.  Tiles of 64 tokens and more have sixteen
+// warps that convert and add (192 tokens 16,384 x 2,048 98 us, 100 with eight; 1,152 tokens 513, 535).
+// Microseconds behind a cleared L2, gemm_f32 in brackets: 16,384 x 2,048, 1, 2, 4, 16 tokens 45 (39, 41, 45, 70), 64 63, 187 98; 2,048 x 8,192 31 (37, 38, 39, 64), 64 38, 187 57.
 //
 // A CTA has one tile of 128 features x BN tokens and some pieces of K.  Warp 0 copies 32-bit blocks of both operands by TMA
-// (128-byte swizzle) into a ring, warp 1 issues the MMAs, eight warps convert a block (of W a row and half of the block a
-// thread, of X a quarter of a row) and add the sums of an earlier block (half of the columns each).  Where CTAs share a tile they are all
+// (128-byte swizzle) into a ring, warp 1 issues the MMAs, eight or sixteen warps convert a block (of W a row and half of the block a
+// thread, of X a quarter of a row) and add the sums of an earlier block.  Where CTAs share a tile they are all
 // resident, wait for one another (bounded) and finish a share of the tokens each.
 #include <mutex>
 
@@ -33,19 +35,24 @@ using namespace sm100;
 
 namespace {
 
-constexpr int FX_BM = 128, FX_BK = 32, FX_THREADS = 320, FX_WORKERS = 256;
+constexpr int FX_BM = 128, FX_BK = 32;
 
 template <int BN> struct FxCfg {
     static constexpr int W_BYTES = FX_BM * 128, X_BYTES = BN * 128, RAW = W_BYTES + X_BYTES;
-    // blocks on their way through the tensor core: terms and sums of DEPTH of them (512 columns of tensor memory in all, 256 where two CTAs share an SM)
-    static constexpr int DEPTH = BN <= 16 ? 3 : BN <= 32 ? 2 : BN <= 64 ? 4 : BN <= 96 ? 3 : 2;
+    // blocks whose terms are on their way through the tensor core
+    static constexpr int DEPTH = BN <= 16 ? 3 : BN <= 32 ? 2 : BN <= 64 ? 4 : 2;
     static constexpr int RING = BN <= 16 ? 5 : BN <= 32 ? 4 : BN <= 64 ? 5 : BN <= 160 ? 4 : 3;
     static constexpr int SMEM = RING * RAW + (DEPTH + (DEPTH + 1) / 2) * X_BYTES + 1024;
-    // W's terms in tensor memory: DEPTH buffers of 64 columns, 32 for each 16 of K: h, m, l and eight columns that nothing reads (one store
+    // Tensor memory, 512 columns (256 where two CTAs share an SM): sums of large products of SUMS blocks, of small products of TAILS pieces of K,
+    // and W's terms of DEPTH blocks in buffers of 64 columns, 32 for each 16 of K: h, m, l and eight columns that nothing reads (one store
     // of 32 columns a warp takes a third of what three of eight do: 57 -> 38 us at 16,384 x 2,048 and 2 tokens)
-    static constexpr int A_COL = DEPTH * BN;
-    static constexpr int TMEM_COLS = DEPTH * (BN + 64) <= 256 ? 256 : 512;
+    static constexpr int SUMS = BN <= 96 ? 2 : 1, TAILS = BN <= 128 ? 2 : 1;
+    static constexpr int T_COL = SUMS * BN, A_COL = T_COL + TAILS * BN;
+    static constexpr int TMEM_COLS = A_COL + DEPTH * 64 <= 256 ? 256 : 512;
     static constexpr int CTAS = BN <= 32 ? 2 : 1;                 // of an SM
+    // Warps that convert and add; a warp adds the sums of a GROUPS-th of the columns.  Of sixteen half convert W, half X.
+    static constexpr int WORKERS = BN < 64 ? 8 : 16, GROUPS = WORKERS / 4, COLS = BN / GROUPS, THREADS = (WORKERS + 2) * 32;
+    static_assert(A_COL + DEPTH * 64 <= 512 && TMEM_COLS * CTAS <= 512 && SUMS <= DEPTH);
 };
 
 struct FxParams {
@@ -61,15 +68,18 @@ struct FxParams {
     int T, N, K, pieces, sharers, t_tiles;
 };
 
-// Two numbers in three bfloat16 terms each, the first in the low halves.
+// Two numbers in three bfloat16 terms each, the first in the low halves: each term the rest, rounded to nearest; nothing is left behind the third.
+__device__ __forceinline__ uint32_t fx_pack(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float fx_low(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float fx_high(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 __device__ __forceinline__ void fx_split(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    const uint32_t ha = __float_as_uint(a), hb = __float_as_uint(b);
-    h = __byte_perm(ha, hb, 0x7632);
-    const float ra = a - __uint_as_float(ha & 0xffff0000u), rb = b - __uint_as_float(hb & 0xffff0000u);
-    const uint32_t ma = __float_as_uint(ra), mb = __float_as_uint(rb);
-    m = __byte_perm(ma, mb, 0x7632);
-    const float la = ra - __uint_as_float(ma & 0xffff0000u), lb = rb - __uint_as_float(mb & 0xffff0000u);
-    l = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+    h = fx_pack(a, b);
+    const float ra = a - fx_low(h), rb = b - fx_high(h);
+    m = fx_pack(ra, rb);
+    l = fx_pack(ra - fx_low(m), rb - fx_high(m));
 }
 __device__ __forceinline__ float4 fx_lds4(uint32_t a) {
     float4 v;
@@ -100,7 +110,20 @@ __device__ __forceinline__ void fx_tmem_ld8(uint32_t taddr, float* v) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void fx_workers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// N columns of this thread's lane, added to acc.
+template <int N> __device__ __forceinline__ void fx_add(float (&acc)[N], uint32_t d) {
+    constexpr int STEP = N % 32 == 0 ? 32 : N % 16 == 0 ? 16 : 8;
+#pragma unroll
+    for (int c = 0; c < N; c += STEP) {
+        float v[STEP];
+        if constexpr (STEP == 32) tmem_ld32(d + c, v);
+        else if constexpr (STEP == 16) tmem_ld16(d + c, v);
+        else fx_tmem_ld8(d + c, v);
+#pragma unroll
+        for (int j = 0; j < STEP; ++j) acc[c + j] += v[j];
+    }
+}
+template <int THREADS> __device__ __forceinline__ void fx_workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
 
 // A sum that is not finite or next to nothing, taken again one product behind another.
 __device__ __noinline__ float fx_again(const float* x, const float* w, int K) {
@@ -114,15 +137,18 @@ __device__ __forceinline__ void fx_store(const FxParams& p, int t, int n, float 
 }
 
 template <int BN>
-__global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                                   const __grid_constant__ CUtensorMap map_x, FxParams p) {
     using Cfg = FxCfg<BN>;
-    constexpr int RING = Cfg::RING, HALF = BN / 2, DEPTH = Cfg::DEPTH;
+    constexpr int RING = Cfg::RING, COLS = Cfg::COLS, WORKERS = Cfg::WORKERS, DEPTH = Cfg::DEPTH, SUMS = Cfg::SUMS, TAILS = Cfg::TAILS;
+    // A block's sums are added SUMS blocks later, before that block's terms are stored, so that the buffer is free when those are there; with
+    // one buffer behind the next block's terms, while its small products run, and the large ones wait for it.
+    constexpr bool LATE = SUMS == 1;
     constexpr bool EARLY = BN <= 64;               // W's terms in registers while the buffer that they go to is still read
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* xs = ring + RING * Cfg::RAW;          // X's terms: rows of 128 bytes, [h | m] of each buffer, then [l of an even buffer | l of an odd one]
-    __shared__ uint64_t raw_full[RING], raw_empty[RING], op_full[DEPTH], done[DEPTH];
+    __shared__ uint64_t raw_full[RING], raw_empty[RING], op_full[DEPTH], done[DEPTH], sum_free, tail_free[TAILS];
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag, all_there;
 
@@ -138,8 +164,10 @@ __global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kerne
     const int b0 = piece_begin(piece0), S = piece_begin(piece1) - b0;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < RING; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
-        for (int i = 0; i < DEPTH; ++i) { mbar_init(&op_full[i], 8); mbar_init(&done[i], 1); }
+        for (int i = 0; i < RING; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WORKERS); }
+        for (int i = 0; i < DEPTH; ++i) { mbar_init(&op_full[i], WORKERS); mbar_init(&done[i], 1); }
+        mbar_init(&sum_free, WORKERS);
+        for (int i = 0; i < TAILS; ++i) mbar_init(&tail_free[i], WORKERS);
         abort_flag = 0;
         fence_barrier_init();
         prefetch_tensormap(&map_w);
@@ -156,11 +184,11 @@ __global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kerne
     gb_grid_launch_dependents();
     gb_grid_wait();
 
-    float acc[HALF];
+    float acc[COLS];
 #pragma unroll
-    for (int i = 0; i < HALF; ++i) acc[i] = 0.f;
-    const int quarter = warp & 3, row = quarter * 32 + lane, half = warp >= 6 ? 1 : 0;       // of the workers
-    const int cols = min(BN, p.T - t0), mine = half * HALF;
+    for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+    const int quarter = warp & 3, row = quarter * 32 + lane, group = (warp - 2) >> 2, half = group & 1;       // of the workers
+    const int cols = min(BN, p.T - t0), mine = group * COLS;
 
     if (warp == 0) {
         if (elect_one()) {
@@ -177,34 +205,86 @@ __global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kerne
         if (elect_one()) {
             constexpr uint32_t idesc = instr_desc_bf16(FX_BM, BN);
             const uint32_t xa = smem_u32(xs);
+            int piece = 0, piece_end = piece_begin(piece0 + 1) - b0, more = 0;         // pieces before this one; whether it has begun
             for (int s = 0; s < S; ++s) {
-                const int b = s % DEPTH;
+                const int b = s % DEPTH, tail = piece % TAILS;
                 if (!mbar_wait(&op_full[b], (s / DEPTH) & 1)) { atomicExch(p.status, 22); abort_flag = 1; break; }
+                // (two buffers for small products: the piece before the last has been read before this block's terms are there, if not LATE)
+                if (LATE && !more && piece >= TAILS && !mbar_wait(&tail_free[tail], (piece / TAILS - 1) & 1)) {
+                    atomicExch(p.status, 26);
+                    abort_flag = 1;
+                    break;
+                }
                 tc_fence_after();
-                const uint32_t d = tmem + b * BN, a = tmem + Cfg::A_COL + b * 64;
+                const uint32_t d = tmem + s % SUMS * BN, t = tmem + Cfg::T_COL + tail * BN, a = tmem + Cfg::A_COL + b * 64;
                 const uint32_t xh = xa + b * Cfg::X_BYTES, xm = xh + 64, xl = xa + (DEPTH + (b >> 1)) * Cfg::X_BYTES + (b & 1) * 64;
-                uint32_t more = 0;
-                auto two = [&](int term, uint32_t xt) {             // both steps of 16 of K
+                auto two = [&](uint32_t to, int term, uint32_t xt, uint32_t add) {             // both steps of 16 of K
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        mma_f16_a_tmem(d, a + k * 32 + term * 8, smem_desc_sw128(xt + k * 32), idesc, more);
-                        more = 1;
-                    }
+                    for (int k = 0; k < 2; ++k) mma_f16_a_tmem(to, a + k * 32 + term * 8, smem_desc_sw128(xt + k * 32), idesc, k ? 1u : add);
                 };
-                two(1, xm);
-                two(2, xh);
-                two(0, xl);
-                two(1, xh);
-                two(0, xm);
-                two(0, xh);
+                two(t, 2, xm, more);
+                two(t, 1, xl, 1u);
+                two(t, 1, xm, 1u);
+                two(t, 2, xh, 1u);
+                two(t, 0, xl, 1u);
+                two(t, 1, xh, 1u);
+                two(t, 0, xm, 1u);
+                if (LATE && s > 0) {
+                    if (!mbar_wait(&sum_free, (s - 1) & 1)) { atomicExch(p.status, 27); abort_flag = 1; break; }
+                    tc_fence_after();
+                }
+                two(d, 0, xh, 0u);
                 mma_commit(&done[b]);
+                more = 1;
+                if (s + 1 == piece_end) {
+                    more = 0;
+                    ++piece;
+                    piece_end = piece_begin(min(piece0 + piece + 1, p.pieces)) - b0;
+                }
             }
         }
     } else {
         const uint32_t ring_a = smem_u32(ring), xs_a = smem_u32(xs);
         const uint32_t lane_base = uint32_t(quarter * 32) << 16;
         int piece = piece0, piece_end = piece_begin(piece0 + 1) - b0;           // the piece whose blocks are being added
-        for (int s = 0; s < S + DEPTH; ++s) {
+        const bool does_w = WORKERS == 8 || warp < 10, does_x = WORKERS == 8 || warp >= 10;
+        const int xw = (warp - 2) & 7;
+        // block s: its sums and, behind a piece's last block, those of the piece's small products
+        auto add = [&](int s) {
+            if (!mbar_wait(&done[s % DEPTH], (s / DEPTH) & 1)) {
+                if (lane == 0) atomicExch(p.status, 23);
+                abort_flag = 1;
+                return false;
+            }
+            tc_fence_after();
+            fx_add<COLS>(acc, tmem + lane_base + s % SUMS * BN + mine);
+            if (LATE) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sum_free);
+            }
+            if (s + 1 == piece_end) {
+                const int tail = (piece - piece0) % TAILS;
+                fx_add<COLS>(acc, tmem + lane_base + Cfg::T_COL + tail * BN + mine);
+                if (LATE) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tail_free[tail]);
+                }
+                if (!(keep && piece + 1 == p.pieces)) {
+                    float* to = p.scratch + (size_t(tile) * p.pieces + piece) * (BN * FX_BM) + row;
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) {
+                        if (mine + c < cols) __stcg(to + size_t(mine + c) * FX_BM, acc[c]);
+                        acc[c] = 0.f;
+                    }
+                }
+                ++piece;
+                piece_end = piece_begin(min(piece + 1, p.pieces)) - b0;
+            }
+            return true;
+        };
+        for (int s = 0; s < S + SUMS; ++s) {
             const int b = s % DEPTH, slot = s % RING;
             uint32_t terms[32];                                                 // h, m, l
             const uint32_t raw = ring_a + slot * Cfg::RAW;
@@ -225,64 +305,40 @@ __global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kerne
                     abort_flag = 1;
                     break;
                 }
-                if (EARLY) split_w();
+                if (EARLY && does_w) split_w();
             }
-            if (s >= DEPTH) {
-                if (!mbar_wait(&done[b], (s / DEPTH - 1) & 1)) {
-                    if (lane == 0) atomicExch(p.status, 23);
-                    abort_flag = 1;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t d = tmem + lane_base + b * BN + mine;
-                constexpr int STEP = HALF % 32 == 0 ? 32 : HALF % 16 == 0 ? 16 : 8;
-#pragma unroll
-                for (int c = 0; c < HALF; c += STEP) {
-                    float v[STEP];
-                    if constexpr (STEP == 32) tmem_ld32(d + c, v);
-                    else if constexpr (STEP == 16) tmem_ld16(d + c, v);
-                    else fx_tmem_ld8(d + c, v);
-#pragma unroll
-                    for (int j = 0; j < STEP; ++j) acc[c + j] += v[j];
-                }
-                if (s - DEPTH + 1 == piece_end && !(keep && piece + 1 == p.pieces)) {        // a piece is complete
-                    float* to = p.scratch + (size_t(tile) * p.pieces + piece) * (BN * FX_BM) + row;
-#pragma unroll
-                    for (int c = 0; c < HALF; ++c) {
-                        if (mine + c < cols) __stcg(to + size_t(mine + c) * FX_BM, acc[c]);
-                        acc[c] = 0.f;
-                    }
-                    ++piece;
-                    piece_end = piece_begin(min(piece + 1, p.pieces)) - b0;
-                }
-            }
+            if (!LATE && s >= SUMS && !add(s - SUMS)) break;
             if (s < S) {
-                if (!EARLY) split_w();
-                fx_tmem_st32(tmem + lane_base + Cfg::A_COL + b * 64 + half * 32, terms);
-                // X: eight of K a thread; the rows of a quarter of a warp are four apart, so that their 64 bytes lie in both halves
-                const int j = lane & 3, sub = (lane >> 3) + (lane & 4);
-                const uint32_t x = raw + Cfg::W_BYTES, hm = xs_a + b * Cfg::X_BYTES, lo = xs_a + (DEPTH + (b >> 1)) * Cfg::X_BYTES;
+                // (the tensor core has read this block's buffers: what lies SUMS <= DEPTH blocks back has been added; LATE: 2 = DEPTH blocks)
+                if (!EARLY && does_w) split_w();
+                if (does_w) fx_tmem_st32(tmem + lane_base + Cfg::A_COL + b * 64 + half * 32, terms);
+                if (does_x) {
+                    // X: eight of K a thread; the rows of a quarter of a warp are four apart, so that their 64 bytes lie in both halves
+                    const int j = lane & 3, sub = (lane >> 3) + (lane & 4);
+                    const uint32_t x = raw + Cfg::W_BYTES, hm = xs_a + b * Cfg::X_BYTES, lo = xs_a + (DEPTH + (b >> 1)) * Cfg::X_BYTES;
 #pragma unroll
-                for (int r0 = 0; r0 < BN; r0 += 64) {
-                    const int r = r0 + (warp - 2) * 8 + sub, sw = r & 7;
-                    if (BN - r0 >= 64 || r < BN) {
-                        const float4 u = fx_lds4(x + r * 128 + ((2 * j ^ sw) << 4)), v = fx_lds4(x + r * 128 + (((2 * j + 1) ^ sw) << 4));
-                        uint32_t xh[4], xm[4], xl[4];
-                        fx_split(u.x, u.y, xh[0], xm[0], xl[0]);
-                        fx_split(u.z, u.w, xh[1], xm[1], xl[1]);
-                        fx_split(v.x, v.y, xh[2], xm[2], xl[2]);
-                        fx_split(v.z, v.w, xh[3], xm[3], xl[3]);
-                        fx_sts4(hm + r * 128 + ((j ^ sw) << 4), xh);
-                        fx_sts4(hm + r * 128 + (((j + 4) ^ sw) << 4), xm);
-                        fx_sts4(lo + r * 128 + (((j + 4 * (b & 1)) ^ sw) << 4), xl);
+                    for (int r0 = 0; r0 < BN; r0 += 64) {
+                        const int r = r0 + xw * 8 + sub, sw = r & 7;
+                        if (BN - r0 >= 64 || r < BN) {
+                            const float4 u = fx_lds4(x + r * 128 + ((2 * j ^ sw) << 4)), v = fx_lds4(x + r * 128 + (((2 * j + 1) ^ sw) << 4));
+                            uint32_t xh[4], xm[4], xl[4];
+                            fx_split(u.x, u.y, xh[0], xm[0], xl[0]);
+                            fx_split(u.z, u.w, xh[1], xm[1], xl[1]);
+                            fx_split(v.x, v.y, xh[2], xm[2], xl[2]);
+                            fx_split(v.z, v.w, xh[3], xm[3], xl[3]);
+                            fx_sts4(hm + r * 128 + ((j ^ sw) << 4), xh);
+                            fx_sts4(hm + r * 128 + (((j + 4) ^ sw) << 4), xm);
+                            fx_sts4(lo + r * 128 + (((j + 4 * (b & 1)) ^ sw) << 4), xl);
+                        }
                     }
+                    fence_proxy_async();
                 }
-                fence_proxy_async();
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) { mbar_arrive(&raw_empty[slot]); mbar_arrive(&op_full[b]); }
             }
+            if (LATE && s >= 1 && !add(s - 1)) break;
         }
     }
     tc_fence_before();
@@ -297,18 +353,18 @@ __global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kerne
         if (p.pieces == 2) {                            // what this thread has stored itself
             const float* first = p.scratch + size_t(tile) * 2 * (BN * FX_BM) + row;
 #pragma unroll
-            for (int c = 0; c < HALF; ++c)
+            for (int c = 0; c < COLS; ++c)
                 if (mine + c < cols) acc[c] = __ldcg(first + size_t(mine + c) * FX_BM) + acc[c];
         }
         if (n < p.N) {
 #pragma unroll
-            for (int c = 0; c < HALF; ++c)
+            for (int c = 0; c < COLS; ++c)
                 if (mine + c < cols) fx_store(p, t0 + mine + c, n, acc[c], bias);
         }
         return;
     }
     __threadfence();
-    fx_workers_sync();
+    fx_workers_sync<Cfg::WORKERS * 32>();
     if (p.sharers > 1) {
         if (threadIdx.x == 64) {
             atomicAdd(&p.counters[tile], 1);
@@ -327,12 +383,12 @@ __global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kerne
             all_there = seen >= p.sharers;
             if (!all_there) atomicExch(p.status, 25);
         }
-        fx_workers_sync();
+        fx_workers_sync<Cfg::WORKERS * 32>();
         if (!all_there) return;
     }
     const int c_lo = me * cols / p.sharers, c_hi = (me + 1) * cols / p.sharers;
     const float* base = p.scratch + size_t(tile) * p.pieces * (BN * FX_BM) + row;
-    for (int c0 = c_lo + half * 4; c0 < c_hi; c0 += 8) {
+    for (int c0 = c_lo + group * 4; c0 < c_hi; c0 += 4 * Cfg::GROUPS) {
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         for (int s0 = 0; s0 < p.pieces; s0 += 8) {
             float ld[8][4];
@@ -354,7 +410,7 @@ __global__ void __launch_bounds__(FX_THREADS, FxCfg<BN>::CTAS) gemm_f32_tc_kerne
     }
     if (p.sharers > 1) {
         // the last of the tile's CTAs to have read the others' sums puts the counter back for the next launch
-        fx_workers_sync();
+        fx_workers_sync<Cfg::WORKERS * 32>();
         if (threadIdx.x == 64 && atomicAdd(&p.counters[tile], 1) == 2 * p.sharers - 1) p.counters[tile] = 0;
     }
 }
@@ -384,7 +440,7 @@ template <int BN> int launch_fx(const CUtensorMap& mw, const CUtensorMap& mx, co
             return gb_fail("gb_gemm_f32_tc: cannot get %d bytes of shared memory", FxCfg<BN>::SMEM);
         configured[dev] = true;
     }
-    gb_launch(gemm_f32_tc_kernel<BN>, dim3(ctas), dim3(FX_THREADS), FxCfg<BN>::SMEM, stream, mw, mx, p);
+    gb_launch(gemm_f32_tc_kernel<BN>, dim3(ctas), dim3(FxCfg<BN>::THREADS), FxCfg<BN>::SMEM, stream, mw, mx, p);
     GB_LAUNCH_OK("gb_gemm_f32_tc");
     return 0;
 }
@@ -404,7 +460,7 @@ int fx_pieces(int N, int K, int sms) {
 struct FxCut { int bn, pieces, sharers; long long tiles; };
 FxCut fx_cut(int T, int N, int K, int sms, bool may_share, int n_counters) {
     static const int BNS[7] = {16, 32, 64, 96, 128, 160, 192};
-    static const double BLOCK[7] = {0.85, 0.95, 0.65, 0.75, 0.85, 1.0, 1.15};
+    static const double BLOCK[7] = {0.9, 1.0, 0.8, 0.87, 0.97, 1.12, 1.3};
     const int blocks = (K + FX_BK - 1) / FX_BK, pieces = fx_pieces(N, K, sms);
     FxCut best = {16, pieces, 1, 0};
     double least = 1e300;

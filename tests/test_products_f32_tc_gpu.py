@@ -32,13 +32,37 @@ def test_closer_to_64_bits_than_one_thread(T, N, K, positive):
     torch.cuda.synchronize()
     k.check_tc_status()
     e, e_plain = [float((a.double() - want).norm() / want.norm()) for a in (got, plain)]
-    # a result is rounded once (2^-25 in the mean of a binade's ends) and the sums of 32 that it adds are; the terms left out are 2^-23
+    # a result is rounded once (2^-25 in the mean of a binade's ends) and the sums of 32 that it adds are; the products left out are 2^-36
     assert e <= max(1.1 * e_plain, 1.5e-7) and e < 4e-7, (e, e_plain)
     assert (got._base[:, N:] == 7.0).all()
     again, low = torch.empty_like(plain), torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
     k.gemm_f32_tc(x, w, bias, again)
     k.gemm_f32_tc(x, w, bias, low)
     assert torch.equal(again, got) and torch.equal(low, got.bfloat16())          # the order of the sums is fixed; counters are back at zero
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 6, 8, 12, 16])
+@pytest.mark.parametrize("apart", [False, True])
+@pytest.mark.parametrize("positive", [False, True])
+def test_rows_of_few_terms(n, apart, positive):
+    """Rows of X with n entries, in one or two blocks of 32 of K or all over it: as close to 64 bits as one 32-bit FMA behind another."""
+    from gguf_rs_cli_b200 import kernels as k
+    T, N, K = 64, 1024, 2048
+    full, w = _operands(T, N, K, 10 * n + apart, positive)
+    x = torch.zeros_like(full)
+    for t in range(T):
+        at = torch.randperm(K, device=DEV)[:n] if apart else (torch.arange(n, device=DEV) + 37 * t) % K
+        x[t, at] = full[t, at]
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    got, plain = torch.empty(T, N, device=DEV), torch.empty(T, N, device=DEV)
+    k.gemm_f32_tc(x, w, None, got)
+    k.gemm_f32(x, w, None, plain)
+    e, e_plain = [float((a.double() - want).norm() / want.norm()) for a in (got, plain)]
+    # Terms far apart are rounded when their piece of K is complete and again when the pieces are added, an FMA once: 1.15 to 1.19 measured for two to four.
+    assert e <= (1.01 if n == 1 else 1.25 if apart else 1.0) * e_plain, (e, e_plain)
+    # one product: its large part is exact, the small ones are cut at 2^-23 of themselves, 2^-8 of it, and the sum is rounded once; n: n sums of either kind
+    # and of pieces, each rounded once
+    assert ((got.double() - want).abs() <= (1 if n == 1 else 3 * n) * (1 + 2.0 ** -6) * 2.0 ** -24 * size).all()
 
 
 def test_rows_of_larger_matrices_and_the_dispatch():
