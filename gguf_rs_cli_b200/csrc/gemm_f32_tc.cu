@@ -3,7 +3,7 @@
 //
 // Every operand is cut into three bfloat16 terms, each the rest rounded to nearest, so that nothing is left behind the third (x = h + m + l: the
 // scheme of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", 2019), and eight
-// of the nine products of terms are taken; l l, 2^-36 of a product, is left out.  The tensor core cuts its 32-bit sums instead of rounding them, so it
+// of the nine products of terms are taken; l l, 2^-34 of a product, is left out.  The tensor core cuts its 32-bit sums instead of rounding them, so it
 // is given little to cut: a block of 32 of K has a sum of its own for h h, whose products have 16 bits, and the blocks' sums are added in
 // registers, rounded to nearest; the seven small products are summed in a second accumulator over a piece of K, where a lost bit is 2^-8 of
 // that, and added behind its last block.  Against 64 bits (2,048 of K, 32-bit FMAs one behind another in brackets, of the result's norm): one term in a row
@@ -24,8 +24,8 @@
 //
 // A CTA has one tile of 128 features x BN tokens and some pieces of K.  Warp 0 copies 32-bit blocks of both operands by TMA
 // (128-byte swizzle) into a ring, warp 1 issues the MMAs, eight or sixteen warps convert a block (of W a row and half of the block a
-// thread, of X a quarter of a row) and add the sums of an earlier block.  Where CTAs share a tile they are all
-// resident, wait for one another (bounded) and finish a share of the tokens each.
+// thread, of X a quarter of a row) and add the sums of an earlier block.  Where a tile is one CTA's, its pieces' sums are added as they come; else they go to
+// scratch memory and a second kernel adds them: no CTA waits for another, whatever runs beside them.
 #include <mutex>
 
 #include "common.cuh"
@@ -36,6 +36,7 @@ using namespace sm100;
 namespace {
 
 constexpr int FX_BM = 128, FX_BK = 32;
+constexpr int FX_PIECES = 16;                   // of K, at most
 
 template <int BN> struct FxCfg {
     static constexpr int W_BYTES = FX_BM * 128, X_BYTES = BN * 128, RAW = W_BYTES + X_BYTES;
@@ -60,12 +61,11 @@ struct FxParams {
     const float* w;
     const void* bias;
     void* out;
-    float* scratch;       // [tiles][pieces][BN][128] sums of the pieces of K
-    int* counters;        // [tiles], zero between launches
+    float* scratch;       // [tiles][pieces][slot_cols][128] sums of the pieces of K, where a tile is not one CTA's
     int* status;
     long long ldx, ldw, ldo;
     int bias_dtype, out_dtype;
-    int T, N, K, pieces, sharers, t_tiles;
+    int T, N, K, pieces, tiles, t_tiles, slot_cols;
 };
 
 // Two numbers in three bfloat16 terms each, the first in the low halves: each term the rest, rounded to nearest; nothing is left behind the third.
@@ -123,7 +123,6 @@ template <int N> __device__ __forceinline__ void fx_add(float (&acc)[N], uint32_
         for (int j = 0; j < STEP; ++j) acc[c + j] += v[j];
     }
 }
-template <int THREADS> __device__ __forceinline__ void fx_workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
 
 // A sum that is not finite or next to nothing, taken again one product behind another.
 __device__ __noinline__ float fx_again(const float* x, const float* w, int K) {
@@ -150,18 +149,17 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
     uint8_t* xs = ring + RING * Cfg::RAW;          // X's terms: rows of 128 bytes, [h | m] of each buffer, then [l of an even buffer | l of an odd one]
     __shared__ uint64_t raw_full[RING], raw_empty[RING], op_full[DEPTH], done[DEPTH], sum_free, tail_free[TAILS];
     __shared__ uint32_t tmem_base;
-    __shared__ int abort_flag, all_there;
+    __shared__ int abort_flag;
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    const int tile = blockIdx.x / p.sharers, me = blockIdx.x - tile * p.sharers;
-    const int n0 = tile / p.t_tiles * FX_BM, t0 = (tile % p.t_tiles) * BN;
+    // This CTA's units, pieces of K of tiles one behind another: all of one tile (whole), or some, and then their sums go to scratch memory.
     const int blocks = (p.K + FX_BK - 1) / FX_BK;
-    // this CTA's pieces of K, and their blocks
-    const int piece0 = me * p.pieces / p.sharers, piece1 = (me + 1) * p.pieces / p.sharers;
-    // one CTA's two pieces: the second stays in registers (and one CTA's only piece does)
-    const bool keep = p.sharers == 1 && p.pieces <= 2;
-    auto piece_begin = [&](int i) { return int((long long)i * blocks / p.pieces); };
-    const int b0 = piece_begin(piece0), S = piece_begin(piece1) - b0;
+    const bool whole = gridDim.x == p.tiles;
+    const int units = p.tiles * p.pieces, unit0 = int((long long)blockIdx.x * units / gridDim.x), unit1 = int((long long)(blockIdx.x + 1) * units / gridDim.x);
+    const int tile0 = unit0 / p.pieces, piece0 = unit0 - tile0 * p.pieces;
+    auto piece_begin = [&](int i) { return i * blocks / p.pieces; };          // i <= 16, blocks < 2^26
+    auto piece_blocks = [&](int unit) { const int i = unit % p.pieces; return piece_begin(i + 1) - piece_begin(i); };
+    const int S = (unit1 / p.pieces - tile0) * blocks + piece_begin(unit1 % p.pieces) - piece_begin(piece0);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < RING; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WORKERS); }
@@ -184,28 +182,33 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
     gb_grid_launch_dependents();
     gb_grid_wait();
 
-    float acc[COLS];
+    constexpr bool TOTAL = BN <= 96;              // a whole tile's pieces are added in registers of their own
+    float acc[COLS], total[TOTAL ? COLS : 1];
 #pragma unroll
     for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+#pragma unroll
+    for (int i = 0; i < (TOTAL ? COLS : 1); ++i) total[i] = 0.f;
     const int quarter = warp & 3, row = quarter * 32 + lane, group = (warp - 2) >> 2, half = group & 1;       // of the workers
-    const int cols = min(BN, p.T - t0), mine = group * COLS;
+    const int mine = group * COLS;
 
     if (warp == 0) {
         if (elect_one()) {
+            int tile = tile0, kb = piece_begin(piece0);
             for (int s = 0; s < S; ++s) {
                 const int slot = s % RING;
                 if (s >= RING && !mbar_wait(&raw_empty[slot], (s / RING - 1) & 1)) { atomicExch(p.status, 21); abort_flag = 1; break; }
                 uint8_t* dst = ring + slot * Cfg::RAW;
                 mbar_expect_tx(&raw_full[slot], Cfg::RAW);
-                tma_load_2d(dst, &map_w, (b0 + s) * FX_BK, n0, &raw_full[slot]);
-                tma_load_2d(dst + Cfg::W_BYTES, &map_x, (b0 + s) * FX_BK, t0, &raw_full[slot]);
+                tma_load_2d(dst, &map_w, kb * FX_BK, tile / p.t_tiles * FX_BM, &raw_full[slot]);
+                tma_load_2d(dst + Cfg::W_BYTES, &map_x, kb * FX_BK, tile % p.t_tiles * BN, &raw_full[slot]);
+                if (++kb == blocks) { kb = 0; ++tile; }
             }
         }
     } else if (warp == 1) {
         if (elect_one()) {
             constexpr uint32_t idesc = instr_desc_bf16(FX_BM, BN);
             const uint32_t xa = smem_u32(xs);
-            int piece = 0, piece_end = piece_begin(piece0 + 1) - b0, more = 0;         // pieces before this one; whether it has begun
+            int piece = 0, piece_end = piece_blocks(unit0), more = 0;         // pieces before this one; whether it has begun
             for (int s = 0; s < S; ++s) {
                 const int b = s % DEPTH, tail = piece % TAILS;
                 if (!mbar_wait(&op_full[b], (s / DEPTH) & 1)) { atomicExch(p.status, 22); abort_flag = 1; break; }
@@ -239,14 +242,14 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
                 if (s + 1 == piece_end) {
                     more = 0;
                     ++piece;
-                    piece_end = piece_begin(min(piece0 + piece + 1, p.pieces)) - b0;
+                    piece_end += piece_blocks(unit0 + piece);
                 }
             }
         }
     } else {
         const uint32_t ring_a = smem_u32(ring), xs_a = smem_u32(xs);
         const uint32_t lane_base = uint32_t(quarter * 32) << 16;
-        int piece = piece0, piece_end = piece_begin(piece0 + 1) - b0;           // the piece whose blocks are being added
+        int unit = unit0, piece_end = piece_blocks(unit0);                      // the piece whose blocks are being added
         const bool does_w = WORKERS == 8 || warp < 10, does_x = WORKERS == 8 || warp >= 10;
         const int xw = (warp - 2) & 7;
         // block s: its sums and, behind a piece's last block, those of the piece's small products
@@ -264,23 +267,49 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
                 if (lane == 0) mbar_arrive(&sum_free);
             }
             if (s + 1 == piece_end) {
-                const int tail = (piece - piece0) % TAILS;
+                const int tail = (unit - unit0) % TAILS;
                 fx_add<COLS>(acc, tmem + lane_base + Cfg::T_COL + tail * BN + mine);
                 if (LATE) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&tail_free[tail]);
                 }
-                if (!(keep && piece + 1 == p.pieces)) {
-                    float* to = p.scratch + (size_t(tile) * p.pieces + piece) * (BN * FX_BM) + row;
+                const int tile = unit / p.pieces, piece = unit - tile * p.pieces, t0 = tile % p.t_tiles * BN, cols = min(BN, p.T - t0);
+                if (!whole) {
+                    float* to = p.scratch + size_t(unit) * (p.slot_cols * FX_BM) + row;
 #pragma unroll
                     for (int c = 0; c < COLS; ++c) {
                         if (mine + c < cols) __stcg(to + size_t(mine + c) * FX_BM, acc[c]);
                         acc[c] = 0.f;
                     }
+                } else if constexpr (TOTAL) {
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) {
+                        total[c] = piece ? total[c] + acc[c] : acc[c];
+                        acc[c] = 0.f;
+                    }
+                } else if (p.pieces > 1) {
+                    // no registers for a second set of sums: they wait in the result's place, which is 32 bits wide then
+                    const int n = tile / p.t_tiles * FX_BM + row;
+                    float* to = reinterpret_cast<float*>(p.out) + size_t(t0 + mine) * p.ldo + n;
+                    const int m = n < p.N ? cols - mine : 0;
+#pragma unroll
+                    for (int c0 = 0; c0 < COLS; c0 += 8) {
+                        float v[8];
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) v[c] = piece && c0 + c < m ? __ldcg(to + (c0 + c) * p.ldo) : 0.f;
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            if (piece) acc[c0 + c] = v[c] + acc[c0 + c];
+                            if (unit + 1 < unit1) {
+                                if (c0 + c < m) __stcg(to + (c0 + c) * p.ldo, acc[c0 + c]);
+                                acc[c0 + c] = 0.f;
+                            }
+                        }
+                    }
                 }
-                ++piece;
-                piece_end = piece_begin(min(piece + 1, p.pieces)) - b0;
+                ++unit;
+                piece_end += piece_blocks(unit);
             }
             return true;
         };
@@ -344,74 +373,36 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, Cfg::TMEM_COLS);
-    if (abort_flag) return;
-    if (warp < 2) return;
+    if (abort_flag || warp < 2 || !whole) return;
 
-    const int n = n0 + row;
+    const int n = tile0 / p.t_tiles * FX_BM + row, t0 = tile0 % p.t_tiles * BN, cols = min(BN, p.T - t0);
     const float bias = p.bias && n < p.N ? gb_load(p.bias, p.bias_dtype, n) : 0.f;
-    if (keep) {
-        if (p.pieces == 2) {                            // what this thread has stored itself
-            const float* first = p.scratch + size_t(tile) * 2 * (BN * FX_BM) + row;
+    if (n < p.N) {
 #pragma unroll
-            for (int c = 0; c < COLS; ++c)
-                if (mine + c < cols) acc[c] = __ldcg(first + size_t(mine + c) * FX_BM) + acc[c];
-        }
-        if (n < p.N) {
-#pragma unroll
-            for (int c = 0; c < COLS; ++c)
-                if (mine + c < cols) fx_store(p, t0 + mine + c, n, acc[c], bias);
-        }
-        return;
+        for (int c = 0; c < COLS; ++c)
+            if (mine + c < cols) fx_store(p, t0 + mine + c, n, TOTAL ? total[TOTAL ? c : 0] : acc[c], bias);
     }
-    __threadfence();
-    fx_workers_sync<Cfg::WORKERS * 32>();
-    if (p.sharers > 1) {
-        if (threadIdx.x == 64) {
-            atomicAdd(&p.counters[tile], 1);
-            int seen = 0;
-            uint64_t start = 0;
-            for (uint32_t i = 0;; ++i) {
-                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.counters + tile) : "memory");
-                if (seen >= p.sharers) break;
-                __nanosleep(40);
-                if ((i & 255) == 255) {
-                    const uint64_t now = global_timer_ns();
-                    if (start == 0) start = now;
-                    else if (now - start > WAIT_NS) break;
-                }
-            }
-            all_there = seen >= p.sharers;
-            if (!all_there) atomicExch(p.status, 25);
-        }
-        fx_workers_sync<Cfg::WORKERS * 32>();
-        if (!all_there) return;
-    }
-    const int c_lo = me * cols / p.sharers, c_hi = (me + 1) * cols / p.sharers;
-    const float* base = p.scratch + size_t(tile) * p.pieces * (BN * FX_BM) + row;
-    for (int c0 = c_lo + group * 4; c0 < c_hi; c0 += 4 * Cfg::GROUPS) {
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int s0 = 0; s0 < p.pieces; s0 += 8) {
-            float ld[8][4];
+}
+
+// The sums of the pieces of tiles that were not one CTA's, added in order: a feature a thread, tokens 2 gridDim.y apart.
+__global__ void __launch_bounds__(2 * FX_BM) gemm_f32_tc_merge_kernel(FxParams p, int bn) {
+    gb_grid_launch_dependents();
+    gb_grid_wait();
+    const int tile = blockIdx.x, row = threadIdx.x & (FX_BM - 1);
+    const int n = tile / p.t_tiles * FX_BM + row, t0 = tile % p.t_tiles * bn, cols = min(bn, p.T - t0);
+    if (n >= p.N) return;
+    const float bias = p.bias ? gb_load(p.bias, p.bias_dtype, n) : 0.f;
+    const size_t slot = size_t(p.slot_cols) * FX_BM;
+    for (int c = 2 * blockIdx.y + (threadIdx.x >> 7); c < cols; c += 2 * gridDim.y) {
+        const float* from = p.scratch + size_t(tile) * p.pieces * slot + size_t(c) * FX_BM + row;
+        float v[FX_PIECES];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < FX_PIECES; ++i) v[i] = i < p.pieces ? __ldcg(from + i * slot) : 0.f;
+        float sum = v[0];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    ld[i][j] = s0 + i < p.pieces && c0 + j < c_hi ? __ldcg(base + (size_t(s0 + i) * BN + c0 + j) * FX_BM) : 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] += ld[i][j];
-        }
-        if (n < p.N) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (c0 + j < c_hi) fx_store(p, t0 + c0 + j, n, v[j], bias);
-        }
-    }
-    if (p.sharers > 1) {
-        // the last of the tile's CTAs to have read the others' sums puts the counter back for the next launch
-        fx_workers_sync<Cfg::WORKERS * 32>();
-        if (threadIdx.x == 64 && atomicAdd(&p.counters[tile], 1) == 2 * p.sharers - 1) p.counters[tile] = 0;
+        for (int i = 1; i < FX_PIECES; ++i)
+            if (i < p.pieces) sum += v[i];
+        fx_store(p, t0 + c, n, sum, bias);
     }
 }
 
@@ -430,8 +421,9 @@ int ensure_status() {
     return 0;
 }
 
+constexpr int MAX_DEVICES = 64;
+
 template <int BN> int launch_fx(const CUtensorMap& mw, const CUtensorMap& mx, const FxParams& p, int ctas, cudaStream_t stream) {
-    constexpr int MAX_DEVICES = 64;
     static bool configured[MAX_DEVICES] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return gb_fail("gb_gemm_f32_tc: no usable current device");
@@ -442,6 +434,12 @@ template <int BN> int launch_fx(const CUtensorMap& mw, const CUtensorMap& mx, co
     }
     gb_launch(gemm_f32_tc_kernel<BN>, dim3(ctas), dim3(FxCfg<BN>::THREADS), FxCfg<BN>::SMEM, stream, mw, mx, p);
     GB_LAUNCH_OK("gb_gemm_f32_tc");
+    if (ctas != p.tiles) {
+        int slices = 1280 / p.tiles;                                 // a token a thread, or a few: up to eight blocks an SM
+        slices = slices > (p.slot_cols + 1) / 2 ? (p.slot_cols + 1) / 2 : slices > 0 ? slices : 1;
+        gb_launch(gemm_f32_tc_merge_kernel, dim3(p.tiles, slices), dim3(2 * FX_BM), 0, stream, p, BN);
+        GB_LAUNCH_OK("gb_gemm_f32_tc (merge)");
+    }
     return 0;
 }
 
@@ -451,26 +449,34 @@ template <int BN> int launch_fx(const CUtensorMap& mw, const CUtensorMap& mx, co
 int fx_pieces(int N, int K, int sms) {
     const int tiles = (N + FX_BM - 1) / FX_BM, blocks = (K + FX_BK - 1) / FX_BK;
     int n = 2 * sms / tiles;
-    if (n > 16) n = 16;
+    if (n > FX_PIECES) n = FX_PIECES;
     if (n > blocks / 4) n = blocks / 4;
     return n > 1 ? n : 1;
 }
-// The tile and the number of CTAs on each that take the least time: rounds over the device times blocks of K times a block's
-// time, with what a CTA takes beside its blocks, and a merge.  A block's time as measured at 16,384 x 2,048, microseconds.
-struct FxCut { int bn, pieces, sharers; long long tiles; };
-FxCut fx_cut(int T, int N, int K, int sms, bool may_share, int n_counters) {
+// The tile and the number of CTAs that take the least time: rounds over the device times blocks of K times a block's time, with what a CTA
+// takes beside its blocks, and where tiles are not one CTA's each the merge behind and the bytes that go there and back.  A block's time as
+// measured at 16,384 x 2,048, microseconds.  The scratch memory of a launch is bounded (FX_SCRATCH floats); one CTA's tile needs none.
+struct FxCut { int bn, pieces, ctas; long long tiles, scratch; };
+constexpr long long FX_SCRATCH = 8LL << 20;
+FxCut fx_cut(int T, int N, int K, int out_dtype, int sms) {
     static const int BNS[7] = {16, 32, 64, 96, 128, 160, 192};
     static const double BLOCK[7] = {0.9, 1.0, 0.8, 0.87, 0.97, 1.12, 1.3};
     const int blocks = (K + FX_BK - 1) / FX_BK, pieces = fx_pieces(N, K, sms);
-    FxCut best = {16, pieces, 1, 0};
+    FxCut best = {16, pieces, 0, 0, 0};
     double least = 1e300;
     for (int i = 0; i < 7; ++i) {
-        const long long tiles = (long long)((N + FX_BM - 1) / FX_BM) * ((T + BNS[i] - 1) / BNS[i]), resident = (BNS[i] <= 32 ? 2LL : 1LL) * sms;
-        for (int sharers = 1; sharers <= pieces; ++sharers) {
-            if (sharers > 1 && (!may_share || tiles * sharers > resident || tiles > n_counters)) break;
-            const int each = (pieces + sharers - 1) / sharers * ((blocks + pieces - 1) / pieces);
-            const double cost = double((tiles * sharers + resident - 1) / resident) * (each * BLOCK[i] + 4.0) + (sharers > 1 ? 3.0 : 0.0);
-            if (cost < least) { least = cost; best = {BNS[i], pieces, sharers, tiles}; }
+        const int bn = BNS[i];
+        const long long tiles = (long long)((N + FX_BM - 1) / FX_BM) * ((T + bn - 1) / bn), places = (bn <= 32 ? 2LL : 1LL) * sms;
+        if (bn <= 96 || pieces == 1 || out_dtype == GB_F32) {       // wider ones keep a piece's sums in a 32-bit result
+            const double cost = double((tiles + places - 1) / places) * (blocks * BLOCK[i] + 4.0);
+            if (cost < least) { least = cost; best = {bn, pieces, int(tiles), tiles, 0}; }
+        }
+        const long long scratch = tiles * pieces * (T < bn ? T : bn) * FX_BM;
+        for (int each = 1; each < pieces; ++each) {                   // pieces a CTA
+            const int sharers = (pieces + each - 1) / each;
+            if (tiles * sharers > places || scratch > FX_SCRATCH) continue;
+            const double cost = each * ((blocks + pieces - 1) / pieces) * BLOCK[i] + 8.0 + 2e-6 * scratch;
+            if (cost < least) { least = cost; best = {bn, pieces, int(tiles * sharers), tiles, scratch}; }
         }
     }
     return best;
@@ -490,33 +496,32 @@ GB_API int gb_gemm_f32_tc_supported(const void* X, long long ldx, const void* W,
            (reinterpret_cast<uintptr_t>(W) & 15) == 0;
 }
 
-// Floats of scratch that a launch of these sizes needs, with counters or without (0: K is one piece).
-GB_API long long gb_gemm_f32_tc_scratch_floats(int T, int N, int K, int sms, int n_counters) {
-    const FxCut c = fx_cut(T, N, K, sms, n_counters > 0, n_counters);
-    return c.pieces > 1 ? c.tiles * c.pieces * c.bn * FX_BM : 0;
+// Floats of scratch that a launch of these sizes needs (0: every tile is one CTA's); never more than gb_gemm_f32_tc_scratch_max.
+GB_API long long gb_gemm_f32_tc_scratch_floats(int T, int N, int K, int out_dtype, int sms) {
+    return T > 0 && N > 0 && K > 0 && sms > 0 ? fx_cut(T, N, K, out_dtype, sms).scratch : 0;
 }
+GB_API long long gb_gemm_f32_tc_scratch_max() { return FX_SCRATCH; }
 
-// scratch: gb_gemm_f32_tc_scratch_floats floats, counters: n_counters zeroed ints (left zero), null with n_counters 0: no two CTAs share a tile.
+// scratch: gb_gemm_f32_tc_scratch_floats floats.
 GB_API int gb_gemm_f32_tc(const float* X, long long ldx, const float* W, long long ldw, const void* bias, int bias_dtype, void* out,
-                          int out_dtype, long long ldo, int T, int N, int K, float* scratch, int* counters, int n_counters, int sms,
-                          cudaStream_t stream) {
+                          int out_dtype, long long ldo, int T, int N, int K, float* scratch, int sms, cudaStream_t stream) {
     GB_REQUIRE(gb_is_dtype(out_dtype) && (!bias || gb_is_dtype(bias_dtype)), "gb_gemm_f32_tc: bad dtype");
     GB_REQUIRE(T >= 0 && N > 0 && K > 0 && ldx >= K && ldw >= K && ldo >= N && sms > 0,
                "gb_gemm_f32_tc: bad sizes T=%d N=%d K=%d ldx=%lld ldw=%lld ldo=%lld", T, N, K, ldx, ldw, ldo);
     GB_REQUIRE(gb_gemm_f32_tc_supported(X, ldx, W, ldw, K), "gb_gemm_f32_tc: rows must start on 16 bytes (K=%d, pitches %lld and %lld)", K, ldx, ldw);
     if (T == 0) return 0;
     if (ensure_status()) return 1;
-    const FxCut cut = fx_cut(T, N, K, sms, counters && n_counters > 0, counters ? n_counters : 0);
-    GB_REQUIRE(cut.pieces == 1 || scratch, "gb_gemm_f32_tc: N=%d K=%d needs scratch memory", N, K);
-    GB_REQUIRE(cut.tiles * cut.sharers < (1LL << 31), "gb_gemm_f32_tc: T=%d N=%d is more work than one launch numbers", T, N);
+    const FxCut cut = fx_cut(T, N, K, out_dtype, sms);
+    GB_REQUIRE(cut.scratch == 0 || scratch, "gb_gemm_f32_tc: T=%d N=%d K=%d needs scratch memory", T, N, K);
+    GB_REQUIRE(cut.tiles * cut.pieces < (1LL << 31), "gb_gemm_f32_tc: T=%d N=%d is more work than one launch numbers", T, N);
     FxParams p;
-    p.x = X; p.w = W; p.bias = bias; p.out = out; p.scratch = scratch; p.counters = counters; p.status = g_status_dev;
+    p.x = X; p.w = W; p.bias = bias; p.out = out; p.scratch = scratch; p.status = g_status_dev;
     p.ldx = ldx; p.ldw = ldw; p.ldo = ldo; p.bias_dtype = bias_dtype; p.out_dtype = out_dtype; p.T = T; p.N = N; p.K = K;
-    p.pieces = cut.pieces; p.sharers = cut.sharers; p.t_tiles = (T + cut.bn - 1) / cut.bn;
+    p.pieces = cut.pieces; p.tiles = int(cut.tiles); p.t_tiles = (T + cut.bn - 1) / cut.bn; p.slot_cols = T < cut.bn ? T : cut.bn;
     CUtensorMap mw, mx;
     if (tensor_map_f32_2d(W, N, K, ldw, FX_BM, &mw)) return 1;
     if (tensor_map_f32_2d(X, T, K, ldx, cut.bn, &mx)) return 1;
-    const int ctas = int(cut.tiles * cut.sharers);
+    const int ctas = cut.ctas;
     switch (cut.bn) {
         case 16: return launch_fx<16>(mw, mx, p, ctas, stream);
         case 32: return launch_fx<32>(mw, mx, p, ctas, stream);

@@ -3,7 +3,6 @@ stream.  Nothing here computes; a missing or failing library raises NativeError.
 """
 from __future__ import annotations
 
-import threading
 from typing import Optional, Tuple
 
 import torch
@@ -1189,39 +1188,15 @@ def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
     T, K = x.shape
     N = w.shape[0]
     assert w.shape[1] == K and x.dtype == w.dtype == torch.float32 and out.shape == (T, N) and out.stride(1) == 1
-    sms = tc_scratch(x.device).sms
-    counters, scratch = _f32_counters(x.device), None
-    need = native.library().gb_gemm_f32_tc_scratch_floats(T, N, K, sms, 0 if counters is None else counters.numel())
+    sms, scratch = tc_scratch(x.device).sms, None
+    need = native.library().gb_gemm_f32_tc_scratch_floats(T, N, K, dtype_code(out), sms)
     if need:
         scratch = torch.empty(need, dtype=torch.float32, device=x.device)
     call("gb_gemm_f32_tc", ptr(x), x.stride(0), ptr(w), w.stride(0), ptr(bias), 0 if bias is None else dtype_code(bias), ptr(out),
-         dtype_code(out), out.stride(0), T, N, K, ptr(scratch), ptr(counters), 0 if counters is None else counters.numel(), sms, stream_ptr())
+         dtype_code(out), out.stride(0), T, N, K, ptr(scratch), sms, stream_ptr())
+    if need:
+        native.count_launches(1)                              # the pieces' sums are added by a second kernel
     return out
-
-
-_f32_counter_buffers, _f32_counter_rows, _f32_counter_lock = {}, {}, threading.Lock()
-F32_COUNTER_STREAMS = 64         # 16 KB each; launches on further streams share no tiles
-
-
-def _f32_counters(device) -> Optional[torch.Tensor]:
-    """Arrival counters of the 32-bit tensor-core products on the current stream, zero between launches.  Products on different
-    streams may run at the same time, so each stream has its own; all are allocated at a device's first product, so that a
-    stream's first may be one that is being captured."""
-    index = torch.device(device).index or 0
-    key = (index, stream_ptr())
-    got = _f32_counter_rows.get(key)
-    if got is not None:
-        return got
-    with _f32_counter_lock:
-        if index not in _f32_counter_buffers:
-            if torch.cuda.is_current_stream_capturing():
-                return None
-            _f32_counter_buffers[index] = torch.zeros(F32_COUNTER_STREAMS, _TcScratch.COUNTERS, dtype=torch.int32, device=device)
-            torch.cuda.synchronize(index)                             # zero for every stream
-        taken = sum(k[0] == index for k in _f32_counter_rows)
-        if key not in _f32_counter_rows and taken < F32_COUNTER_STREAMS:
-            _f32_counter_rows[key] = _f32_counter_buffers[index][taken]
-        return _f32_counter_rows.get(key)
 
 
 GROUPED_TILE = 256               # tokens of a tile of the kernel that pairs two SMs
@@ -1480,8 +1455,6 @@ def check_tc_status() -> None:
     code = lib.gb_gemm_f32_tc_status()
     if code:
         lib.gb_gemm_f32_tc_status_clear()
-        for counters in _f32_counter_buffers.values():
-            counters.zero_()
         raise native.NativeError(f"a 32-bit tensor-core product gave up waiting (code {code}); its output is invalid")
     code = lib.gb_attention_tc_status()
     if code:

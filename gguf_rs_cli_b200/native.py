@@ -225,11 +225,12 @@ _SIGNATURES = {
     "gb_attention_decode_set_two_warps": [_I],
     "gb_attention_decode_set_stamps": [_P],
     "gb_gemm_f32": [_P, _L, _P, _L, _P, _I, _P, _I, _L, _I, _I, _I, _P],
-    "gb_gemm_f32_tc": [_P, _L, _P, _L, _P, _I, _P, _I, _L, _I, _I, _I, _P, _P, _I, _I, _P],
+    "gb_gemm_f32_tc": [_P, _L, _P, _L, _P, _I, _P, _I, _L, _I, _I, _I, _P, _I, _P],
     "gb_gemm_f32_tc_supported": [_P, _L, _P, _L, _I],
     "gb_gemm_f32_tc_status": [],
     "gb_gemm_f32_tc_status_clear": [],
     "gb_gemm_f32_tc_scratch_floats": [_I, _I, _I, _I, _I],
+    "gb_gemm_f32_tc_scratch_max": [],
     "gb_gemm_f32_supported": [_P, _L, _P, _L, _I],
     "gb_gemm_tc_set_pair_tile": [_I],
     "gb_gemm_tc_pair_slots": [],
@@ -247,7 +248,7 @@ _SIGNATURES = {
     "gb_tc_status": [],
     "gb_tc_status_clear": [],
 }
-_RESTYPES = {"gb_gemm_f32_tc_scratch_floats": ctypes.c_longlong, "gb_retention_chunk_floats": ctypes.c_longlong, "gb_rglru_segment_floats": ctypes.c_longlong, "gb_delta_rule_scratch_floats": ctypes.c_longlong, "gb_gla_scratch_floats": ctypes.c_longlong, "gb_gla_segment_floats": ctypes.c_longlong, "gb_selective_scan_segment_floats": ctypes.c_longlong, "gb_linear_walk_scratch_floats": ctypes.c_longlong, "gb_moe_grouped_scratch_ints": ctypes.c_longlong, "gb_latent_decode_scratch_floats": ctypes.c_longlong, "gb_gemm_tc_scratch_floats": ctypes.c_longlong, "gb_attention_decode_scratch_floats": ctypes.c_longlong}
+_RESTYPES = {"gb_gemm_f32_tc_scratch_max": ctypes.c_longlong, "gb_gemm_f32_tc_scratch_floats": ctypes.c_longlong, "gb_retention_chunk_floats": ctypes.c_longlong, "gb_rglru_segment_floats": ctypes.c_longlong, "gb_delta_rule_scratch_floats": ctypes.c_longlong, "gb_gla_scratch_floats": ctypes.c_longlong, "gb_gla_segment_floats": ctypes.c_longlong, "gb_selective_scan_segment_floats": ctypes.c_longlong, "gb_linear_walk_scratch_floats": ctypes.c_longlong, "gb_moe_grouped_scratch_ints": ctypes.c_longlong, "gb_latent_decode_scratch_floats": ctypes.c_longlong, "gb_gemm_tc_scratch_floats": ctypes.c_longlong, "gb_attention_decode_scratch_floats": ctypes.c_longlong}
 
 
 def register_signature(name: str, argtypes) -> None:

@@ -32,7 +32,7 @@ def test_closer_to_64_bits_than_one_thread(T, N, K, positive):
     torch.cuda.synchronize()
     k.check_tc_status()
     e, e_plain = [float((a.double() - want).norm() / want.norm()) for a in (got, plain)]
-    # a result is rounded once (2^-25 in the mean of a binade's ends) and the sums of 32 that it adds are; the products left out are 2^-36
+    # a result is rounded once (2^-25 in the mean of a binade's ends) and the sums of 32 that it adds are; the product left out is 2^-34
     assert e <= max(1.1 * e_plain, 1.5e-7) and e < 4e-7, (e, e_plain)
     assert (got._base[:, N:] == 7.0).all()
     again, low = torch.empty_like(plain), torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
@@ -133,3 +133,52 @@ def test_streams_have_counters_of_their_own():
     torch.cuda.synchronize()
     k.check_tc_status()
     assert all(torch.equal(o, want) for o in outs)
+
+
+@pytest.mark.parametrize("T, N, K", [(2048, 2048, 2048), (2048, 2048, 8192), (1500, 1100, 14336), (5000, 2048, 1024), (187, 16384, 2048), (1, 40000, 1024)])
+def test_scratch_memory_is_bounded(T, N, K):
+    """However many tokens and pieces of K: sums wait in registers, in the result, or in memory of a fixed size; a row's bits stay what they are alone."""
+    from gguf_rs_cli_b200 import kernels as k, native
+    x, w = _operands(T, N, K, N + K)
+    most = native.library().gb_gemm_f32_tc_scratch_max()
+    assert most <= 8 << 20
+    for code in (0, 1):
+        assert native.library().gb_gemm_f32_tc_scratch_floats(T, N, K, code, 148) <= most
+    got, low = torch.empty(T, N, device=DEV), torch.empty(T, N, device=DEV, dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    k.gemm_f32_tc(x, w, None, got)
+    k.gemm_f32_tc(x, w, None, low)
+    torch.cuda.synchronize()
+    k.check_tc_status()
+    assert torch.cuda.max_memory_allocated() - before <= 4 * most + (1 << 20)
+    assert torch.equal(low, got.bfloat16())
+    for lo, hi in ((0, 1), (T // 2, T // 2 + 40), (T - 1, T)):
+        hi = min(hi, T)
+        part = torch.empty(hi - lo, N, device=DEV)
+        k.gemm_f32_tc(x[lo:hi], w, None, part)
+        assert torch.equal(part, got[lo:hi])
+    want = x.double() @ w.double().T
+    assert float((got.double() - want).norm() / want.norm()) < 4e-7
+
+
+def test_products_on_two_streams_wait_for_nobody():
+    """Launches that share the device with one another, of every width, shared tiles among them: nothing waits for CTAs that have not started."""
+    from gguf_rs_cli_b200 import kernels as k
+    cases = [(_operands(T, N, K, T + K), T, N) for T, N, K in ((1, 2048, 8192), (30, 4096, 4096), (100, 2048, 8192), (187, 2048, 2048), (60, 3072, 2048))]
+    want = []
+    for (x, w), T, N in cases:
+        want.append(torch.empty(T, N, device=DEV))
+        k.gemm_f32_tc(x, w, None, want[-1])
+    torch.cuda.synchronize()
+    streams, outs = [torch.cuda.Stream() for _ in range(4)], []
+    for i in range(40):
+        for j, s in enumerate(streams):
+            (x, w), T, N = cases[(i + j) % len(cases)]
+            with torch.cuda.stream(s):
+                outs.append(((i + j) % len(cases), torch.empty(T, N, device=DEV)))
+                k.gemm_f32_tc(x, w, None, outs[-1][1])
+    torch.cuda.synchronize()
+    k.check_tc_status()
+    assert all(torch.equal(o, want[i]) for i, o in outs)
