@@ -1182,15 +1182,18 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     return out
 
 
-def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
-    """32-bit operands on the tensor cores, three bfloat16 terms each; the same operands as gemm_f32."""
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, ws=None) -> torch.Tensor:
+    """32-bit operands on the tensor cores, three bfloat16 terms each; the same operands as gemm_f32.  ws: the engine's buffers
+    (parts.base.Workspace), whose products follow one another; without one the scratch memory is the call's own."""
     _cuda(x, w, bias, out)
     T, K = x.shape
     N = w.shape[0]
     assert w.shape[1] == K and x.dtype == w.dtype == torch.float32 and out.shape == (T, N) and out.stride(1) == 1
     sms, scratch = tc_scratch(x.device).sms, None
     need = native.library().gb_gemm_f32_tc_scratch_floats(T, N, K, dtype_code(out), sms)
-    if need:
+    if need and ws is not None:                               # one buffer for all sizes: it is there before a step is captured
+        scratch = ws.get("gemm_f32.scratch", (native.library().gb_gemm_f32_tc_scratch_max(),), torch.float32)
+    elif need:
         scratch = torch.empty(need, dtype=torch.float32, device=x.device)
     call("gb_gemm_f32_tc", ptr(x), x.stride(0), ptr(w), w.stride(0), ptr(bias), 0 if bias is None else dtype_code(bias), ptr(out),
          dtype_code(out), out.stride(0), T, N, K, ptr(scratch), sms, stream_ptr())
@@ -1473,13 +1476,13 @@ def _f32_on_tensor_cores(w: torch.Tensor) -> bool:
     return K >= 1024 and N * K >= 1 << 20 and N <= 1 << 16
 
 
-def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
+def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, ws=None) -> torch.Tensor:
     """The product path of every projection: a tensor-core kernel when dtype and sizes
-    fit it, else a CUDA-core kernel (two of them, with the same sums bit for bit)."""
+    fit it, else a CUDA-core kernel (two of them, with the same sums bit for bit).  ws: see gemm_f32_tc."""
     if gemm_tc_supported(x, w):
         return gemm_tc(x, w, bias, out)
     if gemm_f32_supported(x, w) and _f32_on_tensor_cores(w):
-        return gemm_f32_tc(x, w, bias, out)
+        return gemm_f32_tc(x, w, bias, out, ws)
     # one block of 16 of K and thousands of features: gemm_generic has nothing to wait for (16 x 16384 x 16 3.2 us, 6.8 in gemm_f32;
     # 1000 x 4096 x 16 9.4 and 12.5), and from K = 20 on gemm_f32 takes 0.7 to 0.8 as long in the mean
     if gemm_f32_supported(x, w) and not (x.shape[1] <= 16 and w.shape[0] > 1000):

@@ -58,5 +58,5 @@ class Linear:
             residual.pending, residual.xb, residual.ssq, residual.ssq_parts = None, xb, ssq, parts
             return None
         out = ctx.ws.get(buffer or self.name, (T, self.out_features), out_dtype or ctx.dtype)
-        out = kernels.gemm_tc(rows, self.weight, self.bias, out, **norm) if norm else kernels.gemm(x, self.weight, self.bias, out)
+        out = kernels.gemm_tc(rows, self.weight, self.bias, out, **norm) if norm else kernels.gemm(x, self.weight, self.bias, out, ctx.ws)
         return kernels.unary_act_(out, activation) if activation else out

@@ -101,7 +101,7 @@ class GatedLinearRecurrence(Part):
         if self.gates_in is not None:
             return kernels.head_matmul(u, n, self.gates_in, z, 2 * n)
         for b in range(self.blocks):
-            kernels.gemm(u[:, b * n:(b + 1) * n], self.gates[b], None, z[:, 2 * b * n:2 * (b + 1) * n])
+            kernels.gemm(u[:, b * n:(b + 1) * n], self.gates[b], None, z[:, 2 * b * n:2 * (b + 1) * n], ctx.ws)
         return z
 
     def forward(self, h, ctx: StepContext, run: RunView, residual=None) -> Optional[torch.Tensor]:

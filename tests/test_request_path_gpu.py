@@ -136,3 +136,34 @@ def test_index_arrays_of_long_and_short_sequences_side_by_side(lens):
         s = eng.open()
         assert torch.equal(row, eng.step([Entry(s, p, (len(p) - 1,))])[0])
         eng.close(s)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_captured_step_allocates_nothing(dtype):
+    """Of matrices that are large enough for the tensor cores in either type: all buffers are there before the capture."""
+    from gguf_rs_cli_b200.api import _build
+    from gguf_rs_cli_b200.engine.backend import EngineBackend
+    from gguf_rs_cli_b200.engine.generate import generate_ids
+    from gguf_rs_cli_b200.engine.step import Engine
+    from gguf_rs_cli_b200.weights import TensorSource
+    from tests import plain_llama as P
+    from tests.tiny import config
+    raw = dict(config("A"), hidden_size=1024, num_attention_heads=16, num_key_value_heads=4, head_dim=64, intermediate_size=2048, num_hidden_layers=1)
+    w = {k: v.to(getattr(torch, dtype)) for k, v in P.random_weights(raw, 0).items()}
+    model = _build(raw, TensorSource(tensors=w, where="one layer"), dtype, "cuda:0")
+    backend, seen = EngineBackend(Engine(model.model, n_tokens=256, n_slots=2)), []
+    real = backend._capture
+
+    def counted(body):
+        allocated = lambda: torch.cuda.memory_stats()["allocation.all.allocated"]
+
+        def inside():
+            before = allocated()
+            body()
+            seen.append(allocated() - before)
+        return real(inside)
+    backend._capture = counted
+    for n in (1, 2):
+        prompts = [tokens_of("A", 5, i) for i in range(n)]
+        assert len(generate_ids(backend, prompts, 6)) == n
+    assert seen == [0] * len(seen) and len(seen) >= 2
