@@ -9,9 +9,10 @@
 // that, and added behind its last block.  Against 64 bits (2,048 of K, 32-bit FMAs one behind another in brackets, of the result's norm): one term in a row
 // 2.5e-8 (2.5e-8), 4 side by side 2.7e-8 (4.2e-8), 4 far apart 4.5e-8 (4.1e-8), 16 3.7e-8 and 6.9e-8 (7.5e-8), all 9.8e-8 (8.1e-7).
 // (One accumulator for all products: one term 4.9e-8, and 2 to 15 % less time.)
-// Results that are not finite (an infinite operand times a term that is zero) and results below 2^-96 (the terms of operands of that size
-// reach the end of the exponents' range: operands of 1e-34 would give 6e-7, of 1e-36 5e-5) are summed again one product behind another, as gemm_generic
-// does; an exact zero stays.
+// Results that are not finite (an infinite operand times a term that is zero) and results below 2^-96 are summed again one product behind another,
+// as gemm_generic does, and so are those from which more than 2^-26 may be missing where an operand below 2^-110 has lost bits (its terms reach the end of
+// the exponents' range: operands of 1e-34 lose 3e-7 of themselves, of 1e-36 3e-5, of 1e-42 everything).  The conversion looks for such operands; only where it
+// finds one are a tile's operands read again for what they may have cost.
 //
 // A row's result does not depend on the rows beside it: a block's sum is the same whatever the tile's width, and K is cut into pieces
 // by the matrix's sizes alone (fx_pieces), whose sums are added in order.
@@ -62,6 +63,7 @@ struct FxParams {
     const void* bias;
     void* out;
     float* scratch;       // [tiles][pieces][slot_cols][128] sums of the pieces of K, where a tile is not one CTA's
+    float* lost;          // [tiles][pieces] behind them: fx_lost of a piece
     int* status;
     long long ldx, ldw, ldo;
     int bias_dtype, out_dtype;
@@ -124,15 +126,71 @@ template <int N> __device__ __forceinline__ void fx_add(float (&acc)[N], uint32_
     }
 }
 
-// A sum that is not finite or next to nothing, taken again one product behind another.
+// A number below this loses bits in its terms: the third one ends at 2^-133, the smallest bfloat16.
+constexpr float FX_TINY = 0x1p-110f;
+// The smallest magnitude that is not zero, as twice its bits less one, in which zero is the largest number there is: no branch stands in the
+// conversion's loop, where one costs what the whole look costs.
+constexpr uint32_t FX_TINY_RANK = ((127u - 110u) << 24) - 1u;
+__device__ __forceinline__ uint32_t fx_rank(float v) { return 2u * __float_as_uint(v) - 1u; }
+__device__ __forceinline__ uint32_t fx_least(uint32_t least, const float4& v) {
+    return __vimin3_u32(__vimin3_u32(least, fx_rank(v.x), fx_rank(v.y)), fx_rank(v.z), fx_rank(v.w));
+}
+
+// A sum that is not finite or next to nothing, or from which too much may be lost, taken again one product behind another.
 __device__ __noinline__ float fx_again(const float* x, const float* w, int K) {
     float v = 0.f;
     for (int k = 0; k < K; ++k) v = fmaf(x[k], w[k], v);
     return v;
 }
-__device__ __forceinline__ void fx_store(const FxParams& p, int t, int n, float v, float bias) {
-    if (!isfinite(v) || (fabsf(v) < 0x1p-96f && v != 0.f)) v = fx_again(p.x + size_t(t) * p.ldx, p.w + size_t(n) * p.ldw, p.K);
+__device__ __forceinline__ void fx_store(const FxParams& p, int t, int n, float v, float bias, float lost = 0.f) {
+    if (!isfinite(v) || (fabsf(v) < 0x1p-96f && v != 0.f) || fabsf(v) < lost) v = fx_again(p.x + size_t(t) * p.ldx, p.w + size_t(n) * p.ldw, p.K);
     gb_store(p.out, p.out_dtype, size_t(t) * p.ldo + n, p.bias ? v + bias : v);
+}
+
+// The largest finite magnitude of a row's K numbers and whether one of them loses bits, by a warp into big and tiny.
+__device__ __forceinline__ void fx_scan(const float* row, int K, int* big, int* tiny) {
+    float most = 0.f;
+    bool any = false;
+    for (int k = 4 * (threadIdx.x & 31); k < K; k += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(row + k);
+        const float a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (fabsf(a[e]) < INFINITY) most = fmaxf(most, fabsf(a[e]));
+            any = any || (a[e] != 0.f && fabsf(a[e]) < FX_TINY);
+        }
+    }
+    if (most > 0.f) atomicMax(big, __float_as_int(most));              // not negative: ordered as whole numbers are
+    if (any) *tiny = 1;
+}
+// What may be missing of a sum over k places of K where operands have lost bits, times 2^26: up to 2^-134 of each, times the largest of the
+// other operand, as often as there are places.  Results below it are summed again.  By all threads of a block, for all rows from x and w on.
+// (A function of its own with values for arguments, called when no sums wait in registers: inlined in front of the stores it cost the block's loop 10 %.)
+__device__ __noinline__ float fx_lost(const float* x, long long ldx, int tokens, const float* w, long long ldw, int features, int k) {
+    __shared__ int big_w, big_x, tiny_w, tiny_x;
+    __syncthreads();
+    if (threadIdx.x == 0) big_w = big_x = tiny_w = tiny_x = 0;
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (int i = warp; i < features; i += warps) fx_scan(w + i * ldw, k, &big_w, &tiny_w);
+    for (int i = warp; i < tokens; i += warps) fx_scan(x + i * ldx, k, &big_x, &tiny_x);
+    __syncthreads();
+    return 0x1p-108f * float(k) * ((tiny_w ? __int_as_float(big_x) : 0.f) + (tiny_x ? __int_as_float(big_w) : 0.f));
+}
+// The results of a whole tile once more, behind their stores.
+__device__ __noinline__ void fx_mend(const float* x, long long ldx, int tokens, const float* w, long long ldw, int features, int K, const void* bias,
+                                     int bias_dtype, void* out, int out_dtype, long long ldo, int n0, int t0) {
+    const float lost = fx_lost(x, ldx, tokens, w, ldw, features, K);
+    for (int i = threadIdx.x; i < tokens * FX_BM; i += blockDim.x) {
+        const int n = i & (FX_BM - 1), c = i / FX_BM;
+        if (n >= features) continue;
+        const size_t at = size_t(t0 + c) * ldo + n0 + n;
+        const float b = bias ? gb_load(bias, bias_dtype, n0 + n) : 0.f;
+        if (fabsf(gb_load(out, out_dtype, at) - b) < 2.f * lost) {                           // (twice: the result may have been rounded to 8 bits)
+            const float v = fx_again(x + c * ldx, w + n * ldw, K);
+            gb_store(out, out_dtype, at, bias ? v + b : v);
+        }
+    }
 }
 
 template <int BN>
@@ -149,7 +207,7 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
     uint8_t* xs = ring + RING * Cfg::RAW;          // X's terms: rows of 128 bytes, [h | m] of each buffer, then [l of an even buffer | l of an odd one]
     __shared__ uint64_t raw_full[RING], raw_empty[RING], op_full[DEPTH], done[DEPTH], sum_free, tail_free[TAILS];
     __shared__ uint32_t tmem_base;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, tiny_seen;
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     // This CTA's units, pieces of K of tiles one behind another: all of one tile (whole), or some, and then their sums go to scratch memory.
@@ -166,7 +224,7 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
         for (int i = 0; i < DEPTH; ++i) { mbar_init(&op_full[i], WORKERS); mbar_init(&done[i], 1); }
         mbar_init(&sum_free, WORKERS);
         for (int i = 0; i < TAILS; ++i) mbar_init(&tail_free[i], WORKERS);
-        abort_flag = 0;
+        abort_flag = tiny_seen = 0;
         fence_barrier_init();
         prefetch_tensormap(&map_w);
         prefetch_tensormap(&map_x);
@@ -252,6 +310,7 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
         int unit = unit0, piece_end = piece_blocks(unit0);                      // the piece whose blocks are being added
         const bool does_w = WORKERS == 8 || warp < 10, does_x = WORKERS == 8 || warp >= 10;
         const int xw = (warp - 2) & 7;
+        uint32_t least[2] = {0xffffffffu, 0xffffffffu};                         // fx_least of all that this thread has converted
         // block s: its sums and, behind a piece's last block, those of the piece's small products
         auto add = [&](int s) {
             if (!mbar_wait(&done[s % DEPTH], (s / DEPTH) & 1)) {
@@ -322,6 +381,7 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float4 v = fx_lds4(raw + row * 128 + (((half * 4 + c) ^ (row & 7)) << 4));
+                    least[c & 1] = fx_least(least[c & 1], v);
                     fx_split(v.x, v.y, terms[2 * c], terms[8 + 2 * c], terms[16 + 2 * c]);
                     fx_split(v.z, v.w, terms[2 * c + 1], terms[9 + 2 * c], terms[17 + 2 * c]);
                 }
@@ -350,6 +410,8 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
                         const int r = r0 + xw * 8 + sub, sw = r & 7;
                         if (BN - r0 >= 64 || r < BN) {
                             const float4 u = fx_lds4(x + r * 128 + ((2 * j ^ sw) << 4)), v = fx_lds4(x + r * 128 + (((2 * j + 1) ^ sw) << 4));
+                            least[0] = fx_least(least[0], u);
+                            least[1] = fx_least(least[1], v);
                             uint32_t xh[4], xm[4], xl[4];
                             fx_split(u.x, u.y, xh[0], xm[0], xl[0]);
                             fx_split(u.z, u.w, xh[1], xm[1], xl[1]);
@@ -369,40 +431,62 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
             }
             if (LATE && s >= 1 && !add(s - 1)) break;
         }
+        if (min(least[0], least[1]) < FX_TINY_RANK) tiny_seen = 1;
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, Cfg::TMEM_COLS);
-    if (abort_flag || warp < 2 || !whole) return;
+    if (abort_flag) return;
+    if (!whole) {
+        for (int unit = unit0; unit < unit1; ++unit) {
+            float lost = 0.f;
+            if (tiny_seen) {
+                const int tile = unit / p.pieces, piece = unit - tile * p.pieces, n0 = tile / p.t_tiles * FX_BM, t0 = tile % p.t_tiles * BN;
+                const int k0 = piece_begin(piece) * FX_BK, k1 = min(p.K, piece_begin(piece + 1) * FX_BK);
+                lost = fx_lost(p.x + t0 * p.ldx + k0, p.ldx, min(BN, p.T - t0), p.w + n0 * p.ldw + k0, p.ldw, min(FX_BM, p.N - n0), k1 - k0);
+            }
+            if (threadIdx.x == 0) p.lost[unit] = lost;
+        }
+        return;
+    }
 
-    const int n = tile0 / p.t_tiles * FX_BM + row, t0 = tile0 % p.t_tiles * BN, cols = min(BN, p.T - t0);
-    const float bias = p.bias && n < p.N ? gb_load(p.bias, p.bias_dtype, n) : 0.f;
-    if (n < p.N) {
+    const int n0 = tile0 / p.t_tiles * FX_BM, t0 = tile0 % p.t_tiles * BN, n = n0 + row, cols = min(BN, p.T - t0);
+    if (warp >= 2 && n < p.N) {
+        const float bias = p.bias ? gb_load(p.bias, p.bias_dtype, n) : 0.f;
 #pragma unroll
         for (int c = 0; c < COLS; ++c)
             if (mine + c < cols) fx_store(p, t0 + mine + c, n, TOTAL ? total[TOTAL ? c : 0] : acc[c], bias);
     }
+    if (tiny_seen)
+        fx_mend(p.x + t0 * p.ldx, p.ldx, cols, p.w + n0 * p.ldw, p.ldw, min(FX_BM, p.N - n0), p.K, p.bias, p.bias_dtype, p.out, p.out_dtype, p.ldo, n0, t0);
 }
 
 // The sums of the pieces of tiles that were not one CTA's, added in order: a feature a thread, tokens 2 gridDim.y apart.
 __global__ void __launch_bounds__(2 * FX_BM) gemm_f32_tc_merge_kernel(FxParams p, int bn) {
     gb_grid_launch_dependents();
     gb_grid_wait();
+    __shared__ float lost_s;
     const int tile = blockIdx.x, row = threadIdx.x & (FX_BM - 1);
     const int n = tile / p.t_tiles * FX_BM + row, t0 = tile % p.t_tiles * bn, cols = min(bn, p.T - t0);
-    if (n >= p.N) return;
-    const float bias = p.bias ? gb_load(p.bias, p.bias_dtype, n) : 0.f;
+    if (threadIdx.x < 32) {                            // one warp asks (by all of them it was 20 us at 2,048 x 2,048 and 187 tokens)
+        const float lost = gb_warp_sum(threadIdx.x < p.pieces ? __ldcg(p.lost + tile * p.pieces + threadIdx.x) : 0.f);
+        if (threadIdx.x == 0) lost_s = lost;
+    }
+    const float bias = p.bias && n < p.N ? gb_load(p.bias, p.bias_dtype, n) : 0.f;
     const size_t slot = size_t(p.slot_cols) * FX_BM;
-    for (int c = 2 * blockIdx.y + (threadIdx.x >> 7); c < cols; c += 2 * gridDim.y) {
+    bool first = true;                                 // every thread's first round, with a token or without: the barrier stands in it
+    for (int c = 2 * blockIdx.y + (threadIdx.x >> 7); first || c < cols; c += 2 * gridDim.y) {
         const float* from = p.scratch + size_t(tile) * p.pieces * slot + size_t(c) * FX_BM + row;
         float v[FX_PIECES];
 #pragma unroll
-        for (int i = 0; i < FX_PIECES; ++i) v[i] = i < p.pieces ? __ldcg(from + i * slot) : 0.f;
+        for (int i = 0; i < FX_PIECES; ++i) v[i] = i < p.pieces && c < cols ? __ldcg(from + i * slot) : 0.f;
         float sum = v[0];
 #pragma unroll
         for (int i = 1; i < FX_PIECES; ++i)
             if (i < p.pieces) sum += v[i];
-        fx_store(p, t0 + c, n, sum, bias);
+        if (first) __syncthreads();                    // lost_s, while the first sums are on their way
+        first = false;
+        if (n < p.N && c < cols) fx_store(p, t0 + c, n, sum, bias, lost_s);
     }
 }
 
@@ -471,7 +555,7 @@ FxCut fx_cut(int T, int N, int K, int out_dtype, int sms) {
             const double cost = double((tiles + places - 1) / places) * (blocks * BLOCK[i] + 4.0);
             if (cost < least) { least = cost; best = {bn, pieces, int(tiles), tiles, 0}; }
         }
-        const long long scratch = tiles * pieces * (T < bn ? T : bn) * FX_BM;
+        const long long scratch = tiles * pieces * ((T < bn ? T : bn) * FX_BM + 1);
         for (int each = 1; each < pieces; ++each) {                   // pieces a CTA
             const int sharers = (pieces + each - 1) / each;
             if (tiles * sharers > places || scratch > FX_SCRATCH) continue;
@@ -518,6 +602,7 @@ GB_API int gb_gemm_f32_tc(const float* X, long long ldx, const float* W, long lo
     p.x = X; p.w = W; p.bias = bias; p.out = out; p.scratch = scratch; p.status = g_status_dev;
     p.ldx = ldx; p.ldw = ldw; p.ldo = ldo; p.bias_dtype = bias_dtype; p.out_dtype = out_dtype; p.T = T; p.N = N; p.K = K;
     p.pieces = cut.pieces; p.tiles = int(cut.tiles); p.t_tiles = (T + cut.bn - 1) / cut.bn; p.slot_cols = T < cut.bn ? T : cut.bn;
+    p.lost = cut.scratch ? scratch + cut.tiles * cut.pieces * p.slot_cols * FX_BM : nullptr;
     CUtensorMap mw, mx;
     if (tensor_map_f32_2d(W, N, K, ldw, FX_BM, &mw)) return 1;
     if (tensor_map_f32_2d(X, T, K, ldx, cut.bn, &mx)) return 1;

@@ -92,6 +92,41 @@ def test_a_rows_result_does_not_depend_on_the_rows_beside_it(N, K):
     k.check_tc_status()
 
 
+@pytest.mark.parametrize("T", [1, 16, 30, 64, 90, 187, 700])
+@pytest.mark.parametrize("N, K", [(300, 1024), (20000, 1028), (2048, 8192)])
+def test_tiny_operands_beside_large_ones(T, N, K):
+    """Rows of X, of W, and single entries too small for three bfloat16 terms, beside operands that make a result of them that counts: what one 32-bit FMA
+    behind another gives.  Beside operands of ordinary size they change nothing, and neither do zeros."""
+    from gguf_rs_cli_b200 import kernels as k
+
+    def run(x, w, bias=None, dtype=torch.float32):
+        got, plain = torch.empty(T, N, device=DEV, dtype=dtype), torch.empty(T, N, device=DEV, dtype=dtype)
+        k.gemm_f32_tc(x, w, bias, got)
+        k.gemm_f32(x, w, bias, plain)
+        return got, plain
+    x0, w0 = _operands(T, N, K, T + K)
+    for tiny, large in ((1e-34, 1e30), (1e-36, 1e12), (1e-38, 1e30), (1e-42, 1e30)):
+        for a, b in ((tiny, large), (large, tiny)):
+            got, plain = run(x0 * a, w0 * b)
+            assert torch.equal(got, plain), (a, b)                              # all of them are summed again
+    bias = torch.randn(N, device=DEV) * 1e-12
+    for dtype in (torch.float32, torch.bfloat16):
+        got, plain = run(x0 * 1e-42, w0 * 1e30, bias, dtype)
+        assert torch.equal(got, plain)
+    ordinary, _ = run(x0, w0)
+    x, w = x0.clone(), w0.clone()
+    x[:, 5::7], w[::3, 11] = 1e-39, -1e-37                                       # what is lost is below 2^-134 times K times 5
+    got, plain = run(x, w)
+    want = x.double() @ w.double().T
+    assert float((got.double() - want).norm()) <= 1.01 * float((plain.double() - want).norm())
+    assert not torch.equal(got, plain) and not torch.equal(got, ordinary)
+    x[T // 2], w[:, 3] = 0.0, 1e33
+    x[T // 2, 3] = 1.23456789e-39                                                # the only term of a row, 1e-6
+    got, plain = run(x, w)
+    assert torch.equal(got[T // 2], plain[T // 2]) and (got[T // 2] != 0).all()
+    k.check_tc_status()
+
+
 def test_operands_that_are_not_finite_and_large_ones():
     """Infinities, NaN (with a payload in its last bits only), numbers next to the largest, and subnormal ones: what one thread's sum gives."""
     from gguf_rs_cli_b200 import kernels as k
