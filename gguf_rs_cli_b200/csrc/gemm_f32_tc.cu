@@ -54,6 +54,8 @@ template <int BN> struct FxCfg {
     static constexpr int CTAS = BN <= 32 ? 2 : 1;                 // of an SM
     // Warps that convert and add; a warp adds the sums of a GROUPS-th of the columns.  Of sixteen half convert W, half X.
     static constexpr int WORKERS = BN < 64 ? 8 : 16, GROUPS = WORKERS / 4, COLS = BN / GROUPS, THREADS = (WORKERS + 2) * 32;
+    static constexpr bool X_BY_COPIER = BN <= 16;                 // the warp that copies converts X too
+    static constexpr int ARRIVALS = WORKERS + (X_BY_COPIER ? 1 : 0);             // for a block that is converted
     static_assert(A_COL + DEPTH * 64 <= 512 && TMEM_COLS * CTAS <= 512 && SUMS <= DEPTH);
 };
 
@@ -67,7 +69,7 @@ struct FxParams {
     int* status;
     long long ldx, ldw, ldo;
     int bias_dtype, out_dtype;
-    int T, N, K, pieces, tiles, t_tiles, slot_cols;
+    int T, N, K, pieces, first_blocks, tiles, t_tiles, slot_cols;       // first_blocks: of the first of two unequal pieces of K (0: equal ones)
 };
 
 // Two numbers in three bfloat16 terms each, the first in the low halves: each term the rest, rounded to nearest; nothing is left behind the third.
@@ -210,18 +212,30 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
     __shared__ int abort_flag, tiny_seen;
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    // This CTA's units, pieces of K of tiles one behind another: all of one tile (whole), or some, and then their sums go to scratch memory.
+    // This CTA's units, pieces of K of tiles: all of one tile (whole), or some, and then their sums go to scratch memory.  With two unequal pieces
+    // (first_blocks) a CTA has the first piece of a tile, or the second ones of several.
     const int blocks = (p.K + FX_BK - 1) / FX_BK;
     const bool whole = gridDim.x == p.tiles;
-    const int units = p.tiles * p.pieces, unit0 = int((long long)blockIdx.x * units / gridDim.x), unit1 = int((long long)(blockIdx.x + 1) * units / gridDim.x);
-    const int tile0 = unit0 / p.pieces, piece0 = unit0 - tile0 * p.pieces;
-    auto piece_begin = [&](int i) { return i * blocks / p.pieces; };          // i <= 16, blocks < 2^26
+    auto piece_begin = [&](int i) { return i == 1 && p.first_blocks ? p.first_blocks : i * blocks / p.pieces; };          // i <= 16, blocks < 2^26
     auto piece_blocks = [&](int unit) { const int i = unit % p.pieces; return piece_begin(i + 1) - piece_begin(i); };
-    const int S = (unit1 / p.pieces - tile0) * blocks + piece_begin(unit1 % p.pieces) - piece_begin(piece0);
+    int unit0, count, step = 1;
+    if (p.first_blocks && !whole) {
+        const int c = blockIdx.x - p.tiles, rest = gridDim.x - p.tiles;
+        unit0 = c < 0 ? 2 * blockIdx.x : 2 * int((long long)c * p.tiles / rest) + 1;
+        count = c < 0 ? 1 : int((long long)(c + 1) * p.tiles / rest) - int((long long)c * p.tiles / rest);
+        step = 2;
+    } else {
+        const int units = p.tiles * p.pieces;
+        unit0 = int((long long)blockIdx.x * units / gridDim.x);
+        count = int((long long)(blockIdx.x + 1) * units / gridDim.x) - unit0;
+    }
+    const int tile0 = unit0 / p.pieces;
+    int S = 0;
+    for (int i = 0; i < count; ++i) S += piece_blocks(unit0 + i * step);
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < RING; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WORKERS); }
-        for (int i = 0; i < DEPTH; ++i) { mbar_init(&op_full[i], WORKERS); mbar_init(&done[i], 1); }
+        for (int i = 0; i < RING; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], Cfg::ARRIVALS); }
+        for (int i = 0; i < DEPTH; ++i) { mbar_init(&op_full[i], Cfg::ARRIVALS); mbar_init(&done[i], 1); }
         mbar_init(&sum_free, WORKERS);
         for (int i = 0; i < TAILS; ++i) mbar_init(&tail_free[i], WORKERS);
         abort_flag = tiny_seen = 0;
@@ -249,18 +263,79 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
     const int quarter = warp & 3, row = quarter * 32 + lane, group = (warp - 2) >> 2, half = group & 1;       // of the workers
     const int mine = group * COLS;
 
+    // X, eight of K (a 16th of the block's rows of 128 bytes: chunk j of its terms) of row r: the terms of block s in buffer b.
+    const uint32_t ring_a = smem_u32(ring), xs_a = smem_u32(xs);
+    uint32_t least[2] = {0xffffffffu, 0xffffffffu};                             // fx_least of all that this thread has converted
+    auto convert_x = [&](uint32_t raw, int b, int r, int j) {
+        const uint32_t x = raw + Cfg::W_BYTES, hm = xs_a + b * Cfg::X_BYTES, lo = xs_a + (DEPTH + (b >> 1)) * Cfg::X_BYTES;
+        const int sw = r & 7;
+        const float4 u = fx_lds4(x + r * 128 + ((2 * j ^ sw) << 4)), v = fx_lds4(x + r * 128 + (((2 * j + 1) ^ sw) << 4));
+        least[0] = fx_least(least[0], u);
+        least[1] = fx_least(least[1], v);
+        uint32_t xh[4], xm[4], xl[4];
+        fx_split(u.x, u.y, xh[0], xm[0], xl[0]);
+        fx_split(u.z, u.w, xh[1], xm[1], xl[1]);
+        fx_split(v.x, v.y, xh[2], xm[2], xl[2]);
+        fx_split(v.z, v.w, xh[3], xm[3], xl[3]);
+        fx_sts4(hm + r * 128 + ((j ^ sw) << 4), xh);
+        fx_sts4(hm + r * 128 + (((j + 4) ^ sw) << 4), xm);
+        fx_sts4(lo + r * 128 + (((j + 4 * (b & 1)) ^ sw) << 4), xl);
+    };
+
     if (warp == 0) {
-        if (elect_one()) {
-            int tile = tile0, kb = piece_begin(piece0);
-            for (int s = 0; s < S; ++s) {
-                const int slot = s % RING;
-                if (s >= RING && !mbar_wait(&raw_empty[slot], (s / RING - 1) & 1)) { atomicExch(p.status, 21); abort_flag = 1; break; }
-                uint8_t* dst = ring + slot * Cfg::RAW;
-                mbar_expect_tx(&raw_full[slot], Cfg::RAW);
-                tma_load_2d(dst, &map_w, kb * FX_BK, tile / p.t_tiles * FX_BM, &raw_full[slot]);
-                tma_load_2d(dst + Cfg::W_BYTES, &map_x, kb * FX_BK, tile % p.t_tiles * BN, &raw_full[slot]);
-                if (++kb == blocks) { kb = 0; ++tile; }
+        int unit = unit0, tile = tile0, kb = piece_begin(unit0 - tile0 * p.pieces), left = piece_blocks(unit0);
+        auto copy = [&](int slot) {
+            uint8_t* dst = ring + slot * Cfg::RAW;
+            mbar_expect_tx(&raw_full[slot], Cfg::RAW);
+            tma_load_2d(dst, &map_w, kb * FX_BK, tile / p.t_tiles * FX_BM, &raw_full[slot]);
+            tma_load_2d(dst + Cfg::W_BYTES, &map_x, kb * FX_BK, tile % p.t_tiles * BN, &raw_full[slot]);
+            ++kb;
+            if (--left == 0) {
+                unit += step;
+                tile = unit / p.pieces;
+                kb = piece_begin(unit - tile * p.pieces);
+                left = piece_blocks(unit);
             }
+        };
+        if constexpr (!Cfg::X_BY_COPIER) {
+            if (elect_one()) {
+                for (int s = 0; s < S; ++s) {
+                    const int slot = s % RING;
+                    if (s >= RING && !mbar_wait(&raw_empty[slot], (s / RING - 1) & 1)) { atomicExch(p.status, 21); abort_flag = 1; break; }
+                    copy(slot);
+                }
+            }
+        } else {
+            // few tokens: this warp converts X beside its copies, or two of the workers' warps would be later than the others with every block (28,672 x
+            // 4,096 at one token 118 -> 114 us; with 32 tokens it would be the last itself: 130 -> 140)
+            if (elect_one())
+                for (int s = 0; s < S && s < RING; ++s) copy(s);
+            for (int s = 0; s < S; ++s) {
+                const int b = s % DEPTH, slot = s % RING;
+                if (!mbar_wait(&raw_full[slot], (s / RING) & 1) || (s >= DEPTH && !mbar_wait(&done[b], (s / DEPTH - 1) & 1))) {
+                    if (lane == 0) atomicExch(p.status, 28);
+                    abort_flag = 1;
+                    break;
+                }
+#pragma unroll
+                for (int i = 0; i < BN / 8; ++i) convert_x(ring_a + slot * Cfg::RAW, b, (i >> 1) * 16 + (lane >> 1), (lane & 1) * 2 + (i & 1));
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) { mbar_arrive(&raw_empty[slot]); mbar_arrive(&op_full[b]); }
+                if (s + RING < S) {
+                    bool late = false;
+                    if (elect_one()) {
+                        late = !mbar_wait(&raw_empty[slot], (s / RING) & 1);
+                        if (!late) copy(slot);
+                    }
+                    if (__any_sync(0xffffffffu, late)) {
+                        if (lane == 0) atomicExch(p.status, 21);
+                        abort_flag = 1;
+                        break;
+                    }
+                }
+            }
+            if (min(least[0], least[1]) < FX_TINY_RANK) tiny_seen = 1;
         }
     } else if (warp == 1) {
         if (elect_one()) {
@@ -300,17 +375,15 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
                 if (s + 1 == piece_end) {
                     more = 0;
                     ++piece;
-                    piece_end += piece_blocks(unit0 + piece);
+                    piece_end += piece_blocks(unit0 + piece * step);
                 }
             }
         }
     } else {
-        const uint32_t ring_a = smem_u32(ring), xs_a = smem_u32(xs);
         const uint32_t lane_base = uint32_t(quarter * 32) << 16;
-        int unit = unit0, piece_end = piece_blocks(unit0);                      // the piece whose blocks are being added
-        const bool does_w = WORKERS == 8 || warp < 10, does_x = WORKERS == 8 || warp >= 10;
+        int unit = unit0, done_units = 0, piece_end = piece_blocks(unit0);      // the piece whose blocks are being added, and those before it
+        const bool does_w = WORKERS == 8 || warp < 10, does_x = !Cfg::X_BY_COPIER && (WORKERS == 8 || warp >= 10);
         const int xw = (warp - 2) & 7;
-        uint32_t least[2] = {0xffffffffu, 0xffffffffu};                         // fx_least of all that this thread has converted
         // block s: its sums and, behind a piece's last block, those of the piece's small products
         auto add = [&](int s) {
             if (!mbar_wait(&done[s % DEPTH], (s / DEPTH) & 1)) {
@@ -326,7 +399,7 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
                 if (lane == 0) mbar_arrive(&sum_free);
             }
             if (s + 1 == piece_end) {
-                const int tail = (unit - unit0) % TAILS;
+                const int tail = done_units % TAILS;
                 fx_add<COLS>(acc, tmem + lane_base + Cfg::T_COL + tail * BN + mine);
                 if (LATE) {
                     tc_fence_before();
@@ -360,14 +433,15 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
 #pragma unroll
                         for (int c = 0; c < 8; ++c) {
                             if (piece) acc[c0 + c] = v[c] + acc[c0 + c];
-                            if (unit + 1 < unit1) {
+                            if (done_units + 1 < count) {
                                 if (c0 + c < m) __stcg(to + (c0 + c) * p.ldo, acc[c0 + c]);
                                 acc[c0 + c] = 0.f;
                             }
                         }
                     }
                 }
-                ++unit;
+                ++done_units;
+                unit += step;
                 piece_end += piece_blocks(unit);
             }
             return true;
@@ -404,24 +478,9 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
                 if (does_x) {
                     // X: eight of K a thread; the rows of a quarter of a warp are four apart, so that their 64 bytes lie in both halves
                     const int j = lane & 3, sub = (lane >> 3) + (lane & 4);
-                    const uint32_t x = raw + Cfg::W_BYTES, hm = xs_a + b * Cfg::X_BYTES, lo = xs_a + (DEPTH + (b >> 1)) * Cfg::X_BYTES;
 #pragma unroll
-                    for (int r0 = 0; r0 < BN; r0 += 64) {
-                        const int r = r0 + xw * 8 + sub, sw = r & 7;
-                        if (BN - r0 >= 64 || r < BN) {
-                            const float4 u = fx_lds4(x + r * 128 + ((2 * j ^ sw) << 4)), v = fx_lds4(x + r * 128 + (((2 * j + 1) ^ sw) << 4));
-                            least[0] = fx_least(least[0], u);
-                            least[1] = fx_least(least[1], v);
-                            uint32_t xh[4], xm[4], xl[4];
-                            fx_split(u.x, u.y, xh[0], xm[0], xl[0]);
-                            fx_split(u.z, u.w, xh[1], xm[1], xl[1]);
-                            fx_split(v.x, v.y, xh[2], xm[2], xl[2]);
-                            fx_split(v.z, v.w, xh[3], xm[3], xl[3]);
-                            fx_sts4(hm + r * 128 + ((j ^ sw) << 4), xh);
-                            fx_sts4(hm + r * 128 + (((j + 4) ^ sw) << 4), xm);
-                            fx_sts4(lo + r * 128 + (((j + 4 * (b & 1)) ^ sw) << 4), xl);
-                        }
-                    }
+                    for (int r0 = 0; r0 < BN; r0 += 64)
+                        if (BN - r0 >= 64 || r0 + xw * 8 + sub < BN) convert_x(raw, b, r0 + xw * 8 + sub, j);
                     fence_proxy_async();
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -438,7 +497,7 @@ __global__ void __launch_bounds__(FxCfg<BN>::THREADS, FxCfg<BN>::CTAS) gemm_f32_
     if (warp == 1) tmem_dealloc(tmem, Cfg::TMEM_COLS);
     if (abort_flag) return;
     if (!whole) {
-        for (int unit = unit0; unit < unit1; ++unit) {
+        for (int i = 0, unit = unit0; i < count; ++i, unit += step) {
             float lost = 0.f;
             if (tiny_seen) {
                 const int tile = unit / p.pieces, piece = unit - tile * p.pieces, n0 = tile / p.t_tiles * FX_BM, t0 = tile % p.t_tiles * BN;
@@ -529,38 +588,51 @@ template <int BN> int launch_fx(const CUtensorMap& mw, const CUtensorMap& mx, co
 
 // Pieces of K whose sums are added at the end, in order.  A function of the matrix alone: whatever the tokens beside it, a
 // row's result is the same sums in the same order.  As many as give every SM two of a step with a single tile of tokens, of at
-// least four blocks each.
-int fx_pieces(int N, int K, int sms) {
-    const int tiles = (N + FX_BM - 1) / FX_BM, blocks = (K + FX_BK - 1) / FX_BK;
+// least four blocks each.  More tiles than that makes two of leave SMs with one of them: there K has two unequal pieces, so that a tile's first is a
+// CTA's and the places left share the second ones (28,672 x 4,096 at one token: 224 whole tiles 139 us, 103 and 25 blocks 113; equal pieces of a fifth
+// 116, but a prompt's tile has to add them: 330 -> 375 us at 187 tokens, with two 346).
+struct FxPieces { int n, first_blocks, shares; };          // shares: second pieces of a CTA, at most
+FxPieces fx_pieces(int N, int K, int sms) {
+    const int tiles = (N + FX_BM - 1) / FX_BM, blocks = (K + FX_BK - 1) / FX_BK, rest = 2 * sms - tiles;
+    if (tiles > sms && rest > 0) {
+        const int q = (tiles + rest - 1) / rest, first = (blocks * q + q) / (q + 1);
+        if (blocks - first >= 4 && 10 * first <= 9 * blocks) return {2, first, q};
+        return {1, 0, 0};
+    }
     int n = 2 * sms / tiles;
     if (n > FX_PIECES) n = FX_PIECES;
     if (n > blocks / 4) n = blocks / 4;
-    return n > 1 ? n : 1;
+    return {n > 1 ? n : 1, 0, 0};
 }
 // The tile and the number of CTAs that take the least time: rounds over the device times blocks of K times a block's time, with what a CTA
 // takes beside its blocks, and where tiles are not one CTA's each the merge behind and the bytes that go there and back.  A block's time as
 // measured at 16,384 x 2,048, microseconds.  The scratch memory of a launch is bounded (FX_SCRATCH floats); one CTA's tile needs none.
-struct FxCut { int bn, pieces, ctas; long long tiles, scratch; };
+struct FxCut { int bn, pieces, first_blocks, ctas; long long tiles, scratch; };
 constexpr long long FX_SCRATCH = 8LL << 20;
 FxCut fx_cut(int T, int N, int K, int out_dtype, int sms) {
     static const int BNS[7] = {16, 32, 64, 96, 128, 160, 192};
     static const double BLOCK[7] = {0.9, 1.0, 0.8, 0.87, 0.97, 1.12, 1.3};
-    const int blocks = (K + FX_BK - 1) / FX_BK, pieces = fx_pieces(N, K, sms);
-    FxCut best = {16, pieces, 0, 0, 0};
+    const FxPieces cut = fx_pieces(N, K, sms);
+    const int blocks = (K + FX_BK - 1) / FX_BK, pieces = cut.n;
+    FxCut best = {16, pieces, cut.first_blocks, 0, 0, 0};
     double least = 1e300;
     for (int i = 0; i < 7; ++i) {
         const int bn = BNS[i];
         const long long tiles = (long long)((N + FX_BM - 1) / FX_BM) * ((T + bn - 1) / bn), places = (bn <= 32 ? 2LL : 1LL) * sms;
         if (bn <= 96 || pieces == 1 || out_dtype == GB_F32) {       // wider ones keep a piece's sums in a 32-bit result
             const double cost = double((tiles + places - 1) / places) * (blocks * BLOCK[i] + 4.0);
-            if (cost < least) { least = cost; best = {bn, pieces, int(tiles), tiles, 0}; }
+            if (cost < least) { least = cost; best = {bn, pieces, cut.first_blocks, int(tiles), tiles, 0}; }
         }
         const long long scratch = tiles * pieces * ((T < bn ? T : bn) * FX_BM + 1);
-        for (int each = 1; each < pieces; ++each) {                   // pieces a CTA
+        for (int each = 1; each < pieces && !cut.first_blocks; ++each) {                   // pieces a CTA
             const int sharers = (pieces + each - 1) / each;
             if (tiles * sharers > places || scratch > FX_SCRATCH) continue;
             const double cost = each * ((blocks + pieces - 1) / pieces) * BLOCK[i] + 8.0 + 2e-6 * scratch;
-            if (cost < least) { least = cost; best = {bn, pieces, int(tiles * sharers), tiles, scratch}; }
+            if (cost < least) { least = cost; best = {bn, pieces, 0, int(tiles * sharers), tiles, scratch}; }
+        }
+        if (cut.first_blocks && bn <= 32 && T <= bn && scratch <= FX_SCRATCH) {
+            const double second = cut.shares * (blocks - cut.first_blocks + 0.33), cost = (second > cut.first_blocks ? second : cut.first_blocks) * BLOCK[i] + 8.0 + 2e-6 * scratch;
+            if (cost < least) { least = cost; best = {bn, pieces, cut.first_blocks, int(places), tiles, scratch}; }
         }
     }
     return best;
@@ -601,7 +673,7 @@ GB_API int gb_gemm_f32_tc(const float* X, long long ldx, const float* W, long lo
     FxParams p;
     p.x = X; p.w = W; p.bias = bias; p.out = out; p.scratch = scratch; p.status = g_status_dev;
     p.ldx = ldx; p.ldw = ldw; p.ldo = ldo; p.bias_dtype = bias_dtype; p.out_dtype = out_dtype; p.T = T; p.N = N; p.K = K;
-    p.pieces = cut.pieces; p.tiles = int(cut.tiles); p.t_tiles = (T + cut.bn - 1) / cut.bn; p.slot_cols = T < cut.bn ? T : cut.bn;
+    p.pieces = cut.pieces; p.first_blocks = cut.first_blocks; p.tiles = int(cut.tiles); p.t_tiles = (T + cut.bn - 1) / cut.bn; p.slot_cols = T < cut.bn ? T : cut.bn;
     p.lost = cut.scratch ? scratch + cut.tiles * cut.pieces * p.slot_cols * FX_BM : nullptr;
     CUtensorMap mw, mx;
     if (tensor_map_f32_2d(W, N, K, ldw, FX_BM, &mw)) return 1;

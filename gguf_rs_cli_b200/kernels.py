@@ -1468,12 +1468,13 @@ def check_tc_status() -> None:
 # ------------------------------------------------------------------ dispatch
 def _f32_on_tensor_cores(w: torch.Tensor) -> bool:
     """Whether 32-bit products with this matrix run on the tensor cores: for every number of tokens or for none, so that a row's
-    result does not depend on the rows beside it.  Tensor cores over CUDA cores at 1, 2, 4, 16 and 187 tokens, us: 3072 x 2048 12.4 / 13.4,
-    12.6 / 12.3, 12.7 / 16.9, 13 / 36, 23 / 123; 2048 x 8192 22 / 36, 22 / 42, 22 / 41, 22 / 80, 45 / 414; 16384 x 2048 35 / 24, 35 / 27,
-    35 / 33, 36 / 63, 80 / 390; 2048 x 2048 11 / 12.5 ... 20 / 114; 1024 x 1024 7.8 / 7.4 ... 16 tokens 7.7 / 8.6, 17 7.8 / 19.6.  Smaller matrices are
-    faster on CUDA cores (512 x 512 7.0 / 4.2), and so is a head, which sees few tokens (128256 x 2048 203 / 180)."""
+    result does not depend on the rows beside it.  Tensor cores over CUDA cores at 1, 4, 16 and 64 tokens, us behind a cleared L2: 2048 x 2048 17.4 / 16.4,
+    17.4 / 16.4, 17.4 / 22.5, 21 / 40; 2048 x 8192 30 / 37, 31 / 39, 32 / 64, 38 / 140; 4096 x 14336 63 / 68, 64 / 84, 65 / 178; 16384 x 2048 46 / 39, 46 / 45,
+    48 / 70, 59 / 130; 28672 x 4096 113 / 100, 114 / 123, 116 / 274; a head of 32000 x 4096 120 / 111, 120 / 129, 124 / 285.  More features than two
+    CTAs an SM hold tiles are a head's, which sees few tokens, and take a second round: 40000 x 2048 115 / 82, 115 / 92, 115 / 168; 64000 x 4096
+    252 / 195, 252 / 248, 254 / 558.  Smaller matrices are faster on CUDA cores (1024 x 1024 15 / 12, 15 / 12, 15 / 12, 17 / 25)."""
     N, K = w.shape
-    return K >= 1024 and N * K >= 1 << 20 and N <= 1 << 16
+    return K >= 1024 and N * K >= 1 << 20 and N <= 37888
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, ws=None) -> torch.Tensor:

@@ -217,3 +217,30 @@ def test_products_on_two_streams_wait_for_nobody():
     torch.cuda.synchronize()
     k.check_tc_status()
     assert all(torch.equal(o, want[i]) for i, o in outs)
+
+
+@pytest.mark.parametrize("N, K", [(19072, 1024), (28672, 1100), (30000, 1060), (37000, 1024), (37888, 1024)])
+def test_two_unequal_pieces_of_k(N, K):
+    """More tiles of features than SMs: few tokens have a tile's first piece of K or several tiles' second ones, prompts whole tiles: the same bits."""
+    from gguf_rs_cli_b200 import kernels as k
+    x, w = _operands(200, N, K, N + K)
+    bias, want = torch.randn(N, device=DEV), torch.empty(200, N, device=DEV)
+    k.gemm_f32_tc(x, w, bias, want)
+    exact = x.double() @ w.double().T + bias.double()
+    assert float((want.double() - exact).norm() / exact.norm()) < 2e-7
+    for T in (1, 15, 16, 17, 32, 33, 96, 97, 128):
+        for dtype in (torch.float32, torch.bfloat16):
+            got = torch.full((T, N + 4), 7.0, device=DEV, dtype=dtype)
+            k.gemm_f32_tc(x[:T], w, bias, got[:, :N])
+            assert torch.equal(got[:, :N], want[:T].to(dtype)) and (got[:, N:] == 7.0).all(), (T, dtype)
+    k.check_tc_status()
+
+
+def test_heads_of_more_features_than_a_round_holds_stay_on_cuda_cores():
+    from gguf_rs_cli_b200 import kernels as k
+    x, w = _operands(3, 37889, 1024, 4)
+    for N, kernel in ((37888, k.gemm_f32_tc), (37889, k.gemm_f32)):
+        got, direct = torch.empty(3, N, device=DEV), torch.empty(3, N, device=DEV)
+        k.gemm(x, w[:N], None, got)
+        kernel(x, w[:N], None, direct)
+        assert torch.equal(got, direct)
