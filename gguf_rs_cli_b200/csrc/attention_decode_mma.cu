@@ -782,12 +782,8 @@ __global__ void __launch_bounds__(PW_WARPS * 32, PW_WARPS == 4 && PW_SLOTS == 2 
 
 template <int HD, int WARPS, int SLOTS> int launch_pw(const DmParams& p, dim3 grid, cudaStream_t stream) {
     constexpr int SMEM = (DM_ROWS + 2 * WARPS * SLOTS * PW_KEYS) * HD * 2;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(attention_decode_pages_kernel<HD, WARPS, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-            return gb_fail("gb_attention_decode_mma: cannot get %d bytes of shared memory", SMEM);
-        configured = true;
-    }
+    static bool configured[GB_MAX_DEVICES] = {};
+    if (gb_allow_smem(attention_decode_pages_kernel<HD, WARPS, SLOTS>, SMEM, configured, "gb_attention_decode_mma")) return 1;
     gb_launch(attention_decode_pages_kernel<HD, WARPS, SLOTS>, grid, dim3(WARPS * 32), SMEM, stream, p);
     GB_LAUNCH_OK("gb_attention_decode_mma");
     return 0;
@@ -795,12 +791,8 @@ template <int HD, int WARPS, int SLOTS> int launch_pw(const DmParams& p, dim3 gr
 
 template <int HD, int WARPS> int launch_dm(const DmParams& p, dim3 grid, cudaStream_t stream) {
     constexpr int SMEM = (DM_ROWS + 2 * DM_STAGES * WARPS * 16) * HD * 2;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(attention_decode_mma_kernel<HD, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-            return gb_fail("gb_attention_decode_mma: cannot get %d bytes of shared memory", SMEM);
-        configured = true;
-    }
+    static bool configured[GB_MAX_DEVICES] = {};
+    if (gb_allow_smem(attention_decode_mma_kernel<HD, WARPS>, SMEM, configured, "gb_attention_decode_mma")) return 1;
     gb_launch(attention_decode_mma_kernel<HD, WARPS>, grid, dim3(WARPS * 32), SMEM, stream, p);
     GB_LAUNCH_OK("gb_attention_decode_mma");
     return 0;

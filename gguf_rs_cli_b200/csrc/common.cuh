@@ -65,6 +65,19 @@ static inline cudaError_t gb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 // four sequences, from its rows prepared to its o product done: 27 -> 23 us); with thousands of blocks each block pays for the wait.
 constexpr int GB_FEW_TOKENS = 64;
 
+// A kernel's limit of shared memory is set once on each device: done[device] of the kernel's launcher.  Returns 0, or leaves a message.
+constexpr int GB_MAX_DEVICES = 64;
+template <typename Kernel> static inline int gb_allow_smem(Kernel kernel, int bytes, bool (&done)[GB_MAX_DEVICES], const char* name) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= GB_MAX_DEVICES) return gb_fail("%s: no usable current device", name);
+    if (!done[dev]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+            return gb_fail("%s: cannot get %d bytes of shared memory", name, bytes);
+        done[dev] = true;
+    }
+    return 0;
+}
+
 static inline bool gb_is_dtype(int d) { return d == GB_F32 || d == GB_BF16; }
 static inline size_t gb_dtype_size(int d) { return d == GB_F32 ? 4 : 2; }
 
