@@ -155,8 +155,10 @@ __device__ __forceinline__ void dm_merge_splits(const DmParams& p, int live, int
 // Four warps take 16 keys each of a page at a time, with a block-wide barrier per page: for heads of 64 with more than two CTAs
 // for each SM (64 sequences of 500 positions, 8 KV heads: 14.4 us where the kernel below takes 18.6) and for
 // heads of 128 with more than four.
-template <int HD, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) attention_decode_mma_kernel(DmParams p) {
+constexpr int DM_WARPS = 4;
+template <int HD>
+__global__ void __launch_bounds__(DM_WARPS * 32) attention_decode_mma_kernel(DmParams p) {
+    constexpr int WARPS = DM_WARPS;
     constexpr int CH = HD / 8, KS = HD / 16, OT = HD / 8, HALF = HD / 2;
     constexpr int THREADS = WARPS * 32, UK = WARPS * 16, UPP = GB_PAGE / UK;      // keys per unit, units per page
     constexpr int PAGE_ELEMS = GB_PAGE * HD, UNIT_ELEMS = UK * HD;
@@ -789,11 +791,11 @@ template <int HD, int WARPS, int SLOTS> int launch_pw(const DmParams& p, dim3 gr
     return 0;
 }
 
-template <int HD, int WARPS> int launch_dm(const DmParams& p, dim3 grid, cudaStream_t stream) {
-    constexpr int SMEM = (DM_ROWS + 2 * DM_STAGES * WARPS * 16) * HD * 2;
+template <int HD> int launch_dm(const DmParams& p, dim3 grid, cudaStream_t stream) {
+    constexpr int SMEM = (DM_ROWS + 2 * DM_STAGES * DM_WARPS * 16) * HD * 2;
     static bool configured[GB_MAX_DEVICES] = {};
-    if (gb_allow_smem(attention_decode_mma_kernel<HD, WARPS>, SMEM, configured, "gb_attention_decode_mma")) return 1;
-    gb_launch(attention_decode_mma_kernel<HD, WARPS>, grid, dim3(WARPS * 32), SMEM, stream, p);
+    if (gb_allow_smem(attention_decode_mma_kernel<HD>, SMEM, configured, "gb_attention_decode_mma")) return 1;
+    gb_launch(attention_decode_mma_kernel<HD>, grid, dim3(DM_WARPS * 32), SMEM, stream, p);
     GB_LAUNCH_OK("gb_attention_decode_mma");
     return 0;
 }
@@ -873,7 +875,7 @@ static int decode_mma(const void* q, long long ldq, void* out, long long ldo, in
         p.slots = 4 * sms;
         return launch_pw<128, 2, 3>(p, grid, stream);
     }
-    return hd == 64 ? launch_dm<64, 4>(p, grid, stream) : launch_dm<128, 4>(p, grid, stream);
+    return hd == 64 ? launch_dm<64>(p, grid, stream) : launch_dm<128>(p, grid, stream);
 }
 
 GB_API int gb_attention_decode_mma(const void* q, long long ldq, void* out, long long ldo, int T, int nh, int nkv, int hd,

@@ -8,7 +8,7 @@
 // registers, rounded to nearest; the seven small products are summed in a second accumulator over a piece of K, where a lost bit is 2^-8 of
 // that, and added behind its last block.  Against 64 bits (2,048 of K, 32-bit FMAs one behind another in brackets, of the result's norm): one term in a row
 // 2.5e-8 (2.5e-8), 4 side by side 2.7e-8 (4.2e-8), 4 far apart 4.5e-8 (4.1e-8), 16 3.7e-8 and 6.9e-8 (7.5e-8), all 9.8e-8 (8.1e-7).
-// (One accumulator for all products: one term 4.9e-8, and 2 to 15 % less time.)
+// (One accumulator for all products took 2 to 15 % less time, and the whole sum was cut.)
 // Results that are not finite (an infinite operand times a term that is zero) and results below 2^-96 are summed again one product behind another,
 // as gemm_generic does, and so are those from which more than 2^-26 may be missing where an operand below 2^-110 has lost bits (its terms reach the end of
 // the exponents' range: operands of 1e-34 lose 3e-7 of themselves, of 1e-36 3e-5, of 1e-42 everything).  The conversion looks for such operands; only where it
@@ -18,13 +18,15 @@
 // by the matrix's sizes alone (fx_pieces), whose sums are added in order.
 //
 // What bounds it: a block of 128 features x 192 tokens x 32 of K takes 1,540 cycles of tensor core (eight products for each 32-bit one), 1,670 of
-// shared memory (the loads, X's conversion, the products' reads of X) and 2,500 in all.  Few tokens: the loads; without conversion and sums 39 us of 41 at 16,384 x 2,048.
+// shared memory (the loads, X's conversion, the products' reads of X) and 2,500 in all.  Few tokens: the warps' chain from a
+// block's copy through its conversion (28,672 x 4,096 at one token with a tile a CTA: 139 us, 96 without the conversion, of which 72 are bytes).
 // W is the A operand from tensor memory because shared memory would be busy for 1,700 cycles more with its reads.  Tiles of 64 tokens and more have sixteen
-// warps that convert and add (192 tokens 16,384 x 2,048 98 us, 100 with eight; 1,152 tokens 513, 535).
-// Microseconds behind a cleared L2, gemm_f32 in brackets: 16,384 x 2,048, 1, 2, 4, 16 tokens 45 (39, 41, 45, 70), 64 63, 187 98; 2,048 x 8,192 31 (37, 38, 39, 64), 64 38, 187 57.
+// warps that convert and add (192 tokens 16,384 x 2,048 98 us, 100 with eight; 1,152 tokens 513, 535; before the look for tiny operands, which takes 3 to 5 %).
+// Microseconds behind a cleared L2, gemm_f32 in brackets: 16,384 x 2,048, 1, 2, 4, 16 tokens 46, 46, 46, 48 (39, 41, 45, 70), 64 59, 187 103; 2,048 x
+// 8,192 30, 30, 31, 32 (37, 38, 39, 64), 64 38, 187 64; 28,672 x 4,096 113, 113, 114, 116 (100, 102, 123, 274), 64 195, 187 346.
 //
-// A CTA has one tile of 128 features x BN tokens and some pieces of K.  Warp 0 copies 32-bit blocks of both operands by TMA
-// (128-byte swizzle) into a ring, warp 1 issues the MMAs, eight or sixteen warps convert a block (of W a row and half of the block a
+// A CTA has one tile of 128 features x BN tokens or some pieces of K of one or several.  Warp 0 copies 32-bit blocks of both operands by TMA
+// (128-byte swizzle) into a ring (and converts X where there are up to 16 tokens), warp 1 issues the MMAs, eight or sixteen warps convert a block (of W a row and half of the block a
 // thread, of X a quarter of a row) and add the sums of an earlier block.  Where a tile is one CTA's, its pieces' sums are added as they come; else they go to
 // scratch memory and a second kernel adds them: no CTA waits for another, whatever runs beside them.
 #include <mutex>

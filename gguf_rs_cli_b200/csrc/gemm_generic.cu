@@ -2,9 +2,9 @@
 // W row-major [out, in] as the reference stores it (src/tensor/dequant.rs:258-259,
 // 315-317).  Every product and sum is a 32-bit FMA; each output element is summed by
 // one thread in ascending k, so a row's result does not depend on which other rows
-// are in the batch.  It is the whole matrix path of the 32-bit mode, the twin that
-// the tensor-core kernel is tested against, and the path for sizes the tensor-core
-// kernel refuses.
+// are in the batch.  It is the twin that the bfloat16 tensor-core kernel is
+// tested against, the path for sizes which that kernel refuses, and in the 32-bit mode the one for rows that
+// do not start on 16 bytes (gemm_f32.cu and gemm_f32_tc.cu take the others).
 #include "common.cuh"
 
 constexpr int GG_BM = 64, GG_BN = 64, GG_BK = 16;

@@ -315,9 +315,9 @@ __global__ void __launch_bounds__(TC_THREADS, ctas_per_sm(BN)) gemm_tc_kernel(co
             }
         }
     } else {
-        // ---- epilogue: 4 warps, warp w reads TMEM lanes 32*(w%4) .. +31.  The code that finishes 16 tokens of
-        // a tile exists once, for tiles of the CTA's own and for shared ones (every SM runs this code from a cold
-        // instruction cache after another kernel: its size is time).
+        // ---- epilogue: 4 warps, warp w reads TMEM lanes 32*(w%4) .. +31.  Tiles of the CTA's own are finished
+        // from tensor memory (tc_finish_chunk), shared ones from their CTAs' sums (finish_shared); every SM runs this code from a cold
+        // instruction cache after another kernel: its size is time.
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;        // feature within the tile = TMEM lane
         int j = 0;
@@ -751,8 +751,7 @@ static int gemm_tc_impl(const void* X, long long ldx, const void* W, long long l
             case 16: return launch_tc<16, true>(mw, mx, p, stream);
             case 32: return launch_tc<32, true>(mw, mx, p, stream);
             case 64: return launch_tc<64, true>(mw, mx, p, stream);
-            case 128: return launch_tc<128, true>(mw, mx, p, stream);
-            default: return launch_tc<256, true>(mw, mx, p, stream);
+            default: return gb_fail("gb_gemm_tc_dyt: no tiles of %d tokens", bn);          // only a tuning override asks for them
         }
     }
     if (bn == 256 && g_pair && cut.cut == CUT_WHOLE) {

@@ -216,15 +216,13 @@ __device__ __forceinline__ float tc_warp_sum16(const float (&v)[16], int lane) {
     return d;
 }
 
-// The last steps for 16 columns (tokens c0 .. c0+15 of the tile, those from c_lo on and below c_end being the
-// caller's to finish) of this thread's feature row n = n0 + row: v[jj] holds the finished sum of column c0 + jj.
+// The last steps for 16 columns (tokens c0 .. c0+15 of the tile, those below c_end being there) of this thread's feature row n = n0 + row: v[jj] holds the finished sum of column c0 + jj.
 // x_early: the 16 values of the residual stream at these places if the caller has read them already, else null.
 template <int BN, bool DYT = false>
 __device__ __forceinline__ void tc_finish_chunk(const TcParams& p, int n0, int t0, int n, int row, int lane, int quarter,
                                                 float bias, bool waited, int c0, int c_end, float (&v)[16],
-                                                const float* rstd_s, float (*ssq_s)[BN], const float* x_early = nullptr,
-                                                int c_lo = 0) {
-    auto mine = [&](int c) { return c >= c_lo && c < c_end; };
+                                                const float* rstd_s, float (*ssq_s)[BN], const float* x_early = nullptr) {
+    auto mine = [&](int c) { return c < c_end; };
     if (p.row_ssq) {
 #pragma unroll
         for (int jj = 0; jj < 16; ++jj) v[jj] *= rstd_s[min(c0 + jj, BN - 1)];

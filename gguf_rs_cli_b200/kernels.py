@@ -1065,7 +1065,8 @@ class _TcScratch:
     holds its address, so a buffer that grew would leave every graph captured before pointing at
     freed memory.  The product needs at most one partial tile per resident CTA (two CTAs per SM with
     tiles of up to 64 tokens, one with wider tiles: 2 * sms * 64 * 128 floats), decode attention
-    (head_dim + 2) floats per head and split with no more CTAs than two per SM.  A launch that would
+    (head_dim + 2) floats per head and split: with no more CTAs than two per SM, or four splits of each of up to four columns an SM (decode_sharing: 4 * 4 * sms
+    * 16 heads * 130 floats, half of the capacity, and 4 * sms counters).  A launch that would
     need more (only a tuning override can ask for it) runs without splitting instead."""
     COUNTERS = 4096
 
